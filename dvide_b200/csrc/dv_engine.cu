@@ -1144,6 +1144,23 @@ int Engine::copy_state_out(int b0, int n, double* p, double* v) {
   return DV_OK;
 }
 
+// As copy_state_out: the body vectors are packed on the device (3 doubles of
+// each double4) and cross in one contiguous copy.  A strided copy instead is
+// bound by its 24-byte rows: 28.9 ms for 200,005 bodies into pageable memory,
+// 0.65 ms this way.
+int Engine::copy_contact_force_out(double* f) {
+  const int n = d.nb;
+  const size_t need = 3 * (size_t)n;
+  if (need > stage3_cap_) {
+    dfree(stage3_);
+    stage3_cap_ = 0;
+    TRY(dalloc(&stage3_, need));
+    stage3_cap_ = need;
+  }
+  k_pack3<<<(n + kThreads - 1) / kThreads, kThreads, 0, st_>>>(d.fc4, n, stage3_);
+  return download(f, stage3_, sizeof(double) * need);
+}
+
 int Engine::copy_state_in(int b0, int n, const double* p, const double* v) {
   if (n <= 0) return DV_OK;
   if (b0 < 0 || b0 + n > d.nb) return DV_ERR_ARG;

@@ -115,6 +115,7 @@ class Engine {
   // plus a pack/unpack kernel (synchronous).  p or v may be null.
   int copy_state_out(int b0, int n, double* p, double* v);
   int copy_state_in(int b0, int n, const double* p, const double* v);
+  int copy_contact_force_out(double* f);  // every body
 
   // Download helpers (synchronous).
   int download(void* dst, const void* src, size_t bytes);

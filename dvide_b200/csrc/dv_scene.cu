@@ -187,11 +187,7 @@ DV_API int dv_set_state(dv_scene* s, const double* p, const double* v) {
 
 DV_API int dv_get_contact_force(dv_scene* s, double* f) {
   if (!s || !f) return DV_ERR_ARG;
-  Engine& E = s->E;
-  DV_CUDA_TRY(cudaMemcpy2DAsync(f, 3 * sizeof(double), E.d.fc4, sizeof(double4), 3 * sizeof(double),
-                                E.d.nb, cudaMemcpyDeviceToHost, E.stream()));
-  DV_CUDA_TRY(cudaStreamSynchronize(E.stream()));
-  return DV_OK;
+  return s->E.copy_contact_force_out(f);
 }
 
 DV_API int dv_get_num_contacts(dv_scene* s, int32_t* nc, int32_t* npossible) {
