@@ -7,13 +7,12 @@
 //   v = Minv (k + D^T gamma), p += h v        System.cu:570-583
 //
 // The reference runs each BLAS-1 call, SpMV and projection as its own launch
-// and brings every dot/nrm2/nrmmax back to the host (APGD.cu:227-350).  Here
-// the scalar control (step size, Lipschitz backtracking, restart, best
-// iterate, convergence) runs on the device, per segment: the CTA that finishes
-// a segment's last tile of a pass folds that segment's per-tile partial sums in
-// a fixed order and executes its control logic; a grid barrier then starts the
-// next pass.  Segments converge independently (their tiles and bodies are
-// skipped once done); the kernel ends when every segment is done.
+// and brings every dot/nrm2/nrmmax back to the host (APGD.cu:227-350).  Here a
+// team of CTAs (dv_team.cuh) takes a scene and runs all of it.  The scalar
+// control (step size, Lipschitz backtracking, restart, best iterate,
+// convergence) runs on the device: after a pass's barrier every member folds
+// the scene's per-tile partial sums in a fixed order and executes the control
+// logic on its own copy of the scalars, in shared memory.
 //
 // Matrix-free N x = D Minv D^T x (D's block of contact c is [+F_c^T | -F_c^T],
 // F_c = [n u v]):
@@ -39,215 +38,229 @@
 // and Lipschitz-test sums, the residual, the final D^T gamma and the
 // integration in FP64.
 //
-// Work is split in tiles of 512 contacts (2 per thread) and 256 bodies.
-// Every wait has a time limit.
+// What the passes read per contact lies in blocks of 32 contacts, one warp's
+// share: the constants of a solve (normal, frame words, r, body ids) in one
+// block, each iterate with its product in another.  A warp brings its next 32
+// contacts with three bulk copies of 0.4 to 2.5 KB.  As separate planes they
+// were twenty copies of 256 bytes, and the copy engine's rate per copy (about
+// 30 cycles), not the bytes, set the pass's time: 52 us in FP64 and 51 us in
+// FP32 on 741,000 contacts.
+//
+// Work is split in tiles of 512 contacts (2 per thread).  Every wait has a
+// time limit.
 #include <algorithm>
 
-#include "dv_solve.cuh"
+#include "dv_team.cuh"
 
 namespace dv {
 
 namespace {
 
-// Per-segment scalars of the step and product passes, kept in shared memory
-// (written by thread 0 when the CTA moves to another segment) so that they
-// take no registers in the contact loops.
-struct ProdScalars {
-  int cur, nw, nw2, restart, exact, rsel;
-  double ya, ym, nt2, gd, gA, gB, mu;
+// A solve's scalar state (APGD.cu:208-223, 266-332), one copy per member in
+// shared memory, and what the passes take from it.  Iterates live in five
+// rotating buffers: cur = gamma_k, prev = gamma_{k-1}, nw = target of
+// gamma_new, best = gamma_hat (-1 before the first accepted iterate), nw2 the
+// next iterate computed ahead.
+struct Solve {
+  double L, t, theta, theta_new, beta, yb;
+  double obj1, obj2, obj2_base, residual, objective, objN;
+  double gdiff, ginv, gneg, L0;        // gd, 1 / gd, -(1 / gd)
+  double step_ya, step_ym, step_nt;    // step pass: 1 + yb, -yb, -t
+  double prod_ya, prod_ym, prod_nt;    // look-ahead: 1 + beta, -beta, -(1 / (0.9 L))
+  Cone<double> cone;
+  Cone<float> conef;
+  double sums[8];
+  int k, restart, cur, prev, nw, nw2, best, yr, first, step;
+  int backtracks, sweeps, iterations, rsel, since_best, done;
+  unsigned err;
 };
-struct StepScalars {
-  int part, first, cur, prev, nw, yr, exact, rsel;
-  double ya, ym, nt, mu;
-};
+
+template <class T> __device__ inline const Cone<T>& cone_of(const Solve& c);
+template <> __device__ inline const Cone<double>& cone_of<double>(const Solve& c) { return c.cone; }
+template <> __device__ inline const Cone<float>& cone_of<float>(const Solve& c) { return c.conef; }
 
 // Mixed precision with refinement: the FP32 phase of a solve ends when its
 // best residual has not improved for this many accepted iterations.
 constexpr int kStallIterations = 50;
 
-// What the segment controllers read and write, passed by value.
-struct CtlArgs {
-  double* part;
-  int tcap;
-  int mixed;  // FP32 iterates: the Lipschitz test allows float-noise differences
-  int ar;     // anti-relaxation: an accepted, unconverged iterate moves r to the next plane
-  int refine; // FP64 refinement launch: only the solves the FP32 launch marked, <= seg.refine iterations
-  SegState* sst;
-  const SegParams* seg;
-  EngineWords* ew;
-  unsigned* donemask;
+// ---- controllers (thread 0 of every member, after fold_team) ----
+
+__device__ inline void pass_scalars(Solve& C) {
+  C.step_ya = 1.0 + C.yb;
+  C.step_ym = -C.yb;
+  C.step_nt = -C.t;
+  C.prod_ya = 1.0 + C.beta;
+  C.prod_ym = -C.beta;
+  C.prod_nt = -(1.0 / (0.9 * C.L));
+}
+
+__device__ __noinline__ void ctl_lipschitz(Solve& C, const SegParams& P, int nc, int cap,
+                                           bool mixed) {
+  const double L = sqrt(C.sums[0]) / C.L0;
+  C.L = L;
+  C.t = 1.0 / L;
+  C.theta = 1.0;
+  const double th = 1.0;
+  const double tn = (-(th * th) + th * sqrt(th * th + 4.0)) / 2.0;
+  C.theta_new = tn;
+  C.beta = th * (1.0 - th) / (th * th + tn);
+  C.residual = 10e30;
+  C.objective = 0.0;
+  // APGD.cu:92: 1 / (contacts + bilateral rows)^2
+  const double ncd = (double)(nc + P.nbil);
+  const double gd = 1.0 / (ncd * ncd);
+  C.gdiff = gd;
+  C.ginv = 1.0 / gd;
+  C.gneg = -1.0 / gd;
+  C.k = 0;
+  C.step = 1;
+  C.iterations = 0;
+  C.sweeps = 0;
+  C.restart = 0;
+  C.cur = 0;
+  C.prev = -1;
+  C.nw = 1;
+  C.best = -1;
+  C.nw2 = free_slot(1, 0, -1, -1);
+  C.yr = 1;
+  C.yb = 0.0;
+  C.first = 1;
+  C.backtracks = 0;
+  C.obj1 = 0.0;
+  C.obj2 = 0.0;
+  C.obj2_base = 0.0;
+  C.rsel = 0;
+  C.objN = 0.0;
+  C.since_best = 0;
+  C.done = cap <= 0 ? 1 : 0;
+  C.cone = make_cone<double>(P.mu);
+  if (mixed) C.conef = make_cone<float>((float)P.mu);
+  pass_scalars(C);
+}
+
+__device__ __noinline__ void ctl_step(Solve& C) {
+  double ob = C.obj2_base;
+  if (C.first) {
+    ob = 0.5 * C.sums[3] + C.sums[4];
+    C.obj2_base = ob;
+  }
+  const double nr = sqrt(C.sums[1]);
+  C.obj2 = ob + (C.sums[0] + 0.5 * C.L * (nr * nr));
+  C.restart = (C.sums[2] > 0) ? 1 : 0;
+  C.first = 0;
+  C.step = 0;
+}
+
+__device__ __noinline__ void ctl_product(Solve& C, const SegParams& P, int cap, bool mixed, bool ar) {
+  const double obj1 = 0.5 * C.sums[0] + C.sums[1];
+  const double res = C.sums[7];
+  C.obj1 = obj1;
+  int k = C.k;
+  bool finished = false;
+  // APGD.cu:240: obj1 >= obj2 means the step was too long.  With FP32
+  // iterates both objectives carry rounding of order 1e-7 |f|; a difference
+  // within that noise is not a failed test (else L doubles on noise alone).
+  const double obj2 = C.obj2;
+  const bool fail = mixed ? (obj1 - obj2 >= 1e-6 * (fabs(obj1) + fabs(obj2))) : (obj1 >= obj2);
+  if (fail) {
+    // (10)-(14): double L and retry the projection
+    if (C.backtracks >= P.max_bt) {
+      C.err |= kErrBacktrackCap;
+      finished = true;
+    } else {
+      C.backtracks += 1;
+      C.L = 2.0 * C.L;
+      C.t = 1.0 / C.L;
+      C.step = 1;
+    }
+  } else {
+    C.sweeps += 1;
+    const int best = C.best;
+    C.since_best += 1;
+    if (res < C.residual) {
+      C.residual = res;
+      C.objective = obj1;
+      if (ar) C.objN = 0.5 * C.sums[0];
+      C.best = C.nw;
+      C.since_best = 0;
+    }
+    if (C.residual < P.tol) {
+      finished = true;
+    } else if (mixed && P.refine > 0 && C.since_best >= kStallIterations) {
+      // FP32 iterates no longer improve: the FP64 refinement continues
+      // from gamma_hat
+      finished = true;
+    } else {
+      // APGD.cu:335-345 after this iteration: r moves to the plane the
+      // product pass wrote for the look-ahead
+      if (ar) C.rsel ^= 1;
+      const double th = C.restart ? 1.0 : C.theta_new;
+      C.yb = C.beta;
+      C.yr = C.restart;
+      const double L = 0.9 * C.L;
+      C.L = L;
+      C.t = 1.0 / L;
+      C.theta = th;
+      const int cur = C.nw, nw = free_slot(C.nw, C.cur, C.prev, best);
+      C.prev = C.cur;
+      C.cur = cur;
+      C.nw = nw;
+      C.nw2 = free_slot(nw, cur, C.prev, C.best);
+      k += 1;
+      C.k = k;
+      if (k >= cap) {
+        finished = true;
+      } else {
+        const double tn = (-(th * th) + th * sqrt(th * th + 4.0)) / 2.0;
+        C.theta_new = tn;
+        C.beta = th * (1.0 - th) / (th * th + tn);
+        // the look-ahead step is now iteration k's step
+        const double ob = 0.5 * C.sums[5] + C.sums[6];
+        C.obj2_base = ob;
+        const double nr = sqrt(C.sums[3]);
+        C.obj2 = ob + (C.sums[2] + 0.5 * L * (nr * nr));
+        C.restart = (C.sums[4] > 0) ? 1 : 0;
+      }
+    }
+  }
+  if (finished) {
+    C.iterations = k;
+    C.done = 1;
+  }
+  pass_scalars(C);
+}
+
+// ---- blocks of 32 contacts ----
+// Constant block: 9 planes of 32 (normal, frame words, r), then the 32 ids A
+// and the 32 ids B.  Iterate block: 3 planes of the iterate, 3 of its product.
+template <class T> struct Block {
+  static constexpr int kIds = 9 * 32;                               // in T
+  static constexpr int kConst = kIds + 256 / (int)sizeof(T);
+  static constexpr unsigned kConstBytes = kConst * sizeof(T);
+  static constexpr unsigned kHalfBytes = 3 * 32 * sizeof(T);        // an iterate or a product
+  // a warp's stage: constants, gamma_new, gamma_k with its product
+  static constexpr unsigned kStageBytes = kConstBytes + 3 * kHalfBytes;
 };
 
-// Segment controllers, run by the CTA that completes a segment's tiles of a
-// pass (all its threads; thread 0 writes).  Kept out of line so that their
-// registers do not weigh on the contact-pass loops.
-__device__ __noinline__ void ctl_setup(CtlArgs a, int s, double* scratch) {
-  double sm[1];
-  fold_tiles<1>(a, a.sst[s].t0, a.sst[s].nt, sm, scratch);
-  if (threadIdx.x == 0) a.sst[s].ctl.L0 = sqrt(sm[0]);
+template <class T>
+__device__ inline T* const_at(const KArgs<T>& a, int c) {
+  return a.blk + (size_t)(c >> 5) * Block<T>::kConst + (c & 31);
 }
-
-__device__ __noinline__ void ctl_lipschitz(CtlArgs a, int s, double* scratch) {
-  double sm[1];
-  fold_tiles<1>(a, a.sst[s].t0, a.sst[s].nt, sm, scratch);
-  if (threadIdx.x == 0) {
-    const SegParams& P = a.seg[s];
-    ApgdCtl* C = &a.sst[s].ctl;
-    // refinement launch: a solve the FP32 phase finished keeps its result
-    if (a.refine && !__ldcg(&C->refined)) return;
-    const double L = sqrt(sm[0]) / __ldcg(&C->L0);
-    C->L = L;
-    C->t = 1.0 / L;
-    C->theta = 1.0;
-    const double th = 1.0;
-    const double tn = (-(th * th) + th * sqrt(th * th + 4.0)) / 2.0;
-    C->theta_new = tn;
-    C->beta = th * (1.0 - th) / (th * th + tn);
-    C->residual = 10e30;
-    C->objective = 0.0;
-    // APGD.cu:92: 1 / (contacts + bilateral rows)^2
-    const double ncd = (double)(a.sst[s].nc + a.seg[s].nbil);
-    const double gd = 1.0 / (ncd * ncd);
-    C->gdiff = gd;
-    C->ginv = 1.0 / gd;
-    C->k = 0;
-    C->mode = 0;
-    C->iterations = 0;
-    C->sweeps = 0;
-    C->restart = 0;
-    C->cur = 0;
-    C->prev = -1;
-    C->nw = 1;
-    C->best = -1;
-    C->yr = 1;
-    C->yb = 0.0;
-    C->first = 1;
-    C->backtracks = 0;
-    C->obj1 = 0.0;
-    C->obj2 = 0.0;
-    C->obj2_base = 0.0;
-    C->rsel = 0;
-    C->objN = 0.0;
-    C->since_best = 0;
-    if ((a.refine ? P.refine : P.max_iter) <= 0) {
-      mark_done(a, s);
-    } else {
-      C->done = 0;
-      atomicAdd(&a.ew->active, 1);
-      atomicAdd(&a.ew->step_count, 1);
-    }
-  }
+constexpr int kIterBlock = 6 * 32;
+template <class T>
+__device__ inline T* iter_at(T* x, int c) {
+  return x + (size_t)(c >> 5) * kIterBlock + (c & 31);
 }
-
-__device__ __noinline__ void ctl_step(CtlArgs a, int s, double* scratch) {
-  double sm[5];
-  fold_tiles<5>(a, a.sst[s].t0, a.sst[s].nt, sm, scratch);
-  if (threadIdx.x == 0) {
-    ApgdCtl* W = &a.sst[s].ctl;
-    const int first = __ldcg(&W->first);
-    const double L = __ldcg(&W->L);
-    double ob = __ldcg(&W->obj2_base);
-    if (first) {
-      ob = 0.5 * sm[3] + sm[4];
-      W->obj2_base = ob;
-    }
-    const double nr = sqrt(sm[1]);
-    W->obj2 = ob + (sm[0] + 0.5 * L * (nr * nr));
-    W->restart = (sm[2] > 0) ? 1 : 0;
-    W->first = 0;
-  }
+template <class T>
+__device__ inline Frame<T> block_frame(const T* p) {
+  return make_frame<T>(p[0], p[32], p[64], FrameWords<T>{p[96], p[128], p[160]});
 }
-
-// `direct`: an engine of one scene, whose controller runs at the product
-// pass's barrier: it sets step_needed itself (no arrival counter to latch).
-__device__ __noinline__ void ctl_product(CtlArgs a, int s, double* scratch, bool direct = false) {
-  double sm[7], res;
-  fold_tiles_sm<7, 1>(a, a.sst[s].t0, a.sst[s].nt, sm, &res, kQMax, scratch);
-  if (threadIdx.x == 0) {
-    const SegParams& P = a.seg[s];
-    ApgdCtl* C = &a.sst[s].ctl;
-    const ApgdCtl c = ctl_read(C);
-    const double obj1 = 0.5 * sm[0] + sm[1];
-    C->obj1 = obj1;
-    bool finished = false;
-    int k = c.k;
-    // APGD.cu:240: obj1 >= obj2 means the step was too long.  With FP32
-    // iterates both objectives carry rounding of order 1e-7 |f|; a difference
-    // within that noise is not a failed test (else L doubles on noise alone).
-    const double obj2 = c.obj2;
-    const bool fail = a.mixed ? (obj1 - obj2 >= 1e-6 * (fabs(obj1) + fabs(obj2))) : (obj1 >= obj2);
-    if (fail) {
-      // (10)-(14): double L and retry the projection
-      if (c.backtracks >= P.max_bt) {
-        seg_error(a, s, kErrBacktrackCap);
-        finished = true;
-      } else {
-        C->backtracks = c.backtracks + 1;
-        const double L = 2.0 * c.L;
-        C->L = L;
-        C->t = 1.0 / L;
-        C->mode = 1;
-        if (direct) *(volatile int*)&a.ew->step_needed = 1;
-        else atomicAdd(&a.ew->step_count, 1);
-      }
-    } else {
-      C->mode = 0;
-      if (direct) *(volatile int*)&a.ew->step_needed = 0;
-      C->sweeps = c.sweeps + 1;
-      double residual = c.residual;
-      int since_best = c.since_best + 1;
-      if (res < residual) {
-        residual = res;
-        C->residual = res;
-        C->objective = obj1;
-        if (a.ar) C->objN = 0.5 * sm[0];
-        C->best = c.nw;
-        since_best = 0;
-      }
-      C->since_best = since_best;
-      if (residual < P.tol) {
-        finished = true;
-      } else if (a.mixed && P.refine > 0 && since_best >= kStallIterations) {
-        // FP32 iterates no longer improve: the FP64 refinement continues
-        // from gamma_hat
-        finished = true;
-      } else {
-        // APGD.cu:335-345 after this iteration: r moves to the plane the
-        // product pass wrote for the look-ahead
-        if (a.ar) C->rsel = c.rsel ^ 1;
-        const double th = c.restart ? 1.0 : c.theta_new;
-        C->yb = c.beta;
-        C->yr = c.restart;
-        const double L = 0.9 * c.L;
-        C->L = L;
-        C->t = 1.0 / L;
-        C->theta = th;
-        C->prev = c.cur;
-        C->cur = c.nw;
-        C->nw = free_slot(c.nw, c.cur, c.prev, c.best);
-        k += 1;
-        C->k = k;
-        if (k >= (a.refine ? P.refine : P.max_iter)) {
-          finished = true;
-        } else {
-          const double tn = (-(th * th) + th * sqrt(th * th + 4.0)) / 2.0;
-          C->theta_new = tn;
-          C->beta = th * (1.0 - th) / (th * th + tn);
-          // the look-ahead step is now iteration k's step
-          const double ob = 0.5 * sm[5] + sm[6];
-          C->obj2_base = ob;
-          const double nr = sqrt(sm[3]);
-          C->obj2 = ob + (sm[2] + 0.5 * L * (nr * nr));
-          C->restart = (sm[4] > 0) ? 1 : 0;
-        }
-      }
-    }
-    if (finished) {
-      C->iterations = k;
-      mark_done(a, s);
-      atomicSub(&a.ew->active, 1);
-    }
-  }
+template <class T>
+__device__ inline uint2 block_ids(const KArgs<T>& a, int c) {
+  const uint32_t* p =
+      reinterpret_cast<const uint32_t*>(a.blk + (size_t)(c >> 5) * Block<T>::kConst + Block<T>::kIds) +
+      (c & 31);
+  return make_uint2(p[0], p[32]);
 }
 
 // The arrays of one bilateral tile in the product pass.
@@ -270,11 +283,10 @@ struct BilRows {
 // it adds no registers to the contact loops).  Returns whether a residual
 // item of this thread was NaN.
 template <class T>
-__device__ inline bool bil_product_tile(BilRows<T> R, const ProdScalars& ps, int r0, int n,
-                                              bool has_contacts, DeferBuf* def, int slot, int tile) {
-  const T ya = (T)ps.ya, ym = (T)ps.ym, nt2 = (T)ps.nt2;
-  double acc[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  double mx = 0.0;
+__device__ inline bool bil_product_tile(BilRows<T> R, const Solve& C, int r0, int n,
+                                        bool has_contacts, ParkBuf* park, int slot, int tile) {
+  const T ya = (T)C.prod_ya, ym = (T)C.prod_ym, nt2 = (T)C.prod_nt;
+  double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   bool bad = false;
   for (int m = 0; m < kItemsPerThread; ++m) {
     const int k = m * kThreads + threadIdx.x;
@@ -290,14 +302,14 @@ __device__ inline bool bil_product_tile(BilRows<T> R, const ProdScalars& ps, int
       double T0 = (double)rr + (double)N0;
       if (has_contacts) {
         const double X0 = x0;
-        T0 = X0 + (-ps.gd) * T0;
-        T0 = ps.gA * X0 + ps.gB * T0;
+        T0 = X0 + (-C.gdiff) * T0;
+        T0 = C.ginv * X0 + C.gneg * T0;
       }
       const double m0 = fabs(T0);
       bad |= (m0 != m0);
-      mx = fmax(mx, m0);
+      acc[7] = fmax(acc[7], m0);
       T y0, M0;
-      if (ps.restart) {
+      if (C.restart) {
         y0 = x0;
         M0 = N0;
       } else {
@@ -316,963 +328,736 @@ __device__ inline bool bil_product_tile(BilRows<T> R, const ProdScalars& ps, int
       acc[6] = acc[6] + (double)y0 * (double)rr;
     }
   }
-  park_tile<7, true>(*def, slot, tile, acc, mx);
+  park8<true>(*park, slot, tile, acc);
   return bad;
 }
+
+// Phases of a one-scene engine, timed by its first member between barriers.
+struct PhaseTimer {
+  unsigned long long last, ns[8];
+  unsigned count[8];
+};
 
 // kAR: APGD's anti-relaxation (APGD.cu:335-345), FP64 one-scene engines.
 template <class T, int kMinB, bool kAR>
 __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
   using V = typename Vec4<T>::type;
-  __shared__ double scratch[kNQ * 8 + 8];
-  __shared__ unsigned s_mask[kMaskWords];
-  __shared__ ProdScalars s_ps;
-  __shared__ StepScalars s_st;
-  __shared__ DeferBuf s_def;
+  using B = Block<T>;
+  constexpr bool kMixed = sizeof(T) != sizeof(double);
+  __shared__ double scratch[64];
+  __shared__ Solve C;
+  __shared__ Team tm;
+  __shared__ ParkBuf park;
+  __shared__ PhaseTimer timer;
+  __shared__ int s_seen, s_copy_fail;
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   const size_t S = a.S;
-  V* wv = reinterpret_cast<V*>(a.wd);
-  V* qv = reinterpret_cast<V*>(a.qd);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Staging stg;
   stg.base = dyn_smem;
-  stg.stage_bytes = warp_stage_bytes<T>();
-  stg.bar = reinterpret_cast<uint64_t*>(dyn_smem + (size_t)kWarps * 2 * stg.stage_bytes);
+  stg.stage_bytes = B::kStageBytes;
+  stg.bar = reinterpret_cast<uint64_t*>(dyn_smem + (size_t)kWarps * 2 * B::kStageBytes);
   stg.phase = 0;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2 * kWarps; ++i) mbar_init(stg.bar + i, 1);
     for (int w = 0; w < kWarps; ++w) reinterpret_cast<unsigned char*>(stg.bar + 2 * kWarps)[w] = 0;
     fence_mbar_init();
+    s_seen = 0;
+    s_copy_fail = 0;
+    timer.last = global_ns();
+    for (int i = 0; i < 8; ++i) {
+      timer.ns[i] = 0;
+      timer.count[i] = 0;
+    }
   }
   __syncthreads();
   if (ld_acquire(&a.ew->err)) return;  // an error of collision detection: nothing to do
-  const int NT = a.ew->ntiles;
-  const int nbt = (a.nb + kThreads - 1) / kThreads;
-  const int mwords = (a.nseg + 31) >> 5;
-  __shared__ SegCache s_sc;  // segment of the CTA's current tile
-  SegCache& sc = s_sc;
-  if (threadIdx.x == 0) {
-    sc.s = -1;
-    sc.t0 = sc.t1 = 0;
-    s_def.fail = 0;
-  }
-  __syncthreads();
-  const CtlArgs ca{a.part,  a.tcap, sizeof(T) != sizeof(double) ? 1 : 0, kAR ? 1 : 0, a.refine,
-                   a.sst,   a.seg,  a.ew, a.donemask};
 
-  // ---- work lists off; per-segment solve state; done mask (bit set: not iterating)
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    a.ew->act_on = 0;
-    a.ew->act_rebuild = 0;
-    a.ew->act_base = a.nseg;
-  }
-  for (int s = blockIdx.x * kThreads + threadIdx.x; s < a.nseg; s += gridDim.x * kThreads) {
-    SegState& X = a.sst[s];
-    X.arrive = 0u;
-    ApgdCtl& C = X.ctl;
-    // System.cu:560: a solve runs with contacts or bilateral rows
-    const bool live = a.seg[s].active && (X.nc > 0 || a.seg[s].nbil > 0);
-    if (a.refine) {
-      // FP64 refinement: only the solves the FP32 launch marked; the others
-      // keep their result, counts and error bits
-      if (!(live && C.refined)) {
-        C.done = 1;
-        continue;
-      }
-      C.it_lo = C.iterations;
-      C.bt_lo = C.backtracks;
-      C.sw_lo = C.sweeps;
-    } else {
-      C.refined = 0;
-      C.refine_it = 0;
+  // a phase ends at a barrier
+  auto sync = [&](int phase, bool joining = false) {
+    const bool ok = team_sync(a, tm, joining);
+    if (a.nseg == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
+      const unsigned long long now = global_ns();
+      timer.ns[phase] += now - timer.last;
+      timer.count[phase] += 1;
+      timer.last = now;
     }
-    X.err = 0u;
-    C.done = live ? 0 : 1;
-    C.iterations = 0;
-    C.sweeps = 0;
-    C.backtracks = 0;
-    C.residual = 0.0;
-    C.objective = 0.0;
-    C.best = -1;
-  }
-  for (int wi = blockIdx.x * kThreads + threadIdx.x; wi < mwords; wi += gridDim.x * kThreads) {
-    unsigned m = 0u;
-    for (int j = 0; j < 32; ++j) {
-      const int s = wi * 32 + j;
-      if (s >= a.nseg || !(a.seg[s].active && (a.sst[s].nc > 0 || a.seg[s].nbil > 0)) ||
-          (a.refine && !a.sst[s].ctl.refined))
-        m |= 1u << j;
-    }
-    a.donemask[wi] = m;
-  }
+    return ok;
+  };
 
-  // ---- applied impulse: k = m v + h f (m = 1/minv, 0 for fixed); w = minv k
-  for (int bt = blockIdx.x; bt < nbt; bt += gridDim.x) {
-    int b = bt * kThreads + threadIdx.x;
-    if (b < a.nb) {
-      const SegParams& P = a.seg[__ldg(a.bseg + b)];
-      if (P.active) {
-        const double h = P.h;
-        double mi = __ldg(a.minv + b);
-        double m = mi;
-        if (m) m = 1.0 / m;
-        double4 v = a.v4[b], f = a.f4[b];
-        double4 k = make_double4(h * f.x + m * v.x, h * f.y + m * v.y, h * f.z + m * v.z, 0.0);
-        a.k4[b] = k;
-        a.wd[b] = make_double4(mi * k.x, mi * k.y, mi * k.z, 0.0);
-      }
+  while (join_team(a, tm, &s_seen)) {
+    const int s = tm.s;
+    const SegParams& P = a.seg[s];
+    const int nc = tm.nc, c0 = tm.c0;
+    // the iterations' w and q: in FP32 they lie over the scene's own FP64 ones
+    // (setup and update), not over another scene's
+    V* wv = reinterpret_cast<V*>(a.wd + P.b0) - P.b0;
+    V* qv = reinterpret_cast<V*>(a.qd + c0) - c0;
+    double* part = a.part + tm.t0;
+    int parity = 0;  // the partials' planes of this pass (a member may be a pass ahead)
+    auto planes = [&]() { return part + (size_t)parity * 8 * a.tcap; };
+    const bool live = nc > 0 || P.nbil > 0;  // System.cu:560: a solve runs with contacts or rows
+    const int cap = a.refine ? P.refine : P.max_iter;
+    int it_lo = 0, bt_lo = 0, sw_lo = 0;
+    if (a.refine && threadIdx.x == 0) {
+      const ApgdCtl& D = a.sst[s].ctl;
+      it_lo = D.iterations;
+      bt_lo = D.backtracks;
+      sw_lo = D.sweeps;
     }
-  }
-  if (!grid_sync(a, kPhaseSetup, [&]() {
-        if (threadIdx.x == 0) {
-          atomicExch(&a.ew->active, 0);
-          atomicExch(&a.ew->step_count, 0);
-          *(volatile int*)&a.ew->step_needed = 0;
-        }
-      }))
-    return;
+    if (threadIdx.x == 0) {
+      C.err = 0u;
+      C.done = 1;
+      C.iterations = C.sweeps = C.backtracks = 0;
+      C.residual = C.objective = 0.0;
+      C.best = -1;
+      C.rsel = 0;
+    }
 
-  // ---- r = D (Minv k) + b; gamma_0 -> G[0]; e = gamma_0 - gamma_hat_0 (= gamma_0 - 1)
-  {
-    SegRun run;
-    int nslot = 0;
-    auto ctl = [&](int s) { ctl_setup(ca, s, scratch); };
-    for (int i = 0;; ++i) {
-      const int t = cta_tile(a, NT, i);
-      if (t < 0) break;
-      locate(a, sc, t);
-      const int s = sc.s;
-      // refinement launch: a solve it does not refine needs no r, start or Lipschitz
-      // estimate (its q and warm start from the FP32 launch stand)
-      if (a.refine && !__ldcg(&a.sst[s].ctl.refined)) continue;
-      if (s != run.s) {
-        if (run.n) {
-          fold_parked<1, false>(a, s_def, nslot);
-          nslot = 0;
-        }
-        flush_run(a, run, ctl);
-        run.s = s;
-      }
-      const SegParams& P = a.seg[s];
-      const int k0 = (t - sc.t0) * kTileItems, nc = sc.nc, c0 = sc.c0, gsize = sc.gsize;
+    // ---- applied impulse: k = m v + h f (m = 1/minv, 0 for fixed); w = minv k
+    for (int b = tm.w0 + threadIdx.x; b < tm.w1; b += kThreads) {
       const double h = P.h;
-      double acc[1] = {0.0};
-      const int kb = a.nbil ? bil_tile_k0(t, sc.t0, nc) : -1;
-      if (kb >= 0) {
-        // bilateral rows: b = violation / h (System.cu:1526-1544) at the
-        // step's start time, r = b + (D Minv k)_row, gamma_0, e = gamma_0 - 1
-        const double* pd = reinterpret_cast<const double*>(a.p4);
-        const double* wdv = reinterpret_cast<const double*>(a.wd);
-        const double tm = a.seg_time[s];
-        for (int m = 0; m < kItemsPerThread; ++m) {
-          const int k = kb + m * kThreads + threadIdx.x;
-          if (k < P.nbil) {
-            const int i = P.bil0 + k;
-            const int2 o = __ldg(a.bil_off + i);
-            const double4 inf = a.bil_info[i];  // velocity, start time, p0
-            double velocity = inf.x;
-            if (tm < inf.y) velocity = 0;
-            const double pa = pd[o.x];
-            const double viol = o.y >= 0 ? pa - pd[o.y] - velocity * (tm - inf.y)
-                                         : pa - inf.z - velocity * (tm - inf.y);
-            const double bb = viol / h;
-            a.bil_b[i] = bb;
-            a.br[i] = (T)(bb + bil_dw<double>(o, wdv));
-            // warm start: the row's last impulse.  Without it the reference's
-            // initialiser writes (1, 0, 0) over flat entries [0, 3 nc) with
-            // the rows first (APGD.cu:114-120, 200): row k takes 1 if k is a
-            // multiple of 3, 0 otherwise, and keeps its last impulse from 3 nc on.
-            double g = a.bil_gam[i];
-            if (!P.warm && k < 3 * nc) g = (k % 3 == 0) ? 1.0 : 0.0;
-            const T x0 = (T)g;
-            a.bG[0][i] = x0;
-            const T e0 = x0 + T(-1);
-            acc[0] = acc[0] + (double)e0 * (double)e0;
-            a.bq[i] = e0;
-          }
-        }
-      }
-      for (int m = 0; m < kItemsPerThread && kb < 0; ++m) {
-        int k = k0 + m * kThreads + threadIdx.x;
-        if (k < nc) {
-          const int c = c0 + k;
-          Frame<double> fd = load_frame_fp64(a, c, P.exact != 0);
-          double4 wa = a.wd[__ldg(a.ida + c)], wb = a.wd[__ldg(a.idb + c)];
-          double d0, d1, d2;
-          ft_times<double, double4>(fd, wa, wb, &d0, &d1, &d2);
-          double bn = __ldg(a.gap + c) / h;
-          a.r[0 * S + c] = (T)(bn + d0);
-          if (kAR) {
-            // r_n and the anti-relaxation vector (0 at the start, APGD.cu:196)
-            a.ar_r0[c] = bn + d0;
-            a.ar_v[c] = 0.0;
-          }
-          a.r[1 * S + c] = (T)(0.0 + d1);
-          a.r[2 * S + c] = (T)(0.0 + d2);
-          double g0, g1, g2;
-          // refinement: positional, from the FP32 phase's gamma_hat of this step
-          const int warm = a.refine ? 1 : P.warm;
-          if (warm == 2) {
-            // matched: the impulse the same (A, B) pair had at the last solve;
-            // A's earlier contacts are sorted by B, so a binary search finds it
-            const uint32_t ia = __ldg(a.ida + c);
-            const uint32_t bl = __ldg(a.idb + c) - (uint32_t)P.b0;
-            int lo = a.ws[ia], hi = lo + a.wc[ia];
-            if (hi > gsize) hi = gsize;
-            while (lo < hi) {
-              const int mid = (lo + hi) >> 1;
-              if (a.wid[(size_t)P.wbase + mid] < bl) lo = mid + 1;
-              else hi = mid;
-            }
-            g0 = 0.0; g1 = 0.0; g2 = 0.0;
-            if (lo < gsize && lo < a.ws[ia] + a.wc[ia] && a.wid[(size_t)P.wbase + lo] == bl) {
-              const size_t wj = (size_t)P.wbase + lo;
-              g0 = a.gamma[0 * a.WS + wj];
-              g1 = a.gamma[1 * a.WS + wj];
-              g2 = a.gamma[2 * a.WS + wj];
-            }
-          } else if (warm) {
-            const size_t wi = (size_t)P.wbase + k;
-            g0 = k < gsize ? a.gamma[0 * a.WS + wi] : 0.0;
-            g1 = k < gsize ? a.gamma[1 * a.WS + wi] : 0.0;
-            g2 = k < gsize ? a.gamma[2 * a.WS + wi] : 0.0;
-          } else if (P.nbil == 0) {
-            g0 = 1.0; g1 = 0.0; g2 = 0.0;
-          } else {
-            // the initialiser's (1, 0, 0) pattern over flat entries [0, 3 nc)
-            // of a vector whose first nbil entries are the bilateral rows;
-            // flat entries from 3 nc on keep what the resize kept
-            const long long f = (long long)P.nbil + 3LL * k, lim = 3LL * nc;
-            const size_t wi = (size_t)P.wbase + k;
-            double gg[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d)
-              gg[d] = (f + d < lim) ? (((f + d) % 3 == 0) ? 1.0 : 0.0)
-                                    : (k < gsize ? a.gamma[d * a.WS + wi] : 0.0);
-            g0 = gg[0]; g1 = gg[1]; g2 = gg[2];
-          }
-          const T x0 = (T)g0, x1 = (T)g1, x2 = (T)g2;
-          a.G[0][0 * S + c] = x0; a.G[0][1 * S + c] = x1; a.G[0][2 * S + c] = x2;
-          const T e0 = x0 + T(-1), e1 = x1 + T(-1), e2 = x2 + T(-1);
-          acc[0] = acc[0] + dot3i(e0, e1, e2, e0, e1, e2);
-          Frame<T> f = load_frame<T>(a, c, P.exact != 0);
-          store_keep(qv + c, f_times<T, V>(f, e0, e1, e2));
-        }
-      }
-      park_tile<1, false>(s_def, nslot, t, acc, 0.0);
-      ++run.n;
-      if (++nslot == kMaxDefer) {
-        fold_parked<1, false>(a, s_def, nslot);
-        nslot = 0;
-      }
+      double mi = __ldg(a.minv + b);
+      double m = mi;
+      if (m) m = 1.0 / m;
+      double4 v = a.v4[b], f = a.f4[b];
+      double4 k = make_double4(h * f.x + m * v.x, h * f.y + m * v.y, h * f.z + m * v.z, 0.0);
+      a.k4[b] = k;
+      a.wd[b] = make_double4(mi * k.x, mi * k.y, mi * k.z, 0.0);
     }
-    fold_parked<1, false>(a, s_def, nslot);
-    flush_run(a, run, ctl);
-  }
-  if (!grid_sync(a, kPhaseSetup, NoCtl{})) return;
-  load_mask(a, s_mask, mwords);
-  body_pass_schur<T, kAR>(a, s_mask);
-  if (!grid_sync(a, kPhaseSetup, NoCtl{})) return;
 
-  // ---- L = ||N e|| / ||e||; q = F gamma_0 for the first N y
-  {
-    SegRun run;
-    int nslot = 0;
-    auto ctl = [&](int s) { ctl_lipschitz(ca, s, scratch); };
-    for (int i = 0;; ++i) {
-      const int t = cta_tile(a, NT, i);
-      if (t < 0) break;
-      locate(a, sc, t);
-      const int s = sc.s;
-      if (a.refine && !__ldcg(&a.sst[s].ctl.refined)) continue;
-      if (s != run.s) {
-        if (run.n) {
-          fold_parked<1, false>(a, s_def, nslot);
-          nslot = 0;
-        }
-        flush_run(a, run, ctl);
-        run.s = s;
-      }
-      const int k0 = (t - sc.t0) * kTileItems, nc = sc.nc, c0 = sc.c0;
-      double acc[1] = {0.0};
-      const int kb = a.nbil ? bil_tile_k0(t, sc.t0, nc) : -1;
-      if (kb >= 0) {
-        // bilateral rows: (N e)_row; q = gamma_0 for the first N y
-        const SegParams& P = a.seg[s];
-        const T* wt = reinterpret_cast<const T*>(a.wd);
-        for (int m = 0; m < kItemsPerThread; ++m) {
-          const int k = kb + m * kThreads + threadIdx.x;
-          if (k < P.nbil) {
-            const int i = P.bil0 + k;
-            const T n0 = bil_dw<T>(__ldg(a.bil_off + i), wt);
-            acc[0] = acc[0] + (double)n0 * (double)n0;
-            a.bq[i] = a.bG[0][i];
-          }
-        }
-      }
-      for (int m = 0; m < kItemsPerThread && kb < 0; ++m) {
-        int k = k0 + m * kThreads + threadIdx.x;
-        if (k < nc) {
-          const int c = c0 + k;
-          Frame<T> f = load_frame<T>(a, c, a.seg[s].exact != 0);
-          V wa = wv[__ldg(a.ida + c)], wb = wv[__ldg(a.idb + c)];
-          T n0, n1, n2;
-          ft_times<T, V>(f, wa, wb, &n0, &n1, &n2);
-          acc[0] = acc[0] + dot3i(n0, n1, n2, n0, n1, n2);
-          T y0 = a.G[0][0 * S + c], y1 = a.G[0][1 * S + c], y2 = a.G[0][2 * S + c];
-          store_keep(qv + c, f_times<T, V>(f, y0, y1, y2));
-        }
-      }
-      park_tile<1, false>(s_def, nslot, t, acc, 0.0);
-      ++run.n;
-      if (++nslot == kMaxDefer) {
-        fold_parked<1, false>(a, s_def, nslot);
-        nslot = 0;
-      }
-    }
-    fold_parked<1, false>(a, s_def, nslot);
-    flush_run(a, run, ctl);
-  }
-  // step_count is raised by atomics of other CTAs: read and clear it atomically
-  auto latch = [&]() {
-    if (threadIdx.x == 0) {
-      int n = atomicExch(&a.ew->step_count, 0);
-      *(volatile int*)&a.ew->step_needed = n;
-    }
-  };
-  if (!grid_sync(a, kPhaseSetup, latch)) return;
-  load_mask(a, s_mask, mwords);
-  body_pass_schur<T, kAR>(a, s_mask);
-  if (!grid_sync(a, kPhaseSetup, NoCtl{})) return;
+    if (live) {
+      if (!sync(kPhaseSetup, true)) return;
 
-  // ---- APGD iterations (APGD.cu:227-350)
-  //
-  // Each iteration is one body pass (w = Minv D^T q of gamma_new) and one
-  // contact pass that computes N gamma_new, the objective and the residual of
-  // iteration k, and -- assuming the Lipschitz test accepts gamma_new -- the
-  // whole step of iteration k+1 (y, N y, g, gamma_new = P(y - t g), q).  When
-  // the test fails (backtracking) the look-ahead is discarded and a step pass
-  // recomputes gamma_new with the doubled L; the arithmetic of every value is
-  // the same either way.  A segment's first step is a step pass too (N y_0
-  // is a product: w of gamma_0).  Segment scalars are loaded once per run of
-  // consecutive tiles of one segment.
-  // one segment: its step and product controllers run at the passes' barriers
-  const bool single = a.nseg == 1;
-  // the product pass's barrier also decides whether the work lists are rebuilt:
-  // once half the segments iterating at the last build have finished
-  auto latch_product = [&]() {
-    if (single) {
-      ctl_product(ca, 0, scratch, true);
-      return;
-    }
-    if (threadIdx.x == 0) {
-      volatile EngineWords* E = a.ew;
-      const int n = atomicExch(&a.ew->step_count, 0);
-      E->step_needed = n;
-      const int act = E->active;
-      if (a.nseg > 1 && act > 0 && 2 * act <= E->act_base) E->act_rebuild = 1;
-    }
-  };
-  for (;;) {
-    if (__ldcg(&a.ew->active) == 0) break;
-    // the done mask at the start of a pass holds for every tile this CTA has
-    // left in the pass: a segment finishes only after all its tiles
-    load_mask(a, s_mask, mwords);
-    const int lon = __ldcg(&a.ew->act_on);
-    const int NTL = lon ? __ldcg(&a.ew->act_nt) : NT;
-    const int NBL = lon ? __ldcg(&a.ew->act_nb) : 0;
-    if (__ldcg(&a.ew->step_needed) > 0) {
-      SegRun run;
-      int nslot = 0;
-      auto ctl = [&](int s) { ctl_step(ca, s, scratch); };
-      int cs = -1;
-      for (int i = 0;; ++i) {
-        const int t = pass_tile(a, lon, NTL, i);
-        if (t < 0) break;
-        locate(a, sc, t);
-        const int s = sc.s;
-        if (s != cs) {
-          cs = s;
-          __syncthreads();
-          if (threadIdx.x == 0) {
-            int part = !mask_done(a, s_mask, mwords, s);
-            if (part) {
-              const ApgdCtl* C = &a.sst[s].ctl;
-              const int first = __ldcg(&C->first);
-              part = first || __ldcg(&C->mode) == 1;
-              s_st.first = first;
-              s_st.cur = __ldcg(&C->cur);
-              s_st.prev = __ldcg(&C->prev);
-              s_st.nw = __ldcg(&C->nw);
-              s_st.yr = __ldcg(&C->yr);
-              const double yb = __ldcg(&C->yb);
-              s_st.ya = 1.0 + yb;
-              s_st.ym = -yb;
-              s_st.nt = -__ldcg(&C->t);
-              s_st.mu = a.seg[s].mu;
-              s_st.exact = a.seg[s].exact;
-              if (kAR) s_st.rsel = __ldcg(&C->rsel);
-            }
-            s_st.part = part;
-          }
-          __syncthreads();
-        }
-        const bool part = s_st.part != 0;
-        if (!part) continue;
-        if (s != run.s) {
-          if (run.n) {
-            fold_parked<5, false>(a, s_def, nslot);
-            nslot = 0;
-          }
-          flush_run(a, run, ctl, single);
-          run.s = s;
-        }
-        const int cur = s_st.cur, prev = s_st.prev, first = s_st.first, yr = s_st.yr;
-        const T ya = (T)s_st.ya, ym = (T)s_st.ym, nt_ = (T)s_st.nt, mu = (T)s_st.mu;
-        const T* Gc = a.G[cur];
-        const T* Gp = a.G[prev < 0 ? cur : prev];
-        T* NGc = a.NG[cur];
-        const T* NGp = a.NG[prev < 0 ? cur : prev];
-        T* Gn = a.G[s_st.nw];
-        const int k0 = (t - sc.t0) * kTileItems, nc = sc.nc, c0 = sc.c0;
-        double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        const int kb = a.nbil ? bil_tile_k0(t, sc.t0, nc) : -1;
-        if (kb >= 0) {
-          // bilateral rows: the same step without the cone projection
-          const SegParams& P = a.seg[s];
-          const T* wt = reinterpret_cast<const T*>(a.wd);
-          const T* bGc = a.bG[cur];
-          const T* bGp = a.bG[prev < 0 ? cur : prev];
-          T* bNGc = a.bNG[cur];
-          const T* bNGp = a.bNG[prev < 0 ? cur : prev];
-          T* bGn = a.bG[s_st.nw];
-          for (int m = 0; m < kItemsPerThread; ++m) {
-            const int k = kb + m * kThreads + threadIdx.x;
-            if (k < P.nbil) {
-              const int i = P.bil0 + k;
-              const T c0v = bGc[i];
-              T y0, N0;
-              if (yr) y0 = c0v;
-              else y0 = ya * c0v + ym * bGp[i];
-              if (first) {
-                N0 = bil_dw<T>(__ldg(a.bil_off + i), wt);
-                bNGc[i] = N0;
-              } else if (yr) {
-                N0 = bNGc[i];
-              } else {
-                N0 = ya * bNGc[i] + ym * bNGp[i];
-              }
-              const T r0 = a.br[i];
-              const T g0 = N0 + r0;
-              const T x0 = y0 + nt_ * g0;
-              bGn[i] = x0;
-              a.bq[i] = x0;
-              const T t0 = x0 + T(-1) * y0, s0 = x0 + T(-1) * c0v;
-              acc[0] = acc[0] + (double)g0 * (double)t0;
-              acc[1] = acc[1] + (double)t0 * (double)t0;
-              acc[2] = acc[2] + (double)g0 * (double)s0;
-              if (first) {
-                acc[3] = acc[3] + (double)y0 * (double)N0;
-                acc[4] = acc[4] + (double)y0 * (double)r0;
-              }
-            }
-          }
-        } else {
-          // the second item's lines into L2 while the first one computes
-          const int k = k0 + kThreads + threadIdx.x;
-          if (k < nc) {
-            const int c = c0 + k;
-            const T* nrm = normal_planes<T>(a);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-              prefetch_l2(nrm + d * S + c);
-              prefetch_l2(Gc + d * S + c);
-              prefetch_l2(a.r + d * S + c);
-              if (!first) prefetch_l2(NGc + d * S + c);
-              if (!yr) {
-                prefetch_l2(Gp + d * S + c);
-                if (!first) prefetch_l2(NGp + d * S + c);
-              }
-            }
-          }
-        }
-        for (int m = 0; m < kItemsPerThread && kb < 0; ++m) {
-          int k = k0 + m * kThreads + threadIdx.x;
-          if (k < nc) {
-            const int c = c0 + k;
-            Frame<T> f = load_frame<T>(a, c, s_st.exact != 0);
-            T c0v = Gc[0 * S + c], c1v = Gc[1 * S + c], c2v = Gc[2 * S + c];
-            T y0, y1, y2, N0, N1, N2;
-            if (yr) {
-              y0 = c0v; y1 = c1v; y2 = c2v;
-            } else {
-              y0 = ya * c0v + ym * Gp[0 * S + c];
-              y1 = ya * c1v + ym * Gp[1 * S + c];
-              y2 = ya * c2v + ym * Gp[2 * S + c];
-            }
-            if (first) {
-              V wa = wv[__ldg(a.ida + c)], wb = wv[__ldg(a.idb + c)];
-              ft_times<T, V>(f, wa, wb, &N0, &N1, &N2);
-              NGc[0 * S + c] = N0; NGc[1 * S + c] = N1; NGc[2 * S + c] = N2;
-            } else if (yr) {
-              N0 = NGc[0 * S + c]; N1 = NGc[1 * S + c]; N2 = NGc[2 * S + c];
-            } else {
-              N0 = ya * NGc[0 * S + c] + ym * NGp[0 * S + c];
-              N1 = ya * NGc[1 * S + c] + ym * NGp[1 * S + c];
-              N2 = ya * NGc[2 * S + c] + ym * NGp[2 * S + c];
-            }
-            T r0 = kAR ? (T)a.ar_r0[(size_t)s_st.rsel * S + c] : a.r[0 * S + c];
-            T r1 = a.r[1 * S + c], r2 = a.r[2 * S + c];
-            T g0 = N0 + r0, g1 = N1 + r1, g2 = N2 + r2;
-            T x0 = y0 + nt_ * g0, x1 = y1 + nt_ * g1, x2 = y2 + nt_ * g2;
-            project_cone<T>(x0, x1, x2, mu);
-            Gn[0 * S + c] = x0; Gn[1 * S + c] = x1; Gn[2 * S + c] = x2;
-            store_keep(qv + c, f_times<T, V>(f, x0, x1, x2));
-            T t0 = x0 + T(-1) * y0, t1 = x1 + T(-1) * y1, t2 = x2 + T(-1) * y2;
-            T s0 = x0 + T(-1) * c0v, s1 = x1 + T(-1) * c1v, s2 = x2 + T(-1) * c2v;
-            acc[0] = acc[0] + dot3i(g0, g1, g2, t0, t1, t2);
-            acc[1] = acc[1] + dot3i(t0, t1, t2, t0, t1, t2);
-            acc[2] = acc[2] + dot3i(g0, g1, g2, s0, s1, s2);
-            if (first) {
-              acc[3] = acc[3] + dot3i(y0, y1, y2, N0, N1, N2);
-              acc[4] = acc[4] + dot3i(y0, y1, y2, r0, r1, r2);
-            }
-          }
-        }
-        park_tile<5, false>(s_def, nslot, t, acc, 0.0);
-        ++run.n;
-        if (++nslot == kMaxDefer) {
-          fold_parked<5, false>(a, s_def, nslot);
-          nslot = 0;
-        }
-      }
-      fold_parked<5, false>(a, s_def, nslot);
-      flush_run(a, run, ctl, single);
-      if (!grid_sync(a, kPhaseStep, [&]() {
-            if (single) ctl_step(ca, 0, scratch);
-          }))
-        return;
-    }
-    body_pass_schur<T, kAR>(a, s_mask, lon, NBL);
-    if (!grid_sync(a, kPhaseBody, NoCtl{})) return;
-
-    // N gamma_new, objective (APGD.cu:237-238), residual (:90-102); then the
-    // next iteration's step assuming gamma_new is accepted (:266-273, 312-332)
-    {
-      const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-      // this CTA's next iterating tile at or after sequence index i (-1: none)
-      auto next_tile = [&](int i, int* tile_out) {
-        for (;; ++i) {
-          int t = pass_tile(a, lon, NTL, i);
-          if (t < 0) return -1;
-          locate(a, sc, t);
-          // contact tiles only (the bilateral rows' tiles have their own loop)
-          if (!mask_done(a, s_mask, mwords, sc.s) &&
-              (!a.nbil || (t - sc.t0) * kTileItems < sc.nc)) {
-            *tile_out = t;
-            return i;
-          }
-        }
-      };
-      // bulk copies of (tile t of segment s, sub-tile sub) for this warp into stage sidx
-      auto issue = [&](int t, int st0, int sc0, int snc, int sub, int sidx, int cur, int nw,
-                       int restart, int rsel) {
-        const int kw = (t - st0) * kTileItems + sub * kSub + warp * 32;
-        if (lane == 0 && kw < snc) {
-          mark_stage_issued(stg, sidx);
-          const int cw = sc0 + kw;
-          const T* nrm = normal_planes<T>(a);
-          const T* src[kStagePlanes];
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            src[k] = nrm + k * S;
-            src[3 + k] = a.G[nw] + k * S;
-            src[6 + k] = a.r + k * S;
-            src[9 + k] = a.G[cur] + k * S;
-            src[12 + k] = a.NG[cur] + k * S;
-          }
-          // anti-relaxation: the current plane of r_n
-          if (kAR) src[6] = reinterpret_cast<const T*>(a.ar_r0 + (size_t)rsel * S);
-          const int nd = restart ? 9 : kStagePlanes;
-          const unsigned pbytes = 32u * (unsigned)sizeof(T);
-          unsigned char* dst = stg.base + (size_t)(2 * warp + sidx) * stg.stage_bytes;
-          uint64_t* bar = stg.bar + 2 * warp + sidx;
-          // order this warp's earlier generic reads of the stage before the copies
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          mbar_arrive_expect_tx(bar, (unsigned)nd * pbytes + 256u);
-          for (int p = 0; p < nd; ++p) bulk_g2s(dst + (size_t)p * pbytes, src[p] + cw, pbytes, bar);
-          unsigned char* ids = dst + (size_t)kStagePlanes * pbytes;
-          bulk_g2s(ids, a.ida + cw, 128, bar);
-          bulk_g2s(ids + 128, a.idb + cw, 128, bar);
-        }
-      };
-      auto load_ps = [&](int s) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          const ApgdCtl* C = &a.sst[s].ctl;
-          const int cur = __ldcg(&C->cur), prev = __ldcg(&C->prev), nw = __ldcg(&C->nw);
-          const int best = __ldcg(&C->best);
-          const double beta = __ldcg(&C->beta), gd = __ldcg(&C->gdiff);
-          s_ps.cur = cur;
-          s_ps.nw = nw;
-          s_ps.nw2 = free_slot(nw, cur, prev, best);
-          s_ps.restart = __ldcg(&C->restart);
-          s_ps.ya = 1.0 + beta;
-          s_ps.ym = -beta;
-          s_ps.nt2 = -(1.0 / (0.9 * __ldcg(&C->L)));
-          s_ps.gd = gd;
-          s_ps.gA = __ldcg(&C->ginv);
-          s_ps.gB = -1.0 / gd;
-          s_ps.mu = a.seg[s].mu;
-          s_ps.exact = a.seg[s].exact;
-          if (kAR) s_ps.rsel = __ldcg(&C->rsel);
-        }
-        __syncthreads();
-      };
-      SegRun run;
-      int nslot = 0;
-      auto ctl = [&](int s) { ctl_product(ca, s, scratch); };
-
-      double acc[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-      double mx = 0.0;
-      bool bad = false, failed = false;
-      int tcur = -1;
-      int seq = next_tile(0, &tcur);
-      int sub = 0, sidx = 0;
-      const ProdScalars& ps = s_ps;
-      int s = -1, sc0 = 0, st0 = 0, snc = 0;
-      if (seq >= 0) {
-        locate(a, sc, tcur);
-        s = sc.s;
-        load_ps(s);
-        sc0 = sc.c0; st0 = sc.t0; snc = sc.nc;
-        issue(tcur, st0, sc0, snc, 0, 0, ps.cur, ps.nw, ps.restart, kAR ? ps.rsel : 0);
-      }
-      while (seq >= 0) {
-        const int ti = tcur;
-        if (sub == 0 && s != run.s) {
-          if (run.n) {
-            if (!fold_parked<7, true>(a, s_def, nslot)) {
-              drain_warp_stages(stg, &a.ew->wait_limit_ns);
-              return;
-            }
-            nslot = 0;
-          }
-          flush_run(a, run, ctl, single);
-          run.s = s;
-        }
-        // the following sub-tile: this tile's second half, or the next tile
-        // (next_tile leaves that tile's segment in sc)
-        int nseq = seq, ntile = tcur, nsub = sub + 1;
-        if (nsub == kItemsPerThread) {
-          nsub = 0;
-          nseq = next_tile(seq + 1, &ntile);
-        }
-        const int ns = (nseq >= 0 && nsub == 0) ? sc.s : s;
-        __syncwarp();  // the warp's reads of stage sidx^1 are done
-        if (nseq >= 0 && !failed) {
-          if (ns == s) {
-            issue(ntile, st0, sc0, snc, nsub, sidx ^ 1, ps.cur, ps.nw, ps.restart,
-                  kAR ? ps.rsel : 0);
-          } else {
-            const ApgdCtl* C = &a.sst[ns].ctl;
-            issue(ntile, sc.t0, sc.c0, sc.nc, nsub, sidx ^ 1, __ldcg(&C->cur), __ldcg(&C->nw),
-                  __ldcg(&C->restart), kAR ? __ldcg(&C->rsel) : 0);
-          }
-        }
-        const int kw = (ti - st0) * kTileItems + sub * kSub + warp * 32;
-        if (kw < snc && !failed) {
-          if (!wait_warp_stage(a, stg, sidx)) failed = true;
-        }
-        const int k = kw + lane;
-        if (k < snc && !failed) {
-          const int c = sc0 + k;
-          const T* sd =
-              reinterpret_cast<const T*>(stg.base + (size_t)(2 * warp + sidx) * stg.stage_bytes);
-          const uint32_t* su = reinterpret_cast<const uint32_t*>(sd + (size_t)kStagePlanes * 32);
-          const int j = lane;
-          Frame<T> f =
-              make_frame<T>(sd[0 * 32 + j], sd[1 * 32 + j], sd[2 * 32 + j], ps.exact != 0);
-          V wa = wv[su[j]], wb = wv[su[32 + j]];
-          T N0, N1, N2;
-          ft_times<T, V>(f, wa, wb, &N0, &N1, &N2);
-          T* NGn = a.NG[ps.nw];
-          NGn[0 * S + c] = N0; NGn[1 * S + c] = N1; NGn[2 * S + c] = N2;
-          T x0 = sd[3 * 32 + j], x1 = sd[4 * 32 + j], x2 = sd[5 * 32 + j];
-          T r0 = sd[6 * 32 + j], r1 = sd[7 * 32 + j], r2 = sd[8 * 32 + j];
-          acc[0] = acc[0] + dot3i(x0, x1, x2, N0, N1, N2);
-          acc[1] = acc[1] + dot3i(x0, x1, x2, r0, r1, r2);
-          {
-            // residual, FP64 in both paths (gd = 1/nc^2 is far below float
-            // resolution).  The mixed path takes it at the FP64 projection of
-            // the FP32 iterate: the residual divides by gd, which would
-            // otherwise magnify the iterate's float rounding off the cone.
-            double X0 = x0, X1 = x1, X2 = x2;
-            if (sizeof(T) != sizeof(double)) project_cone<double>(X0, X1, X2, ps.mu);
-            double T0 = (double)r0 + (double)N0, T1 = (double)r1 + (double)N1,
-                   T2 = (double)r2 + (double)N2;
-            T0 = X0 + (-ps.gd) * T0; T1 = X1 + (-ps.gd) * T1; T2 = X2 + (-ps.gd) * T2;
-            project_cone<double>(T0, T1, T2, ps.mu);
-            const double gA = ps.gA, gB = ps.gB;
-            T0 = gA * X0 + gB * T0; T1 = gA * X1 + gB * T1; T2 = gA * X2 + gB * T2;
-            double m0 = fabs(T0), m1 = fabs(T1), m2 = fabs(T2);
-            bad |= (m0 != m0) || (m1 != m1) || (m2 != m2);
-            mx = fmax(mx, fmax(m0, fmax(m1, m2)));
-          }
-          // look-ahead step of iteration k+1: y = (1+b) x - b gamma_k, or x after a restart
-          const T ya = (T)ps.ya, ym = (T)ps.ym;
-          const T nt2 = (T)ps.nt2;
-          T y0, y1, y2, M0, M1, M2;
-          if (ps.restart) {
-            y0 = x0; y1 = x1; y2 = x2;
-            M0 = N0; M1 = N1; M2 = N2;
-          } else {
-            T c0v = sd[9 * 32 + j], c1v = sd[10 * 32 + j], c2v = sd[11 * 32 + j];
-            y0 = ya * x0 + ym * c0v; y1 = ya * x1 + ym * c1v; y2 = ya * x2 + ym * c2v;
-            M0 = ya * N0 + ym * sd[12 * 32 + j];
-            M1 = ya * N1 + ym * sd[13 * 32 + j];
-            M2 = ya * N2 + ym * sd[14 * 32 + j];
-          }
-          T rn0 = r0;  // r_n of the next iteration
-          if (kAR) {
-            // APGD.cu:335-345 for gamma_new = x: v = Minv (k + D^T x) of the
-            // body pass, s = (D v)_(u, v), ar = sqrt(s_u^2 + s_v^2) mu;
-            // r_n' = ar + (-ar_old + r_n), into the next plane
-            const double4 va = a.v_ar[su[j]], vb = a.v_ar[su[32 + j]];
-            const double d0 = va.x - vb.x, d1 = va.y - vb.y, d2 = va.z - vb.z;
-            const double s_u = (f.u0 * d0 + f.u1 * d1) + f.u2 * d2;
-            const double s_v = (f.v0 * d0 + f.v1 * d1) + f.v2 * d2;
-            const double arn = sqrt(s_u * s_u + s_v * s_v) * ps.mu;
-            const size_t cur_p = (size_t)ps.rsel * S + c, nxt_p = (size_t)(ps.rsel ^ 1) * S + c;
-            const double rnn = arn + (-a.ar_v[cur_p] + (double)r0);
-            a.ar_r0[nxt_p] = rnn;
-            a.ar_v[nxt_p] = arn;
-            rn0 = (T)rnn;
-          }
-          T g0 = M0 + rn0, g1 = M1 + r1, g2 = M2 + r2;
-          T z0 = y0 + nt2 * g0, z1 = y1 + nt2 * g1, z2 = y2 + nt2 * g2;
-          project_cone<T>(z0, z1, z2, (T)ps.mu);
-          T* G2 = a.G[ps.nw2];
-          G2[0 * S + c] = z0; G2[1 * S + c] = z1; G2[2 * S + c] = z2;
-          store_keep(qv + c, f_times<T, V>(f, z0, z1, z2));
-          T t0 = z0 + T(-1) * y0, t1 = z1 + T(-1) * y1, t2 = z2 + T(-1) * y2;
-          T s0 = z0 + T(-1) * x0, s1 = z1 + T(-1) * x1, s2 = z2 + T(-1) * x2;
-          acc[2] = acc[2] + dot3i(g0, g1, g2, t0, t1, t2);
-          acc[3] = acc[3] + dot3i(t0, t1, t2, t0, t1, t2);
-          acc[4] = acc[4] + dot3i(g0, g1, g2, s0, s1, s2);
-          acc[5] = acc[5] + dot3i(y0, y1, y2, M0, M1, M2);
-          acc[6] = acc[6] + dot3i(y0, y1, y2, rn0, r1, r2);
-        }
-        if (sub == kItemsPerThread - 1) {
-          if (__any_sync(0xffffffffu, bad) && lane == 0) seg_error(a, s, kErrNaN);
-          if (failed && lane == 0) s_def.fail = 1;
-          park_tile<7, true>(s_def, nslot, ti, acc, mx);
-          for (int qq = 0; qq < 7; ++qq) acc[qq] = 0.0;
-          mx = 0.0;
-          bad = false;
-          ++run.n;
-          if (++nslot == kMaxDefer) {
-            if (!fold_parked<7, true>(a, s_def, nslot)) {
-              drain_warp_stages(stg, &a.ew->wait_limit_ns);
-              return;
-            }
-            nslot = 0;
-          }
-        }
-        seq = nseq;
-        tcur = ntile;
-        sub = nsub;
-        sidx ^= 1;
-        if (ns != s) {
-          s = ns;
-          load_ps(s);
-          sc0 = sc.c0; st0 = sc.t0; snc = sc.nc;
-        }
-      }
-      if (!fold_parked<7, true>(a, s_def, nslot)) {
-        drain_warp_stages(stg, &a.ew->wait_limit_ns);
-        return;
-      }
-      nslot = 0;
-      flush_run(a, run, ctl, single);
-      if (a.nbil) {
-        // then the bilateral rows' tiles: N gamma_new, the objective and
-        // residual items and the look-ahead step, without the cone projection
-        const T* wt = reinterpret_cast<const T*>(a.wd);
+      // ---- r = D (Minv k) + b; gamma_0 -> G[0]; e = gamma_0 - gamma_hat_0 (= gamma_0 - 1)
+      {
+        int nslot = 0;
         for (int i = 0;; ++i) {
-          const int t = pass_tile(a, lon, NTL, i);
+          const int t = team_tile(tm, tm.nt, i);
           if (t < 0) break;
-          locate(a, sc, t);
-          const int s = sc.s;
-          if (mask_done(a, s_mask, mwords, s)) continue;
-          const int kb = bil_tile_k0(t, sc.t0, sc.nc);
-          if (kb < 0) continue;
-          if (s != run.s) {
-            if (run.n) {
-              fold_parked<7, true>(a, s_def, nslot);
+          const int k0 = t * kTileItems, gsize = tm.gsize;
+          const double h = P.h;
+          double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+          const int kb = a.nbil ? bil_tile_k0(t, 0, nc) : -1;
+          if (kb >= 0) {
+            // bilateral rows: b = violation / h (System.cu:1526-1544) at the
+            // step's start time, r = b + (D Minv k)_row, gamma_0, e = gamma_0 - 1
+            const double* pd = reinterpret_cast<const double*>(a.p4);
+            const double* wdv = reinterpret_cast<const double*>(a.wd);
+            const double tmv = a.seg_time[s];
+            for (int m = 0; m < kItemsPerThread; ++m) {
+              const int k = kb + m * kThreads + threadIdx.x;
+              if (k < P.nbil) {
+                const int i2 = P.bil0 + k;
+                const int2 o = __ldg(a.bil_off + i2);
+                const double4 inf = a.bil_info[i2];  // velocity, start time, p0
+                double velocity = inf.x;
+                if (tmv < inf.y) velocity = 0;
+                const double pa = pd[o.x];
+                const double viol = o.y >= 0 ? pa - pd[o.y] - velocity * (tmv - inf.y)
+                                             : pa - inf.z - velocity * (tmv - inf.y);
+                const double bb = viol / h;
+                a.bil_b[i2] = bb;
+                a.br[i2] = (T)(bb + bil_dw<double>(o, wdv));
+                // warm start: the row's last impulse.  Without it the reference's
+                // initialiser writes (1, 0, 0) over flat entries [0, 3 nc) with
+                // the rows first (APGD.cu:114-120, 200): row k takes 1 if k is a
+                // multiple of 3, 0 otherwise, and keeps its last impulse from 3 nc on.
+                double g = a.bil_gam[i2];
+                if (!P.warm && k < 3 * nc) g = (k % 3 == 0) ? 1.0 : 0.0;
+                const T x0 = (T)g;
+                a.bG[0][i2] = x0;
+                const T e0 = x0 + T(-1);
+                acc[0] = acc[0] + (double)e0 * (double)e0;
+                a.bq[i2] = e0;
+              }
+            }
+          }
+          for (int m = 0; m < kItemsPerThread && kb < 0; ++m) {
+            int k = k0 + m * kThreads + threadIdx.x;
+            if (k < nc) {
+              const int c = c0 + k;
+              const uint32_t ia = __ldg(a.ida + c), ib = __ldg(a.idb + c);
+              double4 wa = a.wd[ia], wb = a.wd[ib];
+              const double n0 = __ldg(a.F + c), n1 = __ldg(a.F + S + c), n2 = __ldg(a.F + 2 * S + c);
+              const FrameWords<double> fw = frame_words(n0, n1, n2, P.exact != 0);
+              const Frame<double> fd = make_frame<double>(n0, n1, n2, fw);
+              double d0, d1, d2;
+              ft_times<double, double4>(fd, wa, wb, &d0, &d1, &d2);
+              double bn = __ldg(a.gap + c) / h;
+              const T r0 = (T)(bn + d0), r1 = (T)(0.0 + d1), r2 = (T)(0.0 + d2);
+              a.r[0 * S + c] = r0;
+              a.r[1 * S + c] = r1;
+              a.r[2 * S + c] = r2;
+              if (kAR) {
+                // r_n and the anti-relaxation vector (0 at the start, APGD.cu:196)
+                a.ar_r0[c] = bn + d0;
+                a.ar_v[c] = 0.0;
+              }
+              double g0, g1, g2;
+              // refinement: positional, from the FP32 phase's gamma_hat of this step
+              const int warm = a.refine ? 1 : P.warm;
+              if (warm == 2) {
+                // matched: the impulse the same (A, B) pair had at the last solve;
+                // A's earlier contacts are sorted by B, so a binary search finds it
+                const uint32_t bl = ib - (uint32_t)P.b0;
+                int lo = a.ws[ia], hi = lo + a.wc[ia];
+                if (hi > gsize) hi = gsize;
+                while (lo < hi) {
+                  const int mid = (lo + hi) >> 1;
+                  if (a.wid[(size_t)P.wbase + mid] < bl) lo = mid + 1;
+                  else hi = mid;
+                }
+                g0 = 0.0; g1 = 0.0; g2 = 0.0;
+                if (lo < gsize && lo < a.ws[ia] + a.wc[ia] && a.wid[(size_t)P.wbase + lo] == bl) {
+                  const size_t wj = (size_t)P.wbase + lo;
+                  g0 = a.gamma[0 * a.WS + wj];
+                  g1 = a.gamma[1 * a.WS + wj];
+                  g2 = a.gamma[2 * a.WS + wj];
+                }
+              } else if (warm) {
+                const size_t wi = (size_t)P.wbase + k;
+                g0 = k < gsize ? a.gamma[0 * a.WS + wi] : 0.0;
+                g1 = k < gsize ? a.gamma[1 * a.WS + wi] : 0.0;
+                g2 = k < gsize ? a.gamma[2 * a.WS + wi] : 0.0;
+              } else if (P.nbil == 0) {
+                g0 = 1.0; g1 = 0.0; g2 = 0.0;
+              } else {
+                // the initialiser's (1, 0, 0) pattern over flat entries [0, 3 nc)
+                // of a vector whose first nbil entries are the bilateral rows;
+                // flat entries from 3 nc on keep what the resize kept
+                const long long f = (long long)P.nbil + 3LL * k, lim = 3LL * nc;
+                const size_t wi = (size_t)P.wbase + k;
+                double gg[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                  gg[d] = (f + d < lim) ? (((f + d) % 3 == 0) ? 1.0 : 0.0)
+                                        : (k < gsize ? a.gamma[d * a.WS + wi] : 0.0);
+                g0 = gg[0]; g1 = gg[1]; g2 = gg[2];
+              }
+              const T x0 = (T)g0, x1 = (T)g1, x2 = (T)g2;
+              T* gi = iter_at(a.G[0], c);
+              gi[0] = x0; gi[32] = x1; gi[64] = x2;
+              const T e0 = x0 + T(-1), e1 = x1 + T(-1), e2 = x2 + T(-1);
+              acc[0] = acc[0] + dot3i(e0, e1, e2, e0, e1, e2);
+              // the contact's constants
+              T* p = const_at(a, c);
+              Frame<T> f;
+              if (kMixed) {
+                const T m0 = (T)n0, m1 = (T)n1, m2 = (T)n2;
+                const FrameWords<T> w = frame_words(m0, m1, m2, false);
+                f = make_frame<T>(m0, m1, m2, w);
+                p[96] = w.a; p[128] = w.b; p[160] = w.iv;
+              } else {
+                f = make_frame<T>((T)n0, (T)n1, (T)n2, FrameWords<T>{(T)fw.a, (T)fw.b, (T)fw.iv});
+                p[96] = (T)fw.a; p[128] = (T)fw.b; p[160] = (T)fw.iv;
+              }
+              p[0] = f.n0; p[32] = f.n1; p[64] = f.n2;
+              p[192] = r0; p[224] = r1; p[256] = r2;
+              uint32_t* pi = reinterpret_cast<uint32_t*>(a.blk + (size_t)(c >> 5) * B::kConst + B::kIds) +
+                             (c & 31);
+              pi[0] = ia;
+              pi[32] = ib;
+              store_keep(qv + c, f_times<T, V>(f, e0, e1, e2));
+            }
+          }
+          park8<false>(park, nslot, t, acc);
+          if (++nslot == kParkSlots) {
+            fold_parked8<false>(park, planes(), a.tcap, nslot);
+            nslot = 0;
+          }
+        }
+        fold_parked8<false>(park, planes(), a.tcap, nslot);
+      }
+      if (!sync(kPhaseSetup)) return;
+      fold_team<1, false>(planes(), a.tcap, tm.nt, scratch, C.sums);
+      if (threadIdx.x == 0) C.L0 = sqrt(C.sums[0]);
+      parity ^= 1;
+      team_body_pass<T, kAR>(a, tm, wv, qv);
+      if (!sync(kPhaseSetup)) return;
+
+      // ---- L = ||N e|| / ||e||; q = F gamma_0 for the first N y
+      {
+        int nslot = 0;
+        for (int i = 0;; ++i) {
+          const int t = team_tile(tm, tm.nt, i);
+          if (t < 0) break;
+          const int k0 = t * kTileItems;
+          double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+          const int kb = a.nbil ? bil_tile_k0(t, 0, nc) : -1;
+          if (kb >= 0) {
+            // bilateral rows: (N e)_row; q = gamma_0 for the first N y
+            const T* wt = reinterpret_cast<const T*>(wv);
+            for (int m = 0; m < kItemsPerThread; ++m) {
+              const int k = kb + m * kThreads + threadIdx.x;
+              if (k < P.nbil) {
+                const int i2 = P.bil0 + k;
+                const T n0 = bil_dw<T>(__ldg(a.bil_off + i2), wt);
+                acc[0] = acc[0] + (double)n0 * (double)n0;
+                a.bq[i2] = a.bG[0][i2];
+              }
+            }
+          }
+          for (int m = 0; m < kItemsPerThread && kb < 0; ++m) {
+            int k = k0 + m * kThreads + threadIdx.x;
+            if (k < nc) {
+              const int c = c0 + k;
+              const Frame<T> f = block_frame<T>(const_at(a, c));
+              const uint2 id = block_ids(a, c);
+              V wa = load_vec(wv + id.x), wb = load_vec(wv + id.y);
+              T n0, n1, n2;
+              ft_times<T, V>(f, wa, wb, &n0, &n1, &n2);
+              acc[0] = acc[0] + dot3i(n0, n1, n2, n0, n1, n2);
+              const T* gi = iter_at(a.G[0], c);
+              store_keep(qv + c, f_times<T, V>(f, gi[0], gi[32], gi[64]));
+            }
+          }
+          park8<false>(park, nslot, t, acc);
+          if (++nslot == kParkSlots) {
+            fold_parked8<false>(park, planes(), a.tcap, nslot);
+            nslot = 0;
+          }
+        }
+        fold_parked8<false>(park, planes(), a.tcap, nslot);
+      }
+      if (!sync(kPhaseSetup)) return;
+      fold_team<1, false>(planes(), a.tcap, tm.nt, scratch, C.sums);
+      if (threadIdx.x == 0) ctl_lipschitz(C, P, nc, cap, kMixed);
+      parity ^= 1;
+      team_body_pass<T, kAR>(a, tm, wv, qv);
+      if (!sync(kPhaseSetup)) return;
+
+      // ---- APGD iterations (APGD.cu:227-350)
+      //
+      // Each iteration is one body pass (w = Minv D^T q of gamma_new) and one
+      // contact pass that computes N gamma_new, the objective and the residual of
+      // iteration k, and -- assuming the Lipschitz test accepts gamma_new -- the
+      // whole step of iteration k+1 (y, N y, g, gamma_new = P(y - t g), q).  When
+      // the test fails (backtracking) the look-ahead is discarded and a step pass
+      // recomputes gamma_new with the doubled L; the arithmetic of every value is
+      // the same either way.  A scene's first step is a step pass too (N y_0
+      // is a product: w of gamma_0).
+      while (!C.done) {
+        if (C.step) {
+          int nslot = 0;
+          const int cur = C.cur, prev = C.prev, first = C.first, yr = C.yr;
+          const T ya = (T)C.step_ya, ym = (T)C.step_ym, nt_ = (T)C.step_nt;
+          T* Xc = a.G[cur];
+          const T* Xp = a.G[prev < 0 ? cur : prev];
+          T* Xn = a.G[C.nw];
+          for (int i = 0;; ++i) {
+            const int t = team_tile(tm, tm.nt, i);
+            if (t < 0) break;
+            const int k0 = t * kTileItems;
+            double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            const int kb = a.nbil ? bil_tile_k0(t, 0, nc) : -1;
+            if (kb >= 0) {
+              // bilateral rows: the same step without the cone projection
+              const T* wt = reinterpret_cast<const T*>(wv);
+              const T* bGc = a.bG[cur];
+              const T* bGp = a.bG[prev < 0 ? cur : prev];
+              T* bNGc = a.bNG[cur];
+              const T* bNGp = a.bNG[prev < 0 ? cur : prev];
+              T* bGn = a.bG[C.nw];
+              for (int m = 0; m < kItemsPerThread; ++m) {
+                const int k = kb + m * kThreads + threadIdx.x;
+                if (k < P.nbil) {
+                  const int i2 = P.bil0 + k;
+                  const T c0v = bGc[i2];
+                  T y0, N0;
+                  if (yr) y0 = c0v;
+                  else y0 = ya * c0v + ym * bGp[i2];
+                  if (first) {
+                    N0 = bil_dw<T>(__ldg(a.bil_off + i2), wt);
+                    bNGc[i2] = N0;
+                  } else if (yr) {
+                    N0 = bNGc[i2];
+                  } else {
+                    N0 = ya * bNGc[i2] + ym * bNGp[i2];
+                  }
+                  const T r0 = a.br[i2];
+                  const T g0 = N0 + r0;
+                  const T x0 = y0 + nt_ * g0;
+                  bGn[i2] = x0;
+                  a.bq[i2] = x0;
+                  const T t0 = x0 + T(-1) * y0, s0 = x0 + T(-1) * c0v;
+                  acc[0] = acc[0] + (double)g0 * (double)t0;
+                  acc[1] = acc[1] + (double)t0 * (double)t0;
+                  acc[2] = acc[2] + (double)g0 * (double)s0;
+                  if (first) {
+                    acc[3] = acc[3] + (double)y0 * (double)N0;
+                    acc[4] = acc[4] + (double)y0 * (double)r0;
+                  }
+                }
+              }
+            } else {
+              // the second item's lines into L2 while the first one computes
+              const int k = k0 + kThreads + threadIdx.x;
+              if (k < nc) {
+                const int c = c0 + k;
+                const T* p = const_at(a, c);
+                const T* x = iter_at(Xc, c);
+                const T* y = iter_at(Xp, c);
+#pragma unroll
+                for (int d = 0; d < 9; ++d) prefetch_l2(p + 32 * d);
+#pragma unroll
+                for (int d = 0; d < 6; ++d) {
+                  prefetch_l2(x + 32 * d);
+                  if (!yr) prefetch_l2(y + 32 * d);
+                }
+              }
+            }
+            for (int m = 0; m < kItemsPerThread && kb < 0; ++m) {
+              int k = k0 + m * kThreads + threadIdx.x;
+              if (k < nc) {
+                const int c = c0 + k;
+                const T* p = const_at(a, c);
+                T* xc = iter_at(Xc, c);
+                const T* xp = iter_at(Xp, c);
+                const Frame<T> f = block_frame<T>(p);
+                T c0v = xc[0], c1v = xc[32], c2v = xc[64];
+                T y0, y1, y2, N0, N1, N2;
+                if (yr) {
+                  y0 = c0v; y1 = c1v; y2 = c2v;
+                } else {
+                  y0 = ya * c0v + ym * xp[0];
+                  y1 = ya * c1v + ym * xp[32];
+                  y2 = ya * c2v + ym * xp[64];
+                }
+                if (first) {
+                  const uint2 id = block_ids(a, c);
+                  V wa = load_vec(wv + id.x), wb = load_vec(wv + id.y);
+                  ft_times<T, V>(f, wa, wb, &N0, &N1, &N2);
+                  xc[96] = N0; xc[128] = N1; xc[160] = N2;
+                } else if (yr) {
+                  N0 = xc[96]; N1 = xc[128]; N2 = xc[160];
+                } else {
+                  N0 = ya * xc[96] + ym * xp[96];
+                  N1 = ya * xc[128] + ym * xp[128];
+                  N2 = ya * xc[160] + ym * xp[160];
+                }
+                T r0 = kAR ? (T)a.ar_r0[(size_t)C.rsel * S + c] : p[192];
+                T r1 = p[224], r2 = p[256];
+                T g0 = N0 + r0, g1 = N1 + r1, g2 = N2 + r2;
+                T x0 = y0 + nt_ * g0, x1 = y1 + nt_ * g1, x2 = y2 + nt_ * g2;
+                project_cone<T>(x0, x1, x2, cone_of<T>(C));
+                T* xn = iter_at(Xn, c);
+                xn[0] = x0; xn[32] = x1; xn[64] = x2;
+                store_keep(qv + c, f_times<T, V>(f, x0, x1, x2));
+                T t0 = x0 + T(-1) * y0, t1 = x1 + T(-1) * y1, t2 = x2 + T(-1) * y2;
+                T s0 = x0 + T(-1) * c0v, s1 = x1 + T(-1) * c1v, s2 = x2 + T(-1) * c2v;
+                acc[0] = acc[0] + dot3i(g0, g1, g2, t0, t1, t2);
+                acc[1] = acc[1] + dot3i(t0, t1, t2, t0, t1, t2);
+                acc[2] = acc[2] + dot3i(g0, g1, g2, s0, s1, s2);
+                if (first) {
+                  acc[3] = acc[3] + dot3i(y0, y1, y2, N0, N1, N2);
+                  acc[4] = acc[4] + dot3i(y0, y1, y2, r0, r1, r2);
+                }
+              }
+            }
+            park8<false>(park, nslot, t, acc);
+            if (++nslot == kParkSlots) {
+              fold_parked8<false>(park, planes(), a.tcap, nslot);
               nslot = 0;
             }
-            flush_run(a, run, ctl, single);
-            run.s = s;
           }
-          load_ps(s);
-          const SegParams& P = a.seg[s];
-          const ProdScalars& ps = s_ps;
-          BilRows<T> br_{a.bil_off, wt, a.bG[ps.cur], a.bG[ps.nw], a.bG[ps.nw2], a.bNG[ps.cur],
-                         a.bNG[ps.nw], a.br, a.bq};
-          const bool bad = bil_product_tile<T>(br_, ps, P.bil0 + kb, P.nbil - kb, sc.nc > 0,
-                                               &s_def, nslot, t);
-          if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) seg_error(a, s, kErrNaN);
-          ++run.n;
-          if (++nslot == kMaxDefer) {
-            fold_parked<7, true>(a, s_def, nslot);
+          fold_parked8<false>(park, planes(), a.tcap, nslot);
+          if (!sync(kPhaseStep)) return;
+          fold_team<5, false>(planes(), a.tcap, tm.nt, scratch, C.sums);
+          if (threadIdx.x == 0) ctl_step(C);
+          parity ^= 1;
+          __syncthreads();
+        }
+
+        // ---- the contact pass's sub-tiles of this member; its first two are
+        // copied while the body pass runs
+        const int cur = C.cur, nw = C.nw, restart = C.restart;
+        auto issue = [&](int j) {  // sub-tile j of this member into stage j & 1
+          const int t = team_tile(tm, tm.ntc, j >> 1);
+          const int kw = t * kTileItems + (j & 1) * kSub + warp * 32;
+          if (t >= 0 && kw < nc && lane == 0) {
+            const int sidx = j & 1;
+            const size_t blk = (size_t)(c0 + kw) >> 5;
+            unsigned char* dst = stg.base + (size_t)(2 * warp + sidx) * B::kStageBytes;
+            uint64_t* bar = stg.bar + 2 * warp + sidx;
+            mark_stage_issued(stg, sidx);
+            // gamma_k and N gamma_k only enter without a restart
+            mbar_arrive_expect_tx(bar, B::kConstBytes + (restart ? 1u : 3u) * B::kHalfBytes);
+            bulk_g2s(dst, a.blk + blk * B::kConst, B::kConstBytes, bar);
+            bulk_g2s(dst + B::kConstBytes, a.G[nw] + blk * kIterBlock, B::kHalfBytes, bar);
+            if (!restart)
+              bulk_g2s(dst + B::kConstBytes + B::kHalfBytes, a.G[cur] + blk * kIterBlock,
+                       2 * B::kHalfBytes, bar);
+          }
+        };
+        // this warp's earlier writes of the iterates, and its reads of the
+        // stages, come before the copies
+        asm volatile("fence.proxy.async;" ::: "memory");
+        __syncwarp();
+        issue(0);
+        issue(1);
+        team_body_pass<T, kAR>(a, tm, wv, qv);
+        if (!sync(kPhaseBody)) {
+          drain_warp_stages(stg, &a.ew->wait_limit_ns);
+          return;
+        }
+
+        // N gamma_new, objective (APGD.cu:237-238), residual (:90-102); then the
+        // next iteration's step assuming gamma_new is accepted (:266-273, 312-332)
+        {
+          int nslot = 0;
+          double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+          bool bad = false, failed = false;
+          T* Xn = a.G[nw];
+          T* X2 = a.G[C.nw2];
+          for (int j = 0;; ++j) {
+            const int t = team_tile(tm, tm.ntc, j >> 1);
+            if (t < 0) break;
+            const int sidx = j & 1;
+            if (j && !failed) {
+              __syncwarp();  // the warp's reads of stage sidx^1 are done
+              asm volatile("fence.proxy.async;" ::: "memory");
+              issue(j + 1);
+            }
+            const int kw = t * kTileItems + sidx * kSub + warp * 32;
+            if (kw < nc && !failed && !wait_warp_stage(a, stg, sidx)) {
+              failed = true;
+              s_copy_fail = 1;
+            }
+            const int k = kw + lane;
+            if (k < nc && !failed) {
+              const int c = c0 + k;
+              const T* sd =
+                  reinterpret_cast<const T*>(stg.base + (size_t)(2 * warp + sidx) * B::kStageBytes) + lane;
+              const uint32_t* su = reinterpret_cast<const uint32_t*>(
+                  stg.base + (size_t)(2 * warp + sidx) * B::kStageBytes + B::kIds * sizeof(T)) + lane;
+              const uint32_t ia = su[0], ib = su[32];
+              const V wa = load_vec(wv + ia), wb = load_vec(wv + ib);
+              const Frame<T> f = block_frame<T>(sd);
+              const T* sx = sd + B::kConst;
+              T N0, N1, N2;
+              ft_times<T, V>(f, wa, wb, &N0, &N1, &N2);
+              T* xn = iter_at(Xn, c);
+              xn[96] = N0; xn[128] = N1; xn[160] = N2;
+              const T x0 = sx[0], x1 = sx[32], x2 = sx[64];
+              T r0 = sd[192];
+              const T r1 = sd[224], r2 = sd[256];
+              if (kAR) r0 = (T)a.ar_r0[(size_t)C.rsel * S + c];
+              acc[0] = acc[0] + dot3i(x0, x1, x2, N0, N1, N2);
+              acc[1] = acc[1] + dot3i(x0, x1, x2, r0, r1, r2);
+              {
+                // residual, FP64 in both paths (gd = 1/nc^2 is far below float
+                // resolution).  The mixed path takes it at the FP64 projection of
+                // the FP32 iterate: the residual divides by gd, which would
+                // otherwise magnify the iterate's float rounding off the cone.
+                double X0 = x0, X1 = x1, X2v = x2;
+                if (kMixed) project_cone<double>(X0, X1, X2v, C.cone);
+                const double gd = C.gdiff, gA = C.ginv, gB = C.gneg;
+                double T0 = (double)r0 + (double)N0, T1 = (double)r1 + (double)N1,
+                       T2 = (double)r2 + (double)N2;
+                T0 = X0 + (-gd) * T0; T1 = X1 + (-gd) * T1; T2 = X2v + (-gd) * T2;
+                project_cone<double>(T0, T1, T2, C.cone);
+                T0 = gA * X0 + gB * T0; T1 = gA * X1 + gB * T1; T2 = gA * X2v + gB * T2;
+                double m0 = fabs(T0), m1 = fabs(T1), m2 = fabs(T2);
+                bad |= (m0 != m0) || (m1 != m1) || (m2 != m2);
+                acc[7] = fmax(acc[7], fmax(m0, fmax(m1, m2)));
+              }
+              // look-ahead step of iteration k+1: y = (1+b) x - b gamma_k, or x after a restart
+              T y0, y1, y2, M0, M1, M2;
+              if (restart) {
+                y0 = x0; y1 = x1; y2 = x2;
+                M0 = N0; M1 = N1; M2 = N2;
+              } else {
+                const T ya = (T)C.prod_ya, ym = (T)C.prod_ym;
+                y0 = ya * x0 + ym * sx[96]; y1 = ya * x1 + ym * sx[128]; y2 = ya * x2 + ym * sx[160];
+                M0 = ya * N0 + ym * sx[192];
+                M1 = ya * N1 + ym * sx[224];
+                M2 = ya * N2 + ym * sx[256];
+              }
+              T rn0 = r0;  // r_n of the next iteration
+              if (kAR) {
+                // APGD.cu:335-345 for gamma_new = x: v = Minv (k + D^T x) of the
+                // body pass, s = (D v)_(u, v), ar = sqrt(s_u^2 + s_v^2) mu;
+                // r_n' = ar + (-ar_old + r_n), into the next plane
+                const double4 va = a.v_ar[ia], vb = a.v_ar[ib];
+                const double d0 = va.x - vb.x, d1 = va.y - vb.y, d2 = va.z - vb.z;
+                const double s_u = (f.u0 * d0 + f.u1 * d1) + f.u2 * d2;
+                const double s_v = (f.v0 * d0 + f.v1 * d1) + f.v2 * d2;
+                const double arn = sqrt(s_u * s_u + s_v * s_v) * C.cone.mu;
+                const size_t cur_p = (size_t)C.rsel * S + c, nxt_p = (size_t)(C.rsel ^ 1) * S + c;
+                const double rnn = arn + (-a.ar_v[cur_p] + (double)r0);
+                a.ar_r0[nxt_p] = rnn;
+                a.ar_v[nxt_p] = arn;
+                rn0 = (T)rnn;
+              }
+              const T nt2 = (T)C.prod_nt;
+              T g0 = M0 + rn0, g1 = M1 + r1, g2 = M2 + r2;
+              T z0 = y0 + nt2 * g0, z1 = y1 + nt2 * g1, z2 = y2 + nt2 * g2;
+              project_cone<T>(z0, z1, z2, cone_of<T>(C));
+              T* x2p = iter_at(X2, c);
+              x2p[0] = z0; x2p[32] = z1; x2p[64] = z2;
+              store_keep(qv + c, f_times<T, V>(f, z0, z1, z2));
+              T t0 = z0 + T(-1) * y0, t1 = z1 + T(-1) * y1, t2 = z2 + T(-1) * y2;
+              T s0 = z0 + T(-1) * x0, s1 = z1 + T(-1) * x1, s2 = z2 + T(-1) * x2;
+              acc[2] = acc[2] + dot3i(g0, g1, g2, t0, t1, t2);
+              acc[3] = acc[3] + dot3i(t0, t1, t2, t0, t1, t2);
+              acc[4] = acc[4] + dot3i(g0, g1, g2, s0, s1, s2);
+              acc[5] = acc[5] + dot3i(y0, y1, y2, M0, M1, M2);
+              acc[6] = acc[6] + dot3i(y0, y1, y2, rn0, r1, r2);
+            }
+            if (sidx == kItemsPerThread - 1) {
+              if (__any_sync(0xffffffffu, bad) && lane == 0) seg_error(a, s, kErrNaN);
+              park8<true>(park, nslot, t, acc);
+#pragma unroll
+              for (int q = 0; q < 8; ++q) acc[q] = 0.0;
+              bad = false;
+              if (++nslot == kParkSlots) {
+                fold_parked8<true>(park, planes(), a.tcap, nslot);
+                nslot = 0;
+              }
+            }
+          }
+          fold_parked8<true>(park, planes(), a.tcap, nslot);
+          if (s_copy_fail) {
+            drain_warp_stages(stg, &a.ew->wait_limit_ns);
+            return;
+          }
+          if (a.nbil) {
+            // then the bilateral rows' tiles: N gamma_new, the objective and
+            // residual items and the look-ahead step, without the cone projection
+            nslot = 0;
+            const T* wt = reinterpret_cast<const T*>(wv);
+            for (int i = 0;; ++i) {
+              const int t = team_tile(tm, tm.nt, i);
+              if (t < 0) break;
+              const int kb = bil_tile_k0(t, 0, nc);
+              if (kb < 0) continue;
+              BilRows<T> br_{a.bil_off, wt, a.bG[cur], a.bG[nw], a.bG[C.nw2], a.bNG[cur],
+                             a.bNG[nw], a.br, a.bq};
+              const bool bad2 = bil_product_tile<T>(br_, C, P.bil0 + kb, P.nbil - kb, nc > 0,
+                                                    &park, nslot, t);
+              if (__any_sync(0xffffffffu, bad2) && lane == 0) seg_error(a, s, kErrNaN);
+              if (++nslot == kParkSlots) {
+                fold_parked8<true>(park, planes(), a.tcap, nslot);
+                nslot = 0;
+              }
+            }
+            fold_parked8<true>(park, planes(), a.tcap, nslot);
+          }
+        }
+        if (!sync(kPhaseProduct)) return;
+        fold_team<7, true>(planes(), a.tcap, tm.nt, scratch, C.sums);
+        if (threadIdx.x == 0) ctl_product(C, P, cap, kMixed, kAR);
+        parity ^= 1;
+        __syncthreads();
+      }
+
+      // ---- anti-relaxation: objectiveCCP = 1/2 gamma_hat' N gamma_hat + gamma_hat' r
+      // with the last r (APGD.cu:353-354); the first term was kept when gamma_hat was
+      // found, the second is folded over the tiles here (one scene)
+      if (kAR) {
+        int nslot = 0;
+        const int best = C.best;
+        for (int i = 0;; ++i) {
+          const int t = team_tile(tm, tm.nt, i);
+          if (t < 0) break;
+          double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+          if (best >= 0) {
+            for (int m = 0; m < kItemsPerThread; ++m) {
+              const int k = t * kTileItems + m * kThreads + threadIdx.x;
+              if (k < nc) {
+                const int c = c0 + k;
+                const T* x = iter_at(a.G[best], c);
+                const T* p = const_at(a, c);
+                acc[0] = acc[0] + dot3i(x[0], x[32], x[64], a.ar_r0[(size_t)C.rsel * S + c],
+                                        (double)p[224], (double)p[256]);
+              }
+            }
+          }
+          park8<false>(park, nslot, t, acc);
+          if (++nslot == kParkSlots) {
+            fold_parked8<false>(park, planes(), a.tcap, nslot);
             nslot = 0;
           }
         }
-        fold_parked<7, true>(a, s_def, nslot);
-        nslot = 0;
-        flush_run(a, run, ctl, single);
+        fold_parked8<false>(park, planes(), a.tcap, nslot);
+        if (!sync(kPhaseFinal)) return;
+        fold_team<1, false>(planes(), a.tcap, tm.nt, scratch, C.sums);
+        if (threadIdx.x == 0 && best >= 0) C.objective = C.objN + C.sums[0];
+        parity ^= 1;
+        __syncthreads();
       }
 
-    }
-    if (!grid_sync(a, kPhaseProduct, latch_product)) {
-      drain_warp_stages(stg, &a.ew->wait_limit_ns);
-      return;
-    }
-    if (__ldcg(&a.ew->act_rebuild)) {
-      if (blockIdx.x == 0) rebuild_work_lists(a, reinterpret_cast<int*>(scratch));
-      if (!grid_sync(a, kPhaseRebuild, [&]() {
-            if (threadIdx.x == 0) {
-              volatile EngineWords* E = a.ew;
-              E->act_rebuild = 0;
-              E->act_on = 1;
-              E->act_base = E->active;
+      // ---- gamma = gamma_hat (APGD.cu:358) into the warm-start region; q = F gamma (FP64)
+      {
+        const int best = C.best;
+        // a refinement whose FP64 phase accepted no iterate keeps the FP32
+        // launch's gamma_hat; q is formed again (the setup wrote over it)
+        const bool keep = a.refine && best < 0;
+        const T* src = best >= 0 ? a.G[best] : nullptr;
+        for (int i = 0;; ++i) {
+          const int t = team_tile(tm, tm.nt, i);
+          if (t < 0) break;
+          const int kb = a.nbil ? bil_tile_k0(t, 0, nc) : -1;
+          if (kb >= 0) {
+            // the rows' gamma_hat (ones before the first accepted iterate)
+            for (int m = 0; m < kItemsPerThread; ++m) {
+              const int k = kb + m * kThreads + threadIdx.x;
+              if (k < P.nbil) {
+                const int r = P.bil0 + k;
+                a.bil_gam[r] = best >= 0 ? (double)a.bG[best][r] : 1.0;
+              }
             }
-          }))
-        return;
-    }
-  }
-
-  // ---- anti-relaxation: objectiveCCP = 1/2 gamma_hat' N gamma_hat + gamma_hat' r
-  // with the last r (APGD.cu:353-354); the first term was kept when gamma_hat was
-  // found, the second is folded over the tiles here (one scene)
-  if (kAR) {
-    int nslot = 0;
-    for (int i = 0;; ++i) {
-      const int t = cta_tile(a, NT, i);
-      if (t < 0) break;
-      locate(a, sc, t);
-      const ApgdCtl* C = &a.sst[sc.s].ctl;
-      const int best = __ldcg(&C->best), rsel = __ldcg(&C->rsel);
-      const int k0 = (t - sc.t0) * kTileItems, nc = sc.nc, c0 = sc.c0;
-      double acc[1] = {0.0};
-      if (best >= 0) {
-        const T* B = a.G[best];
-        for (int m = 0; m < kItemsPerThread; ++m) {
-          const int k = k0 + m * kThreads + threadIdx.x;
-          if (k < nc) {
-            const int c = c0 + k;
-            acc[0] = acc[0] + dot3i(B[c], B[S + c], B[2 * S + c], a.ar_r0[(size_t)rsel * S + c],
-                                    (double)a.r[S + c], (double)a.r[2 * S + c]);
+            continue;
           }
-        }
-      }
-      park_tile<1, false>(s_def, nslot, t, acc, 0.0);
-      if (++nslot == kMaxDefer) {
-        fold_parked<1, false>(a, s_def, nslot);
-        nslot = 0;
-      }
-    }
-    fold_parked<1, false>(a, s_def, nslot);
-    if (!grid_sync(a, kPhaseFinal, [&]() {
-          double sm[1];
-          fold_tiles<1>(a, a.sst[0].t0, a.sst[0].nt, sm, scratch);
-          if (threadIdx.x == 0) {
-            ApgdCtl* C = &a.sst[0].ctl;
-            if (__ldcg(&C->best) >= 0) C->objective = __ldcg(&C->objN) + sm[0];
-          }
-        }))
-      return;
-  }
-
-  // ---- gamma = gamma_hat (APGD.cu:358) into the warm-start region; q = F gamma (FP64)
-  {
-    int cs = -1, cbest = -1;
-    bool keep = false, skip = false;
-    const T* src = nullptr;
-    for (int i = 0;; ++i) {
-      const int t = cta_tile(a, NT, i);
-      if (t < 0) break;
-      locate(a, sc, t);
-      const int s = sc.s;
-      if (s != cs) {
-        cs = s;
-        cbest = __ldcg(&a.sst[s].ctl.best);
-        src = cbest >= 0 ? a.G[cbest] : nullptr;
-        // refinement launch: a solve it did not refine keeps the FP32 launch's
-        // gamma_hat and q = F gamma_hat, written by that launch's final pass; one
-        // whose FP64 phase accepted no iterate keeps that gamma_hat, and q is
-        // formed again (this launch's setup passes wrote over it)
-        skip = a.refine && !__ldcg(&a.sst[s].ctl.refined);
-        keep = a.refine && cbest < 0;
-      }
-      if (skip) continue;
-      const SegParams& P = a.seg[s];
-      const int k0 = (t - sc.t0) * kTileItems, nc = sc.nc, c0 = sc.c0;
-      const int kb = a.nbil ? bil_tile_k0(t, sc.t0, nc) : -1;
-      if (kb >= 0) {
-        // the rows' gamma_hat (ones before the first accepted iterate)
-        for (int m = 0; m < kItemsPerThread; ++m) {
-          const int k = kb + m * kThreads + threadIdx.x;
-          if (k < P.nbil) {
-            const int r = P.bil0 + k;
-            a.bil_gam[r] = cbest >= 0 ? (double)a.bG[cbest][r] : 1.0;
-          }
-        }
-        continue;
-      }
-      for (int m = 0; m < kItemsPerThread; ++m) {
-        int k = k0 + m * kThreads + threadIdx.x;
-        if (k < nc) {
-          const int c = c0 + k;
-          double x0 = 1.0, x1 = 1.0, x2 = 1.0;
-          const size_t wi = (size_t)P.wbase + k;
-          if (keep) {
-            x0 = a.gamma[0 * a.WS + wi]; x1 = a.gamma[1 * a.WS + wi]; x2 = a.gamma[2 * a.WS + wi];
-          } else {
-            if (src) {
-              x0 = (double)src[0 * S + c]; x1 = (double)src[1 * S + c]; x2 = (double)src[2 * S + c];
+          for (int m = 0; m < kItemsPerThread; ++m) {
+            int k = t * kTileItems + m * kThreads + threadIdx.x;
+            if (k < nc) {
+              const int c = c0 + k;
+              double x0 = 1.0, x1 = 1.0, x2 = 1.0;
+              const size_t wi = (size_t)P.wbase + k;
+              if (keep) {
+                x0 = a.gamma[0 * a.WS + wi]; x1 = a.gamma[1 * a.WS + wi]; x2 = a.gamma[2 * a.WS + wi];
+              } else {
+                if (src) {
+                  const T* x = iter_at(src, c);
+                  x0 = (double)x[0]; x1 = (double)x[32]; x2 = (double)x[64];
+                }
+                a.gamma[0 * a.WS + wi] = x0;
+                a.gamma[1 * a.WS + wi] = x1;
+                a.gamma[2 * a.WS + wi] = x2;
+              }
+              a.wid[wi] = __ldg(a.idb + c) - (uint32_t)P.b0;
+              Frame<double> f;
+              if (kMixed) f = load_frame_fp64(a, c, P.exact != 0);
+              else {
+                const T* p = const_at(a, c);
+                f = make_frame<double>((double)p[0], (double)p[32], (double)p[64],
+                                       FrameWords<double>{(double)p[96], (double)p[128], (double)p[160]});
+              }
+              a.qd[c] = f_times<double, double4>(f, x0, x1, x2);
             }
-            a.gamma[0 * a.WS + wi] = x0;
-            a.gamma[1 * a.WS + wi] = x1;
-            a.gamma[2 * a.WS + wi] = x2;
           }
-          a.wid[wi] = __ldg(a.idb + c) - (uint32_t)P.b0;
-          Frame<double> f = load_frame_fp64(a, c, P.exact != 0);
-          a.qd[c] = f_times<double, double4>(f, x0, x1, x2);
         }
       }
+      if (!sync(kPhaseFinal)) return;
     }
-  }
-  if (!grid_sync(a, kPhaseFinal, [&]() {
-        if (threadIdx.x == 0 && !a.solve_only) atomicAdd(&a.ew->steps_done, 1);
-      }))
-    return;
 
-  // ---- f_c = D^T gamma; v = Minv (k + f_c); f_contact = f_c / h; p += h v.
-  // Segments with neither contacts nor bilateral rows: v = Minv k, f_contact = 0
-  // (System.cu:577-581); the rows' impulses enter f_c like the contacts'.
-  for (int bt = blockIdx.x; bt < nbt && !a.solve_only; bt += gridDim.x) {
-    int b = bt * kThreads + threadIdx.x;
-    if (b < a.nb) {
-      const int s = __ldg(a.bseg + b);
-      const SegParams& P = a.seg[s];
-      if (P.active) {
+    // mixed precision: a solve that ended above the tolerance without an error
+    // is refined in FP64 by the launch that follows, which also updates it
+    const unsigned err = C.err | (live ? __ldcg(&a.sst[s].err) : 0u);
+    const bool refine_next = kMixed && P.refine > 0 && live && err == 0u && !(C.residual < P.tol);
+
+    // ---- f_c = D^T gamma; v = Minv (k + f_c); f_contact = f_c / h; p += h v.
+    // Scenes with neither contacts nor bilateral rows: v = Minv k, f_contact = 0
+    // (System.cu:577-581); the rows' impulses enter f_c like the contacts'.
+    if (!a.solve_only && !refine_next) {
+      for (int b = tm.w0 + threadIdx.x; b < tm.w1; b += kThreads) {
         const double h = P.h;
-        const int nc = a.sst[s].nc;
         double4 k = a.k4[b];
         double mi = __ldg(a.minv + b);
         double4 v, fcv;
-        if (nc > 0 || P.nbil > 0) {
+        if (live) {
           double4 fc = gather_q<double, double4>(a, a.qd, b);
           if (a.nbil) add_bilateral<double, double4>(a.bil_inc_start, a.bil_inc, a.bil_gam, b, fc);
           v = make_double4(mi * (k.x + fc.x), mi * (k.y + fc.y), mi * (k.z + fc.z), 0.0);
@@ -1288,36 +1073,133 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
         a.p4[b] = make_double4(h * v.x + p.x, h * v.y + p.y, h * v.z + p.z, 0.0);
       }
     }
-  }
-  // warm-start length of every segment that solved (System::gamma_d resize)
-  for (int s = blockIdx.x * kThreads + threadIdx.x; s < a.nseg; s += gridDim.x * kThreads) {
-    SegState& X = a.sst[s];
-    const bool live = a.seg[s].active && (X.nc > 0 || a.seg[s].nbil > 0);
-    if (live) X.gsize = X.nc;
-    ApgdCtl& C = X.ctl;
-    if (sizeof(T) != sizeof(double) && a.seg[s].refine > 0 && live) {
-      // mixed precision: a solve that ended above the tolerance is refined
-      // in FP64 by the launch that follows
-      C.refined = (X.err == 0u && !(C.residual < a.seg[s].tol)) ? 1 : 0;
+    // matched warm start: where each body's A-contacts went in the warm region
+    if (live) {
+      const int shift = a.sst[s].delta - c0;
+      for (int b = tm.w0 + threadIdx.x; b < tm.w1; b += kThreads) {
+        a.ws[b] = a.cbase[b] + shift;
+        a.wc[b] = a.cnt_cont[b];
+      }
     }
-    if (a.refine && live && C.refined) {
-      C.refine_it = C.iterations;
-      C.iterations += C.it_lo;
-      C.backtracks += C.bt_lo;
-      C.sweeps += C.sw_lo;
+    // the scene's results, and its warm-start length (System::gamma_d resize)
+    if (tm.rank == 0 && threadIdx.x == 0) {
+      SegState& X = a.sst[s];
+      ApgdCtl& D = X.ctl;
+      if (C.err) {
+        X.err = err;
+        if (a.ew->stop_on_seg_err) atomicOr(&a.ew->err, C.err);
+      }
+      D.iterations = C.iterations + it_lo;
+      D.backtracks = C.backtracks + bt_lo;
+      D.sweeps = C.sweeps + sw_lo;
+      D.residual = C.residual;
+      D.objective = C.objective;
+      D.best = C.best;
+      D.done = 1;
+      D.refine_it = a.refine ? C.iterations : 0;
+      if (!a.refine) D.refined = refine_next ? 1 : 0;
+      if (live) X.gsize = nc;
+      // System::time += h (System.cu:584), read by the next step's rows
+      if (a.nbil && !a.solve_only) a.seg_time[s] = a.seg_time[s] + P.h;
     }
-    // System::time += h (System.cu:584), read by the next step's rows
-    if (a.nbil && a.seg[s].active && !a.solve_only) a.seg_time[s] = a.seg_time[s] + a.seg[s].h;
   }
-  // matched warm start: where each body's A-contacts went in the warm region
-  for (int b = blockIdx.x * kThreads + threadIdx.x; b < a.nb; b += gridDim.x * kThreads) {
-    const int s = __ldg(a.bseg + b);
-    const SegState& X = a.sst[s];
-    if (a.seg[s].active && (X.nc > 0 || a.seg[s].nbil > 0)) {
-      a.ws[b] = a.cbase[b] + X.delta - X.c0;
-      a.wc[b] = a.cnt_cont[b];
+  if (a.nseg == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
+    for (int i = 0; i < 8; ++i) {
+      a.ew->phase_ns[i] += timer.ns[i];
+      a.ew->phase_count[i] += timer.count[i];
     }
   }
+}
+
+// The scenes of one launch in teams (engines of several scenes): those that
+// are active (in a refinement launch, those the FP32 launch marked), by size,
+// largest first, each with one member per `per` tiles; slots[] lists (scene,
+// rank) in that order.  One CTA.
+__global__ void __launch_bounds__(1024) k_team_plan(int nseg, const SegParams* __restrict__ seg,
+                                                    SegState* __restrict__ sst, int refine, int grid,
+                                                    int2* __restrict__ slots, int slot_cap,
+                                                    int* __restrict__ order,
+                                                    unsigned* __restrict__ team_bar,
+                                                    EngineWords* __restrict__ ew) {
+  constexpr int kBins = 128;
+  __shared__ int s_bin[kBins], s_tiles, s_warp[32], s_carry;
+  if (ew->err) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < kBins; i += 1024) s_bin[i] = 0;
+  if (tid == 0) {
+    s_tiles = 0;
+    s_carry = 0;
+  }
+  __syncthreads();
+  // bins of four per octave of the tiles, largest first
+  auto bin_of = [](int nt) {
+    if (nt < 4) return kBins - 1 - nt;
+    const int e = 31 - __clz(nt);
+    return kBins - 1 - (4 * (e - 1) + ((nt >> (e - 2)) & 3));
+  };
+  auto takes = [&](int s) { return seg[s].active && (!refine || sst[s].ctl.refined); };
+  for (int s = tid; s < nseg; s += 1024) {
+    if (!refine) sst[s].err = 0u;
+    if (!takes(s)) continue;
+    atomicAdd(&s_bin[bin_of(sst[s].nt)], 1);
+    atomicAdd(&s_tiles, sst[s].nt);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    int at = 0;
+    for (int i = 0; i < kBins; ++i) {
+      const int n = s_bin[i];
+      s_bin[i] = at;
+      at += n;
+    }
+    s_warp[0] = at;
+  }
+  __syncthreads();
+  const int n = s_warp[0];
+  // tiles per member: one while the grid has a CTA for each, then as many as
+  // fill the grid, four at most (a team's barriers and folds cost about 8 us an
+  // iteration, a tile about 5)
+  const int per = max(1, min(kTeamTiles, (s_tiles + grid - 1) / grid));
+  for (int s = tid; s < nseg; s += 1024) {
+    if (!takes(s)) continue;
+    order[atomicAdd(&s_bin[bin_of(sst[s].nt)], 1)] = s;
+    sst[s].members = team_size(sst[s].nt, seg[s].b1 - seg[s].b0, per, grid);
+    for (int i = 0; i < kTeamBarStride; i += kTeamBarStride) team_bar[(size_t)s * kTeamBarStride + i] = 0u;
+  }
+  __syncthreads();
+  for (int base = 0; base < n; base += 1024) {
+    const int i = base + tid;
+    const int s = i < n ? order[i] : -1;
+    const int m = s >= 0 ? sst[s].members : 0;
+    int x = m;
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, off);
+      if (lane >= off) x += y;
+    }
+    __syncthreads();
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    int before = s_carry, total = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) before += s_warp[w];
+      total += s_warp[w];
+    }
+    const int at = before + x - m;
+    for (int r = 0; r < m; ++r)
+      if (at + r < slot_cap) slots[at + r] = make_int2(s, r);
+    __syncthreads();
+    if (tid == 0) s_carry += total;
+    __syncthreads();
+  }
+  if (tid == 0) {
+    ew->ticket = 0u;
+    ew->nslots = min(s_carry, slot_cap);
+  }
+}
+
+template <class T>
+constexpr size_t solve_smem_bytes() {
+  return (size_t)kWarps * 2 * Block<T>::kStageBytes + (size_t)kWarps * 2 * 8 + 16;
 }
 
 template <class T, int MB, bool AR>
@@ -1325,21 +1207,29 @@ void prepare_kernel() {
   static bool done = false;
   if (done) return;
   cudaFuncSetAttribute(k_step_solve<T, MB, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)dyn_smem_bytes<T>());
+                       (int)solve_smem_bytes<T>());
   done = true;
 }
 
-
 template <class T, int MB, bool AR = false>
-void launch_typed(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, bool solve_only,
-                  bool refine = false) {
+void launch_typed(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t* launches,
+                  bool solve_only, bool refine = false) {
   prepare_kernel<T, MB, AR>();
   KArgs<T> a = make_kargs<T>(sd, cfg);
   a.solve_only = solve_only ? 1 : 0;
   a.refine = refine ? 1 : 0;
+  if (sd.nseg > 1) {
+    k_team_plan<<<1, 1024, 0, st>>>(sd.nseg, sd.seg, sd.sst, a.refine, cfg.grid, sd.slots, sd.slot_cap,
+                                    sd.order, sd.team_bar, sd.ew);
+    ++*launches;
+  } else {
+    cudaMemsetAsync(sd.team_bar, 0, sizeof(unsigned), st);
+    if (!refine) cudaMemsetAsync(&sd.sst->err, 0, sizeof(unsigned), st);
+  }
   void* params[] = {&a};
   cudaLaunchCooperativeKernel((const void*)k_step_solve<T, MB, AR>, cfg.grid, kThreads, params,
-                              dyn_smem_bytes<T>(), st);
+                              solve_smem_bytes<T>(), st);
+  ++*launches;
 }
 
 template <class T, int MB>
@@ -1349,7 +1239,7 @@ int max_ctas_of() {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   prepare_kernel<T, MB, false>();
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_solve<T, MB, false>, kThreads,
-                                                dyn_smem_bytes<T>());
+                                                solve_smem_bytes<T>());
   if (per_sm < 1) per_sm = 1;
   return sms * per_sm;
 }
@@ -1366,33 +1256,28 @@ int apgd_max_ctas(int precision, int blocks_per_sm) {
 
 void launch_step_solve(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t* launches,
                        bool solve_only) {
-  cudaMemsetAsync(sd.ew->bar, 0, sizeof(sd.ew->bar), st);
-  cudaMemsetAsync(&sd.ew->last_release, 0, sizeof(unsigned long long), st);
-  if (sd.solver == DV_SOLVER_PGJ) {
-    launch_pgj_solve(sd, cfg, st, solve_only);
-  } else if (sd.solver == DV_SOLVER_PGS) {
-    launch_pgs_solve(sd, cfg, st, solve_only);
+  if (sd.solver == DV_SOLVER_PGJ || sd.solver == DV_SOLVER_PGS) {
+    cudaMemsetAsync(sd.ew->bar, 0, sizeof(sd.ew->bar), st);
+    cudaMemsetAsync(&sd.ew->last_release, 0, sizeof(unsigned long long), st);
+    if (sd.solver == DV_SOLVER_PGJ) launch_pgj_solve(sd, cfg, st, solve_only);
+    else launch_pgs_solve(sd, cfg, st, solve_only);
+    ++*launches;
   } else if (sd.precision == DV_PREC_MIXED) {
-    // with refinement the FP32 launch stops before the update, and an FP64
-    // launch refines the solves it marked, then updates
-    const bool refine = sd.refine_any != 0;
-    if (cfg.blocks_per_sm == 3) launch_typed<float, 3>(sd, cfg, st, solve_only || refine);
-    else launch_typed<float, 2>(sd, cfg, st, solve_only || refine);
-    if (refine) {
-      ++*launches;
+    // with refinement the FP32 launch leaves the update of the solves it marks
+    // to an FP64 launch, which refines them first
+    if (cfg.blocks_per_sm == 3) launch_typed<float, 3>(sd, cfg, st, launches, solve_only);
+    else launch_typed<float, 2>(sd, cfg, st, launches, solve_only);
+    if (sd.refine_any) {
       SolveConfig c2 = cfg;
       c2.blocks_per_sm = 2;
       c2.grid = std::min(cfg.grid, std::max(1, sd.refine_grid));
-      cudaMemsetAsync(sd.ew->bar, 0, sizeof(sd.ew->bar), st);
-      cudaMemsetAsync(&sd.ew->last_release, 0, sizeof(unsigned long long), st);
-      launch_typed<double, 2>(sd, c2, st, solve_only, true);
+      launch_typed<double, 2>(sd, c2, st, launches, solve_only, true);
     }
   } else if (sd.anti_relax) {
-    launch_typed<double, 2, true>(sd, cfg, st, solve_only);
+    launch_typed<double, 2, true>(sd, cfg, st, launches, solve_only);
   } else {
-    launch_typed<double, 2>(sd, cfg, st, solve_only);
+    launch_typed<double, 2>(sd, cfg, st, launches, solve_only);
   }
-  ++*launches;
 }
 
 }  // namespace dv

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "dv_div.h"
 #include "dvide.h"
 
 namespace dv {
@@ -68,25 +69,49 @@ __device__ inline void frame_from_normal(d3 n, d3* u, d3* v, bool exact = false)
   *v = normalize3x(cross3(n, uu), exact);
 }
 
+// 1 / |a| as normalize3x forms it.
+__device__ inline double inv_length3x(d3 a, bool exact) {
+  if (exact) return 1.0 / sqrt(dot3(a, a));
+  return (double)__fdiv_rn(1.0f, __fsqrt_rn((float)dot3(a, a)));
+}
+
+// A scene's friction cone: mu and what the projection forms from it alone, once
+// per scene instead of once per contact.
+template <class R>
+struct Cone {
+  R mu, ninv;   // -(1 / mu)
+  R den, rden;  // mu^2 + 1 and its reciprocal for div_by
+};
+
+template <class R>
+__device__ inline Cone<R> make_cone(R mu) {
+  Cone<R> c;
+  c.mu = mu;
+  c.ninv = -(R(1) / mu);
+  c.den = mu * mu + R(1);
+  c.rden = div_reciprocal(c.den);
+  return c;
+}
+
 // APGD.cu:47-78: projection of one contact impulse onto the friction cone.
 // pow(x, 2.0) is evaluated as x * x.
 template <class R>
-__device__ inline void project_cone(R& g0, R& g1, R& g2, R mu) {
+__device__ inline void project_cone(R& g0, R& g1, R& g2, const Cone<R>& k) {
   R gn = g0;
   R gt = sqrt(g1 * g1 + g2 * g2);
-  if (mu == R(0)) {
+  if (k.mu == R(0)) {
     g1 = R(0);
     g2 = R(0);
     if (gn < R(0)) g0 = R(0);
-  } else if (gt < mu * gn) {
+  } else if (gt < k.mu * gn) {
     // inside the cone
-  } else if ((gt < -(R(1) / mu) * gn) || (fabs(gn) < R(10e-15))) {
+  } else if ((gt < k.ninv * gn) || (fabs(gn) < R(10e-15))) {
     g0 = R(0);
     g1 = R(0);
     g2 = R(0);
   } else {
-    R gnp = (gt * mu + gn) / (mu * mu + R(1));
-    R gtp = gnp * mu;
+    R gnp = div_by(gt * k.mu + gn, k.den, k.rden);
+    R gtp = gnp * k.mu;
     R ratio = gtp / gt;
     g0 = gnp;
     g1 = ratio * g1;

@@ -99,12 +99,9 @@ int Engine::alloc_contacts(size_t cap) {
   // 32-contact plane segments with bulk asynchronous copies
   cap = (cap + kContactAlign - 1) / kContactAlign * kContactAlign;
   dfree(q.ida); dfree(q.idb); dfree(q.F); dfree(q.nf); dfree(q.gap); dfree(q.loc);
-  dfree(q.r);
-  for (int k = 0; k < 5; ++k) {
-    dfree(q.G[k]);
-    dfree(q.NG[k]);
-  }
-  dfree(q.q); dfree(q.inc); dfree(q.part); dfree(q.tseg); dfree(q.act_tiles);
+  dfree(q.r); dfree(q.blk);
+  for (int k = 0; k < 5; ++k) dfree(q.G[k]);
+  dfree(q.q); dfree(q.inc); dfree(q.part); dfree(q.tseg);
   dfree(q.ar_r0); dfree(q.ar_v);
   q.ccap = cap;
   q.tcap = (int)(cap / kTileItems) + q.nseg + 1 + (q.nbil + kTileItems - 1) / kTileItems;
@@ -115,19 +112,17 @@ int Engine::alloc_contacts(size_t cap) {
   TRY(dalloc(&q.gap, cap));
   TRY(dalloc(&q.loc, 3 * cap));
   TRY(dalloc(&q.r, 3 * cap));
-  for (int k = 0; k < 5; ++k) {
-    TRY(dalloc(&q.G[k], 3 * cap));
-    TRY(dalloc(&q.NG[k], 3 * cap));
-  }
+  TRY(dalloc(&q.blk, 10 * cap));
+  for (int k = 0; k < 5; ++k) TRY(dalloc(&q.G[k], 6 * cap));
   TRY(dalloc(&q.q, cap));
   TRY(dalloc(&q.inc, 2 * cap));
   if (q.anti_relax) {
     TRY(dalloc(&q.ar_r0, 2 * cap));
     TRY(dalloc(&q.ar_v, 2 * cap));
   }
-  TRY(dalloc(&q.part, (size_t)8 * q.tcap));
+  TRY(dalloc(&q.part, (size_t)16 * q.tcap));
   TRY(dalloc(&q.tseg, (size_t)q.tcap));
-  TRY(dalloc(&q.act_tiles, (size_t)q.tcap));
+  TRY(ensure_slots());
   size_t rc = std::max((size_t)q.nb, cap);
   if (rc > q.radix_cap) {
     dfree(q.keyA); dfree(q.valA); dfree(q.keyB); dfree(q.valB); dfree(q.radix_hist);
@@ -140,6 +135,26 @@ int Engine::alloc_contacts(size_t cap) {
     TRY(dalloc(&q.radix_hist, q.radix_hist_cap));
   }
   return DV_OK;
+}
+
+// The teams of a launch have a slot per member: at most one per tile, one per
+// 256 bodies and one more per segment.
+int Engine::ensure_slots() {
+  const size_t need = (size_t)d.tcap + (size_t)d.nb / kThreads + 2 * (size_t)d.nseg + 2;
+  if (need <= (size_t)d.slot_cap) return DV_OK;
+  dfree(d.slots);
+  d.slot_cap = 0;
+  TRY(dalloc(&d.slots, need));
+  d.slot_cap = (int)need;
+  drop_graph();
+  return DV_OK;
+}
+
+// One CTA per contact tile of a settled scene and some to spare, up to the
+// co-resident maximum: a settled body has 3.7 contacts, so its tiles are nearly
+// twice its 256-body ranges; CTAs without a tile leave at once.
+int Engine::default_grid(int max_ctas) const {
+  return std::max(1, std::min(max_ctas, d.nb / 64 + 1));
 }
 
 int Engine::upload_segments() {
@@ -235,7 +250,7 @@ int Engine::init(const std::vector<SceneInput>& scenes, int precision) {
   if (scenes.size() == 1 && scenes[0].P.anti_relaxation) TRY(enable_anti_relax());
   max_ctas_ = apgd_max_ctas(precision, 2);
   DV_CUDA_TRY(cudaGetLastError());
-  cfg_.grid = std::max(1, std::min(max_ctas_, (d.nb + kThreads - 1) / kThreads));
+  cfg_.grid = default_grid(max_ctas_);
   cfg_.chunk = 1;
   cfg_.contiguous = 0;
   cfg_.blocks_per_sm = 2;
@@ -501,24 +516,20 @@ int Engine::reconfigure(const std::vector<SlotSpec>& slots) {
     TRY(dalloc(&d.bseg, cap));
     nb_cap_ = cap;
   }
-  // body ranges of the solve's work lists: at most one partial range per segment
-  const size_t need_ab = (size_t)nb2 / kThreads + (size_t)nseg2 + 1;
-  if (need_ab > d.act_bcap) {
-    dfree(d.act_bodies);
-    TRY(dalloc(&d.act_bodies, need_ab));
-    d.act_bcap = need_ab;
-  }
   DV_CUDA_TRY(cudaMemsetAsync(d.k4, 0, sizeof(double4) * nbz, st));
   DV_CUDA_TRY(cudaMemsetAsync(d.w4, 0, sizeof(double4) * nbz, st));
   DV_CUDA_TRY(cudaMemsetAsync(d.fc4, 0, sizeof(double4) * nbz, st));
   if (nseg2 > seg_cap_) {
     int cap = std::max(nseg2, seg_cap_ + seg_cap_ / 4);
     dfree(d.seg); dfree(d.sst); dfree(d.grid); dfree(d.seg_tstart); dfree(d.donemask);
+    dfree(d.order); dfree(d.team_bar);
     TRY(dalloc(&d.seg, cap));
     TRY(dalloc(&d.sst, cap));
     TRY(dalloc(&d.grid, cap));
     TRY(dalloc(&d.seg_tstart, (size_t)cap + 1));
     TRY(dalloc(&d.donemask, (size_t)(cap + 31) / 32));
+    TRY(dalloc(&d.order, cap));
+    TRY(dalloc(&d.team_bar, (size_t)cap * kTeamBarStride));
     if (h_sst_) cudaFreeHost(h_sst_);
     h_sst_ = nullptr;
     if (cudaMallocHost(&h_sst_, sizeof(SegState) * cap) != cudaSuccess)
@@ -569,6 +580,7 @@ int Engine::reconfigure(const std::vector<SlotSpec>& slots) {
   d.ncell_cap = ncell2;
   if (ccap2 > d.ccap || (int)(d.ccap / kTileItems) + nseg2 + 1 > d.tcap || !d.ida)
     TRY(alloc_contacts(std::max(ccap2, d.ccap)));
+  TRY(ensure_slots());
   hseg_ = hs2;
   P_ = P2;
   time_ = t2;
@@ -592,7 +604,7 @@ int Engine::reconfigure(const std::vector<SlotSpec>& slots) {
   DV_CUDA_TRY(cudaStreamSynchronize(st));
   DV_CUDA_TRY(cudaGetLastError());
   if (!cfg_user_ && max_ctas_ > 0)
-    cfg_.grid = std::max(1, std::min(max_ctas_, (d.nb + kThreads - 1) / kThreads));
+    cfg_.grid = default_grid(max_ctas_);
   return DV_OK;
 }
 
@@ -606,7 +618,7 @@ void Engine::set_launch(int grid, int chunk, int contiguous, int blocks_per_sm) 
   const int mx = max_ctas_for(bps);
   if (grid <= 0) {
     cfg_user_ = false;
-    cfg_.grid = std::max(1, std::min(mx, (d.nb + kThreads - 1) / kThreads));
+    cfg_.grid = default_grid(mx);
   } else {
     cfg_user_ = true;
     cfg_.grid = std::min(grid, mx);

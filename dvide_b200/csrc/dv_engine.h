@@ -74,7 +74,7 @@ class Engine {
   int sync_state();  // waits and refreshes words()/seg_state()
 
   // Launch shape of the persistent solve kernel (blocks_per_sm 3 only with
-  // FP32 iterates; grid <= 0: one CTA per 256 bodies up to the co-resident maximum).
+  // FP32 iterates; grid <= 0: default_grid).
   void set_launch(int grid, int chunk, int contiguous, int blocks_per_sm = 2);
   int max_ctas_for(int blocks_per_sm) const;
   SolveConfig launch() const { return cfg_; }
@@ -150,6 +150,8 @@ class Engine {
   template <class T>
   void dfree(T*& p);
   int alloc_contacts(size_t cap);
+  int ensure_slots();
+  int default_grid(int max_ctas) const;
   template <class T>
   int ensure(T** p, int* cap, size_t need);
   int grow_warm(double factor, int min_seg_cap, int which);

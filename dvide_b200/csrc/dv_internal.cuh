@@ -117,7 +117,7 @@ struct SegState {
   int gsize;            // warm-start length (System::gamma_d / 3); kept when nc = 0
   unsigned arrive;      // tile arrivals in the current pass
   unsigned err;         // error bits of this segment's last step
-  int pad_;
+  int members;          // CTAs of its team in this launch (engines of several segments)
   ApgdCtl ctl;
 };
 
@@ -130,7 +130,6 @@ struct EngineWords {
   int n_small;          // gridded bodies (constant)
   int stop_on_seg_err;  // 1: a segment's solver error also sets err (plain System semantics)
   unsigned err;         // error bits (kErr*); sticky: every kernel of a step skips its work while set
-  int steps_done;       // steps completed since creation
   int active;           // segments still iterating (solve kernel)
   int step_count;       // segments that request a step pass next iteration
   int step_needed;      // latched step_count for the current iteration
@@ -139,16 +138,12 @@ struct EngineWords {
   unsigned long long phase_ns[8];
   unsigned long long phase_count[8];
   unsigned long long wait_limit_ns;  // every bounded wait (grid barrier, bulk copy) ends after this
-  // Work lists of the iterating passes (solve kernel): once half the segments
-  // that were iterating at the last rebuild have finished, the contact tiles
-  // and body ranges of the segments still iterating are gathered into
-  // SceneDev::act_tiles / act_bodies, and the passes walk those instead of
-  // every tile and body.
-  int act_on;           // 1: the lists are in use
-  int act_nt;           // entries of act_tiles
-  int act_nb;           // entries of act_bodies
-  int act_base;         // segments iterating when the lists were last built (nseg before)
-  int act_rebuild;      // 1: rebuild the lists before the next pass
+  // Teams of the solve kernel (engines of several segments): slots of the plan,
+  // the next one to take, and the passes that all teams have finished (a CTA
+  // that waits for its team to form sees from it that the others go on).
+  int nslots;
+  unsigned ticket;
+  unsigned progress;
   int n_wide;           // spheres of this step with more partners than the warp pair kernel lists
 };
 
@@ -158,6 +153,11 @@ struct EngineWords {
 constexpr int kWideSpheres = 65536;
 constexpr int kWideGrid = 256;
 constexpr int kWidePartners = 8192;
+
+// Tiles that a team's member takes at most when there are more than the grid
+// has CTAs, and the distance of the teams' arrival counters (a line each).
+constexpr int kTeamTiles = 4;
+constexpr int kTeamBarStride = 32;
 
 struct SceneDev {
   int nb = 0, nseg = 0;
@@ -209,18 +209,21 @@ struct SceneDev {
   double* gap = nullptr;
   double* loc = nullptr;      // 3 planes
   double* r = nullptr;        // 3 planes (float planes in the mixed solve)
+  double* blk = nullptr;      // 10 per contact: APGD's constants in blocks of 32 contacts (normal,
+                              // frame words, r, ids); PGJ and PGS: frame words, 3 planes
   int* binc_start = nullptr;  // nb + 1
   uint32_t* binc = nullptr;   // contact ids sorted by B
   int* inc_start = nullptr;   // nb + 1
   uint32_t* inc = nullptr;    // 2 * ccap
-  // APGD work: iterates and their Schur products, 3 planes each (stride ccap)
+  // APGD work: five iterates with their Schur products, in blocks of 32
+  // contacts (3 planes of 32 of the iterate, then 3 of the product)
   double* G[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-  double* NG[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   double4* q = nullptr;
-  int* act_tiles = nullptr;   // tcap: contact tiles of the segments still iterating
-  int4* act_bodies = nullptr; // act_bcap: (first body, end body, segment, 0), at most 256 bodies each
-  size_t act_bcap = 0;
-  double* part = nullptr;     // reduction partials, 9 x tcap
+  int2* slots = nullptr;      // plan of the teams: (segment, rank) per slot
+  int slot_cap = 0;
+  int* order = nullptr;       // nseg: the plan's segments by size
+  unsigned* team_bar = nullptr;  // nseg x kTeamBarStride: arrivals of each segment's team
+  double* part = nullptr;     // reduction partials, 2 x 8 x tcap
   // bilateral DOF rows (FP64 APGD only)
   int nbil = 0;               // rows of all segments
   int2* bil_off = nullptr;    // per row: element offsets 4 body + axis of DOF A, B (-1: none)

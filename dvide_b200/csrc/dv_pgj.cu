@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
         sum = sum + fd.v2 * fd.v2;
         const double mia = __ldg(a.minv + ia), mib = __ldg(a.minv + ib);
         Bc[c] = (T)(3.0 / ((mia + mib) * sum));
-        Frame<T> f = load_frame<T>(a, c, P.exact != 0);
+        Frame<T> f = start_frame<T>(a, c, P.exact != 0);
         qv[c] = f_times<T, V>(f, T(1), T(0), T(0));
       }
     }
@@ -201,9 +201,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
       int nslot = 0;
       auto ctl = [&](int s) { pgj_ctl(ca, s, scratch); };
       int cs = -1, cur = 0, kk = 0;
-      T mu = T(0);
+      Cone<T> cone{};
       double mud = 0.0;
-      bool ex = false;
       for (int i = 0;; ++i) {
         const int t = cta_tile(a, NT, i);
         if (t < 0) break;
@@ -215,8 +214,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
           cur = __ldcg(&a.sst[s].ctl.cur);
           kk = __ldcg(&a.sst[s].ctl.k);
           mud = a.seg[s].mu;
-          mu = (T)mud;
-          ex = a.seg[s].exact != 0;
+          cone = make_cone<T>((T)mud);
         }
         if (s != run.s) {
           if (run.n) {
@@ -234,7 +232,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
           int k = k0 + m * kThreads + threadIdx.x;
           if (k < nc) {
             const int c = c0 + k;
-            Frame<T> f = load_frame<T>(a, c, ex);
+            Frame<T> f = load_frame<T>(a, c);
             V wa = wv[__ldg(a.ida + c)], wb = wv[__ldg(a.idb + c)];
             T N0, N1, N2;
             ft_times<T, V>(f, wa, wb, &N0, &N1, &N2);
@@ -251,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
             const T b = Bc[c];
             const T om = (T)(-kPgjOmega);
             T h0 = x0 + om * (b * g0), h1 = x1 + om * (b * g1), h2 = x2 + om * (b * g2);
-            project_cone<T>(h0, h1, h2, mu);
+            project_cone<T>(h0, h1, h2, cone);
             const T la = (T)kPgjLambda, lb = (T)(1.0 - kPgjLambda);
             const T y0 = la * h0 + lb * x0, y1 = la * h1 + lb * x1, y2 = la * h2 + lb * x2;
             Gn[0 * S + c] = y0; Gn[1 * S + c] = y1; Gn[2 * S + c] = y2;
@@ -303,10 +301,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
       }
     }
   }
-  if (!grid_sync(a, kPhaseFinal, [&]() {
-        if (threadIdx.x == 0 && !a.solve_only) atomicAdd(&a.ew->steps_done, 1);
-      }))
-    return;
+  if (!grid_sync(a, kPhaseFinal, NoCtl{})) return;
 
   // ---- f_c = D^T gamma; v = Minv (k + f_c); f_contact = f_c / h; p += h v
   for (int bt = blockIdx.x; bt < nbt && !a.solve_only; bt += gridDim.x) {

@@ -76,7 +76,8 @@ __device__ int pgs_sweep_chunk(const KArgs<double>& a, int s, int from) {
   const size_t S = a.S;
   const int nc = X.nc, c0 = X.c0;
   const int to = min(nc, from + kPgsChunk);
-  const double mu = P.mu, h = P.h;
+  const Cone<double> cone = make_cone<double>(P.mu);
+  const double h = P.h;
   double* G = a.G[0];
   const double* Bc = a.G[4];
   double4* v = a.v4;
@@ -97,7 +98,7 @@ __device__ int pgs_sweep_chunk(const KArgs<double>& a, int s, int from) {
                            f.u2 * vb.z);
     double g2 = o2 - ob * (f.v0 * va.x + f.v1 * va.y + f.v2 * va.z - f.v0 * vb.x - f.v1 * vb.y -
                            f.v2 * vb.z);
-    project_cone<double>(g0, g1, g2, mu);
+    project_cone<double>(g0, g1, g2, cone);
     const double la = kPgsLambda, lb = 1.0 - kPgsLambda;
     const double y0 = la * g0 + lb * o0, y1 = la * g1 + lb * o1, y2 = la * g2 + lb * o2;
     G[0 * S + c] = y0;
@@ -229,6 +230,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
         sum = sum + fd.v2 * fd.v2;
         const double mia = __ldg(a.minv + ia), mib = __ldg(a.minv + ib);
         Bc[c] = 3.0 / ((mia + mib) * sum);
+        start_frame<double>(a, c, P.exact != 0);
         qv[c] = f_times<double, double4>(fd, 1.0, 0.0, 0.0);
       }
     }
@@ -288,7 +290,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
       auto ctl = [&](int s) { pgs_ctl(ca, s, scratch); };
       int cs = -1;
       double mu = 0.0;
-      bool ex = false;
       for (int i = 0;; ++i) {
         const int t = cta_tile(a, NT, i);
         if (t < 0) break;
@@ -298,7 +299,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
         if (s != cs) {
           cs = s;
           mu = a.seg[s].mu;
-          ex = a.seg[s].exact != 0;
         }
         if (s != run.s) {
           if (run.n) {
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
           int k = k0 + m * kThreads + threadIdx.x;
           if (k < nc) {
             const int c = c0 + k;
-            Frame<double> f = load_frame<double>(a, c, ex);
+            Frame<double> f = load_frame<double>(a, c);
             V wa = wv[__ldg(a.ida + c)], wb = wv[__ldg(a.idb + c)];
             double N0, N1, N2;
             ft_times<double, V>(f, wa, wb, &N0, &N1, &N2);
@@ -362,10 +362,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
       }
     }
   }
-  if (!grid_sync(a, kPhaseFinal, [&]() {
-        if (threadIdx.x == 0 && !a.solve_only) atomicAdd(&a.ew->steps_done, 1);
-      }))
-    return;
+  if (!grid_sync(a, kPhaseFinal, NoCtl{})) return;
 
   // ---- f_c = D^T gamma; v = Minv (k + f_c); f_contact = f_c / h; p += h v
   for (int bt = blockIdx.x; bt < nbt && !a.solve_only; bt += gridDim.x) {

@@ -58,10 +58,11 @@ struct KArgs {
   const float* __restrict__ nf;
   const double* __restrict__ gap;
   T* r;
+  T* fr;              // PGJ, PGS: frame words (FrameWords), 3 planes, written by the setup pass
+  T* blk;             // APGD: the contacts' constants in blocks of 32 (the same memory)
   const int* __restrict__ inc_start;
   const uint32_t* __restrict__ inc;
-  T* G[5];
-  T* NG[5];
+  T* G[5];            // APGD: iterate blocks (3 planes of 32, then the product's 3); PGJ, PGS: planes
   double4* qd;        // contact vector q, double4 (final pass); Vec4<T> in iterations
   double* gamma;
   uint32_t* wid;      // matched warm start: B of the pair per warm slot (segment-relative)
@@ -75,8 +76,8 @@ struct KArgs {
   const int* __restrict__ tseg;
   unsigned* donemask;
   EngineWords* ew;
-  int* act_tiles;          // work lists of the iterating passes (EngineWords::act_on)
-  int4* act_bodies;
+  const int2* slots;       // the plan of the teams: (scene, rank) per slot
+  unsigned* team_bar;      // arrivals of each scene's team, kTeamBarStride words apart
   // bilateral DOF rows (nbil = 0: none; FP64 iterates only)
   int nbil;
   const int2* __restrict__ bil_off;
@@ -102,25 +103,6 @@ struct Frame {
   T n0, n1, n2, u0, u1, u2, v0, v1, v2;
 };
 
-// System.cu:753-762 in float arithmetic (mixed path).
-__device__ inline void frame_from_normal_f(float n0, float n1, float n2, Frame<float>& f) {
-  float ux, uy, uz;
-  if (n2 != 0.0f) {
-    ux = 1.0f; uy = 0.0f; uz = __fdiv_rn(-n0, n2);
-  } else if (n0 != 0.0f) {
-    ux = __fdiv_rn(-n2, n0); uy = 0.0f; uz = 1.0f;
-  } else {
-    ux = 1.0f; uy = __fdiv_rn(-n0, n1); uz = 0.0f;
-  }
-  float iu = __fdiv_rn(1.0f, __fsqrt_rn(ux * ux + uy * uy + uz * uz));
-  ux *= iu; uy *= iu; uz *= iu;
-  float vx = n1 * uz - n2 * uy, vy = n2 * ux - n0 * uz, vz = n0 * uy - n1 * ux;
-  float iv = __fdiv_rn(1.0f, __fsqrt_rn(vx * vx + vy * vy + vz * vz));
-  f.n0 = n0; f.n1 = n1; f.n2 = n2;
-  f.u0 = ux; f.u1 = uy; f.u2 = uz;
-  f.v0 = vx * iv; f.v1 = vy * iv; f.v2 = vz * iv;
-}
-
 // The FP64 frame, recomputed from the stored normal with the narrowphase's own
 // function and the scene's mode (same bits as the stored u, v planes).
 __device__ inline Frame<double> frame_d(double n0, double n1, double n2, bool exact) {
@@ -133,15 +115,63 @@ __device__ inline Frame<double> frame_d(double n0, double n1, double n2, bool ex
   return f;
 }
 
-// `exact`: the scene's FP64 narrowphase mode (the FP32 frame ignores it).
-template <class T> __device__ inline Frame<T> make_frame(T n0, T n1, T n2, bool exact);
-template <>
-__device__ inline Frame<double> make_frame<double>(double n0, double n1, double n2, bool exact) {
-  return frame_d(n0, n1, n2, exact);
+// What a frame cannot cheaply be rebuilt without, per contact: u has one zero
+// component by construction (System.cu:753-762), so its other two and the
+// reciprocal length of n x u give the frame back with twelve multiplications,
+// in the same order as frame_from_normal (the same bits), where rebuilding it
+// from the normal alone takes a division, two square roots and two reciprocals
+// in one dependent chain.
+template <class T>
+struct FrameWords {
+  T a, b;  // u_x, and u_z (or u_y when n is along y)
+  T iv;    // 1 / |n x u|
+};
+
+__device__ inline FrameWords<double> frame_words(double n0, double n1, double n2, bool exact) {
+  const bool along = n2 == 0 && n0 == 0;
+  d3 r;
+  if (n2 != 0) r = mk3(1, 0, -n0 / n2);
+  else if (n0 != 0) r = mk3(-n2 / n0, 0, 1);
+  else r = mk3(1, -n0 / n1, 0);
+  const d3 u = scale3(r, inv_length3x(r, exact));
+  FrameWords<double> w;
+  w.a = u.x;
+  w.b = along ? u.y : u.z;
+  w.iv = inv_length3x(cross3(mk3(n0, n1, n2), u), exact);
+  return w;
 }
-template <> __device__ inline Frame<float> make_frame<float>(float n0, float n1, float n2, bool) {
-  Frame<float> f;
-  frame_from_normal_f(n0, n1, n2, f);
+// System.cu:753-762 in float arithmetic (mixed path; it has no exact mode).
+__device__ inline FrameWords<float> frame_words(float n0, float n1, float n2, bool) {
+  const bool along = n2 == 0.0f && n0 == 0.0f;
+  float ux, uy, uz;
+  if (n2 != 0.0f) {
+    ux = 1.0f; uy = 0.0f; uz = __fdiv_rn(-n0, n2);
+  } else if (n0 != 0.0f) {
+    ux = __fdiv_rn(-n2, n0); uy = 0.0f; uz = 1.0f;
+  } else {
+    ux = 1.0f; uy = __fdiv_rn(-n0, n1); uz = 0.0f;
+  }
+  const float iu = __fdiv_rn(1.0f, __fsqrt_rn(ux * ux + uy * uy + uz * uz));
+  ux *= iu; uy *= iu; uz *= iu;
+  const float vx = n1 * uz - n2 * uy, vy = n2 * ux - n0 * uz, vz = n0 * uy - n1 * ux;
+  FrameWords<float> w;
+  w.a = ux;
+  w.b = along ? uy : uz;
+  w.iv = __fdiv_rn(1.0f, __fsqrt_rn(vx * vx + vy * vy + vz * vz));
+  return w;
+}
+
+template <class T>
+__device__ inline Frame<T> make_frame(T n0, T n1, T n2, const FrameWords<T>& w) {
+  const bool along = n2 == T(0) && n0 == T(0);
+  Frame<T> f;
+  f.n0 = n0; f.n1 = n1; f.n2 = n2;
+  f.u0 = w.a;
+  f.u1 = along ? w.b : T(0);
+  f.u2 = along ? T(0) : w.b;
+  f.v0 = (n1 * f.u2 - n2 * f.u1) * w.iv;
+  f.v1 = (n2 * f.u0 - n0 * f.u2) * w.iv;
+  f.v2 = (n0 * f.u1 - n1 * f.u0) * w.iv;
   return f;
 }
 
@@ -154,10 +184,25 @@ template <> __device__ inline const float* normal_planes<float>(const KArgs<floa
   return a.nf;
 }
 
+// The frame of contact c from the normal and the words that a solve's setup
+// pass left in the fr planes.
 template <class T>
-__device__ inline Frame<T> load_frame(const KArgs<T>& a, int c, bool exact) {
+__device__ inline Frame<T> load_frame(const KArgs<T>& a, int c) {
   const T* n = normal_planes<T>(a);
-  return make_frame<T>(n[c], n[a.S + c], n[2 * a.S + c], exact);
+  const FrameWords<T> w{a.fr[c], a.fr[a.S + c], a.fr[2 * a.S + c]};
+  return make_frame<T>(n[c], n[a.S + c], n[2 * a.S + c], w);
+}
+
+// Setup: forms the words of contact c, keeps them and returns the frame.
+template <class T>
+__device__ inline Frame<T> start_frame(const KArgs<T>& a, int c, bool exact) {
+  const T* n = normal_planes<T>(a);
+  const T n0 = n[c], n1 = n[a.S + c], n2 = n[2 * a.S + c];
+  const FrameWords<T> w = frame_words(n0, n1, n2, exact);
+  a.fr[c] = w.a;
+  a.fr[a.S + c] = w.b;
+  a.fr[2 * a.S + c] = w.iv;
+  return make_frame<T>(n0, n1, n2, w);
 }
 
 template <class T>
@@ -190,11 +235,9 @@ __device__ inline uint64_t l2_evict_last_policy() {
 }
 __device__ inline void store_keep(double4* addr, const double4& v) {
   const uint64_t pol = l2_evict_last_policy();
-  asm volatile(
-      "st.global.L2::cache_hint.v2.f64 [%0], {%1, %2}, %5;\n\t"
-      "st.global.L2::cache_hint.v2.f64 [%0+16], {%3, %4}, %5;" ::"l"(addr),
-      "d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w), "l"(pol)
-      : "memory");
+  asm volatile("st.global.L2::cache_hint.v4.f64 [%0], {%1, %2, %3, %4}, %5;" ::"l"(addr),
+               "d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w), "l"(pol)
+               : "memory");
 }
 __device__ inline void store_keep(float4* addr, const float4& v) {
   const uint64_t pol = l2_evict_last_policy();
@@ -202,6 +245,16 @@ __device__ inline void store_keep(float4* addr, const float4& v) {
                "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "l"(pol)
                : "memory");
 }
+// One 4-vector by one load (32 bytes in FP64: a sector, where two 16-byte
+// loads would each ask for it).
+__device__ inline double4 load_vec(const double4* p) {
+  double4 v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+               : "l"(p));
+  return v;
+}
+__device__ inline float4 load_vec(const float4* p) { return *p; }
 
 // q = F x : q_k = (n_k x0 + u_k x1) + v_k x2
 template <class T, class V>
@@ -229,31 +282,7 @@ __device__ inline double dot3i(A a0, A a1, A a2, B b0, B b1, B b2) {
   return ((double)a0 * (double)b0 + (double)a1 * (double)b1) + (double)a2 * (double)b2;
 }
 
-// Folds NQ values of each thread; thread 0 gets the results.
-template <int NQ>
-__device__ inline void block_fold_multi(double (&v)[NQ], double* scratch) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int qi = 0; qi < NQ; ++qi) v[qi] = warp_fold(v[qi]);
-  __syncthreads();
-  if (lane == 0) {
-#pragma unroll
-    for (int qi = 0; qi < NQ; ++qi) scratch[qi * 8 + warp] = v[qi];
-  }
-  __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int qi = 0; qi < NQ; ++qi) {
-      double w = (lane < 8) ? scratch[qi * 8 + lane] : 0.0;
-#pragma unroll
-      for (int off = 4; off >= 1; off >>= 1) w = w + __shfl_down_sync(0xffffffffu, w, off);
-      v[qi] = w;
-    }
-  }
-  __syncthreads();
-}
-
-// Folds NS sums (the order of block_fold_multi) and NM maxima of each thread
+// Folds NS sums (warp_fold, then the 8-warp tree) and NM maxima of each thread
 // with one exchange through shared memory (NS + NM <= 8); thread 0 gets the
 // results.
 template <int NS, int NM>
@@ -339,68 +368,14 @@ __device__ inline void fold_tiles_sm(const K& a, int t0, int nt, double* sum_out
   for (int qi = 0; qi < NM; ++qi) max_out[qi] = mx[qi];
 }
 
-template <int NQ, class K>
-__device__ inline void fold_tiles(const K& a, int t0, int nt, double (&out)[NQ], double* scratch) {
-  fold_tiles_sm<NQ, 0>(a, t0, nt, out, nullptr, 0, scratch);
-}
-
-template <int NQ, class K>
-__device__ inline void write_partials(const K& a, int tile, const double (&v)[NQ]) {
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int qi = 0; qi < NQ; ++qi) a.part[(size_t)qi * a.tcap + tile] = v[qi];
-  }
-}
-
-// Deferred tile folds.  At the end of a tile each warp folds its partial sums
-// with shuffles (strides 16..1) and parks the eight warp results in shared
-// memory; fold_parked() later completes the 8-warp tree of every parked tile
-// ((w0+w4)+(w2+w6)) + ((w1+w5)+(w3+w7)) -- the order of block_fold_multi --
-// and writes the tile partials.  Warps thus run their copy pipelines across
-// tiles without a CTA barrier per tile.
-constexpr int kMaxDefer = 16;
+// Deferred tile folds: the warps park their maxima of a tile and go on to the
+// next; fold_parked_max() completes the parked tiles.
+constexpr int kMaxDefer = 8;
 struct DeferBuf {
   double w[kMaxDefer][kNQ + 1][kWarps];  // [slot][quantity][warp]
   int tile[kMaxDefer];
   int fail;                              // a warp's copy wait timed out
 };
-
-template <int NQ, bool kMax>
-__device__ inline void park_tile(DeferBuf& B, int slot, int tile, const double (&acc)[NQ], double mx) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NQ; ++q) {
-    const double v = warp_fold(acc[q]);
-    if (lane == 0) B.w[slot][q][warp] = v;
-  }
-  if (kMax) {
-    const double m = warp_max(mx);
-    if (lane == 0) B.w[slot][NQ][warp] = m;
-  }
-  if (threadIdx.x == 0) B.tile[slot] = tile;
-}
-
-// Completes the parked tiles (NQ sums into planes 0..NQ-1, the max into
-// plane kQMax); returns false if a warp's copy wait had timed out.
-template <int NQ, bool kMax, class K>
-__device__ inline bool fold_parked(const K& a, DeferBuf& B, int n) {
-  __syncthreads();
-  const int nq = NQ + (kMax ? 1 : 0);
-  for (int i = threadIdx.x; i < n * nq; i += kThreads) {
-    const int slot = i / nq, q = i - slot * nq;
-    const double* w = B.w[slot][q];
-    double r;
-    if (kMax && q == NQ)
-      r = fmax(fmax(fmax(w[0], w[4]), fmax(w[2], w[6])), fmax(fmax(w[1], w[5]), fmax(w[3], w[7])));
-    else
-      r = ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
-    const int plane = (kMax && q == NQ) ? kQMax : q;
-    a.part[(size_t)plane * a.tcap + B.tile[slot]] = r;
-  }
-  __threadfence();
-  __syncthreads();
-  return B.fail == 0;
-}
 
 // Tile arrivals of one segment: a CTA delivers the count of its consecutive
 // tiles of segment s at once (after their partials are written).  True, in
@@ -586,15 +561,6 @@ __device__ inline int cta_tile(const K& a, int nt, int i) {
   return t < nt ? (int)t : -1;
 }
 
-// Tile at sequence index i of this CTA in an iterating pass: position i of the
-// work list when it is in use (n = its length; the list is rewritten inside
-// the kernel, so it is read through L2), else tile i of all n tiles.
-template <class K>
-__device__ inline int pass_tile(const K& a, int lon, int n, int i) {
-  const int t = cta_tile(a, n, i);
-  return (t < 0 || !lon) ? t : __ldcg(a.act_tiles + t);
-}
-
 // Eight incidence entries c[0, n) of a body's run (n <= 8): their q gathered
 // together, then added to (ax, ay, az) in order, -q for a B side.
 template <class T, class V>
@@ -603,7 +569,7 @@ __device__ inline void add_q8(const V* q, const uint32_t* c, int n, T& ax, T& ay
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     if (j < n) {
-      qq[j] = q[c[j] & 0x7fffffffu];
+      qq[j] = load_vec(q + (c[j] & 0x7fffffffu));
     } else {
       qq[j].x = T(0); qq[j].y = T(0); qq[j].z = T(0); qq[j].w = T(0);
     }
@@ -773,24 +739,23 @@ struct BodyHead {
   int s, e, seg;
 };
 
-template <class K>
+template <bool kSeg = true, class K>
 __device__ inline BodyHead body_head(const K& a, int b) {
   BodyHead h;
   h.mi = __ldg(a.minv + b);
   h.s = __ldg(a.inc_start + b);
   h.e = __ldg(a.inc_start + b + 1);
-  h.seg = a.nseg > 1 ? __ldg(a.bseg + b) : 0;
+  h.seg = kSeg && a.nseg > 1 ? __ldg(a.bseg + b) : 0;
   return h;
 }
 
 // kPre: c0 holds the body's first eight incidence entries, loaded a round
 // ahead by the body pass (zero past its run).
 template <class T, bool kAR = false, bool kPre = false>
-__device__ inline void body_w(const KArgs<T>& a, int b, const BodyHead& h,
+__device__ inline void body_w(const KArgs<T>& a, typename Vec4<T>::type* w,
+                              const typename Vec4<T>::type* q, int b, const BodyHead& h,
                               const uint32_t* c0 = nullptr) {
   using V = typename Vec4<T>::type;
-  V* w = reinterpret_cast<V*>(a.wd);
-  const V* q = reinterpret_cast<const V*>(a.qd);
   const double mi = h.mi;
   if (mi != 0.0) {
     V s = kPre ? gather_q_pre<T, V>(a, q, h.s, h.e, c0) : gather_q<T, V>(a, q, h.s, h.e);
@@ -815,21 +780,13 @@ __device__ inline void body_w(const KArgs<T>& a, int b, const BodyHead& h,
 }
 
 // Schur body pass: w_b = minv_b * (D^T x)_b for bodies of iterating
-// segments; fixed bodies keep w = 0.  With the work lists in use (lon), over
-// the listed body ranges (one segment each) instead of every body.
-template <class T, bool kAR = false>
-__device__ inline void body_pass_schur(const KArgs<T>& a, const unsigned* s_mask, int lon = 0,
-                                       int nlist = 0) {
+// segments; fixed bodies keep w = 0.
+template <class T>
+__device__ inline void body_pass_schur(const KArgs<T>& a, const unsigned* s_mask) {
+  using V = typename Vec4<T>::type;
+  V* w = reinterpret_cast<V*>(a.wd);
+  const V* q = reinterpret_cast<const V*>(a.qd);
   const int mwords = (a.nseg + 31) >> 5;
-  if (lon) {
-    for (int p = blockIdx.x; p < nlist; p += gridDim.x) {
-      const int4 r = __ldcg(a.act_bodies + p);
-      if (mask_done(a, s_mask, mwords, r.z)) continue;
-      const int b = r.x + threadIdx.x;
-      if (b < r.y) body_w<T, kAR>(a, b, body_head(a, b));
-    }
-    return;
-  }
   // heads load into registers two rounds ahead, and each body's first eight
   // incidence entries one round ahead, while the current round gathers
   const int stride = gridDim.x * kThreads;
@@ -847,7 +804,7 @@ __device__ inline void body_pass_schur(const KArgs<T>& a, const unsigned* s_mask
     uint32_t cn[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) cn[j] = (hn.s + j < hn.e) ? __ldg(a.inc + hn.s + j) : 0u;
-    if (a.nseg == 1 || !mask_done(a, s_mask, mwords, h.seg)) body_w<T, kAR, true>(a, b, h, c);
+    if (a.nseg == 1 || !mask_done(a, s_mask, mwords, h.seg)) body_w<T, false, true>(a, w, q, b, h, c);
     h = hn;
     hn = hnn;
 #pragma unroll
@@ -855,64 +812,11 @@ __device__ inline void body_pass_schur(const KArgs<T>& a, const unsigned* s_mask
   }
 }
 
-// Work lists of the segments still iterating (CTA 0, all its threads): their
-// contact tiles in segment order into act_tiles and their bodies, in ranges of
-// at most kThreads within one segment, into act_bodies.  Reads the done mask
-// as the last product pass left it.
-template <class T>
-__device__ inline void rebuild_work_lists(const KArgs<T>& a, int* sbuf) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int base_t = 0, base_b = 0;
-  for (int s0 = 0; s0 < a.nseg; s0 += kThreads) {
-    const int s = s0 + tid;
-    int ct = 0, cb = 0, t0 = 0, b0 = 0, b1 = 0;
-    if (s < a.nseg && !((__ldcg(a.donemask + (s >> 5)) >> (s & 31)) & 1u)) {
-      ct = a.sst[s].nt;
-      t0 = a.sst[s].t0;
-      b0 = a.seg[s].b0;
-      b1 = a.seg[s].b1;
-      cb = (b1 - b0 + kThreads - 1) / kThreads;
-    }
-    // exclusive scans of ct and cb over the block (warp shuffles, then warp totals)
-    int it = ct, ib = cb;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int ut = __shfl_up_sync(0xffffffffu, it, off);
-      const int ub = __shfl_up_sync(0xffffffffu, ib, off);
-      if (lane >= off) {
-        it += ut;
-        ib += ub;
-      }
-    }
-    __syncthreads();
-    if (lane == 31) {
-      sbuf[warp] = it;
-      sbuf[kWarps + warp] = ib;
-    }
-    __syncthreads();
-    int wt = 0, wb = 0, tt = 0, tb = 0;
-    for (int k = 0; k < kWarps; ++k) {
-      if (k < warp) {
-        wt += sbuf[k];
-        wb += sbuf[kWarps + k];
-      }
-      tt += sbuf[k];
-      tb += sbuf[kWarps + k];
-    }
-    const int et = base_t + wt + it - ct, eb = base_b + wb + ib - cb;
-    for (int j = 0; j < ct; ++j) a.act_tiles[et + j] = t0 + j;
-    for (int j = 0; j < cb; ++j) {
-      const int lo = b0 + j * kThreads;
-      a.act_bodies[eb + j] = make_int4(lo, min(b1, lo + kThreads), s, 0);
-    }
-    base_t += tt;
-    base_b += tb;
-  }
-  __threadfence();
-  if (tid == 0) {
-    a.ew->act_nt = base_t;
-    a.ew->act_nb = base_b;
-  }
+// Members of a team: one per `per` contact tiles or 256 * per bodies, as many
+// as the grid has at most.
+__device__ inline int team_size(int nt, int nb, int per, int grid) {
+  const int m = max((nt + per - 1) / per, (nb + kThreads * per - 1) / (kThreads * per));
+  return max(1, min(m, grid));
 }
 
 // A buffer holding none of the iterates in use (5 buffers, at most 4 in use).
@@ -923,27 +827,15 @@ __device__ inline int free_slot(int a, int b, int c, int d) {
 }
 
 // ---------------------------------------------------------------------------
-// Shared-memory staging of the look-ahead pass, per warp.  A CTA walks its
+// Shared-memory staging of the contact pass, per warp.  A CTA walks its
 // sub-tiles (256 consecutive contacts, kItemsPerThread per reduction tile) in
 // order; warp w owns contacts [32w, 32w+32) of each sub-tile and two stages of
-// its own.  While the warp computes sub-tile i from one stage, its lane 0 has
-// already issued the bulk copies of sub-tile i+1's plane segments (32 values
-// per plane) into the other stage, completed on the warp's own mbarrier, so
-// warps never wait for each other except at the per-tile reduction.
-// Planes: n (3), gamma_new (3), r (3), gamma_k (3), N gamma_k (3); ids A, B.
+// its own.  While the warp works on one, its lane 0 has already issued the
+// bulk copies of the next sub-tile into the other, completed on the warp's own
+// mbarrier, so warps never wait for each other except at the reductions.
 // A segment's contacts start on a multiple of 256, so every copy starts on a
 // 128-byte boundary.
 // ---------------------------------------------------------------------------
-constexpr int kStagePlanes = 15;
-template <class T>
-__host__ __device__ constexpr unsigned warp_stage_bytes() {
-  return (unsigned)kStagePlanes * 32u * (unsigned)sizeof(T) + 2u * 32u * 4u;
-}
-template <class T>
-__host__ __device__ constexpr size_t dyn_smem_bytes() {
-  return (size_t)kWarps * 2 * warp_stage_bytes<T>() + (size_t)kWarps * 2 * 8 + 16;
-}
-
 struct Staging {
   unsigned char* base;  // warp w, stage s at base + (2w + s) * stage_bytes
   unsigned stage_bytes;
@@ -1035,12 +927,10 @@ KArgs<T> make_kargs(SceneDev& sd, const SolveConfig& cfg) {
   a.nf = sd.nf;
   a.gap = sd.gap;
   a.r = reinterpret_cast<T*>(sd.r);
+  a.fr = a.blk = reinterpret_cast<T*>(sd.blk);
   a.inc_start = sd.inc_start;
   a.inc = sd.inc;
-  for (int k = 0; k < 5; ++k) {
-    a.G[k] = reinterpret_cast<T*>(sd.G[k]);
-    a.NG[k] = reinterpret_cast<T*>(sd.NG[k]);
-  }
+  for (int k = 0; k < 5; ++k) a.G[k] = reinterpret_cast<T*>(sd.G[k]);
   a.qd = sd.q;
   a.gamma = sd.gamma;
   a.wid = sd.wid;
@@ -1054,8 +944,8 @@ KArgs<T> make_kargs(SceneDev& sd, const SolveConfig& cfg) {
   a.tseg = sd.tseg;
   a.donemask = sd.donemask;
   a.ew = sd.ew;
-  a.act_tiles = sd.act_tiles;
-  a.act_bodies = sd.act_bodies;
+  a.slots = sd.slots;
+  a.team_bar = sd.team_bar;
   a.nbil = sizeof(T) == sizeof(double) ? sd.nbil : 0;
   a.bil_off = sd.bil_off;
   a.bil_info = sd.bil_info;

@@ -1,0 +1,298 @@
+// dv_team.cuh -- teams: the CTAs of a persistent solve kernel that work on one
+// scene together, from its setup to its update, and leave it only when it is
+// solved.
+//
+// A scene's passes are separated by barriers.  With one barrier for the whole
+// grid every scene of a batch waits for every other in every pass, and all
+// scenes' vectors stream through L2 between two visits.  A team has a barrier
+// of its own and keeps to one scene, so scenes run at their own pace, a scene's
+// vectors stay in L2 while it iterates, and the CTAs that a finished scene
+// frees take the next one.
+//
+// The plan (k_team_plan) lists the scenes by size, largest first, and gives
+// each a run of slots, one per member.  A CTA takes the next slot by one atomic.
+// Slots are handed out in order, so only the team formed last can lack
+// members; it waits for CTAs of earlier teams, which have all theirs and
+// finish.  A team is at most the grid, and the grid is co-resident.
+#pragma once
+
+#include "dv_solve.cuh"
+
+namespace dv {
+
+namespace {
+
+// What a member knows of its team and its share of the scene (shared memory,
+// written by thread 0).
+struct Team {
+  int s;            // scene
+  int rank, m;      // this CTA's place among the team's m members
+  int c0, nc;       // contacts [c0, c0 + nc)
+  int t0, ntc, nt;  // first tile; contact tiles; with the bilateral rows' tiles
+  int w0, w1;       // this member's bodies
+  int gsize;
+  int chunk, contiguous;
+  int fail;
+  unsigned target;  // arrivals that open the next barrier
+  unsigned* bar;
+};
+
+// Tile i of this member's share of n tiles (-1 past the end): round robin in
+// chunks of `chunk` consecutive tiles, or one contiguous range per member.
+__device__ inline int team_tile(const Team& t, int n, int i) {
+  if (t.contiguous) {
+    const int lo = (int)((long long)n * t.rank / t.m);
+    const int hi = (int)((long long)n * (t.rank + 1) / t.m);
+    return lo + i < hi ? lo + i : -1;
+  }
+  const int k = t.chunk;
+  const int x = k == 1 ? t.rank + i * t.m : (t.rank + (i / k) * t.m) * k + i % k;
+  return x < n ? x : -1;
+}
+
+__device__ inline void red_add_release(unsigned* p, unsigned v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ inline void red_add(unsigned* p, unsigned v) {
+  asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Barrier of a team.  Arrivals are counted without a result (the counter only
+// rises: barrier k opens at k m), so a member waits for one trip to L2 and the
+// polls after it.  False after a time limit or another CTA's.  The first
+// barrier of a team (`joining`) may wait for members that are still busy with
+// earlier scenes: there the limit starts again while any team makes progress.
+template <class K>
+__device__ inline bool team_sync(const K& a, Team& t, bool joining = false) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (a.nseg > 1 && t.rank == 0) red_add(&a.ew->progress, 1u);
+    if (t.m > 1) {
+      t.target += (unsigned)t.m;
+      const unsigned target = t.target;
+      red_add_release(t.bar, 1u);
+      unsigned polls = 0, seen = 0;
+      uint64_t t0 = 0;
+      while ((int)(ld_acquire(t.bar) - target) < 0) {
+        if (joining) __nanosleep(200);
+        if ((++polls & 1023u) == 0u) {
+          if (ld_acquire(&a.ew->err) & (kErrBarrierTimeout | kErrCopyTimeout)) {
+            t.fail = 1;
+            break;
+          }
+          const uint64_t now = global_ns();
+          if (t0 == 0) t0 = now;
+          if (joining) {
+            const unsigned p = ld_acquire(&a.ew->progress);
+            if (p != seen) t0 = now;
+            seen = p;
+          }
+          if (now - t0 > a.ew->wait_limit_ns) {
+            atomicOr(&a.ew->err, kErrBarrierTimeout);
+            t.fail = 1;
+            break;
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  return t.fail == 0;
+}
+
+// Takes the next slot of the plan; false when there is none left.  One scene
+// needs no plan: its team is the first m CTAs.
+template <class K>
+__device__ inline bool join_team(const K& a, Team& t, int* slot_seen) {
+  __syncthreads();  // the last scene's reads of the team are done
+  if (threadIdx.x == 0) {
+    int s = -1, rank = 0, m = 0;
+    if (a.nseg == 1) {
+      m = *slot_seen ? 0 : team_size(a.sst[0].nt, a.nb, 1, gridDim.x);
+      rank = blockIdx.x;
+      if (rank < m && (a.seg[0].active != 0) && (!a.refine || a.sst[0].ctl.refined)) s = 0;
+    } else {
+      const unsigned slot = atomicAdd(&a.ew->ticket, 1u);
+      if (slot < (unsigned)__ldcg(&a.ew->nslots)) {
+        const int2 e = __ldcg(a.slots + slot);
+        s = e.x;
+        rank = e.y;
+        m = __ldcg(&a.sst[s].members);
+      }
+    }
+    *slot_seen = 1;
+    t.s = s;
+    if (s >= 0) {
+      const SegState& X = a.sst[s];
+      const SegParams& P = a.seg[s];
+      t.rank = rank;
+      t.m = m;
+      t.c0 = X.c0;
+      t.nc = X.nc;
+      t.t0 = X.t0;
+      t.nt = X.nt;
+      t.ntc = (X.nc + kTileItems - 1) / kTileItems;
+      const int n = P.b1 - P.b0;
+      const int per = ((n + m - 1) / m + 31) & ~31;
+      t.w0 = P.b0 + min(n, rank * per);
+      t.w1 = P.b0 + min(n, (rank + 1) * per);
+      t.gsize = X.gsize;
+      t.chunk = a.chunk;
+      t.contiguous = a.contiguous;
+      t.fail = 0;
+      t.target = 0;
+      t.bar = a.team_bar + (size_t)s * kTeamBarStride;
+    }
+  }
+  __syncthreads();
+  return t.s >= 0;
+}
+
+// Folds the eight quantities of a warp's lanes together, each in the order of
+// warp_fold (strides 16, 8, 4, 2, 1; addition commutes, so which of two lanes
+// adds does not matter).  At each of the first three strides a lane hands half
+// of its quantities to its partner and keeps the other half: 9 exchanges for
+// the eight instead of 40.  Lane l returns quantity l / 4; with kMax the last
+// one is a maximum.
+template <bool kMax>
+__device__ inline double warp_fold8(const double (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+  const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
+  const bool last = kMax && u16 && u8 && u4;
+  double r[4], s[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double keep = u16 ? v[i + 4] : v[i];
+    const double x = __shfl_xor_sync(0xffffffffu, u16 ? v[i] : v[i + 4], 16);
+    r[i] = (kMax && i == 3 && u16) ? fmax(keep, x) : keep + x;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const double keep = u8 ? r[i + 2] : r[i];
+    const double x = __shfl_xor_sync(0xffffffffu, u8 ? r[i] : r[i + 2], 8);
+    s[i] = (kMax && i == 1 && u16 && u8) ? fmax(keep, x) : keep + x;
+  }
+  const double keep = u4 ? s[1] : s[0];
+  double x = __shfl_xor_sync(0xffffffffu, u4 ? s[0] : s[1], 4);
+  double t = last ? fmax(keep, x) : keep + x;
+  x = __shfl_xor_sync(0xffffffffu, t, 2);
+  t = last ? fmax(t, x) : t + x;
+  x = __shfl_xor_sync(0xffffffffu, t, 1);
+  return last ? fmax(t, x) : t + x;
+}
+
+// The warps' folds of the tiles a member has finished, until fold_tiles_out
+// completes them: warps go on to the next tile without a CTA barrier.
+constexpr int kParkSlots = 8;
+struct ParkBuf {
+  double w[kParkSlots][8][kWarps];  // [slot][quantity][warp]
+  int tile[kParkSlots];
+};
+
+template <bool kMax>
+__device__ inline void park8(ParkBuf& B, int slot, int tile, const double (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+  const double t = warp_fold8<kMax>(v);
+  if ((lane & 3) == 0) B.w[slot][lane >> 2][threadIdx.x >> 5] = t;
+  if (threadIdx.x == 0) B.tile[slot] = tile;
+}
+
+// Completes the 8-warp tree of the n parked tiles' quantities into
+// part[quantity][tile].
+template <bool kMax>
+__device__ inline void fold_parked8(ParkBuf& B, double* part, int tcap, int n) {
+  __syncthreads();
+  for (int i = threadIdx.x; i < n * 8; i += kThreads) {
+    const int slot = i >> 3, q = i & 7;
+    const double* w = B.w[slot][q];
+    double r;
+    if (kMax && q == 7)
+      r = fmax(fmax(fmax(w[0], w[4]), fmax(w[2], w[6])), fmax(fmax(w[1], w[5]), fmax(w[3], w[7])));
+    else
+      r = ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+    part[(size_t)q * tcap + B.tile[slot]] = r;
+  }
+  __syncthreads();
+}
+
+// Folds a scene's tile partials (the order of fold_tiles_sm: slot j sums tiles
+// j, j + 256, ..., then the 256-slot tree), NS sums and, with kMax, a maximum
+// in plane 7, into out[].  Every member of a team calls it after the pass's
+// barrier and runs the scene's controller on its own copy of the scalars: the
+// partials cross L2 once more per member, and the result needs no second trip
+// through a word that one CTA writes and the others wait for.
+template <int NS, bool kMax>
+__device__ __noinline__ void fold_team(const double* part, int tcap, int nt, double* scratch,
+                                       double* out) {
+  constexpr int U = 4;
+  double v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) v[q] = 0.0;
+  for (int t = threadIdx.x; t < nt; t += U * kThreads) {
+    double x[8][U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int at = t + u * kThreads;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (q < NS || (kMax && q == 7)) x[q][u] = at < nt ? __ldcg(part + (size_t)q * tcap + at) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (t + u * kThreads < nt) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          if (q < NS) v[q] = v[q] + x[q][u];
+          if (kMax && q == 7) v[q] = fmax(v[q], x[q][u]);
+        }
+      }
+    }
+  }
+  const int lane = threadIdx.x & 31;
+  const double f = warp_fold8<kMax>(v);
+  if ((lane & 3) == 0) scratch[(lane >> 2) * 8 + (threadIdx.x >> 5)] = f;
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    const double* w = scratch + threadIdx.x * 8;
+    double r;
+    if (kMax && threadIdx.x == 7)
+      r = fmax(fmax(fmax(w[0], w[4]), fmax(w[2], w[6])), fmax(fmax(w[1], w[5]), fmax(w[3], w[7])));
+    else
+      r = ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+    out[threadIdx.x] = r;
+  }
+  __syncwarp();  // warp 0 runs the controller
+}
+
+// Body pass of a member: w_b = minv_b (D^T x)_b for its bodies.  Heads load two
+// rounds ahead and each body's first eight incidence entries one round ahead,
+// while the current round gathers.
+template <class T, bool kAR>
+__device__ inline void team_body_pass(const KArgs<T>& a, const Team& t, typename Vec4<T>::type* w,
+                                      const typename Vec4<T>::type* q) {
+  const int e = t.w1;
+  int b = t.w0 + threadIdx.x;
+  BodyHead h{0.0, 0, 0, 0}, hn{0.0, 0, 0, 0};
+  if (b < e) h = body_head<false>(a, b);
+  if (b + kThreads < e) hn = body_head<false>(a, b + kThreads);
+  uint32_t c[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) c[j] = (h.s + j < h.e) ? __ldg(a.inc + h.s + j) : 0u;
+  for (; b < e; b += kThreads) {
+    const int bnn = b + 2 * kThreads;
+    BodyHead hnn{0.0, 0, 0, 0};
+    if (bnn < e) hnn = body_head<false>(a, bnn);
+    uint32_t cn[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) cn[j] = (hn.s + j < hn.e) ? __ldg(a.inc + hn.s + j) : 0u;
+    body_w<T, kAR, true>(a, w, q, b, h, c);
+    h = hn;
+    hn = hnn;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) c[j] = cn[j];
+  }
+}
+
+}  // namespace
+
+}  // namespace dv
