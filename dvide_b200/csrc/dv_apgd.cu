@@ -332,12 +332,6 @@ __device__ inline bool bil_product_tile(BilRows<T> R, const Solve& C, int r0, in
   return bad;
 }
 
-// Phases of a one-scene engine, timed by its first member between barriers.
-struct PhaseTimer {
-  unsigned long long last, ns[8];
-  unsigned count[8];
-};
-
 // kAR: APGD's anti-relaxation (APGD.cu:335-345), FP64 one-scene engines.
 template <class T, int kMinB, bool kAR>
 __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
@@ -364,11 +358,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
     fence_mbar_init();
     s_seen = 0;
     s_copy_fail = 0;
-    timer.last = global_ns();
-    for (int i = 0; i < 8; ++i) {
-      timer.ns[i] = 0;
-      timer.count[i] = 0;
-    }
+    timer.start();
   }
   __syncthreads();
   if (ld_acquire(&a.ew->err)) return;  // an error of collision detection: nothing to do
@@ -376,12 +366,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
   // a phase ends at a barrier
   auto sync = [&](int phase, bool joining = false) {
     const bool ok = team_sync(a, tm, joining);
-    if (a.nseg == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
-      const unsigned long long now = global_ns();
-      timer.ns[phase] += now - timer.last;
-      timer.count[phase] += 1;
-      timer.last = now;
-    }
+    timer.mark(a, phase);
     return ok;
   };
 
@@ -400,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
     const int cap = a.refine ? P.refine : P.max_iter;
     int it_lo = 0, bt_lo = 0, sw_lo = 0;
     if (a.refine && threadIdx.x == 0) {
-      const ApgdCtl& D = a.sst[s].ctl;
+      const SolveResult& D = a.sst[s].ctl;
       it_lo = D.iterations;
       bt_lo = D.backtracks;
       sw_lo = D.sweeps;
@@ -1084,7 +1069,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
     // the scene's results, and its warm-start length (System::gamma_d resize)
     if (tm.rank == 0 && threadIdx.x == 0) {
       SegState& X = a.sst[s];
-      ApgdCtl& D = X.ctl;
+      SolveResult& D = X.ctl;
       if (C.err) {
         X.err = err;
         if (a.ew->stop_on_seg_err) atomicOr(&a.ew->err, C.err);
@@ -1094,8 +1079,6 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
       D.sweeps = C.sweeps + sw_lo;
       D.residual = C.residual;
       D.objective = C.objective;
-      D.best = C.best;
-      D.done = 1;
       D.refine_it = a.refine ? C.iterations : 0;
       if (!a.refine) D.refined = refine_next ? 1 : 0;
       if (live) X.gsize = nc;
@@ -1103,12 +1086,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
       if (a.nbil && !a.solve_only) a.seg_time[s] = a.seg_time[s] + P.h;
     }
   }
-  if (a.nseg == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
-    for (int i = 0; i < 8; ++i) {
-      a.ew->phase_ns[i] += timer.ns[i];
-      a.ew->phase_count[i] += timer.count[i];
-    }
-  }
+  timer.store(a);
 }
 
 // The scenes of one launch in teams (engines of several scenes): those that
@@ -1218,14 +1196,7 @@ void launch_typed(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t
   KArgs<T> a = make_kargs<T>(sd, cfg);
   a.solve_only = solve_only ? 1 : 0;
   a.refine = refine ? 1 : 0;
-  if (sd.nseg > 1) {
-    k_team_plan<<<1, 1024, 0, st>>>(sd.nseg, sd.seg, sd.sst, a.refine, cfg.grid, sd.slots, sd.slot_cap,
-                                    sd.order, sd.team_bar, sd.ew);
-    ++*launches;
-  } else {
-    cudaMemsetAsync(sd.team_bar, 0, sizeof(unsigned), st);
-    if (!refine) cudaMemsetAsync(&sd.sst->err, 0, sizeof(unsigned), st);
-  }
+  plan_teams(sd, cfg.grid, refine, st, launches);
   void* params[] = {&a};
   cudaLaunchCooperativeKernel((const void*)k_step_solve<T, MB, AR>, cfg.grid, kThreads, params,
                               solve_smem_bytes<T>(), st);
@@ -1254,14 +1225,23 @@ int apgd_max_ctas(int precision, int blocks_per_sm) {
   return max_ctas_of<double, 2>();
 }
 
+void plan_teams(SceneDev& sd, int grid, bool refine, cudaStream_t st, int64_t* launches) {
+  if (sd.nseg > 1) {
+    k_team_plan<<<1, 1024, 0, st>>>(sd.nseg, sd.seg, sd.sst, refine ? 1 : 0, grid, sd.slots,
+                                    sd.slot_cap, sd.order, sd.team_bar, sd.ew);
+    ++*launches;
+  } else {
+    cudaMemsetAsync(sd.team_bar, 0, sizeof(unsigned), st);
+    if (!refine) cudaMemsetAsync(&sd.sst->err, 0, sizeof(unsigned), st);
+  }
+}
+
 void launch_step_solve(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t* launches,
                        bool solve_only) {
-  if (sd.solver == DV_SOLVER_PGJ || sd.solver == DV_SOLVER_PGS) {
-    cudaMemsetAsync(sd.ew->bar, 0, sizeof(sd.ew->bar), st);
-    cudaMemsetAsync(&sd.ew->last_release, 0, sizeof(unsigned long long), st);
-    if (sd.solver == DV_SOLVER_PGJ) launch_pgj_solve(sd, cfg, st, solve_only);
-    else launch_pgs_solve(sd, cfg, st, solve_only);
-    ++*launches;
+  if (sd.solver == DV_SOLVER_PGJ) {
+    launch_pgj_solve(sd, cfg, st, launches, solve_only);
+  } else if (sd.solver == DV_SOLVER_PGS) {
+    launch_pgs_solve(sd, cfg, st, launches, solve_only);
   } else if (sd.precision == DV_PREC_MIXED) {
     // with refinement the FP32 launch leaves the update of the solves it marks
     // to an FP64 launch, which refines them first

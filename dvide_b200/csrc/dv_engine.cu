@@ -521,13 +521,12 @@ int Engine::reconfigure(const std::vector<SlotSpec>& slots) {
   DV_CUDA_TRY(cudaMemsetAsync(d.fc4, 0, sizeof(double4) * nbz, st));
   if (nseg2 > seg_cap_) {
     int cap = std::max(nseg2, seg_cap_ + seg_cap_ / 4);
-    dfree(d.seg); dfree(d.sst); dfree(d.grid); dfree(d.seg_tstart); dfree(d.donemask);
+    dfree(d.seg); dfree(d.sst); dfree(d.grid); dfree(d.seg_tstart);
     dfree(d.order); dfree(d.team_bar);
     TRY(dalloc(&d.seg, cap));
     TRY(dalloc(&d.sst, cap));
     TRY(dalloc(&d.grid, cap));
     TRY(dalloc(&d.seg_tstart, (size_t)cap + 1));
-    TRY(dalloc(&d.donemask, (size_t)(cap + 31) / 32));
     TRY(dalloc(&d.order, cap));
     TRY(dalloc(&d.team_bar, (size_t)cap * kTeamBarStride));
     if (h_sst_) cudaFreeHost(h_sst_);

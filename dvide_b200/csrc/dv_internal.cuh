@@ -71,41 +71,18 @@ struct SegParams {
   int refine;               // mixed precision: FP64 iterations after a stalled FP32 phase (0: off)
 };
 
-// Scalar state of one APGD solve (APGD.cu:208-223, 266-332).  Iterates live in
-// five rotating buffers G[0..4] with their Schur products NG[0..4]: cur =
-// gamma_k, prev = gamma_{k-1}, nw = target of gamma_new, best = gamma_hat (-1
-// before the first accepted iterate); the fifth holds the next iterate computed
-// ahead.
-struct ApgdCtl {
-  double L, t, theta, theta_new, beta;
-  double obj1, obj2, obj2_base;
-  double residual;      // best residual so far (APGD.cu:214, 293-301)
+// Results of one solve.
+struct SolveResult {
+  double residual;      // best residual (APGD.cu:214, 293-301)
   double objective;     // objective of the best iterate (APGD.cu:353-354)
-  double gdiff, ginv;   // 1 / nc^2 and its reciprocal (APGD.cu:92, 98)
-  double L0;
-  double fx;            // PGJ: primal feasibility of the iterate computed last
-  double yb;            // beta used for y_k = (1+yb) gamma_k - yb gamma_{k-1}
-  int k;                // iteration index
-  int mode;             // next contact pass: 0 full iteration, 1 backtrack
-  int done;
-  int restart;          // g.(gamma_new - gamma) > 0 for the current gamma_new
-  int cur, prev, nw, best;
-  int yr;               // y_k = gamma_k (first iteration or after a restart)
-  int first;            // first iteration: N y_0 is a Schur product
-  int backtracks;
-  unsigned err;
   int iterations;
+  int backtracks;
   int sweeps;           // iterations executed
-  int rsel;             // anti-relaxation: plane of the current r_n and ar (the other: next)
-  double objN;          // anti-relaxation: half of gamma_hat . N gamma_hat
-  // mixed precision with FP64 refinement: accepted iterations since the best
-  // residual last improved (FP32 phase); whether the FP64 phase refines this
-  // solve (set at the end of the FP32 phase); the FP64 phase's iterations; the
-  // FP32 phase's counts while the FP64 phase runs
-  int since_best;
+  int mode;             // PGS: the sweep starts again (in order at fixed bodies too)
+  // mixed precision with FP64 refinement: whether the FP64 launch refines this
+  // solve (set by the FP32 launch), and its iterations
   int refined;
   int refine_it;
-  int it_lo, bt_lo, sw_lo;
 };
 
 // Per-segment results of the current step (device-written).
@@ -115,10 +92,9 @@ struct SegState {
   int t0, nt;           // tiles
   int delta;            // c0 - (unpadded global offset of the segment's first contact)
   int gsize;            // warm-start length (System::gamma_d / 3); kept when nc = 0
-  unsigned arrive;      // tile arrivals in the current pass
   unsigned err;         // error bits of this segment's last step
   int members;          // CTAs of its team in this launch (engines of several segments)
-  ApgdCtl ctl;
+  SolveResult ctl;
 };
 
 // Engine-wide words (device).
@@ -130,14 +106,9 @@ struct EngineWords {
   int n_small;          // gridded bodies (constant)
   int stop_on_seg_err;  // 1: a segment's solver error also sets err (plain System semantics)
   unsigned err;         // error bits (kErr*); sticky: every kernel of a step skips its work while set
-  int active;           // segments still iterating (solve kernel)
-  int step_count;       // segments that request a step pass next iteration
-  int step_needed;      // latched step_count for the current iteration
-  unsigned bar[4];      // grid barrier: [0] arrivals, [1] generation, [2] error bits
-  unsigned long long last_release;
   unsigned long long phase_ns[8];
   unsigned long long phase_count[8];
-  unsigned long long wait_limit_ns;  // every bounded wait (grid barrier, bulk copy) ends after this
+  unsigned long long wait_limit_ns;  // every bounded wait (team barrier, bulk copy) ends after this
   // Teams of the solve kernel (engines of several segments): slots of the plan,
   // the next one to take, and the passes that all teams have finished (a CTA
   // that waits for its team to form sees from it that the others go on).
@@ -170,7 +141,6 @@ struct SceneDev {
   GridInfo* grid = nullptr;     // nseg
   int* seg_tstart = nullptr;    // nseg + 1 tile starts (for tile -> segment lookup)
   int* tseg = nullptr;          // tile -> segment
-  unsigned* donemask = nullptr; // (nseg + 31) / 32 words: segments not iterating
   EngineWords* ew = nullptr;
   // bodies
   double4 *p4 = nullptr, *v4 = nullptr, *k4 = nullptr, *f4 = nullptr, *w4 = nullptr, *fc4 = nullptr;
@@ -292,10 +262,12 @@ int apgd_max_ctas(int precision, int blocks_per_sm);
 // own solve(): v, p, f_contact and the clock are left as they are)
 void launch_step_solve(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t* launches,
                        bool solve_only = false);
-// ---- PGJ (dv_pgj.cu) ----
-int pgj_max_ctas(int precision);
-void launch_pgj_solve(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, bool solve_only);
-int pgs_max_ctas();
-void launch_pgs_solve(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, bool solve_only);
+// The teams of one solve launch (refine: of the solves the FP32 launch marked).
+void plan_teams(SceneDev& sd, int grid, bool refine, cudaStream_t st, int64_t* launches);
+// ---- PGJ (dv_pgj.cu), PGS (dv_pgs.cu) ----
+void launch_pgj_solve(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t* launches,
+                      bool solve_only);
+void launch_pgs_solve(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t* launches,
+                      bool solve_only);
 
 }  // namespace dv

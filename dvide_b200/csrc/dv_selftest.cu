@@ -1,10 +1,9 @@
 // dv_selftest.cu -- makes the solve kernels' bounded waits run out on
-// purpose, without a fault: a cooperative launch of two CTAs where CTA 1
-// never arrives at the grid barrier, and an mbarrier that expects 16 bytes no
-// copy will bring.  The waits are the ones the solve kernels use (grid_sync,
-// bounded_mbar_wait); each must end after the limit with its error bit set,
-// and the context stays usable.
-#include "dv_solve.cuh"
+// purpose, without a fault: a team of two whose second member never arrives at
+// its barrier, and an mbarrier that expects 16 bytes no copy will bring.  The
+// waits are the ones the solve kernels use (team_sync, bounded_mbar_wait); each
+// must end after the limit with its error bit set, and the context stays usable.
+#include "dv_team.cuh"
 
 #include "dvide.h"
 
@@ -14,12 +13,23 @@ namespace {
 
 struct WaitTestArgs {
   EngineWords* ew;
+  unsigned* team_bar;
+  int nseg;
 };
 
 __global__ void __launch_bounds__(kThreads) k_selftest_waits(WaitTestArgs a, int* out) {
   __shared__ __align__(8) uint64_t bar[1];
-  if (blockIdx.x != 0) return;  // the CTA that never reaches the barrier
-  const bool barrier_ok = grid_sync(a, kPhaseSetup, NoCtl{});
+  __shared__ Team tm;
+  if (threadIdx.x == 0) {
+    // a team of two whose second member never arrives
+    tm.rank = 0;
+    tm.m = 2;
+    tm.fail = 0;
+    tm.target = 0;
+    tm.bar = a.team_bar;
+  }
+  __syncthreads();
+  const bool barrier_ok = team_sync(a, tm);
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
@@ -48,21 +58,21 @@ DV_API int dv_selftest_bounded_waits(int32_t limit_ms, int32_t* barrier_timed_ou
                                      int32_t* copy_timed_out, uint32_t* error_bits) {
   if (limit_ms <= 0) return DV_ERR_ARG;
   EngineWords* ew = nullptr;
-  int* out = nullptr;
+  int* out = nullptr;  // two results, then the barrier's counter
   if (cudaMalloc(&ew, sizeof(EngineWords)) != cudaSuccess) return DV_ERR_OOM;
-  if (cudaMalloc(&out, 2 * sizeof(int)) != cudaSuccess) {
+  if (cudaMalloc(&out, 3 * sizeof(int)) != cudaSuccess) {
     cudaFree(ew);
     return DV_ERR_OOM;
   }
   EngineWords h;
   memset(&h, 0, sizeof(h));
   h.wait_limit_ns = (unsigned long long)limit_ms * 1000000ull;
-  int host_out[2] = {-1, -1};
+  int host_out[3] = {-1, -1, 0};
   cudaMemcpy(ew, &h, sizeof(h), cudaMemcpyHostToDevice);
   cudaMemcpy(out, host_out, sizeof(host_out), cudaMemcpyHostToDevice);
-  WaitTestArgs a{ew};
-  void* params[] = {&a, &out};
-  cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_selftest_waits, 2, kThreads, params, 0, 0);
+  WaitTestArgs a{ew, reinterpret_cast<unsigned*>(out + 2), 1};
+  k_selftest_waits<<<1, kThreads>>>(a, out);
+  cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaMemcpy(host_out, out, sizeof(host_out), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemcpy(&h, ew, sizeof(h), cudaMemcpyDeviceToHost);

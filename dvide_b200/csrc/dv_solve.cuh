@@ -1,10 +1,8 @@
 // dv_solve.cuh -- device machinery shared by the persistent solve kernels
-// (APGD in dv_apgd.cu, PGJ in dv_pgj.cu): kernel arguments, the tangent frame
-// and the matrix-free products with the frame, the ordered tile reductions
-// (per-warp shuffle folds parked in shared memory, per-scene tile folds), the
-// per-scene arrival counters, the grid barrier, the CTA tile sequence and
-// segment cache, the body gather, the done mask, and the per-warp staging of
-// bulk asynchronous copies.  Every wait has a time limit.
+// (APGD in dv_apgd.cu, PGJ in dv_pgj.cu, PGS in dv_pgs.cu): kernel arguments,
+// the tangent frame and the matrix-free products with the frame, the ordered
+// tile reductions, the body gather, bilateral rows, and the per-warp staging
+// of bulk asynchronous copies.  Every wait has a time limit.
 #pragma once
 
 #include <stdio.h>
@@ -21,11 +19,10 @@ constexpr int kQMax = kNQ;  // slot of the per-tile maximum
 constexpr int kWarps = kThreads / 32;
 constexpr int kSub = kThreads;  // contacts per sub-tile
 
-// Phases timed between grid-barrier releases (EngineWords::phase_ns).
+// Phases timed between barriers (EngineWords::phase_ns).
 enum Phase : int {
   kPhaseSetup = 0,     // k, r, Lipschitz estimate
   kPhaseStep = 1,      // gamma_new = P(y - t g): first iteration or backtrack
-  kPhaseRebuild = 2,   // work lists of the segments still iterating
   kPhaseBody = 3,      // body gather w = Minv D^T q
   kPhaseProduct = 4,   // N gamma_new, objective, residual, look-ahead step
   kPhaseFinal = 5,     // gamma = gamma_hat, update
@@ -51,7 +48,6 @@ struct KArgs {
   double4* fc4;
   double4* wd;        // body vector, double4 (setup); reinterpreted as Vec4<T> in iterations
   const double* __restrict__ minv;
-  const int* __restrict__ bseg;
   const uint32_t* __restrict__ ida;
   const uint32_t* __restrict__ idb;
   const double* __restrict__ F;
@@ -70,11 +66,10 @@ struct KArgs {
   int* wc;            // ... and their count
   const int* __restrict__ cbase;     // this step's contact offsets (unpadded) per body
   const int* __restrict__ cnt_cont;  // this step's contacts with A = body
+  int* body_count;    // PGS: contacts of each body that the sweep has updated (scratch)
   double* part;
   const SegParams* __restrict__ seg;
   SegState* sst;
-  const int* __restrict__ tseg;
-  unsigned* donemask;
   EngineWords* ew;
   const int2* slots;       // the plan of the teams: (scene, rank) per slot
   unsigned* team_bar;      // arrivals of each scene's team, kTeamBarStride words apart
@@ -208,19 +203,6 @@ __device__ inline Frame<T> start_frame(const KArgs<T>& a, int c, bool exact) {
 template <class T>
 __device__ inline Frame<double> load_frame_fp64(const KArgs<T>& a, int c, bool exact) {
   return frame_d(__ldg(a.F + c), __ldg(a.F + a.S + c), __ldg(a.F + 2 * a.S + c), exact);
-}
-
-// The nine stored frame planes (n, u, v) of contact c, as the narrowphase
-// wrote them: the same bits as load_frame_fp64, read instead of rebuilt.
-template <class T>
-__device__ inline Frame<double> stored_frame(const KArgs<T>& a, int c) {
-  const double* F = a.F;
-  const size_t S = a.S;
-  Frame<double> f;
-  f.n0 = __ldg(F + c); f.n1 = __ldg(F + S + c); f.n2 = __ldg(F + 2 * S + c);
-  f.u0 = __ldg(F + 3 * S + c); f.u1 = __ldg(F + 4 * S + c); f.u2 = __ldg(F + 5 * S + c);
-  f.v0 = __ldg(F + 6 * S + c); f.v1 = __ldg(F + 7 * S + c); f.v2 = __ldg(F + 8 * S + c);
-  return f;
 }
 
 // Stores of the vectors a pass writes and the next pass reads at once (q for
@@ -377,9 +359,6 @@ struct DeferBuf {
   int fail;                              // a warp's copy wait timed out
 };
 
-// Tile arrivals of one segment: a CTA delivers the count of its consecutive
-// tiles of segment s at once (after their partials are written).  True, in
-// every thread, in the CTA whose delivery completes the segment's tiles.
 // ---- maxima reductions of PGJ and PGS (only maxima: no summation order) ----
 // max_c -min(0, scale * x_n - |x_t|), a NaN term counting 0 (PGJ.cu:112-142, PGS.cu:335-365)
 __device__ inline double pgj_feasible(double xn, double xt1, double xt2, double scale) {
@@ -413,152 +392,6 @@ __device__ inline void fold_parked_max(const K& a, DeferBuf& B, int n) {
   }
   __threadfence();
   __syncthreads();
-}
-
-
-template <class K>
-__device__ inline bool seg_arrive(const K& a, int s, int n) {
-  __shared__ int s_flag;
-  // the tiles' partials were written (and fenced) before the CTA barrier that
-  // ends fold_parked
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned nt = (unsigned)a.sst[s].nt;
-    unsigned old = atom_add_acq_rel(&a.sst[s].arrive, (unsigned)n);
-    int last = (old + (unsigned)n == nt);
-    if (last) a.sst[s].arrive = 0u;  // the next pass starts after a grid barrier
-    s_flag = last;
-  }
-  __syncthreads();
-  const bool last = s_flag != 0;
-  if (last) __threadfence();
-  return last;
-}
-
-// The segment of a tile and its ranges, cached per CTA for the whole kernel
-// (they do not change during a step): tiles of the cached segment need no
-// loads to find their contacts.
-struct SegCache {
-  int s;
-  int t0, t1;   // tiles [t0, t1)
-  int c0, nc;   // contacts [c0, c0 + nc)
-  int gsize;
-};
-
-// c is in shared memory; every thread of the CTA calls this with the same t.
-template <class K>
-__device__ inline void locate(const K& a, SegCache& c, int t) {
-  if (t >= c.t0 && t < c.t1) return;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int s = a.tseg[t];
-    const SegState& X = a.sst[s];
-    c.s = s;
-    c.t0 = X.t0;
-    c.t1 = X.t0 + X.nt;
-    c.c0 = X.c0;
-    c.nc = X.nc;
-    c.gsize = X.gsize;
-  }
-  __syncthreads();
-}
-
-struct SegRun {
-  int s = -1;  // segment of the current run of tiles
-  int n = 0;   // tiles of it processed since the last delivery
-};
-
-// Delivers the run's arrivals; the CTA that completes the segment runs ctl(s).
-template <class K, class Fn>
-// `deferred`: the pass's grid barrier runs the controller instead (an engine
-// with one segment: its controller follows the last arrival anyway, so the
-// arrival counter would only add a serialized atomic to every CTA's exit).
-__device__ inline void flush_run(const K& a, SegRun& run, Fn ctl, bool deferred = false) {
-  if (run.n == 0) return;
-  const int s = run.s, n = run.n;
-  run.n = 0;
-  if (deferred) return;
-  if (seg_arrive(a, s, n)) ctl(s);
-}
-
-// Grid barrier.  The last CTA to arrive runs `ctl_fn` (all its threads),
-// then releases the generation word.  Returns false after a timeout or an
-// error raised by another CTA; the caller then leaves the kernel.
-template <class K, class Fn>
-__device__ inline bool grid_sync(const K& a, int phase, Fn ctl_fn) {
-  __shared__ unsigned s_last, s_target;
-  __shared__ int s_fail;
-  unsigned* bar = a.ew->bar;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    unsigned ticket = atom_add_acq_rel(&bar[0], 1u);
-    s_target = ticket / gridDim.x + 1u;
-    s_last = (ticket % gridDim.x) == gridDim.x - 1u;
-    s_fail = 0;
-  }
-  __syncthreads();
-  if (s_last) {
-    __threadfence();
-    ctl_fn();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const unsigned long long now = global_ns();
-      __threadfence();
-      st_release(&bar[1], s_target);
-      // Phase timers, after the release so that their round trips to L2 are
-      // off the barrier's critical path.  Written by whichever CTA arrives
-      // last (no L1-cached copies); the next barrier's last CTA reads them
-      // only after this CTA's next arrival, which follows in program order.
-      volatile EngineWords* E = a.ew;
-      const unsigned long long prev = E->last_release;
-      if (prev) {
-        E->phase_ns[phase] += now - prev;
-        E->phase_count[phase] += 1;
-      }
-      E->last_release = now;
-    }
-  } else if (threadIdx.x == 0) {
-    const uint64_t limit = a.ew->wait_limit_ns;
-    uint64_t t0 = global_ns();
-    unsigned polls = 0;
-    while (ld_acquire(&bar[1]) < s_target) {
-      __nanosleep(20);
-      if ((++polls & 1023u) == 0u) {
-        if (ld_acquire(&a.ew->err) & (kErrBarrierTimeout | kErrCopyTimeout)) {
-          s_fail = 1;
-          break;
-        }
-        if (global_ns() - t0 > limit) {
-          atomicOr(&a.ew->err, kErrBarrierTimeout);
-          s_fail = 1;
-          break;
-        }
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return !s_fail;
-}
-
-struct NoCtl {
-  __device__ void operator()() const {}
-};
-
-// Tile i of this CTA's sequence (-1 past the end): round robin in chunks of
-// `chunk` consecutive tiles, or one contiguous range per CTA.
-template <class K>
-__device__ inline int cta_tile(const K& a, int nt, int i) {
-  if (a.contiguous) {
-    long long lo = (long long)nt * blockIdx.x / gridDim.x;
-    long long hi = (long long)nt * (blockIdx.x + 1) / gridDim.x;
-    long long t = lo + i;
-    return t < hi ? (int)t : -1;
-  }
-  const int k = a.chunk;
-  long long t = ((long long)blockIdx.x + (long long)(i / k) * gridDim.x) * k + (i % k);
-  return t < nt ? (int)t : -1;
 }
 
 // Eight incidence entries c[0, n) of a body's run (n <= 8): their q gathered
@@ -669,83 +502,28 @@ __device__ inline void add_bilateral(const int* __restrict__ start, const uint32
 
 // A solver error of segment s; with stop_on_seg_err it also stops the steps
 // that follow (every kernel checks EngineWords::err first).
-// A segment's APGD words as its controller finds them: controllers of earlier
-// passes ran on other CTAs, so every field is read through L2, with all the
-// loads in flight together (one round trip instead of one per field).
-__device__ inline ApgdCtl ctl_read(const ApgdCtl* C) {
-  ApgdCtl c;
-  c.L = __ldcg(&C->L); c.t = __ldcg(&C->t); c.theta = __ldcg(&C->theta);
-  c.theta_new = __ldcg(&C->theta_new); c.beta = __ldcg(&C->beta);
-  c.obj1 = __ldcg(&C->obj1); c.obj2 = __ldcg(&C->obj2); c.obj2_base = __ldcg(&C->obj2_base);
-  c.residual = __ldcg(&C->residual); c.objective = __ldcg(&C->objective);
-  c.gdiff = __ldcg(&C->gdiff); c.ginv = __ldcg(&C->ginv); c.L0 = __ldcg(&C->L0);
-  c.fx = __ldcg(&C->fx); c.yb = __ldcg(&C->yb);
-  c.k = __ldcg(&C->k); c.mode = __ldcg(&C->mode); c.done = __ldcg(&C->done);
-  c.restart = __ldcg(&C->restart); c.cur = __ldcg(&C->cur); c.prev = __ldcg(&C->prev);
-  c.nw = __ldcg(&C->nw); c.best = __ldcg(&C->best); c.yr = __ldcg(&C->yr);
-  c.first = __ldcg(&C->first); c.backtracks = __ldcg(&C->backtracks); c.err = __ldcg(&C->err);
-  c.iterations = __ldcg(&C->iterations); c.sweeps = __ldcg(&C->sweeps);
-  c.rsel = __ldcg(&C->rsel);
-  c.since_best = __ldcg(&C->since_best);
-  return c;
-}
-
 template <class K>
 __device__ inline void seg_error(const K& a, int s, unsigned bit) {
   atomicOr(&a.sst[s].err, bit);
   if (a.ew->stop_on_seg_err) atomicOr(&a.ew->err, bit);
 }
 
-// Done mask: bit s set when segment s is not iterating.  Each pass starts
-// with a copy in shared memory (segments beyond kMaskWords * 32 read it from
-// global memory).
-constexpr int kMaskWords = 256;
-
-template <class K>
-__device__ inline void load_mask(const K& a, unsigned* s_mask, int mwords) {
-  if (a.nseg == 1) return;  // a single segment iterates while the loop runs
-  __syncthreads();
-  for (int i = threadIdx.x; i < mwords && i < kMaskWords; i += kThreads)
-    s_mask[i] = __ldcg(a.donemask + i);
-  __syncthreads();
-}
-
-template <class K>
-__device__ inline bool mask_done(const K& a, const unsigned* s_mask, int mwords, int s) {
-  if (a.nseg == 1) return false;
-  const int w = s >> 5;
-  const unsigned m = (w < kMaskWords) ? s_mask[w] : __ldcg(a.donemask + w);
-  return (m >> (s & 31)) & 1u;
-}
-
-// Segment s stops iterating (controller thread).
-template <class K>
-__device__ inline void mark_done(const K& a, int s) {
-  volatile ApgdCtl* C = &a.sst[s].ctl;
-  C->done = 1;
-  atomicOr(a.donemask + (s >> 5), 1u << (s & 31));
-}
-
-// Schur body pass: w_b = minv_b * (D^T x)_b for bodies of iterating
-// segments; fixed bodies keep w = 0.
-// w_b of one body of an iterating segment.
+// w_b = minv_b * (D^T x)_b of one body; fixed bodies keep w = 0.
 // kAR: also v = Minv (k + D^T x) for the anti-relaxation (APGD.cu:338-340;
 // 0 for fixed bodies, whose v enters only as squares).
-// The words a body's gather starts from: its inverse mass, the bounds of its
-// incidence run and (batches) its segment, loaded together so that they cost
-// one memory round trip, and loaded a round ahead by the body pass.
+// The words a body's gather starts from, its inverse mass and the bounds of its
+// incidence run, loaded together so that they cost one memory round trip.
 struct BodyHead {
   double mi;
-  int s, e, seg;
+  int s, e;
 };
 
-template <bool kSeg = true, class K>
+template <class K>
 __device__ inline BodyHead body_head(const K& a, int b) {
   BodyHead h;
   h.mi = __ldg(a.minv + b);
   h.s = __ldg(a.inc_start + b);
   h.e = __ldg(a.inc_start + b + 1);
-  h.seg = kSeg && a.nseg > 1 ? __ldg(a.bseg + b) : 0;
   return h;
 }
 
@@ -776,39 +554,6 @@ __device__ inline void body_w(const KArgs<T>& a, typename Vec4<T>::type* w,
     V o;
     o.x = T(0); o.y = T(0); o.z = T(0); o.w = T(0);
     store_keep(w + b, o);
-  }
-}
-
-// Schur body pass: w_b = minv_b * (D^T x)_b for bodies of iterating
-// segments; fixed bodies keep w = 0.
-template <class T>
-__device__ inline void body_pass_schur(const KArgs<T>& a, const unsigned* s_mask) {
-  using V = typename Vec4<T>::type;
-  V* w = reinterpret_cast<V*>(a.wd);
-  const V* q = reinterpret_cast<const V*>(a.qd);
-  const int mwords = (a.nseg + 31) >> 5;
-  // heads load into registers two rounds ahead, and each body's first eight
-  // incidence entries one round ahead, while the current round gathers
-  const int stride = gridDim.x * kThreads;
-  int b = blockIdx.x * kThreads + threadIdx.x;
-  BodyHead h{0.0, 0, 0, 0}, hn{0.0, 0, 0, 0};
-  if (b < a.nb) h = body_head(a, b);
-  if (b + stride < a.nb) hn = body_head(a, b + stride);
-  uint32_t c[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) c[j] = (h.s + j < h.e) ? __ldg(a.inc + h.s + j) : 0u;
-  for (; b < a.nb; b += stride) {
-    const int bnn = b + 2 * stride;
-    BodyHead hnn{0.0, 0, 0, 0};
-    if (bnn < a.nb) hnn = body_head(a, bnn);
-    uint32_t cn[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) cn[j] = (hn.s + j < hn.e) ? __ldg(a.inc + hn.s + j) : 0u;
-    if (a.nseg == 1 || !mask_done(a, s_mask, mwords, h.seg)) body_w<T, false, true>(a, w, q, b, h, c);
-    h = hn;
-    hn = hnn;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) c[j] = cn[j];
   }
 }
 
@@ -920,7 +665,6 @@ KArgs<T> make_kargs(SceneDev& sd, const SolveConfig& cfg) {
   a.fc4 = sd.fc4;
   a.wd = sd.w4;
   a.minv = sd.minv;
-  a.bseg = sd.bseg;
   a.ida = sd.ida;
   a.idb = sd.idb;
   a.F = sd.F;
@@ -938,11 +682,10 @@ KArgs<T> make_kargs(SceneDev& sd, const SolveConfig& cfg) {
   a.wc = sd.wc;
   a.cbase = sd.cbase;
   a.cnt_cont = sd.cnt_cont;
+  a.body_count = sd.cnt_cand;
   a.part = sd.part;
   a.seg = sd.seg;
   a.sst = sd.sst;
-  a.tseg = sd.tseg;
-  a.donemask = sd.donemask;
   a.ew = sd.ew;
   a.slots = sd.slots;
   a.team_bar = sd.team_bar;

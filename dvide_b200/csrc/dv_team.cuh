@@ -148,6 +148,38 @@ __device__ inline bool join_team(const K& a, Team& t, int* slot_seen) {
   return t.s >= 0;
 }
 
+// Phases of a one-scene engine, timed by its first member between barriers (in
+// shared memory).
+struct PhaseTimer {
+  unsigned long long last, ns[8];
+  unsigned count[8];
+  __device__ void start() {
+    last = global_ns();
+    for (int i = 0; i < 8; ++i) {
+      ns[i] = 0;
+      count[i] = 0;
+    }
+  }
+  template <class K>
+  __device__ void mark(const K& a, int phase) {
+    if (a.nseg == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
+      const unsigned long long now = global_ns();
+      ns[phase] += now - last;
+      count[phase] += 1;
+      last = now;
+    }
+  }
+  template <class K>
+  __device__ void store(const K& a) const {
+    if (a.nseg == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
+      for (int i = 0; i < 8; ++i) {
+        a.ew->phase_ns[i] += ns[i];
+        a.ew->phase_count[i] += count[i];
+      }
+    }
+  }
+};
+
 // Folds the eight quantities of a warp's lanes together, each in the order of
 // warp_fold (strides 16, 8, 4, 2, 1; addition commutes, so which of two lanes
 // adds does not matter).  At each of the first three strides a lane hands half
@@ -272,16 +304,16 @@ __device__ inline void team_body_pass(const KArgs<T>& a, const Team& t, typename
                                       const typename Vec4<T>::type* q) {
   const int e = t.w1;
   int b = t.w0 + threadIdx.x;
-  BodyHead h{0.0, 0, 0, 0}, hn{0.0, 0, 0, 0};
-  if (b < e) h = body_head<false>(a, b);
-  if (b + kThreads < e) hn = body_head<false>(a, b + kThreads);
+  BodyHead h{0.0, 0, 0}, hn{0.0, 0, 0};
+  if (b < e) h = body_head(a, b);
+  if (b + kThreads < e) hn = body_head(a, b + kThreads);
   uint32_t c[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) c[j] = (h.s + j < h.e) ? __ldg(a.inc + h.s + j) : 0u;
   for (; b < e; b += kThreads) {
     const int bnn = b + 2 * kThreads;
-    BodyHead hnn{0.0, 0, 0, 0};
-    if (bnn < e) hnn = body_head<false>(a, bnn);
+    BodyHead hnn{0.0, 0, 0};
+    if (bnn < e) hnn = body_head(a, bnn);
     uint32_t cn[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) cn[j] = (hn.s + j < hn.e) ? __ldg(a.inc + hn.s + j) : 0u;
