@@ -36,6 +36,55 @@ __global__ void __launch_bounds__(kThreads) k_items_final(const double* __restri
   if (threadIdx.x == 0) *out = v;
 }
 
+// Minimum of n items as a loop over them in order finds it with std::min: the
+// first of equal values (zeros of either sign), NaN items after the first
+// passed over, a NaN first item kept.  blockIdx.y: which of two item rows.
+struct MinAt {
+  double x;
+  int i;  // n: none
+};
+__device__ inline MinAt min_at(MinAt a, MinAt b) {
+  return (b.x < a.x || (b.x == a.x && b.i < a.i)) ? b : a;
+}
+__device__ inline MinAt block_min_at(MinAt m) {
+  __shared__ MinAt s_m[kThreads / 32];
+  for (int off = 16; off >= 1; off >>= 1) {
+    MinAt o;
+    o.x = __shfl_down_sync(0xffffffffu, m.x, off);
+    o.i = __shfl_down_sync(0xffffffffu, m.i, off);
+    m = min_at(m, o);
+  }
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
+  __syncthreads();
+  m = s_m[0];
+  for (int w = 1; w < kThreads / 32; ++w) m = min_at(m, s_m[w]);
+  return m;
+}
+constexpr int kMinBlocks = 64;
+__global__ void __launch_bounds__(kThreads) k_min_partials(const double* __restrict__ items, int n,
+                                                           MinAt* __restrict__ part) {
+  const double* x = items + (size_t)blockIdx.y * n;
+  MinAt m{(double)INFINITY, n};
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += kMinBlocks * kThreads) {
+    const double v = x[i];
+    if (v == v) m = min_at(m, MinAt{v, i});
+  }
+  m = block_min_at(m);
+  if (threadIdx.x == 0) part[blockIdx.y * kMinBlocks + blockIdx.x] = m;
+}
+__global__ void __launch_bounds__(kThreads) k_min_final(const double* __restrict__ items, int n,
+                                                        const MinAt* __restrict__ part,
+                                                        double* __restrict__ out) {
+  MinAt m{(double)INFINITY, n};
+  if (threadIdx.x < kMinBlocks) m = part[blockIdx.y * kMinBlocks + threadIdx.x];
+  m = block_min_at(m);
+  if (threadIdx.x == 0) {
+    const double first = items[(size_t)blockIdx.y * n];
+    out[blockIdx.y] = first == first ? m.x : first;
+  }
+}
+
 // System.cu:1590-1643 per-contact items: gamma_n, v_n, gamma_n v_n, cone violation^2.
 __global__ void __launch_bounds__(kThreads) k_violation_items(
     int nc, int c0, size_t S, int w0, size_t WS, const double* __restrict__ gamma,
@@ -151,7 +200,8 @@ int Engine::ccp_violation(int s, double* out4) {
   const int nc = X.nc;
   if (nc == 0) return DV_OK;
   const int nt = (nc + kTileItems - 1) / kTileItems;
-  if (ensure_red(4 * (size_t)nc + 2 * (size_t)(nt + 2)) != DV_OK) return DV_ERR_OOM;
+  const size_t nmin = 2 * 2 * kMinBlocks + 2;  // the minima's partials and results
+  if (ensure_red(4 * (size_t)nc + 2 * (size_t)(nt + 2) + nmin) != DV_OK) return DV_ERR_OOM;
   double* items = d_red_;
   double* part = d_red_ + 4 * (size_t)nc;
   if (hseg_[s].nbil > 0)
@@ -166,16 +216,15 @@ int Engine::ccp_violation(int s, double* out4) {
   ++launches_;
   ordered_sum_dev(items + 2 * (size_t)nc, nc, part, 0);
   ordered_sum_dev(items + 3 * (size_t)nc, nc, part + nt + 2, 1);
-  std::vector<double> gn(nc), vn(nc);
-  DV_CUDA_TRY(cudaMemcpyAsync(gn.data(), items, sizeof(double) * nc, cudaMemcpyDeviceToHost, st_));
-  DV_CUDA_TRY(cudaMemcpyAsync(vn.data(), items + nc, sizeof(double) * nc, cudaMemcpyDeviceToHost, st_));
+  double* mins = part + 2 * (nt + 2);
+  MinAt* mpart = reinterpret_cast<MinAt*>(mins + 2);
+  k_min_partials<<<dim3(kMinBlocks, 2), kThreads, 0, st_>>>(items, nc, mpart);
+  k_min_final<<<dim3(1, 2), kThreads, 0, st_>>>(items, nc, mpart, mins);
+  launches_ += 2;
+  DV_CUDA_TRY(cudaMemcpyAsync(h_red_ + 4, mins, 2 * sizeof(double), cudaMemcpyDeviceToHost, st_));
   DV_CUDA_TRY(cudaStreamSynchronize(st_));
   DV_CUDA_TRY(cudaGetLastError());
-  double x = gn[0], y = vn[0];
-  for (int i = 1; i < nc; ++i) {
-    x = std::min(x, gn[i]);
-    y = std::min(y, vn[i]);
-  }
+  double x = h_red_[4], y = h_red_[5];
   if (x > 0) x = 0;
   if (y > 0) y = 0;
   out4[0] = x;

@@ -119,10 +119,14 @@ class Engine {
 
   // Download helpers (synchronous).
   int download(void* dst, const void* src, size_t bytes);
-  int download_planes(const double* dev, size_t stride, int k, int first, int n,
-                      std::vector<double>& out);  // out: k x n
-  int download_planes_f(const float* dev, size_t stride, int k, int first, int n,
-                        std::vector<double>& out);
+  // k planes of n values (stride apart, from item `first`) as n rows of k.
+  int copy_rows_out(const double* planes, size_t stride, size_t first, int n, int k, double* out);
+  // Contact quantities in the reference's layouts, interleaved on the device:
+  // normal and gap (4 per contact), the Schur vector (3), and the forces per
+  // contact of segment s (3 each; either may be null).
+  int copy_normals_out(int c0, int nc, double* nP);
+  int copy_schur_vector_out(int c0, int nc, double* r);
+  int copy_contact_forces_out(int s, double* normal, double* friction);
 
   // System::getCCPViolation (System.cu:1590-1643) and the energies
   // (System.cu:1645-1658) of segment s, with the solver's reduction order.
@@ -150,6 +154,10 @@ class Engine {
   template <class T>
   void dfree(T*& p);
   int alloc_contacts(size_t cap);
+  int ensure_stage(size_t n);
+  int rows_to_stage(const double* planes, size_t stride, size_t first, int n, int k, int width,
+                    int col);
+  int stage_to_gamma(int s, int n);
   int ensure_slots();
   int default_grid(int max_ctas) const;
   template <class T>
@@ -209,7 +217,7 @@ class Engine {
   std::vector<int> snap_gsize_;
   std::vector<double> snap_time_;
   std::vector<int> snap_time_index_;
-  // state transfer staging (3 doubles per body)
+  // staging of host transfers: bodies or contacts as rows
   double* stage3_ = nullptr;
   size_t stage3_cap_ = 0;
   // diagnostics scratch

@@ -41,12 +41,6 @@ namespace {
     if (rc_ != DV_OK) return rc_; \
   } while (0)
 
-// Interleaves k planes of n values into n rows of `width`.
-void interleave(const std::vector<double>& planes, int n, int k, double* out, int width) {
-  for (int i = 0; i < n; ++i)
-    for (int c = 0; c < k; ++c) out[(size_t)i * width + c] = planes[(size_t)c * n + i];
-}
-
 void absorb_records(dv_scene* s) {
   for (const StepRecord& r : s->E.records()) {
     dv_step_stats st;
@@ -206,18 +200,8 @@ DV_API int dv_get_contacts(dv_scene* s, uint32_t* a, uint32_t* b, double* nP, do
   if (nc == 0) return DV_OK;
   if (a) TRY(E.download(a, E.d.ida + c0, sizeof(uint32_t) * nc));
   if (b) TRY(E.download(b, E.d.idb + c0, sizeof(uint32_t) * nc));
-  std::vector<double> h;
-  if (nP) {
-    TRY(E.download_planes(E.d.F, E.d.ccap, 3, c0, nc, h));
-    interleave(h, nc, 3, nP, 4);
-    std::vector<double> g(nc);
-    TRY(E.download(g.data(), E.d.gap + c0, sizeof(double) * nc));
-    for (int i = 0; i < nc; ++i) nP[4 * (size_t)i + 3] = g[i];
-  }
-  if (loc) {
-    TRY(E.download_planes(E.d.loc, E.d.ccap, 3, c0, nc, h));
-    interleave(h, nc, 3, loc, 3);
-  }
+  if (nP) TRY(E.copy_normals_out(c0, nc, nP));
+  if (loc) TRY(E.copy_rows_out(E.d.loc, E.d.ccap, c0, nc, 3, loc));
   return DV_OK;
 }
 
@@ -226,10 +210,7 @@ DV_API int dv_get_frames(dv_scene* s, double* F) {
   Engine& E = s->E;
   TRY(E.sync_state());
   const int nc = E.seg_state(0).nc, c0 = E.seg_state(0).c0;
-  std::vector<double> h;
-  TRY(E.download_planes(E.d.F, E.d.ccap, 9, c0, nc, h));
-  interleave(h, nc, 9, F, 9);
-  return DV_OK;
+  return E.copy_rows_out(E.d.F, E.d.ccap, c0, nc, 9, F);
 }
 
 DV_API int dv_get_schur_vector(dv_scene* s, double* r) {
@@ -237,13 +218,7 @@ DV_API int dv_get_schur_vector(dv_scene* s, double* r) {
   Engine& E = s->E;
   TRY(E.sync_state());
   const int nc = E.seg_state(0).nc, c0 = E.seg_state(0).c0;
-  std::vector<double> h;
-  if (E.precision() == DV_PREC_MIXED)
-    TRY(E.download_planes_f(reinterpret_cast<const float*>(E.d.r), E.d.ccap, 3, c0, nc, h));
-  else
-    TRY(E.download_planes(E.d.r, E.d.ccap, 3, c0, nc, h));
-  interleave(h, nc, 3, r, 3);
-  return DV_OK;
+  return E.copy_schur_vector_out(c0, nc, r);
 }
 
 DV_API int dv_get_step_vectors(dv_scene* s, double* r, double* b, double* k) {
@@ -252,15 +227,8 @@ DV_API int dv_get_step_vectors(dv_scene* s, double* r, double* b, double* k) {
   TRY(E.sync_state());
   const int nc = E.seg_state(0).nc, c0 = E.seg_state(0).c0, nbil = E.num_bilateral(0);
   const double h = s->P.h;
-  std::vector<double> hv;
   if (r) {
-    if (nc) {
-      if (E.precision() == DV_PREC_MIXED)
-        TRY(E.download_planes_f(reinterpret_cast<const float*>(E.d.r), E.d.ccap, 3, c0, nc, hv));
-      else
-        TRY(E.download_planes(E.d.r, E.d.ccap, 3, c0, nc, hv));
-      interleave(hv, nc, 3, r + nbil, 3);
-    }
+    TRY(E.copy_schur_vector_out(c0, nc, r + nbil));
     if (nbil) TRY(E.download(r, E.d.bil_work + 10 * (size_t)E.d.nbil, sizeof(double) * nbil));
   }
   if (b) {
@@ -333,24 +301,7 @@ DV_API int dv_contact_forces_per_collision(dv_scene* s, double* normal, double* 
   if (!s) return DV_ERR_ARG;
   Engine& E = s->E;
   TRY(E.sync_state());
-  const int nc = E.seg_state(0).nc, c0 = E.seg_state(0).c0;
-  if (nc == 0) return DV_OK;
-  std::vector<double> F, g;
-  TRY(E.download_planes(E.d.F, E.d.ccap, 9, c0, nc, F));
-  int m = 0;
-  TRY(E.get_gamma(0, g, &m));
-  const double h = s->P.h;
-  for (int c = 0; c < nc; ++c) {
-    double g0 = c < m ? g[3 * (size_t)c] : 0.0, g1 = c < m ? g[3 * (size_t)c + 1] : 0.0,
-           g2 = c < m ? g[3 * (size_t)c + 2] : 0.0;
-    for (int k = 0; k < 3; ++k) {
-      double nn = F[(size_t)k * nc + c], u = F[(size_t)(3 + k) * nc + c],
-             v = F[(size_t)(6 + k) * nc + c];
-      if (normal) normal[3 * (size_t)c + k] = (g0 * nn) / h;
-      if (friction) friction[3 * (size_t)c + k] = (g1 * u + g2 * v) / h;
-    }
-  }
-  return DV_OK;
+  return E.copy_contact_forces_out(0, normal, friction);
 }
 
 DV_API int dv_get_step_stats(dv_scene* s, dv_step_stats* out) {
