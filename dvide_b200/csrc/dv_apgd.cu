@@ -62,14 +62,18 @@ namespace {
 // gamma_new, best = gamma_hat (-1 before the first accepted iterate), nw2 the
 // next iterate computed ahead.
 struct Solve {
-  double L, t, theta, theta_new, beta, yb;
+  double L, theta_new;
   double obj1, obj2, obj2_base, residual, objective, objN;
   double gdiff, ginv, gneg, L0;        // gd, 1 / gd, -(1 / gd)
   double step_ya, step_ym, step_nt;    // step pass: 1 + yb, -yb, -t
-  double prod_ya, prod_ym, prod_nt;    // look-ahead: 1 + beta, -beta, -(1 / (0.9 L))
+  double prod_ya, prod_ym, prod_nt;    // look-ahead: 1 + b, -b, -(1 / (0.9 L))
+  // the scalars after the product pass, formed ahead: after an accepted iterate
+  // (a_) and after a failed test (f_)
+  double a_theta, a_theta_new, a_beta, a_L, a_t, a_nt, f_L, f_t, f_nt;
   Cone<double> cone;
   Cone<float> conef;
   double sums[8];
+  int a_nw2_kept, a_nw2_best;  // the next look-ahead's buffer: gamma_hat kept, or gamma_new
   int k, restart, cur, prev, nw, nw2, best, yr, first, step;
   int backtracks, sweeps, iterations, rsel, since_best, done;
   unsigned err;
@@ -85,25 +89,20 @@ constexpr int kStallIterations = 50;
 
 // ---- controllers (thread 0 of every member, after fold_team) ----
 
-__device__ inline void pass_scalars(Solve& C) {
-  C.step_ya = 1.0 + C.yb;
-  C.step_ym = -C.yb;
-  C.step_nt = -C.t;
-  C.prod_ya = 1.0 + C.beta;
-  C.prod_ym = -C.beta;
-  C.prod_nt = -(1.0 / (0.9 * C.L));
-}
-
 __device__ __noinline__ void ctl_lipschitz(Solve& C, const SegParams& P, int nc, int cap,
                                            bool mixed) {
   const double L = sqrt(C.sums[0]) / C.L0;
   C.L = L;
-  C.t = 1.0 / L;
-  C.theta = 1.0;
   const double th = 1.0;
   const double tn = (-(th * th) + th * sqrt(th * th + 4.0)) / 2.0;
   C.theta_new = tn;
-  C.beta = th * (1.0 - th) / (th * th + tn);
+  const double beta = th * (1.0 - th) / (th * th + tn);
+  C.step_ya = 1.0;  // y_0 = gamma_0
+  C.step_ym = -0.0;
+  C.step_nt = -(1.0 / L);
+  C.prod_ya = 1.0 + beta;
+  C.prod_ym = -beta;
+  C.prod_nt = -(1.0 / (0.9 * L));
   C.residual = 10e30;
   C.objective = 0.0;
   // APGD.cu:92: 1 / (contacts + bilateral rows)^2
@@ -123,7 +122,6 @@ __device__ __noinline__ void ctl_lipschitz(Solve& C, const SegParams& P, int nc,
   C.best = -1;
   C.nw2 = free_slot(1, 0, -1, -1);
   C.yr = 1;
-  C.yb = 0.0;
   C.first = 1;
   C.backtracks = 0;
   C.obj1 = 0.0;
@@ -135,7 +133,6 @@ __device__ __noinline__ void ctl_lipschitz(Solve& C, const SegParams& P, int nc,
   C.done = cap <= 0 ? 1 : 0;
   C.cone = make_cone<double>(P.mu);
   if (mixed) C.conef = make_cone<float>((float)P.mu);
-  pass_scalars(C);
 }
 
 __device__ __noinline__ void ctl_step(Solve& C) {
@@ -149,6 +146,26 @@ __device__ __noinline__ void ctl_step(Solve& C) {
   C.restart = (C.sums[2] > 0) ? 1 : 0;
   C.first = 0;
   C.step = 0;
+}
+
+// Formed by one thread while the barrier before the product pass waits: every
+// value that does not depend on the pass's sums (a square root and four
+// divisions in a row otherwise stand between the sums and the next pass).
+__device__ __noinline__ void ctl_ahead(Solve& C) {
+  const double th = C.restart ? 1.0 : C.theta_new;
+  const double tn = (-(th * th) + th * sqrt(th * th + 4.0)) / 2.0;
+  C.a_theta = th;
+  C.a_theta_new = tn;
+  C.a_beta = th * (1.0 - th) / (th * th + tn);
+  const double aL = 0.9 * C.L, fL = 2.0 * C.L;
+  C.a_L = aL;
+  C.a_t = 1.0 / aL;
+  C.a_nt = -(1.0 / (0.9 * aL));
+  C.f_L = fL;
+  C.f_t = 1.0 / fL;
+  C.f_nt = -(1.0 / (0.9 * fL));
+  C.a_nw2_kept = free_slot(C.nw2, C.nw, C.cur, C.best);
+  C.a_nw2_best = free_slot(C.nw2, C.nw, C.cur, C.nw);
 }
 
 __device__ __noinline__ void ctl_product(Solve& C, const SegParams& P, int cap, bool mixed, bool ar) {
@@ -169,20 +186,22 @@ __device__ __noinline__ void ctl_product(Solve& C, const SegParams& P, int cap, 
       finished = true;
     } else {
       C.backtracks += 1;
-      C.L = 2.0 * C.L;
-      C.t = 1.0 / C.L;
+      C.L = C.f_L;
+      C.step_nt = -C.f_t;
+      C.prod_nt = C.f_nt;
       C.step = 1;
     }
   } else {
     C.sweeps += 1;
-    const int best = C.best;
     C.since_best += 1;
+    bool better = false;
     if (res < C.residual) {
       C.residual = res;
       C.objective = obj1;
       if (ar) C.objN = 0.5 * C.sums[0];
       C.best = C.nw;
       C.since_best = 0;
+      better = true;
     }
     if (C.residual < P.tol) {
       finished = true;
@@ -194,31 +213,30 @@ __device__ __noinline__ void ctl_product(Solve& C, const SegParams& P, int cap, 
       // APGD.cu:335-345 after this iteration: r moves to the plane the
       // product pass wrote for the look-ahead
       if (ar) C.rsel ^= 1;
-      const double th = C.restart ? 1.0 : C.theta_new;
-      C.yb = C.beta;
+      // y of the next step pass is this pass's look-ahead y
+      C.step_ya = C.prod_ya;
+      C.step_ym = C.prod_ym;
       C.yr = C.restart;
-      const double L = 0.9 * C.L;
-      C.L = L;
-      C.t = 1.0 / L;
-      C.theta = th;
-      const int cur = C.nw, nw = free_slot(C.nw, C.cur, C.prev, best);
+      C.L = C.a_L;
+      C.step_nt = -C.a_t;
+      C.prod_nt = C.a_nt;
       C.prev = C.cur;
-      C.cur = cur;
-      C.nw = nw;
-      C.nw2 = free_slot(nw, cur, C.prev, C.best);
+      C.cur = C.nw;
+      C.nw = C.nw2;
+      C.nw2 = better ? C.a_nw2_best : C.a_nw2_kept;
       k += 1;
       C.k = k;
       if (k >= cap) {
         finished = true;
       } else {
-        const double tn = (-(th * th) + th * sqrt(th * th + 4.0)) / 2.0;
-        C.theta_new = tn;
-        C.beta = th * (1.0 - th) / (th * th + tn);
+        C.theta_new = C.a_theta_new;
+        C.prod_ya = 1.0 + C.a_beta;
+        C.prod_ym = -C.a_beta;
         // the look-ahead step is now iteration k's step
         const double ob = 0.5 * C.sums[5] + C.sums[6];
         C.obj2_base = ob;
         const double nr = sqrt(C.sums[3]);
-        C.obj2 = ob + (C.sums[2] + 0.5 * L * (nr * nr));
+        C.obj2 = ob + (C.sums[2] + 0.5 * C.L * (nr * nr));
         C.restart = (C.sums[4] > 0) ? 1 : 0;
       }
     }
@@ -227,7 +245,6 @@ __device__ __noinline__ void ctl_product(Solve& C, const SegParams& P, int cap, 
     C.iterations = k;
     C.done = 1;
   }
-  pass_scalars(C);
 }
 
 // ---- blocks of 32 contacts ----
@@ -341,6 +358,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
   __shared__ double scratch[64];
   __shared__ Solve C;
   __shared__ Team tm;
+  __shared__ BodyCache bodies;
   __shared__ ParkBuf park;
   __shared__ PhaseTimer timer;
   __shared__ int s_seen, s_copy_fail;
@@ -412,6 +430,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
     }
 
     if (live) {
+      fill_body_cache(a, tm, bodies);
       if (!sync(kPhaseSetup, true)) return;
 
       // ---- r = D (Minv k) + b; gamma_0 -> G[0]; e = gamma_0 - gamma_hat_0 (= gamma_0 - 1)
@@ -558,7 +577,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
       fold_team<1, false>(planes(), a.tcap, tm.nt, scratch, C.sums);
       if (threadIdx.x == 0) C.L0 = sqrt(C.sums[0]);
       parity ^= 1;
-      team_body_pass<T, kAR>(a, tm, wv, qv);
+      team_body_pass<T, kAR>(a, tm, bodies, wv, qv);
       if (!sync(kPhaseSetup)) return;
 
       // ---- L = ||N e|| / ||e||; q = F gamma_0 for the first N y
@@ -609,7 +628,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
       fold_team<1, false>(planes(), a.tcap, tm.nt, scratch, C.sums);
       if (threadIdx.x == 0) ctl_lipschitz(C, P, nc, cap, kMixed);
       parity ^= 1;
-      team_body_pass<T, kAR>(a, tm, wv, qv);
+      team_body_pass<T, kAR>(a, tm, bodies, wv, qv);
       if (!sync(kPhaseSetup)) return;
 
       // ---- APGD iterations (APGD.cu:227-350)
@@ -630,6 +649,41 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
           T* Xc = a.G[cur];
           const T* Xp = a.G[prev < 0 ? cur : prev];
           T* Xn = a.G[C.nw];
+          // A member of several tiles brings the constants and gamma_k with its
+          // product through the stages; of gamma_{k-1}, and with one tile of all
+          // (nothing would hide the copies), the lines of the next sub-tile go to L2.
+          const bool staged = tm.ntc > tm.m;
+          auto bring = [&](int j) {
+            const int t = team_tile(tm, tm.ntc, j >> 1);
+            const int kw = t * kTileItems + (j & 1) * kSub + warp * 32;
+            if (t < 0 || kw >= nc) return;
+            const size_t blk = (size_t)(c0 + kw) >> 5;
+            const auto lines = [&](const T* p, unsigned bytes) {
+              if (lane * 128u < bytes) prefetch_l2(reinterpret_cast<const unsigned char*>(p) + lane * 128);
+            };
+            if (!yr) lines(Xp + blk * kIterBlock, 2 * B::kHalfBytes);
+            if (!staged) {
+              lines(a.blk + blk * B::kConst, B::kConstBytes);
+              lines(Xc + blk * kIterBlock, 2 * B::kHalfBytes);
+            } else if (lane == 0) {
+              const int sidx = j & 1;
+              unsigned char* dst = stg.base + (size_t)(2 * warp + sidx) * B::kStageBytes;
+              uint64_t* bar = stg.bar + 2 * warp + sidx;
+              mark_stage_issued(stg, sidx);
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+              mbar_arrive_expect_tx(bar, B::kConstBytes + 2u * B::kHalfBytes);
+              bulk_g2s(dst, a.blk + blk * B::kConst, B::kConstBytes, bar);
+              bulk_g2s(dst + B::kConstBytes, Xc + blk * kIterBlock, 2 * B::kHalfBytes, bar);
+            }
+          };
+          if (staged) {
+            asm volatile("fence.proxy.async;" ::: "memory");
+            __syncwarp();
+            bring(0);
+          }
+          bring(1);
+          bool failed = false;
+          int j = 0;  // sub-tile of this member
           for (int i = 0;; ++i) {
             const int t = team_tile(tm, tm.nt, i);
             if (t < 0) break;
@@ -675,62 +729,66 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
                   }
                 }
               }
-            } else {
-              // the second item's lines into L2 while the first one computes
-              const int k = k0 + kThreads + threadIdx.x;
-              if (k < nc) {
-                const int c = c0 + k;
+            }
+            for (int m = 0; m < kItemsPerThread && kb < 0; ++m, ++j) {
+              const int sidx = j & 1;
+              if (j > 0 && !failed) {
+                __syncwarp();  // the warp's reads of the other stage are done
+                bring(j + 1);
+              }
+              const int kw = k0 + m * kSub + warp * 32;
+              const int k = kw + lane;
+              const int c = c0 + k;
+              T p0 = T(0), p1 = T(0), p2 = T(0), q0 = T(0), q1 = T(0), q2 = T(0);
+              if (k < nc && !yr) {
+                const T* xp = iter_at(Xp, c);
+                p0 = xp[0]; p1 = xp[32]; p2 = xp[64];
+                q0 = xp[96]; q1 = xp[128]; q2 = xp[160];
+              }
+              if (staged && kw < nc && !failed && !wait_warp_stage(a, stg, sidx)) {
+                failed = true;
+                s_copy_fail = 1;
+              }
+              if (k < nc && !failed) {
                 const T* p = const_at(a, c);
                 const T* x = iter_at(Xc, c);
-                const T* y = iter_at(Xp, c);
-#pragma unroll
-                for (int d = 0; d < 9; ++d) prefetch_l2(p + 32 * d);
-#pragma unroll
-                for (int d = 0; d < 6; ++d) {
-                  prefetch_l2(x + 32 * d);
-                  if (!yr) prefetch_l2(y + 32 * d);
+                if (staged) {
+                  p = reinterpret_cast<const T*>(stg.base + (size_t)(2 * warp + sidx) * B::kStageBytes) + lane;
+                  x = p + B::kConst;
                 }
-              }
-            }
-            for (int m = 0; m < kItemsPerThread && kb < 0; ++m) {
-              int k = k0 + m * kThreads + threadIdx.x;
-              if (k < nc) {
-                const int c = c0 + k;
-                const T* p = const_at(a, c);
-                T* xc = iter_at(Xc, c);
-                const T* xp = iter_at(Xp, c);
                 const Frame<T> f = block_frame<T>(p);
-                T c0v = xc[0], c1v = xc[32], c2v = xc[64];
+                const T c0v = x[0], c1v = x[32], c2v = x[64];
                 T y0, y1, y2, N0, N1, N2;
                 if (yr) {
                   y0 = c0v; y1 = c1v; y2 = c2v;
                 } else {
-                  y0 = ya * c0v + ym * xp[0];
-                  y1 = ya * c1v + ym * xp[32];
-                  y2 = ya * c2v + ym * xp[64];
+                  y0 = ya * c0v + ym * p0;
+                  y1 = ya * c1v + ym * p1;
+                  y2 = ya * c2v + ym * p2;
                 }
                 if (first) {
                   const uint2 id = block_ids(a, c);
                   V wa = load_vec(wv + id.x), wb = load_vec(wv + id.y);
                   ft_times<T, V>(f, wa, wb, &N0, &N1, &N2);
+                  T* xc = iter_at(Xc, c);
                   xc[96] = N0; xc[128] = N1; xc[160] = N2;
                 } else if (yr) {
-                  N0 = xc[96]; N1 = xc[128]; N2 = xc[160];
+                  N0 = x[96]; N1 = x[128]; N2 = x[160];
                 } else {
-                  N0 = ya * xc[96] + ym * xp[96];
-                  N1 = ya * xc[128] + ym * xp[128];
-                  N2 = ya * xc[160] + ym * xp[160];
+                  N0 = ya * x[96] + ym * q0;
+                  N1 = ya * x[128] + ym * q1;
+                  N2 = ya * x[160] + ym * q2;
                 }
-                T r0 = kAR ? (T)a.ar_r0[(size_t)C.rsel * S + c] : p[192];
-                T r1 = p[224], r2 = p[256];
-                T g0 = N0 + r0, g1 = N1 + r1, g2 = N2 + r2;
+                const T r0 = kAR ? (T)a.ar_r0[(size_t)C.rsel * S + c] : p[192];
+                const T r1 = p[224], r2 = p[256];
+                const T g0 = N0 + r0, g1 = N1 + r1, g2 = N2 + r2;
                 T x0 = y0 + nt_ * g0, x1 = y1 + nt_ * g1, x2 = y2 + nt_ * g2;
                 project_cone<T>(x0, x1, x2, cone_of<T>(C));
                 T* xn = iter_at(Xn, c);
                 xn[0] = x0; xn[32] = x1; xn[64] = x2;
                 store_keep(qv + c, f_times<T, V>(f, x0, x1, x2));
-                T t0 = x0 + T(-1) * y0, t1 = x1 + T(-1) * y1, t2 = x2 + T(-1) * y2;
-                T s0 = x0 + T(-1) * c0v, s1 = x1 + T(-1) * c1v, s2 = x2 + T(-1) * c2v;
+                const T t0 = x0 + T(-1) * y0, t1 = x1 + T(-1) * y1, t2 = x2 + T(-1) * y2;
+                const T s0 = x0 + T(-1) * c0v, s1 = x1 + T(-1) * c1v, s2 = x2 + T(-1) * c2v;
                 acc[0] = acc[0] + dot3i(g0, g1, g2, t0, t1, t2);
                 acc[1] = acc[1] + dot3i(t0, t1, t2, t0, t1, t2);
                 acc[2] = acc[2] + dot3i(g0, g1, g2, s0, s1, s2);
@@ -747,6 +805,10 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
             }
           }
           fold_parked8<false>(park, planes(), a.tcap, nslot);
+          if (s_copy_fail) {
+            drain_warp_stages(stg, &a.ew->wait_limit_ns);
+            return;
+          }
           if (!sync(kPhaseStep)) return;
           fold_team<5, false>(planes(), a.tcap, tm.nt, scratch, C.sums);
           if (threadIdx.x == 0) ctl_step(C);
@@ -776,16 +838,19 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
           }
         };
         // this warp's earlier writes of the iterates, and its reads of the
-        // stages, come before the copies
+        // stages, come before the copies (once for the pass: a fence of global
+        // memory waits for the warp's stores)
         asm volatile("fence.proxy.async;" ::: "memory");
         __syncwarp();
         issue(0);
         issue(1);
-        team_body_pass<T, kAR>(a, tm, wv, qv);
-        if (!sync(kPhaseBody)) {
+        team_body_pass<T, kAR>(a, tm, bodies, wv, qv);
+        if (!team_sync(a, tm, false, [&]() { ctl_ahead(C); })) {
           drain_warp_stages(stg, &a.ew->wait_limit_ns);
           return;
         }
+
+        timer.mark(a, kPhaseBody);
 
         // N gamma_new, objective (APGD.cu:237-238), residual (:90-102); then the
         // next iteration's step assuming gamma_new is accepted (:266-273, 312-332)
@@ -801,7 +866,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
             const int sidx = j & 1;
             if (j && !failed) {
               __syncwarp();  // the warp's reads of stage sidx^1 are done
-              asm volatile("fence.proxy.async;" ::: "memory");
+              if (lane == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
               issue(j + 1);
             }
             const int kw = t * kTileItems + sidx * kSub + warp * 32;

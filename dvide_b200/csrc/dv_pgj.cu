@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
   __shared__ double scratch[kNQ * 8 + 8];
   __shared__ DeferBuf s_def;
   __shared__ Team tm;
+  __shared__ BodyCache bodies;
   __shared__ PhaseTimer timer;
   __shared__ PgjSolve C;
   __shared__ int s_seen;
@@ -108,6 +109,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
     }
 
     if (live) {
+      fill_body_cache(a, tm, bodies);
       if (!sync(kPhaseSetup, true)) return;
       // ---- r = D (Minv k) + b; gamma_0 = (1, 0, 0) -> G[0]; B; q = F gamma_0
       for (int i = 0;; ++i) {
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
       // ---- iterations: one body pass (w of q = F gamma_k) and one contact pass
       // (N gamma_k, residual terms of gamma_k, step to gamma_{k+1}) each
       while (!C.done) {
-        team_body_pass<T, false>(a, tm, wv, qv);
+        team_body_pass<T, false>(a, tm, bodies, wv, qv);
         if (!sync(kPhaseBody)) return;
         int nslot = 0;
         const int kk = C.k;

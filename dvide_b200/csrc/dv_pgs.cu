@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
   __shared__ double scratch[kNQ * 8 + 8];
   __shared__ DeferBuf s_def;
   __shared__ Team tm;
+  __shared__ BodyCache bodies;
   __shared__ PhaseTimer timer;
   __shared__ PgsSolve C;
   __shared__ int s_seen;
@@ -193,6 +194,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
     }
 
     if (live) {
+      fill_body_cache(a, tm, bodies);
       if (!sync(kPhaseSetup, true)) return;
       // ---- r = D (Minv k) + b; gamma_0 = (1, 0, 0) -> G[0]; B; q = F gamma_0
       const int shift = a.sst[s].delta;
@@ -287,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
           }
           if (__ldcg(&a.sst[s].ctl.mode) == 0) break;
         }
-        team_body_pass<double, false>(a, tm, wv, qv);
+        team_body_pass<double, false>(a, tm, bodies, wv, qv);
         if (!sync(kPhaseBody)) return;
         int nslot = 0;
         for (int i = 0;; ++i) {

@@ -62,9 +62,14 @@ __device__ inline void red_add(unsigned* p, unsigned v) {
 // polls after it.  False after a time limit or another CTA's.  The first
 // barrier of a team (`joining`) may wait for members that are still busy with
 // earlier scenes: there the limit starts again while any team makes progress.
-template <class K>
-__device__ inline bool team_sync(const K& a, Team& t, bool joining = false) {
+// Meanwhile one thread of another warp runs `other`.
+struct Nothing {
+  __device__ void operator()() const {}
+};
+template <class K, class Fn = Nothing>
+__device__ inline bool team_sync(const K& a, Team& t, bool joining = false, Fn other = Fn{}) {
   __syncthreads();
+  if (threadIdx.x == 32) other();
   if (threadIdx.x == 0) {
     if (a.nseg > 1 && t.rank == 0) red_add(&a.ew->progress, 1u);
     if (t.m > 1) {
@@ -296,20 +301,40 @@ __device__ __noinline__ void fold_team(const double* part, int tcap, int nt, dou
   __syncwarp();  // warp 0 runs the controller
 }
 
-// Body pass of a member: w_b = minv_b (D^T x)_b for its bodies.  Heads load two
-// rounds ahead and each body's first eight incidence entries one round ahead,
-// while the current round gathers.
+// The heads and first eight incidence entries of a member's first 256 bodies,
+// one per thread, kept for all body passes of a solve: they do not change, and
+// reading them is two trips to L2 that the gathers of q wait for.
+struct BodyCache {
+  double mi[kThreads];
+  int s[kThreads], e[kThreads];
+  uint32_t c[8][kThreads];
+};
+template <class K>
+__device__ inline void fill_body_cache(const K& a, const Team& t, BodyCache& k) {
+  const int b = t.w0 + threadIdx.x;
+  BodyHead h{0.0, 0, 0};
+  if (b < t.w1) h = body_head(a, b);
+  k.mi[threadIdx.x] = h.mi;
+  k.s[threadIdx.x] = h.s;
+  k.e[threadIdx.x] = h.e;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) k.c[j][threadIdx.x] = (h.s + j < h.e) ? __ldg(a.inc + h.s + j) : 0u;
+}
+
+// Body pass of a member: w_b = minv_b (D^T x)_b for its bodies.  Past the kept
+// ones, heads load two rounds ahead and each body's first eight incidence
+// entries one round ahead, while the current round gathers.
 template <class T, bool kAR>
-__device__ inline void team_body_pass(const KArgs<T>& a, const Team& t, typename Vec4<T>::type* w,
-                                      const typename Vec4<T>::type* q) {
+__device__ inline void team_body_pass(const KArgs<T>& a, const Team& t, const BodyCache& k,
+                                      typename Vec4<T>::type* w, const typename Vec4<T>::type* q) {
   const int e = t.w1;
   int b = t.w0 + threadIdx.x;
-  BodyHead h{0.0, 0, 0}, hn{0.0, 0, 0};
-  if (b < e) h = body_head(a, b);
+  if (b >= e) return;
+  BodyHead h{k.mi[threadIdx.x], k.s[threadIdx.x], k.e[threadIdx.x]}, hn{0.0, 0, 0};
   if (b + kThreads < e) hn = body_head(a, b + kThreads);
   uint32_t c[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) c[j] = (h.s + j < h.e) ? __ldg(a.inc + h.s + j) : 0u;
+  for (int j = 0; j < 8; ++j) c[j] = k.c[j][threadIdx.x];
   for (; b < e; b += kThreads) {
     const int bnn = b + 2 * kThreads;
     BodyHead hnn{0.0, 0, 0};
