@@ -18,6 +18,8 @@
 //     segment's box list;
 //   * boxes tested against every body of their segment by a block-parallel
 //     compaction.
+// The pair kernels read spheres as (x, y, z, r) in cell order, one 32-byte
+// sector each: box, overlap test and narrowphase all come from it.
 // Each body's partners with larger id are sorted, so a segment's contacts come
 // out in lexicographic (A, B) order, the order of the reference's sorted unique
 // 64-bit pair keys (CollisionDetector.cu:319-325).  The narrowphase
@@ -26,7 +28,9 @@
 //
 // Sizes that change every step (contacts, tiles) are read on the device, so
 // the whole pipeline runs without a host round trip and can be captured in a
-// CUDA graph.  EngineWords::err is sticky: once set, every later kernel of the
+// CUDA graph.  Engines of at most kFewBodies bodies take short forms of it, one
+// CTA each, for everything before, between and after the pair kernels: there a
+// step of some fifty launches is bound by the launches themselves (2 us each).  EngineWords::err is sticky: once set, every later kernel of the
 // step returns at once.
 #include <stdio.h>
 
@@ -40,6 +44,7 @@ namespace {
 
 constexpr int kWarpsPerCta = kThreads / 32;
 constexpr int kMaxPerBody = 128;  // partners with larger id per sphere
+constexpr int kKeep = kKeepPartners;
 
 __device__ inline unsigned long long ordered_bits(double x) {
   unsigned long long u = (unsigned long long)__double_as_longlong(x);
@@ -78,16 +83,11 @@ __global__ void k_seg_reset(int nseg, GridInfo* __restrict__ grid, SegState* __r
 // CollisionDetector.cu:24-79 (rigid-body branch): aabb = pos -+ (extent +
 // envelope); per-segment AABB union by warp folds when the warp's bodies share
 // a segment, per-body atomics otherwise.
-__global__ void __launch_bounds__(kThreads) k_aabb(const double4* __restrict__ p4,
-                                                  const double4* __restrict__ g4,
-                                                  const int* __restrict__ bseg,
-                                                  const SegParams* __restrict__ seg, int nb,
-                                                  double4* __restrict__ amin,
-                                                  double4* __restrict__ amax,
-                                                  GridInfo* __restrict__ grid,
-                                                  const EngineWords* __restrict__ ew) {
-  if (ew->err) return;
-  const int i = blockIdx.x * kThreads + threadIdx.x;
+// One body per lane (whole warps; i past nb: no body).
+__device__ inline void body_aabb(int i, const double4* __restrict__ p4, const double4* __restrict__ g4,
+                                 const int* __restrict__ bseg, const SegParams* __restrict__ seg, int nb,
+                                 double4* __restrict__ amin, double4* __restrict__ amax,
+                                 GridInfo* __restrict__ grid) {
   const int lane = threadIdx.x & 31;
   int s = -1;
   unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0ull, 0ull, 0ull};
@@ -129,19 +129,27 @@ __global__ void __launch_bounds__(kThreads) k_aabb(const double4* __restrict__ p
   }
 }
 
+__global__ void __launch_bounds__(kThreads) k_aabb(const double4* __restrict__ p4,
+                                                  const double4* __restrict__ g4,
+                                                  const int* __restrict__ bseg,
+                                                  const SegParams* __restrict__ seg, int nb,
+                                                  double4* __restrict__ amin,
+                                                  double4* __restrict__ amax,
+                                                  GridInfo* __restrict__ grid,
+                                                  const EngineWords* __restrict__ ew) {
+  if (ew->err) return;
+  body_aabb(blockIdx.x * kThreads + threadIdx.x, p4, g4, bseg, seg, nb, amin, amax, grid);
+}
+
 // CollisionDetector.cu:566-568: origin = union min - 0.01; grid sized for the
 // widest sphere AABB of the segment, capped at its `cell_cap` cells (a wider
 // cell only adds candidates).
-__global__ void k_grid_setup(int nseg, const SegParams* __restrict__ seg,
-                             GridInfo* __restrict__ grid, const EngineWords* __restrict__ ew) {
-  if (ew->err) return;
-  int s = blockIdx.x * kThreads + threadIdx.x;
-  if (s >= nseg || !seg[s].active) return;
+__device__ inline void set_up_grid(int s, const SegParams* __restrict__ seg, GridInfo* grid) {
   GridInfo* g = grid + s;
   double lo[3], hi[3];
   for (int d = 0; d < 3; ++d) {
-    lo[d] = from_ordered(g->lo[d]);
-    hi[d] = from_ordered(g->hi[d]);
+    lo[d] = from_ordered(__ldcg(&g->lo[d]));
+    hi[d] = from_ordered(__ldcg(&g->hi[d]));
   }
   g->ox = lo[0] - 0.01;
   g->oy = lo[1] - 0.01;
@@ -174,7 +182,25 @@ __global__ void k_grid_setup(int nseg, const SegParams* __restrict__ seg,
   g->ncells = dims[0] * dims[1] * dims[2];
 }
 
+__global__ void k_grid_setup(int nseg, const SegParams* __restrict__ seg,
+                             GridInfo* __restrict__ grid, const EngineWords* __restrict__ ew) {
+  if (ew->err) return;
+  int s = blockIdx.x * kThreads + threadIdx.x;
+  if (s < nseg && seg[s].active) set_up_grid(s, seg, grid);
+}
+
 __device__ inline int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
+
+__device__ inline int4 cell_of(double4 p, double4 geom, const SegParams& P, const GridInfo* g) {
+  double4 a, b;
+  aabb_of(p, geom, P.env, &a, &b);
+  a = make_double4(a.x - g->ox, a.y - g->oy, a.z - g->oz, 0.0);
+  const double iw = g->inv_w;
+  const int cx = clampi((int)floor(a.x * iw), 0, g->dx - 1);
+  const int cy = clampi((int)floor(a.y * iw), 0, g->dy - 1);
+  const int cz = clampi((int)floor(a.z * iw), 0, g->dz - 1);
+  return make_int4(cx, cy, cz, P.cell_base + cx + g->dx * (cy + g->dy * cz));
+}
 
 // CollisionDetector.cu:574: aabb -= origin.  Spheres also get their cell key;
 // spheres of inactive segments go to the parking cell `park`.
@@ -201,30 +227,33 @@ __global__ void __launch_bounds__(kThreads) k_shift_and_bin(
     int s = bseg[body];
     uint32_t key = (uint32_t)park;
     if (seg[s].active) {
-      const GridInfo* g = grid + s;
-      double4 a, b;
-      aabb_of(p4[body], g4[body], seg[s].env, &a, &b);
-      a = make_double4(a.x - g->ox, a.y - g->oy, a.z - g->oz, 0.0);
-      double iw = g->inv_w;
-      int cx = clampi((int)floor(a.x * iw), 0, g->dx - 1);
-      int cy = clampi((int)floor(a.y * iw), 0, g->dy - 1);
-      int cz = clampi((int)floor(a.z * iw), 0, g->dz - 1);
-      int id = seg[s].cell_base + cx + g->dx * (cy + g->dy * cz);
-      cell[body] = make_int4(cx, cy, cz, id);
-      key = (uint32_t)id;
+      const int4 c = cell_of(p4[body], g4[body], seg[s], grid + s);
+      cell[body] = c;
+      key = (uint32_t)c.w;
     }
     keys[i] = key;
     vals[i] = (uint32_t)body;
   }
 }
 
+__device__ inline double4 sphere_of(const double4* __restrict__ p4, const double4* __restrict__ g4,
+                                    int body) {
+  const double4 p = p4[body];
+  return make_double4(p.x, p.y, p.z, g4[body].x);
+}
+
 __global__ void __launch_bounds__(kThreads) k_cell_ranges(const uint32_t* __restrict__ keys,
-                                                         int n, int* __restrict__ cstart,
+                                                         const uint32_t* __restrict__ bodies, int n,
+                                                         int* __restrict__ cstart,
                                                          int* __restrict__ cend, int ncap,
+                                                         const double4* __restrict__ p4,
+                                                         const double4* __restrict__ g4,
+                                                         double4* __restrict__ spheres,
                                                          const EngineWords* __restrict__ ew) {
   if (ew->err) return;
   int j = blockIdx.x * kThreads + threadIdx.x;
   if (j >= n) return;
+  spheres[j] = sphere_of(p4, g4, (int)bodies[j]);
   uint32_t k = keys[j];
   if (k >= (uint32_t)ncap) return;
   if (j == 0 || keys[j - 1] != k) cstart[k] = j;
@@ -313,6 +342,8 @@ struct CollideArgs {
   const int* small_ids;
   const int* large_ids;
   const uint32_t* sorted_bodies;  // small bodies sorted by cell
+  const double4* spheres;         // (x, y, z, r) in the same order
+  uint32_t* kept;                 // kKeep partners per small body, from the count pass
   const int* cstart;
   const int* cend;
   const GridInfo* grid;
@@ -350,120 +381,162 @@ __device__ inline void write_contact(const CollideArgs& a, size_t c, int ia, int
   a.loc[2 * S + c] = o.loc.z;
 }
 
-// One warp per sphere A: partners B > A from the 27 neighbour cells (lane =
-// cell) and from the segment's box list (lanes 27..31).  kWrite = false
-// counts, kWrite = true emits the sorted partner list at the body's slot.
-template <bool kWrite>
-__global__ void __launch_bounds__(kThreads) k_sphere_pairs(CollideArgs a) {
-  __shared__ int s_buf[kWarpsPerCta][kMaxPerBody];
-  __shared__ int s_cnt[kWarpsPerCta];
-  if (a.ew->err) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int j = blockIdx.x * kWarpsPerCta + warp;
-  if (j >= a.n_small) return;
-  const int A = a.small_ids[j];
-  const int sg = a.bseg[A];
+// Two spheres (CollisionDetector.cu:187-331, 333-501, the sphere-sphere case).
+__device__ inline bool spheres_touch(d3 pa, double ra, d3 pb, double rb, double env, bool exact) {
+  return (ra + rb) - length3x(sub3(pb, pa), exact) >= -env;
+}
+
+// Partners B > A of sphere A, found by a warp: lanes 0..26 scan a neighbour
+// cell each, lanes 27..31 the segment's box list.  The first kMaxPerBody go to
+// buf in no order; returns their number and the candidates' (both summed over
+// the warp).
+__device__ inline int find_partners(const CollideArgs& a, int A, int sg, int* buf, int* cnt, int* ncand) {
+  const int lane = threadIdx.x & 31;
   const SegParams& P = a.seg[sg];
-  if (!P.active) return;
-  if (kWrite && a.cnt_cont[A] > kMaxPerBody) return;  // k_sphere_pairs_wide's
   const double env = P.env;
   const bool exact = P.exact != 0;
-  if (lane == 0) s_cnt[warp] = 0;
+  if (lane == 0) *cnt = 0;
   __syncwarp();
-  int ncand = 0, ncont = 0;
+  int nc = 0;
   if (lane < 27) {
-    int4 cA = a.cell[A];
-    int x = cA.x + (lane % 3) - 1, y = cA.y + ((lane / 3) % 3) - 1, z = cA.z + (lane / 9) - 1;
+    const int4 cA = a.cell[A];
+    const int x = cA.x + (lane % 3) - 1, y = cA.y + ((lane / 3) % 3) - 1, z = cA.z + (lane / 9) - 1;
     const GridInfo* g = a.grid + sg;
     if (x >= 0 && y >= 0 && z >= 0 && x < g->dx && y < g->dy && z < g->dz) {
-      int id = P.cell_base + x + g->dx * (y + g->dy * z);
+      const int id = P.cell_base + x + g->dx * (y + g->dy * z);
       int s = a.cstart[id];
       if (s >= 0) {
-        int e = a.cend[id];
+        const int e = a.cend[id];
+        const double4 A0 = a.amin[A], A1 = a.amax[A];
+        const double4 p = a.p4[A];
+        const d3 pA = mk3(p.x, p.y, p.z);
+        const double rA = a.g4[A].x;
+        const int fa = a.fam[A];
+        const double ox = g->ox, oy = g->oy, oz = g->oz;
         for (; s < e; ++s) {
-          int B = (int)a.sorted_bodies[s];
+          const int B = (int)a.sorted_bodies[s];
           if (B <= A) continue;
-          if (!is_candidate(a.amin, a.amax, a.fam, A, B)) continue;
-          ++ncand;
-          NpOut o;
-          if (narrowphase(a.p4, a.g4, A, B, env, exact, &o)) {
-            ++ncont;
-            if (kWrite) {
-              int slot = atomicAdd(&s_cnt[warp], 1);
-              if (slot < kMaxPerBody) s_buf[warp][slot] = B;
-            }
+          // CollisionDetector.cu:124-130 / 161-167, the partner's box from its sphere
+          const double4 q = a.spheres[s];
+          const double ex = q.w + env;
+          const bool in =
+              (A0.x <= (q.x + ex) - ox && (q.x - ex) - ox <= A1.x) &&
+              (A0.y <= (q.y + ex) - oy && (q.y - ex) - oy <= A1.y) &&
+              (A0.z <= (q.z + ex) - oz && (q.z - ex) - oz <= A1.z);
+          if (!in || (fa != -1 && fa == a.fam[B])) continue;
+          ++nc;
+          if (spheres_touch(pA, rA, mk3(q.x, q.y, q.z), q.w, env, exact)) {
+            const int slot = atomicAdd(cnt, 1);
+            if (slot < kMaxPerBody) buf[slot] = B;
           }
         }
       }
     }
   } else {
     for (int m = P.l0 + lane - 27; m < P.l1; m += 5) {
-      int B = a.large_ids[m];
+      const int B = a.large_ids[m];
       if (B <= A) continue;
       if (!is_candidate(a.amin, a.amax, a.fam, A, B)) continue;
-      ++ncand;
+      ++nc;
       NpOut o;
       if (narrowphase(a.p4, a.g4, A, B, env, exact, &o)) {
-        ++ncont;
-        if (kWrite) {
-          int slot = atomicAdd(&s_cnt[warp], 1);
-          if (slot < kMaxPerBody) s_buf[warp][slot] = B;
-        }
+        const int slot = atomicAdd(cnt, 1);
+        if (slot < kMaxPerBody) buf[slot] = B;
       }
     }
   }
-  if (!kWrite) {
-    for (int off = 16; off >= 1; off >>= 1) {
-      ncand += __shfl_down_sync(0xffffffffu, ncand, off);
-      ncont += __shfl_down_sync(0xffffffffu, ncont, off);
-    }
-    if (lane == 0) {
-      a.cnt_cand[A] = ncand;
-      a.cnt_cont[A] = ncont;
-      // more partners than this kernel lists: k_sphere_pairs_wide writes them
-      if (ncont > kMaxPerBody) {
-        const int k = atomicAdd(&a.ew->n_wide, 1);
-        if (k < kWideSpheres && ncont <= kWidePartners) {
-          a.wide_ids[k] = A;
-        } else {
-          atomicOr(&a.ew->err, kErrPartners);
-          atomicOr(&a.sst[sg].err, kErrPartners);  // whose scene (a server retires it)
-        }
-      }
-      if (ncand) {
-        atomicAdd(&a.sst[sg].npossible, ncand);
-        atomicAdd(&a.ew->npossible, ncand);
-      }
-    }
-    return;
-  }
+  *ncand = (int)__reduce_add_sync(0xffffffffu, (unsigned)nc);
   __syncwarp();
-  int n = s_cnt[warp];
-  if (n > kMaxPerBody) n = kMaxPerBody;
-  // rank sort of the (distinct) partner ids, then emit in ascending order
-  int mine[kMaxPerBody / 32];
-  int rk[kMaxPerBody / 32];
-#pragma unroll
-  for (int t = 0; t < kMaxPerBody / 32; ++t) {
-    int e = lane + 32 * t;
-    mine[t] = (e < n) ? s_buf[warp][e] : 0x7fffffff;
-    rk[t] = 0;
+  return *cnt;
+}
+
+// Count pass, one warp per sphere; up to kKeep partners (in a settled pile 3.7
+// on average) are kept in ascending order for the write pass, which otherwise
+// would search again.  On 200,000 settled spheres the two passes took 369 and 451
+// us when each read boxes and spheres body by body, and take 306 and 95.
+__global__ void __launch_bounds__(kThreads) k_sphere_count(CollideArgs a) {
+  __shared__ int s_buf[kWarpsPerCta][kMaxPerBody];
+  __shared__ int s_cnt[kWarpsPerCta];
+  if (a.ew->err) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int j = blockIdx.x * kWarpsPerCta + warp;
+  if (j >= a.n_small) return;
+  const int A = a.small_ids[j];
+  const int sg = a.bseg[A];
+  if (!a.seg[sg].active) return;
+  int ncand;
+  const int n = find_partners(a, A, sg, s_buf[warp], &s_cnt[warp], &ncand);
+  if (n <= kKeep) {
+    const int mine = lane < n ? s_buf[warp][lane] : 0x7fffffff;
+    int rank = 0;
+    for (int e = 0; e < n; ++e) rank += s_buf[warp][e] < mine ? 1 : 0;
+    if (lane < n) a.kept[(size_t)j * kKeep + rank] = (uint32_t)mine;
   }
-  for (int e = 0; e < n; ++e) {
-    int other = s_buf[warp][e];
-#pragma unroll
-    for (int t = 0; t < kMaxPerBody / 32; ++t) rk[t] += (other < mine[t]) ? 1 : 0;
+  if (lane == 0) {
+    a.cnt_cand[A] = ncand;
+    a.cnt_cont[A] = n;
+    // more partners than the write pass lists: k_sphere_pairs_wide writes them
+    if (n > kMaxPerBody) {
+      const int k = atomicAdd(&a.ew->n_wide, 1);
+      if (k < kWideSpheres && n <= kWidePartners) {
+        a.wide_ids[k] = A;
+      } else {
+        atomicOr(&a.ew->err, kErrPartners);
+        atomicOr(&a.sst[sg].err, kErrPartners);  // whose scene (a server retires it)
+      }
+    }
+    if (ncand) {
+      atomicAdd(&a.sst[sg].npossible, ncand);
+      atomicAdd(&a.ew->npossible, ncand);
+    }
   }
-  __syncwarp();
-  size_t base = (size_t)(a.cbase[A] + a.sst[sg].delta);
-#pragma unroll
-  for (int t = 0; t < kMaxPerBody / 32; ++t) {
-    int e = lane + 32 * t;
-    if (e < n) {
+}
+
+// Write pass, eight lanes per sphere: the contacts of the kept partners at the
+// sphere's slot.  A sphere with more than kKeep and at most kMaxPerBody
+// partners is searched again by its whole warp.
+__global__ void __launch_bounds__(kThreads) k_sphere_write(CollideArgs a) {
+  __shared__ int s_buf[kWarpsPerCta][kMaxPerBody];
+  __shared__ int s_cnt[kWarpsPerCta];
+  if (a.ew->err) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int j0 = (blockIdx.x * kWarpsPerCta + warp) * 4;
+  if (j0 >= a.n_small) return;
+  const int j = j0 + (lane >> 3);
+  int A = -1, sg = 0, n = 0;
+  if (j < a.n_small) {
+    A = a.small_ids[j];
+    sg = a.bseg[A];
+    if (a.seg[sg].active) n = a.cnt_cont[A];
+  }
+  if (n > 0 && n <= kKeep) {
+    const SegParams& P = a.seg[sg];
+    const size_t base = (size_t)(a.cbase[A] + a.sst[sg].delta);
+    for (int e = lane & 7; e < n; e += 8) {
+      const int B = (int)a.kept[(size_t)j * kKeep + e];
       NpOut o;
-      narrowphase(a.p4, a.g4, A, mine[t], env, exact, &o);
-      write_contact(a, base + rk[t], A, mine[t], o, exact);
+      narrowphase(a.p4, a.g4, A, B, P.env, P.exact != 0, &o);
+      write_contact(a, base + e, A, B, o, P.exact != 0);
     }
+  }
+  unsigned more = __ballot_sync(0xffffffffu, n > kKeep && n <= kMaxPerBody && (lane & 7) == 0);
+  while (more) {
+    const int l = __ffs(more) - 1;
+    more &= more - 1;
+    const int A2 = __shfl_sync(0xffffffffu, A, l), sg2 = __shfl_sync(0xffffffffu, sg, l);
+    const SegParams& P = a.seg[sg2];
+    int ncand;
+    const int n2 = min(find_partners(a, A2, sg2, s_buf[warp], &s_cnt[warp], &ncand), kMaxPerBody);
+    const size_t base = (size_t)(a.cbase[A2] + a.sst[sg2].delta);
+    for (int e = lane; e < n2; e += 32) {
+      const int B = s_buf[warp][e];
+      int rank = 0;
+      for (int k = 0; k < n2; ++k) rank += s_buf[warp][k] < B ? 1 : 0;
+      NpOut o;
+      narrowphase(a.p4, a.g4, A2, B, P.env, P.exact != 0, &o);
+      write_contact(a, base + rank, A2, B, o, P.exact != 0);
+    }
+    __syncwarp();
   }
 }
 
@@ -623,18 +696,66 @@ __global__ void __launch_bounds__(kThreads) k_box_pairs(CollideArgs a, int* __re
   write_contact(a, pos, L, B, o, P.exact != 0);
 }
 
+// Binary search of the tile starts: the last segment with tstart <= t and tiles.
+__device__ inline int segment_of_tile(int nseg, const int* seg_tstart, int t) {
+  int lo = 0, hi = nseg - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (seg_tstart[mid] <= t) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// out[i] = sum of in(j), j < i; out[n] = the total.  One CTA of 1024 threads,
+// each with a run of consecutive items.
+template <class Fn>
+__device__ inline void scan_one_cta(int n, Fn in, int* out) {
+  __shared__ int s_w[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (n + 1023) / 1024, i0 = min(n, (int)threadIdx.x * per), i1 = min(n, i0 + per);
+  int sum = 0;
+  for (int i = i0; i < i1; ++i) sum += in(i);
+  int x = sum;
+  for (int off = 1; off < 32; off <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, off);
+    if (lane >= off) x += y;
+  }
+  __syncthreads();
+  if (lane == 31) s_w[warp] = x;
+  __syncthreads();
+  int at = x - sum;
+  for (int w = 0; w < warp; ++w) at += s_w[w];
+  if (threadIdx.x == 1023) out[n] = at + sum;
+  for (int i = i0; i < i1; ++i) {
+    const int v = in(i);
+    out[i] = at;
+    at += v;
+  }
+}
+
 // Contact layout: segment s gets nc_s = contacts of its bodies, slots
 // [c0, c0 + nc_s) with c0 a multiple of kContactAlign, tiles [t0, t0 + nt).
 // One CTA scans the segments in order.
+// kFew (engines of few bodies): the scans of the bodies' and box chunks' counts
+// before it and the tile table after it too.
+template <bool kFew>
 __global__ void __launch_bounds__(1024) k_seg_layout(int nseg, int nb,
                                                      const SegParams* __restrict__ seg,
-                                                     SegState* __restrict__ sst,
-                                                     const int* __restrict__ cbase,
+                                                     SegState* __restrict__ sst, int* cbase,
                                                      int* __restrict__ seg_tstart, size_t ccap,
-                                                     int tcap, EngineWords* __restrict__ ew) {
+                                                     int tcap, EngineWords* __restrict__ ew,
+                                                     const int* cnt_cont = nullptr,
+                                                     const int* chunk_cnt = nullptr,
+                                                     int* chunk_off = nullptr, int nchunks = 0,
+                                                     int* tseg = nullptr) {
   __shared__ long long s_c[32], s_t[32];
   __shared__ long long s_carry_c, s_carry_t;
   if (ew->err) return;
+  if (kFew) {
+    scan_one_cta(nb, [&](int i) { return cnt_cont[i]; }, cbase);
+    if (nchunks) scan_one_cta(nchunks, [&](int i) { return chunk_cnt[i]; }, chunk_off);
+    __syncthreads();
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     s_carry_c = 0;
@@ -695,21 +816,21 @@ __global__ void __launch_bounds__(1024) k_seg_layout(int nseg, int nb,
     ew->ntiles = (int)s_carry_t;
     if (s_carry_c > (long long)ccap || s_carry_t > (long long)tcap) atomicOr(&ew->err, kErrCapacity);
   }
+  if (kFew && s_carry_t <= (long long)tcap) {
+    __syncthreads();
+    const int nt = (int)s_carry_t;
+    for (int t = threadIdx.x; t < nt; t += 1024) tseg[t] = segment_of_tile(nseg, seg_tstart, t);
+  }
 }
 
-// tile -> segment (binary search of the tile starts)
+// tile -> segment
 __global__ void __launch_bounds__(kThreads) k_tile_table(int nseg, const int* __restrict__ seg_tstart,
                                                         int* __restrict__ tseg, int tcap,
                                                         const EngineWords* __restrict__ ew) {
   if (ew->err) return;
   const int nt = ew->ntiles;
   for (int t = blockIdx.x * kThreads + threadIdx.x; t < nt; t += gridDim.x * kThreads) {
-    int lo = 0, hi = nseg - 1;  // last segment with tstart <= t and tiles
-    while (lo < hi) {
-      int mid = (lo + hi + 1) >> 1;
-      if (seg_tstart[mid] <= t) lo = mid; else hi = mid - 1;
-    }
-    tseg[t] = lo;
+    tseg[t] = segment_of_tile(nseg, seg_tstart, t);
   }
 }
 
@@ -773,6 +894,134 @@ __global__ void __launch_bounds__(kThreads) k_inc_fill(int nb, const int* __rest
   }
 }
 
+// ---- engines of few bodies: one CTA of 1024 threads ----
+
+// Everything before the pair kernels: counters, AABBs, grids, and the spheres
+// by cell.  Within a cell the order is that of the atomics; the partners of a
+// sphere are sorted by id wherever they are listed.
+__global__ void __launch_bounds__(1024) k_front_few(
+    int nseg, int nb, const int* __restrict__ small_ids, int n_small, const int* __restrict__ bseg,
+    const SegParams* __restrict__ seg, const double4* __restrict__ p4, const double4* __restrict__ g4,
+    double4* amin, double4* amax, GridInfo* grid, int4* cell, int* cstart, int* cend, int ncell,
+    uint32_t* slot, uint32_t* __restrict__ sorted, double4* __restrict__ spheres,
+    int* __restrict__ cnt_cont, int* __restrict__ cnt_cand, SegState* __restrict__ sst, EngineWords* ew) {
+  if (ew->err) return;
+  const int tid = threadIdx.x;
+  for (int i = tid; i < nb; i += 1024) {
+    cnt_cont[i] = 0;
+    cnt_cand[i] = 0;
+  }
+  for (int i = tid; i < ncell; i += 1024) cend[i] = 0;
+  for (int s = tid; s < nseg; s += 1024) {
+    for (int d = 0; d < 3; ++d) {
+      grid[s].lo[d] = ~0ull;
+      grid[s].hi[d] = 0ull;
+    }
+    sst[s].nc = 0;
+    sst[s].npossible = 0;
+  }
+  if (tid == 0) {
+    ew->npossible = 0;
+    ew->n_wide = 0;
+  }
+  __syncthreads();
+  for (int i0 = 0; i0 < nb; i0 += 1024) body_aabb(i0 + tid, p4, g4, bseg, seg, nb, amin, amax, grid);
+  __syncthreads();
+  for (int s = tid; s < nseg; s += 1024)
+    if (seg[s].active) set_up_grid(s, seg, grid);
+  __syncthreads();
+  for (int i = tid; i < nb; i += 1024) {
+    const int s = bseg[i];
+    if (!seg[s].active) continue;
+    const GridInfo* g = grid + s;
+    const double ox = g->ox, oy = g->oy, oz = g->oz;
+    const double4 a = amin[i], b = amax[i];
+    amin[i] = make_double4(a.x - ox, a.y - oy, a.z - oz, 0.0);
+    amax[i] = make_double4(b.x - ox, b.y - oy, b.z - oz, 0.0);
+  }
+  for (int i = tid; i < n_small; i += 1024) {
+    const int body = small_ids[i], s = bseg[body];
+    int4 c = make_int4(0, 0, 0, ncell - 1);  // the parking cell of inactive segments
+    if (seg[s].active) c = cell_of(p4[body], g4[body], seg[s], grid + s);
+    cell[body] = c;
+    slot[i] = (uint32_t)atomicAdd(&cend[c.w], 1);
+  }
+  __syncthreads();
+  scan_one_cta(ncell, [&](int k) { return __ldcg(cend + k); }, cstart);
+  __syncthreads();
+  for (int k = tid; k < ncell; k += 1024) cend[k] = __ldcg(cend + k) + cstart[k];
+  for (int i = tid; i < n_small; i += 1024) {
+    const int body = small_ids[i];
+    const int at = cstart[cell[body].w] + (int)slot[i];
+    sorted[at] = (uint32_t)body;
+    spheres[at] = sphere_of(p4, g4, body);
+  }
+}
+
+// The incidence: per body its contacts as B, then as A, ascending.
+__global__ void __launch_bounds__(1024) k_incidence_few(
+    int nb, const uint32_t* __restrict__ idb, const int* __restrict__ tseg,
+    const SegState* __restrict__ sst, const int* __restrict__ bseg, const int* __restrict__ cbase,
+    const int* __restrict__ acnt, int* cnt, uint32_t* slot, uint32_t* scratch, int* istart, uint32_t* inc,
+    const EngineWords* __restrict__ ew) {
+  constexpr int kShort = 24;  // longest run that one thread sorts
+  __shared__ int s_long;
+  if (ew->err) return;
+  const int tid = threadIdx.x;
+  const int nt = ew->ntiles;
+  if (tid == 0) s_long = 0;
+  for (int b = tid; b < nb; b += 1024) cnt[b] = 0;
+  __syncthreads();
+  auto each_contact = [&](auto fn) {
+    for (int i = tid; i < nt * kTileItems; i += 1024) {
+      const int t = i / kTileItems;
+      const SegState& S = sst[tseg[t]];
+      const int k = (t - S.t0) * kTileItems + i % kTileItems;
+      if (k < S.nc) fn(S.c0 + k);
+    }
+  };
+  each_contact([&](int c) { slot[c] = (uint32_t)atomicAdd(&cnt[idb[c]], 1); });
+  __syncthreads();
+  scan_one_cta(nb, [&](int b) { return __ldcg(cnt + b) + acnt[b]; }, istart);
+  __syncthreads();
+  each_contact([&](int c) { inc[istart[idb[c]] + (int)slot[c]] = (uint32_t)c | 0x80000000u; });
+  __syncthreads();
+  for (int b = tid; b < nb; b += 1024) {
+    const int n = __ldcg(cnt + b), na = acnt[b];
+    uint32_t* run = inc + istart[b];
+    if (n > kShort) {
+      s_long = 1;
+    } else {
+      for (int i = 1; i < n; ++i) {
+        const uint32_t x = run[i];
+        int k = i - 1;
+        for (; k >= 0 && run[k] > x; --k) run[k + 1] = run[k];
+        run[k + 1] = x;
+      }
+    }
+    if (na) {
+      const int first = cbase[b] + sst[bseg[b]].delta;
+      for (int k = 0; k < na; ++k) run[n + k] = (uint32_t)(first + k);
+    }
+  }
+  __syncthreads();
+  if (!s_long) return;
+  for (int b = 0; b < nb; ++b) {  // long runs: the whole CTA, by rank
+    const int n = __ldcg(cnt + b);
+    if (n <= kShort) continue;
+    uint32_t* run = inc + istart[b];
+    for (int i = tid; i < n; i += 1024) scratch[i] = run[i];
+    __syncthreads();
+    for (int i = tid; i < n; i += 1024) {
+      const uint32_t x = scratch[i];
+      int rank = 0;
+      for (int k = 0; k < n; ++k) rank += scratch[k] < x ? 1 : 0;
+      run[rank] = x;
+    }
+    __syncthreads();
+  }
+}
+
 CollideArgs make_args(SceneDev& sd) {
   CollideArgs a;
   a.nb = sd.nb;
@@ -791,6 +1040,8 @@ CollideArgs make_args(SceneDev& sd) {
   a.small_ids = sd.small_ids;
   a.large_ids = sd.large_ids;
   a.sorted_bodies = sd.valA;
+  a.spheres = sd.spheres;
+  a.kept = sd.kept;
   a.cstart = sd.cell_start;
   a.cend = sd.cell_end;
   a.grid = sd.grid;
@@ -823,51 +1074,77 @@ void collide(SceneDev& sd, cudaStream_t st, int64_t* launches) {
   const int nb = sd.nb;
   if (nb == 0) return;
   const int park = sd.ncell_cap - 1;  // cell of spheres in inactive segments
-  cudaMemsetAsync(sd.cnt_cont, 0, sizeof(int) * (size_t)nb, st);
-  cudaMemsetAsync(sd.cnt_cand, 0, sizeof(int) * (size_t)nb, st);
-  k_seg_reset<<<blocks_for(sd.nseg), kThreads, 0, st>>>(sd.nseg, sd.grid, sd.sst, sd.ew);
-  k_aabb<<<blocks_for(nb), kThreads, 0, st>>>(sd.p4, sd.geom4, sd.bseg, sd.seg, nb, sd.amin,
-                                              sd.amax, sd.grid, sd.ew);
-  k_grid_setup<<<blocks_for(sd.nseg), kThreads, 0, st>>>(sd.nseg, sd.seg, sd.grid, sd.ew);
-  k_shift_and_bin<<<blocks_for(std::max(nb, sd.n_small)), kThreads, 0, st>>>(
-      nb, sd.small_ids, sd.n_small, sd.bseg, sd.seg, sd.p4, sd.geom4, sd.amin, sd.amax, sd.grid,
-      sd.cell, sd.keyA, sd.valA, park, sd.ew);
-  *launches += 4;
-  if (sd.n_small > 0) {
-    radix_sort_pairs(sd.keyA, sd.valA, sd.keyB, sd.valB, sd.radix_hist, &sd.ew->n_small,
-                     sd.n_small, bits_for(sd.ncell_cap), st, launches);
-    cudaMemsetAsync(sd.cell_start, 0xff, sizeof(int) * (size_t)sd.ncell_cap, st);
-    k_cell_ranges<<<blocks_for(sd.n_small), kThreads, 0, st>>>(sd.keyA, sd.n_small, sd.cell_start,
-                                                               sd.cell_end, park, sd.ew);
+  // Short or long form, device time of detection: 1,000 spheres 80 or 183 us,
+  // 5,003 spheres 186 or 213, 64 scenes of 20,500 bodies 0.45 ms more than long.
+  const bool few = nb <= kFewBodies && sd.ncell_cap <= 16 * kFewBodies;
+  if (few) {
+    k_front_few<<<1, 1024, 0, st>>>(sd.nseg, nb, sd.small_ids, sd.n_small, sd.bseg, sd.seg, sd.p4,
+                                    sd.geom4, sd.amin, sd.amax, sd.grid, sd.cell, sd.cell_start,
+                                    sd.cell_end, sd.ncell_cap, sd.keyA, sd.valA, sd.spheres,
+                                    sd.cnt_cont, sd.cnt_cand, sd.sst, sd.ew);
     ++*launches;
+  } else {
+    cudaMemsetAsync(sd.cnt_cont, 0, sizeof(int) * (size_t)nb, st);
+    cudaMemsetAsync(sd.cnt_cand, 0, sizeof(int) * (size_t)nb, st);
+    k_seg_reset<<<blocks_for(sd.nseg), kThreads, 0, st>>>(sd.nseg, sd.grid, sd.sst, sd.ew);
+    k_aabb<<<blocks_for(nb), kThreads, 0, st>>>(sd.p4, sd.geom4, sd.bseg, sd.seg, nb, sd.amin,
+                                                sd.amax, sd.grid, sd.ew);
+    k_grid_setup<<<blocks_for(sd.nseg), kThreads, 0, st>>>(sd.nseg, sd.seg, sd.grid, sd.ew);
+    k_shift_and_bin<<<blocks_for(std::max(nb, sd.n_small)), kThreads, 0, st>>>(
+        nb, sd.small_ids, sd.n_small, sd.bseg, sd.seg, sd.p4, sd.geom4, sd.amin, sd.amax, sd.grid,
+        sd.cell, sd.keyA, sd.valA, park, sd.ew);
+    *launches += 4;
+    if (sd.n_small > 0) {
+      radix_sort_pairs(sd.keyA, sd.valA, sd.keyB, sd.valB, sd.radix_hist, &sd.ew->n_small,
+                       sd.n_small, bits_for(sd.ncell_cap), st, launches);
+      cudaMemsetAsync(sd.cell_start, 0xff, sizeof(int) * (size_t)sd.ncell_cap, st);
+      k_cell_ranges<<<blocks_for(sd.n_small), kThreads, 0, st>>>(sd.keyA, sd.valA, sd.n_small,
+                                                                 sd.cell_start, sd.cell_end, park,
+                                                                 sd.p4, sd.geom4, sd.spheres, sd.ew);
+      ++*launches;
+    }
   }
   CollideArgs a = make_args(sd);
-  const int pair_blocks = (sd.n_small + kWarpsPerCta - 1) / kWarpsPerCta;
   dim3 box_grid(sd.max_seg_chunks, sd.n_large);
+  const int nchunks = sd.max_seg_chunks * sd.n_large;
   if (sd.n_small > 0) {
-    k_sphere_pairs<false><<<pair_blocks, kThreads, 0, st>>>(a);
+    k_sphere_count<<<(sd.n_small + kWarpsPerCta - 1) / kWarpsPerCta, kThreads, 0, st>>>(a);
     ++*launches;
   }
   if (sd.n_large > 0) {
     k_box_pairs<false><<<box_grid, kThreads, 0, st>>>(a, sd.large_chunk, nullptr);
     ++*launches;
   }
-  exclusive_scan_i32(sd.cnt_cont, sd.cbase, nb, sd.scan_tmp, st, launches);
-  k_seg_layout<<<1, 1024, 0, st>>>(sd.nseg, nb, sd.seg, sd.sst, sd.cbase, sd.seg_tstart, sd.ccap,
-                                   sd.tcap, sd.ew);
-  k_tile_table<<<std::max(1, std::min(sd.tcap / kThreads + 1, 1184)), kThreads, 0, st>>>(
-      sd.nseg, sd.seg_tstart, sd.tseg, sd.tcap, sd.ew);
-  *launches += 2;
+  if (few) {
+    k_seg_layout<true><<<1, 1024, 0, st>>>(sd.nseg, nb, sd.seg, sd.sst, sd.cbase, sd.seg_tstart,
+                                           sd.ccap, sd.tcap, sd.ew, sd.cnt_cont, sd.large_chunk,
+                                           sd.large_chunk_off, nchunks, sd.tseg);
+    ++*launches;
+  } else {
+    exclusive_scan_i32(sd.cnt_cont, sd.cbase, nb, sd.scan_tmp, st, launches);
+    k_seg_layout<false><<<1, 1024, 0, st>>>(sd.nseg, nb, sd.seg, sd.sst, sd.cbase, sd.seg_tstart,
+                                            sd.ccap, sd.tcap, sd.ew);
+    k_tile_table<<<std::max(1, std::min(sd.tcap / kThreads + 1, 1184)), kThreads, 0, st>>>(
+        sd.nseg, sd.seg_tstart, sd.tseg, sd.tcap, sd.ew);
+    *launches += 2;
+    if (sd.n_large > 0)
+      exclusive_scan_i32(sd.large_chunk, sd.large_chunk_off, nchunks, sd.scan_tmp, st, launches);
+  }
   if (sd.n_small > 0) {
-    k_sphere_pairs<true><<<pair_blocks, kThreads, 0, st>>>(a);
-    k_sphere_pairs_wide<<<kWideGrid, kThreads, 0, st>>>(a);
+    const int per_cta = 4 * kWarpsPerCta;
+    k_sphere_write<<<(sd.n_small + per_cta - 1) / per_cta, kThreads, 0, st>>>(a);
+    k_sphere_pairs_wide<<<std::min(kWideGrid, sd.n_small), kThreads, 0, st>>>(a);
     *launches += 2;
   }
   if (sd.n_large > 0) {
-    exclusive_scan_i32(sd.large_chunk, sd.large_chunk_off, sd.max_seg_chunks * sd.n_large,
-                       sd.scan_tmp, st, launches);
     k_box_pairs<true><<<box_grid, kThreads, 0, st>>>(a, nullptr, sd.large_chunk_off);
     ++*launches;
+  }
+  if (few) {
+    k_incidence_few<<<1, 1024, 0, st>>>(nb, sd.idb, sd.tseg, sd.sst, sd.bseg, sd.cbase, sd.cnt_cont,
+                                        sd.cnt_cand, sd.keyA, sd.valA, sd.inc_start, sd.inc, sd.ew);
+    ++*launches;
+    return;
   }
   // B-side incidence: stable radix sort of (B, contact) keeps ascending contact order.
   cudaMemsetAsync(sd.cnt_cand, 0, sizeof(int) * (size_t)nb, st);

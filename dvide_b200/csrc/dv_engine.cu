@@ -500,6 +500,7 @@ int Engine::reconfigure(const std::vector<SlotSpec>& slots) {
   if (nb2 > nb_cap_) {
     int cap = std::max(nb2, nb_cap_ + nb_cap_ / 4);
     dfree(d.k4); dfree(d.w4); dfree(d.fc4); dfree(d.amin); dfree(d.amax); dfree(d.cell);
+    dfree(d.spheres); dfree(d.kept);
     dfree(d.cnt_cont); dfree(d.cnt_cand); dfree(d.cbase); dfree(d.binc_start); dfree(d.inc_start);
     dfree(d.bseg);
     TRY(dalloc(&d.k4, cap));
@@ -508,6 +509,8 @@ int Engine::reconfigure(const std::vector<SlotSpec>& slots) {
     TRY(dalloc(&d.amin, cap));
     TRY(dalloc(&d.amax, cap));
     TRY(dalloc(&d.cell, cap));
+    TRY(dalloc(&d.spheres, cap));
+    TRY(dalloc(&d.kept, (size_t)cap * kKeepPartners));
     TRY(dalloc(&d.cnt_cont, cap));
     TRY(dalloc(&d.cnt_cand, cap));
     TRY(dalloc(&d.cbase, (size_t)cap + 1));
@@ -547,7 +550,7 @@ int Engine::reconfigure(const std::vector<SlotSpec>& slots) {
     int cap = std::max(ncell2, ncell_alloc_ + ncell_alloc_ / 4);
     dfree(d.cell_start);
     dfree(d.cell_end);
-    TRY(dalloc(&d.cell_start, cap));
+    TRY(dalloc(&d.cell_start, (size_t)cap + 1));
     TRY(dalloc(&d.cell_end, cap));
     DV_CUDA_TRY(cudaMemsetAsync(d.cell_end, 0, sizeof(int) * cap, st));
     ncell_alloc_ = cap;

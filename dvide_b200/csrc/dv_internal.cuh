@@ -124,6 +124,10 @@ struct EngineWords {
 constexpr int kWideSpheres = 65536;
 constexpr int kWideGrid = 256;
 constexpr int kWidePartners = 8192;
+// Partners per sphere that the count pass keeps for the write pass, and the
+// bodies up to which an engine takes the short forms of collision detection.
+constexpr int kKeepPartners = 16;
+constexpr int kFewBodies = 6144;
 
 // Tiles that a team's member takes at most when there are more than the grid
 // has CTAs, and the distance of the teams' arrival counters (a line each).
@@ -154,6 +158,8 @@ struct SceneDev {
   // collision scratch
   double4 *amin = nullptr, *amax = nullptr;   // shifted AABBs
   int4* cell = nullptr;                       // cell coords + global linear id
+  double4* spheres = nullptr;                 // gridded spheres (x, y, z, r) in cell order
+  uint32_t* kept = nullptr;                   // kKeepPartners partners per gridded sphere
   uint32_t *keyA = nullptr, *valA = nullptr, *keyB = nullptr, *valB = nullptr;  // radix buffers
   size_t radix_cap = 0;
   uint32_t* radix_hist = nullptr;
