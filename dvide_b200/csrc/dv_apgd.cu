@@ -295,18 +295,17 @@ struct BilRows {
 };
 
 // Product pass on rows [r0, r0 + min(n, 512)): N gamma_new, the objective and
-// residual items, the look-ahead step, without the cone projection; the tile's
-// partials are parked in slot `slot`.  Called after the contact tiles (where
+// residual items, the look-ahead step, without the cone projection; the sums
+// into acc.  Called after the contact tiles (where
 // it adds no registers to the contact loops).  Returns whether a residual
 // item of this thread was NaN.
-template <class T>
+template <class T, int kGroups>
 __device__ inline bool bil_product_tile(BilRows<T> R, const Solve& C, int r0, int n,
-                                        bool has_contacts, ParkBuf* park, int slot, int tile) {
+                                        bool has_contacts, double (&acc)[8]) {
   const T ya = (T)C.prod_ya, ym = (T)C.prod_ym, nt2 = (T)C.prod_nt;
-  double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   bool bad = false;
-  for (int m = 0; m < kItemsPerThread; ++m) {
-    const int k = m * kThreads + threadIdx.x;
+  for (int m = kGroups == 2 ? (int)(threadIdx.x >> 8) : 0; m < kItemsPerThread; m += kGroups) {
+    const int k = m * kThreads + (threadIdx.x & (kThreads - 1));
     if (k < n) {
       const int r = r0 + k;
       const T N0 = bil_dw<T>(__ldg(R.off + r), R.w);
@@ -345,34 +344,52 @@ __device__ inline bool bil_product_tile(BilRows<T> R, const Solve& C, int r0, in
       acc[6] = acc[6] + (double)y0 * (double)rr;
     }
   }
-  park8<true>(*park, slot, tile, acc);
   return bad;
 }
 
+// The end of a tile: its partials into slot `slot`.
+template <int kGroups, int NQ, bool kMax>
+__device__ __forceinline__ void park_group(ParkBuf& park, PairBuf& pair, int& flip, int slot, int tile,
+                                           double (&acc)[8]) {
+  if constexpr (kGroups == 2) park_pair8<NQ, kMax>(park, pair, flip, slot, tile, acc);
+  else park8<kMax>(park, slot, tile, acc);
+}
+
+// kGroups 2: CTAs of 512 threads, one per SM, whose second group of 256 takes
+// the second sub-tile of every tile: a scene with a tile per member waits for
+// the contact arithmetic once a pass instead of twice.  kGroups 1: CTAs of 256
+// threads, kMinB per SM, which hide each other's waits where there is work for
+// all of them.
 // kAR: APGD's anti-relaxation (APGD.cu:335-345), FP64 one-scene engines.
-template <class T, int kMinB, bool kAR>
-__global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
+template <class T, int kGroups, int kMinB, bool kAR>
+__global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T> a) {
   using V = typename Vec4<T>::type;
   using B = Block<T>;
   constexpr bool kMixed = sizeof(T) != sizeof(double);
+  constexpr int kT = kThreads * kGroups;
   __shared__ double scratch[64];
   __shared__ Solve C;
   __shared__ Team tm;
-  __shared__ BodyCache bodies;
+  __shared__ BodyCache<kT> bodies;
   __shared__ ParkBuf park;
   __shared__ PhaseTimer timer;
   __shared__ int s_seen, s_copy_fail;
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   const size_t S = a.S;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // this thread's sub-tile of a tile (kGroups 2) and its place in it
+  const int group = kGroups == 2 ? (int)(threadIdx.x >> 8) : 0;
+  const int tid = threadIdx.x & (kThreads - 1), gwarp = tid >> 5;
   Staging stg;
   stg.base = dyn_smem;
   stg.stage_bytes = B::kStageBytes;
-  stg.bar = reinterpret_cast<uint64_t*>(dyn_smem + (size_t)kWarps * 2 * B::kStageBytes);
+  stg.bar = reinterpret_cast<uint64_t*>(dyn_smem + (size_t)kWarps * kGroups * 2 * B::kStageBytes);
+  PairBuf& pair = *reinterpret_cast<PairBuf*>(stg.bar + 2 * kMaxWarps + kMaxWarps / 8);
+  int flip = 0;
   stg.phase = 0;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 2 * kWarps; ++i) mbar_init(stg.bar + i, 1);
-    for (int w = 0; w < kWarps; ++w) reinterpret_cast<unsigned char*>(stg.bar + 2 * kWarps)[w] = 0;
+    for (int i = 0; i < 2 * kWarps * kGroups; ++i) mbar_init(stg.bar + i, 1);
+    for (int w = 0; w < kMaxWarps; ++w) reinterpret_cast<unsigned char*>(stg.bar + 2 * kMaxWarps)[w] = 0;
     fence_mbar_init();
     s_seen = 0;
     s_copy_fail = 0;
@@ -381,6 +398,9 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
   __syncthreads();
   if (ld_acquire(&a.ew->err)) return;  // an error of collision detection: nothing to do
 
+  // a warp's sub-tile j: of the member's tile tile_of(j) its part sub_of(j)
+  auto tile_of = [](int j) { return kGroups == 2 ? j : j >> 1; };
+  auto sub_of = [&](int j) { return kGroups == 2 ? group : j & 1; };
   // a phase ends at a barrier
   auto sync = [&](int phase, bool joining = false) {
     const bool ok = team_sync(a, tm, joining);
@@ -418,7 +438,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
     }
 
     // ---- applied impulse: k = m v + h f (m = 1/minv, 0 for fixed); w = minv k
-    for (int b = tm.w0 + threadIdx.x; b < tm.w1; b += kThreads) {
+    for (int b = tm.w0 + threadIdx.x; b < tm.w1; b += kT) {
       const double h = P.h;
       double mi = __ldg(a.minv + b);
       double m = mi;
@@ -449,8 +469,8 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
             const double* pd = reinterpret_cast<const double*>(a.p4);
             const double* wdv = reinterpret_cast<const double*>(a.wd);
             const double tmv = a.seg_time[s];
-            for (int m = 0; m < kItemsPerThread; ++m) {
-              const int k = kb + m * kThreads + threadIdx.x;
+            for (int m = group; m < kItemsPerThread; m += kGroups) {
+              const int k = kb + m * kThreads + tid;
               if (k < P.nbil) {
                 const int i2 = P.bil0 + k;
                 const int2 o = __ldg(a.bil_off + i2);
@@ -477,8 +497,8 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
               }
             }
           }
-          for (int m = 0; m < kItemsPerThread && kb < 0; ++m) {
-            int k = k0 + m * kThreads + threadIdx.x;
+          for (int m = group; m < kItemsPerThread && kb < 0; m += kGroups) {
+            int k = k0 + m * kThreads + tid;
             if (k < nc) {
               const int c = c0 + k;
               const uint32_t ia = __ldg(a.ida + c), ib = __ldg(a.idb + c);
@@ -565,16 +585,16 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
               store_keep(qv + c, f_times<T, V>(f, e0, e1, e2));
             }
           }
-          park8<false>(park, nslot, t, acc);
+          park_group<kGroups, 1, false>(park, pair, flip, nslot, t, acc);
           if (++nslot == kParkSlots) {
-            fold_parked8<false>(park, planes(), a.tcap, nslot);
+            fold_parked8<false, kT>(park, planes(), a.tcap, nslot);
             nslot = 0;
           }
         }
-        fold_parked8<false>(park, planes(), a.tcap, nslot);
+        fold_parked8<false, kT>(park, planes(), a.tcap, nslot);
       }
       if (!sync(kPhaseSetup)) return;
-      fold_team<1, false>(planes(), a.tcap, tm.nt, scratch, C.sums);
+      fold_team<1, false, kGroups>(planes(), a.tcap, tm.nt, scratch, C.sums);
       if (threadIdx.x == 0) C.L0 = sqrt(C.sums[0]);
       parity ^= 1;
       team_body_pass<T, kAR>(a, tm, bodies, wv, qv);
@@ -592,8 +612,8 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
           if (kb >= 0) {
             // bilateral rows: (N e)_row; q = gamma_0 for the first N y
             const T* wt = reinterpret_cast<const T*>(wv);
-            for (int m = 0; m < kItemsPerThread; ++m) {
-              const int k = kb + m * kThreads + threadIdx.x;
+            for (int m = group; m < kItemsPerThread; m += kGroups) {
+              const int k = kb + m * kThreads + tid;
               if (k < P.nbil) {
                 const int i2 = P.bil0 + k;
                 const T n0 = bil_dw<T>(__ldg(a.bil_off + i2), wt);
@@ -602,8 +622,8 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
               }
             }
           }
-          for (int m = 0; m < kItemsPerThread && kb < 0; ++m) {
-            int k = k0 + m * kThreads + threadIdx.x;
+          for (int m = group; m < kItemsPerThread && kb < 0; m += kGroups) {
+            int k = k0 + m * kThreads + tid;
             if (k < nc) {
               const int c = c0 + k;
               const Frame<T> f = block_frame<T>(const_at(a, c));
@@ -616,16 +636,16 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
               store_keep(qv + c, f_times<T, V>(f, gi[0], gi[32], gi[64]));
             }
           }
-          park8<false>(park, nslot, t, acc);
+          park_group<kGroups, 1, false>(park, pair, flip, nslot, t, acc);
           if (++nslot == kParkSlots) {
-            fold_parked8<false>(park, planes(), a.tcap, nslot);
+            fold_parked8<false, kT>(park, planes(), a.tcap, nslot);
             nslot = 0;
           }
         }
-        fold_parked8<false>(park, planes(), a.tcap, nslot);
+        fold_parked8<false, kT>(park, planes(), a.tcap, nslot);
       }
       if (!sync(kPhaseSetup)) return;
-      fold_team<1, false>(planes(), a.tcap, tm.nt, scratch, C.sums);
+      fold_team<1, false, kGroups>(planes(), a.tcap, tm.nt, scratch, C.sums);
       if (threadIdx.x == 0) ctl_lipschitz(C, P, nc, cap, kMixed);
       parity ^= 1;
       team_body_pass<T, kAR>(a, tm, bodies, wv, qv);
@@ -654,8 +674,8 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
           // (nothing would hide the copies), the lines of the next sub-tile go to L2.
           const bool staged = tm.ntc > tm.m;
           auto bring = [&](int j) {
-            const int t = team_tile(tm, tm.ntc, j >> 1);
-            const int kw = t * kTileItems + (j & 1) * kSub + warp * 32;
+            const int t = team_tile(tm, tm.ntc, tile_of(j));
+            const int kw = t * kTileItems + sub_of(j) * kSub + gwarp * 32;
             if (t < 0 || kw >= nc) return;
             const size_t blk = (size_t)(c0 + kw) >> 5;
             const auto lines = [&](const T* p, unsigned bytes) {
@@ -698,8 +718,8 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
               T* bNGc = a.bNG[cur];
               const T* bNGp = a.bNG[prev < 0 ? cur : prev];
               T* bGn = a.bG[C.nw];
-              for (int m = 0; m < kItemsPerThread; ++m) {
-                const int k = kb + m * kThreads + threadIdx.x;
+              for (int m = group; m < kItemsPerThread; m += kGroups) {
+                const int k = kb + m * kThreads + tid;
                 if (k < P.nbil) {
                   const int i2 = P.bil0 + k;
                   const T c0v = bGc[i2];
@@ -730,13 +750,13 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
                 }
               }
             }
-            for (int m = 0; m < kItemsPerThread && kb < 0; ++m, ++j) {
+            for (int m = group; m < kItemsPerThread && kb < 0; m += kGroups, ++j) {
               const int sidx = j & 1;
               if (j > 0 && !failed) {
                 __syncwarp();  // the warp's reads of the other stage are done
                 bring(j + 1);
               }
-              const int kw = k0 + m * kSub + warp * 32;
+              const int kw = k0 + m * kSub + gwarp * 32;
               const int k = kw + lane;
               const int c = c0 + k;
               T p0 = T(0), p1 = T(0), p2 = T(0), q0 = T(0), q1 = T(0), q2 = T(0);
@@ -798,19 +818,19 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
                 }
               }
             }
-            park8<false>(park, nslot, t, acc);
+            park_group<kGroups, 5, false>(park, pair, flip, nslot, t, acc);
             if (++nslot == kParkSlots) {
-              fold_parked8<false>(park, planes(), a.tcap, nslot);
+              fold_parked8<false, kT>(park, planes(), a.tcap, nslot);
               nslot = 0;
             }
           }
-          fold_parked8<false>(park, planes(), a.tcap, nslot);
+          fold_parked8<false, kT>(park, planes(), a.tcap, nslot);
           if (s_copy_fail) {
             drain_warp_stages(stg, &a.ew->wait_limit_ns);
             return;
           }
           if (!sync(kPhaseStep)) return;
-          fold_team<5, false>(planes(), a.tcap, tm.nt, scratch, C.sums);
+          fold_team<5, false, kGroups>(planes(), a.tcap, tm.nt, scratch, C.sums);
           if (threadIdx.x == 0) ctl_step(C);
           parity ^= 1;
           __syncthreads();
@@ -819,9 +839,9 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
         // ---- the contact pass's sub-tiles of this member; its first two are
         // copied while the body pass runs
         const int cur = C.cur, nw = C.nw, restart = C.restart;
-        auto issue = [&](int j) {  // sub-tile j of this member into stage j & 1
-          const int t = team_tile(tm, tm.ntc, j >> 1);
-          const int kw = t * kTileItems + (j & 1) * kSub + warp * 32;
+        auto issue = [&](int j) {  // this warp's sub-tile j into stage j & 1
+          const int t = team_tile(tm, tm.ntc, tile_of(j));
+          const int kw = t * kTileItems + sub_of(j) * kSub + gwarp * 32;
           if (t >= 0 && kw < nc && lane == 0) {
             const int sidx = j & 1;
             const size_t blk = (size_t)(c0 + kw) >> 5;
@@ -861,15 +881,15 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
           T* Xn = a.G[nw];
           T* X2 = a.G[C.nw2];
           for (int j = 0;; ++j) {
-            const int t = team_tile(tm, tm.ntc, j >> 1);
+            const int t = team_tile(tm, tm.ntc, tile_of(j));
             if (t < 0) break;
-            const int sidx = j & 1;
+            const int sidx = j & 1, sub = sub_of(j);
             if (j && !failed) {
               __syncwarp();  // the warp's reads of stage sidx^1 are done
               if (lane == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
               issue(j + 1);
             }
-            const int kw = t * kTileItems + sidx * kSub + warp * 32;
+            const int kw = t * kTileItems + sub * kSub + gwarp * 32;
             if (kw < nc && !failed && !wait_warp_stage(a, stg, sidx)) {
               failed = true;
               s_copy_fail = 1;
@@ -955,19 +975,19 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
               acc[5] = acc[5] + dot3i(y0, y1, y2, M0, M1, M2);
               acc[6] = acc[6] + dot3i(y0, y1, y2, rn0, r1, r2);
             }
-            if (sidx == kItemsPerThread - 1) {
+            if (kGroups == 2 || sub == kItemsPerThread - 1) {
               if (__any_sync(0xffffffffu, bad) && lane == 0) seg_error(a, s, kErrNaN);
-              park8<true>(park, nslot, t, acc);
+              park_group<kGroups, 7, true>(park, pair, flip, nslot, t, acc);
 #pragma unroll
               for (int q = 0; q < 8; ++q) acc[q] = 0.0;
               bad = false;
               if (++nslot == kParkSlots) {
-                fold_parked8<true>(park, planes(), a.tcap, nslot);
+                fold_parked8<true, kT>(park, planes(), a.tcap, nslot);
                 nslot = 0;
               }
             }
           }
-          fold_parked8<true>(park, planes(), a.tcap, nslot);
+          fold_parked8<true, kT>(park, planes(), a.tcap, nslot);
           if (s_copy_fail) {
             drain_warp_stages(stg, &a.ew->wait_limit_ns);
             return;
@@ -984,19 +1004,21 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
               if (kb < 0) continue;
               BilRows<T> br_{a.bil_off, wt, a.bG[cur], a.bG[nw], a.bG[C.nw2], a.bNG[cur],
                              a.bNG[nw], a.br, a.bq};
-              const bool bad2 = bil_product_tile<T>(br_, C, P.bil0 + kb, P.nbil - kb, nc > 0,
-                                                    &park, nslot, t);
+              double racc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+              const bool bad2 =
+                  bil_product_tile<T, kGroups>(br_, C, P.bil0 + kb, P.nbil - kb, nc > 0, racc);
+              park_group<kGroups, 7, true>(park, pair, flip, nslot, t, racc);
               if (__any_sync(0xffffffffu, bad2) && lane == 0) seg_error(a, s, kErrNaN);
               if (++nslot == kParkSlots) {
-                fold_parked8<true>(park, planes(), a.tcap, nslot);
+                fold_parked8<true, kT>(park, planes(), a.tcap, nslot);
                 nslot = 0;
               }
             }
-            fold_parked8<true>(park, planes(), a.tcap, nslot);
+            fold_parked8<true, kT>(park, planes(), a.tcap, nslot);
           }
         }
         if (!sync(kPhaseProduct)) return;
-        fold_team<7, true>(planes(), a.tcap, tm.nt, scratch, C.sums);
+        fold_team<7, true, kGroups>(planes(), a.tcap, tm.nt, scratch, C.sums);
         if (threadIdx.x == 0) ctl_product(C, P, cap, kMixed, kAR);
         parity ^= 1;
         __syncthreads();
@@ -1013,8 +1035,8 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
           if (t < 0) break;
           double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
           if (best >= 0) {
-            for (int m = 0; m < kItemsPerThread; ++m) {
-              const int k = t * kTileItems + m * kThreads + threadIdx.x;
+            for (int m = group; m < kItemsPerThread; m += kGroups) {
+              const int k = t * kTileItems + m * kThreads + tid;
               if (k < nc) {
                 const int c = c0 + k;
                 const T* x = iter_at(a.G[best], c);
@@ -1024,15 +1046,15 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
               }
             }
           }
-          park8<false>(park, nslot, t, acc);
+          park_group<kGroups, 1, false>(park, pair, flip, nslot, t, acc);
           if (++nslot == kParkSlots) {
-            fold_parked8<false>(park, planes(), a.tcap, nslot);
+            fold_parked8<false, kT>(park, planes(), a.tcap, nslot);
             nslot = 0;
           }
         }
-        fold_parked8<false>(park, planes(), a.tcap, nslot);
+        fold_parked8<false, kT>(park, planes(), a.tcap, nslot);
         if (!sync(kPhaseFinal)) return;
-        fold_team<1, false>(planes(), a.tcap, tm.nt, scratch, C.sums);
+        fold_team<1, false, kGroups>(planes(), a.tcap, tm.nt, scratch, C.sums);
         if (threadIdx.x == 0 && best >= 0) C.objective = C.objN + C.sums[0];
         parity ^= 1;
         __syncthreads();
@@ -1051,8 +1073,8 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
           const int kb = a.nbil ? bil_tile_k0(t, 0, nc) : -1;
           if (kb >= 0) {
             // the rows' gamma_hat (ones before the first accepted iterate)
-            for (int m = 0; m < kItemsPerThread; ++m) {
-              const int k = kb + m * kThreads + threadIdx.x;
+            for (int m = group; m < kItemsPerThread; m += kGroups) {
+              const int k = kb + m * kThreads + tid;
               if (k < P.nbil) {
                 const int r = P.bil0 + k;
                 a.bil_gam[r] = best >= 0 ? (double)a.bG[best][r] : 1.0;
@@ -1060,8 +1082,8 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
             }
             continue;
           }
-          for (int m = 0; m < kItemsPerThread; ++m) {
-            int k = t * kTileItems + m * kThreads + threadIdx.x;
+          for (int m = group; m < kItemsPerThread; m += kGroups) {
+            int k = t * kTileItems + m * kThreads + tid;
             if (k < nc) {
               const int c = c0 + k;
               double x0 = 1.0, x1 = 1.0, x2 = 1.0;
@@ -1102,7 +1124,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
     // Scenes with neither contacts nor bilateral rows: v = Minv k, f_contact = 0
     // (System.cu:577-581); the rows' impulses enter f_c like the contacts'.
     if (!a.solve_only && !refine_next) {
-      for (int b = tm.w0 + threadIdx.x; b < tm.w1; b += kThreads) {
+      for (int b = tm.w0 + threadIdx.x; b < tm.w1; b += kT) {
         const double h = P.h;
         double4 k = a.k4[b];
         double mi = __ldg(a.minv + b);
@@ -1126,7 +1148,7 @@ __global__ void __launch_bounds__(kThreads, kMinB) k_step_solve(KArgs<T> a) {
     // matched warm start: where each body's A-contacts went in the warm region
     if (live) {
       const int shift = a.sst[s].delta - c0;
-      for (int b = tm.w0 + threadIdx.x; b < tm.w1; b += kThreads) {
+      for (int b = tm.w0 + threadIdx.x; b < tm.w1; b += kT) {
         a.ws[b] = a.cbase[b] + shift;
         a.wc[b] = a.cnt_cont[b];
       }
@@ -1240,32 +1262,49 @@ __global__ void __launch_bounds__(1024) k_team_plan(int nseg, const SegParams* _
   }
 }
 
-template <class T>
+template <class T, int kGroups>
 constexpr size_t solve_smem_bytes() {
-  return (size_t)kWarps * 2 * Block<T>::kStageBytes + (size_t)kWarps * 2 * 8 + 16;
+  return (size_t)kWarps * kGroups * 2 * Block<T>::kStageBytes + (size_t)kMaxWarps * 2 * 8 + kMaxWarps +
+         (kGroups == 2 ? sizeof(PairBuf) : 0);
 }
 
-template <class T, int MB, bool AR>
+template <class T, int G, int MB, bool AR>
 void prepare_kernel() {
   static bool done = false;
   if (done) return;
-  cudaFuncSetAttribute(k_step_solve<T, MB, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)solve_smem_bytes<T>());
+  cudaFuncSetAttribute(k_step_solve<T, G, MB, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)solve_smem_bytes<T, G>());
   done = true;
 }
 
-template <class T, int MB, bool AR = false>
+template <class T, int G, int MB, bool AR = false>
 void launch_typed(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t* launches,
-                  bool solve_only, bool refine = false) {
-  prepare_kernel<T, MB, AR>();
+                  bool solve_only, bool refine) {
+  prepare_kernel<T, G, MB, AR>();
   KArgs<T> a = make_kargs<T>(sd, cfg);
   a.solve_only = solve_only ? 1 : 0;
   a.refine = refine ? 1 : 0;
-  plan_teams(sd, cfg.grid, refine, st, launches);
+  const int grid = G == 2 ? std::max(1, cfg.grid / 2) : cfg.grid;
+  plan_teams(sd, grid, refine, st, launches);
   void* params[] = {&a};
-  cudaLaunchCooperativeKernel((const void*)k_step_solve<T, MB, AR>, cfg.grid, kThreads, params,
-                              solve_smem_bytes<T>(), st);
+  cudaLaunchCooperativeKernel((const void*)k_step_solve<T, G, MB, AR>, grid, kThreads * G, params,
+                              solve_smem_bytes<T, G>(), st);
   ++*launches;
+}
+
+// Which form of the kernel a launch takes (128 registers per thread in both):
+// 512-thread CTAs for one scene of at most kPairBodies bodies, whose tiles are
+// then at most about one per SM.  Solve per step in 512- and 256-thread CTAs:
+// 1,000 spheres 1.63 and 1.73 ms, 20,011 mixed 8.16 and 8.95; 200,000 spheres
+// 44 and 34 ms (their stages leave the body pass a sixth of the L1); 64 scenes
+// 2.9 and 2.7 ms (their 160 tiles need a second wave).
+template <class T, bool AR = false>
+void launch_form(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t* launches,
+                 bool solve_only, bool refine = false) {
+  if (sd.nseg == 1 && sd.nb <= kPairBodies)
+    launch_typed<T, 2, 1, AR>(sd, cfg, st, launches, solve_only, refine);
+  else
+    launch_typed<T, 1, 2, AR>(sd, cfg, st, launches, solve_only, refine);
 }
 
 template <class T, int MB>
@@ -1273,9 +1312,9 @@ int max_ctas_of() {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  prepare_kernel<T, MB, false>();
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_solve<T, MB, false>, kThreads,
-                                                solve_smem_bytes<T>());
+  prepare_kernel<T, 1, MB, false>();
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_solve<T, 1, MB, false>, kThreads,
+                                                solve_smem_bytes<T, 1>());
   if (per_sm < 1) per_sm = 1;
   return sms * per_sm;
 }
@@ -1310,18 +1349,18 @@ void launch_step_solve(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, in
   } else if (sd.precision == DV_PREC_MIXED) {
     // with refinement the FP32 launch leaves the update of the solves it marks
     // to an FP64 launch, which refines them first
-    if (cfg.blocks_per_sm == 3) launch_typed<float, 3>(sd, cfg, st, launches, solve_only);
-    else launch_typed<float, 2>(sd, cfg, st, launches, solve_only);
+    if (cfg.blocks_per_sm == 3) launch_typed<float, 1, 3>(sd, cfg, st, launches, solve_only, false);
+    else launch_form<float>(sd, cfg, st, launches, solve_only);
     if (sd.refine_any) {
       SolveConfig c2 = cfg;
       c2.blocks_per_sm = 2;
       c2.grid = std::min(cfg.grid, std::max(1, sd.refine_grid));
-      launch_typed<double, 2>(sd, c2, st, launches, solve_only, true);
+      launch_form<double>(sd, c2, st, launches, solve_only, true);
     }
   } else if (sd.anti_relax) {
-    launch_typed<double, 2, true>(sd, cfg, st, launches, solve_only);
+    launch_form<double, true>(sd, cfg, st, launches, solve_only);
   } else {
-    launch_typed<double, 2>(sd, cfg, st, launches, solve_only);
+    launch_form<double>(sd, cfg, st, launches, solve_only);
   }
 }
 

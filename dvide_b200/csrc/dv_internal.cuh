@@ -131,6 +131,7 @@ constexpr int kFewBodies = 6144;
 
 // Tiles that a team's member takes at most when there are more than the grid
 // has CTAs, and the distance of the teams' arrival counters (a line each).
+constexpr int kPairBodies = 20480;  // bodies of a scene that 512-thread CTAs solve
 constexpr int kTeamTiles = 4;
 constexpr int kTeamBarStride = 32;
 

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
   __shared__ double scratch[kNQ * 8 + 8];
   __shared__ DeferBuf s_def;
   __shared__ Team tm;
-  __shared__ BodyCache bodies;
+  __shared__ BodyCache<kThreads> bodies;
   __shared__ PhaseTimer timer;
   __shared__ PgjSolve C;
   __shared__ int s_seen;

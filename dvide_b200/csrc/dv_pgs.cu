@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
   __shared__ double scratch[kNQ * 8 + 8];
   __shared__ DeferBuf s_def;
   __shared__ Team tm;
-  __shared__ BodyCache bodies;
+  __shared__ BodyCache<kThreads> bodies;
   __shared__ PhaseTimer timer;
   __shared__ PgsSolve C;
   __shared__ int s_seen;

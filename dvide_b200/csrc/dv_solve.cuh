@@ -17,6 +17,7 @@ namespace {
 constexpr int kNQ = 7;      // partial-sum slots per tile
 constexpr int kQMax = kNQ;  // slot of the per-tile maximum
 constexpr int kWarps = kThreads / 32;
+constexpr int kMaxWarps = 16;  // warps of the largest CTA that has stages
 constexpr int kSub = kThreads;  // contacts per sub-tile
 
 // Phases timed between barriers (EngineWords::phase_ns).
@@ -591,7 +592,7 @@ struct Staging {
 // Per warp, bit s: copies issued into stage s and not yet seen complete; one
 // byte per warp after the mbarriers (lane 0 writes it).
 __device__ inline volatile unsigned char* stage_pending(const Staging& st) {
-  return reinterpret_cast<volatile unsigned char*>(st.bar + 2 * kWarps) + (threadIdx.x >> 5);
+  return reinterpret_cast<volatile unsigned char*>(st.bar + 2 * kMaxWarps) + (threadIdx.x >> 5);
 }
 __device__ inline void mark_stage_issued(const Staging& st, int s) {
   if ((threadIdx.x & 31) == 0) *stage_pending(st) |= (unsigned char)(1u << s);

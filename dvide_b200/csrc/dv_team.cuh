@@ -192,7 +192,7 @@ struct PhaseTimer {
 // the eight instead of 40.  Lane l returns quantity l / 4; with kMax the last
 // one is a maximum.
 template <bool kMax>
-__device__ inline double warp_fold8(const double (&v)[8]) {
+__device__ __forceinline__ double warp_fold8(const double (&v)[8]) {
   const int lane = threadIdx.x & 31;
   const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
   const bool last = kMax && u16 && u8 && u4;
@@ -227,7 +227,7 @@ struct ParkBuf {
 };
 
 template <bool kMax>
-__device__ inline void park8(ParkBuf& B, int slot, int tile, const double (&v)[8]) {
+__device__ __forceinline__ void park8(ParkBuf& B, int slot, int tile, const double (&v)[8]) {
   const int lane = threadIdx.x & 31;
   const double t = warp_fold8<kMax>(v);
   if ((lane & 3) == 0) B.w[slot][lane >> 2][threadIdx.x >> 5] = t;
@@ -236,10 +236,10 @@ __device__ inline void park8(ParkBuf& B, int slot, int tile, const double (&v)[8
 
 // Completes the 8-warp tree of the n parked tiles' quantities into
 // part[quantity][tile].
-template <bool kMax>
+template <bool kMax, int kT>
 __device__ inline void fold_parked8(ParkBuf& B, double* part, int tcap, int n) {
   __syncthreads();
-  for (int i = threadIdx.x; i < n * 8; i += kThreads) {
+  for (int i = threadIdx.x; i < n * 8; i += kT) {
     const int slot = i >> 3, q = i & 7;
     const double* w = B.w[slot][q];
     double r;
@@ -258,36 +258,45 @@ __device__ inline void fold_parked8(ParkBuf& B, double* part, int tcap, int n) {
 // barrier and runs the scene's controller on its own copy of the scalars: the
 // partials cross L2 once more per member, and the result needs no second trip
 // through a word that one CTA writes and the others wait for.
-template <int NS, bool kMax>
-__device__ __noinline__ void fold_team(const double* part, int tcap, int nt, double* scratch,
-                                       double* out) {
+// In a CTA of two groups of 256 threads the second one folds quantities 4 to 7.
+template <int Q0, int Q1, int NS, bool kMax>
+__device__ __forceinline__ void sum_tiles(const double* part, int tcap, int nt, int tid, double (&v)[8]) {
   constexpr int U = 4;
-  double v[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) v[q] = 0.0;
-  for (int t = threadIdx.x; t < nt; t += U * kThreads) {
+  for (int t = tid; t < nt; t += U * kThreads) {
     double x[8][U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int at = t + u * kThreads;
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
+      for (int q = Q0; q < Q1; ++q)
         if (q < NS || (kMax && q == 7)) x[q][u] = at < nt ? __ldcg(part + (size_t)q * tcap + at) : 0.0;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (t + u * kThreads < nt) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
+        for (int q = Q0; q < Q1; ++q) {
           if (q < NS) v[q] = v[q] + x[q][u];
           if (kMax && q == 7) v[q] = fmax(v[q], x[q][u]);
         }
       }
     }
   }
-  const int lane = threadIdx.x & 31;
-  const double f = warp_fold8<kMax>(v);
-  if ((lane & 3) == 0) scratch[(lane >> 2) * 8 + (threadIdx.x >> 5)] = f;
+}
+template <int NS, bool kMax, int kGroups>
+__device__ __noinline__ void fold_team(const double* part, int tcap, int nt, double* scratch,
+                                       double* out) {
+  const int tid = threadIdx.x & (kThreads - 1);
+  const bool second = kGroups == 2 && threadIdx.x >= kThreads;
+  double v[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) v[q] = 0.0;
+  if (kGroups == 1) sum_tiles<0, 8, NS, kMax>(part, tcap, nt, tid, v);
+  else if (second) sum_tiles<4, 8, NS, kMax>(part, tcap, nt, tid, v);
+  else sum_tiles<0, 4, NS, kMax>(part, tcap, nt, tid, v);
+  const int lane = threadIdx.x & 31, warp = tid >> 5;
+  const double f = warp_fold8<kMax>(v);  // of a group, its own quantities
+  if ((lane & 3) == 0 && (kGroups == 1 || (lane >= 16) == second)) scratch[(lane >> 2) * 8 + warp] = f;
   __syncthreads();
   if (threadIdx.x < 8) {
     const double* w = scratch + threadIdx.x * 8;
@@ -301,16 +310,47 @@ __device__ __noinline__ void fold_team(const double* part, int tcap, int nt, dou
   __syncwarp();  // warp 0 runs the controller
 }
 
-// The heads and first eight incidence entries of a member's first 256 bodies,
-// one per thread, kept for all body passes of a solve: they do not change, and
-// reading them is two trips to L2 that the gathers of q wait for.
-struct BodyCache {
-  double mi[kThreads];
-  int s[kThreads], e[kThreads];
-  uint32_t c[8][kThreads];
+// A tile of a CTA of two groups: each thread of the second group hands its
+// values of the tile's second 256 items to its partner, which adds them to
+// those of the first 256 -- a thread's own order -- and parks the tile.  Four
+// warps, two of each group, meet at a named barrier; of the two buffers one is
+// still being read when the next tile's values go to the other.
+struct PairBuf {
+  double x[2][8][kThreads];
 };
-template <class K>
-__device__ inline void fill_body_cache(const K& a, const Team& t, BodyCache& k) {
+template <int NQ, bool kMax>
+__device__ __forceinline__ void park_pair8(ParkBuf& B, PairBuf& X, int& flip, int slot, int tile, double (&acc)[8]) {
+  const int tid = threadIdx.x & (kThreads - 1);
+  const int id = 1 + (tid >> 6);
+  double (*x)[kThreads] = X.x[flip];
+  flip ^= 1;
+  if (threadIdx.x >= kThreads) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < NQ || (kMax && q == 7)) x[q][tid] = acc[q];
+    asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory");
+  } else {
+    asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory");
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      if (q < NQ) acc[q] = acc[q] + x[q][tid];
+      if (kMax && q == 7) acc[q] = fmax(acc[q], x[q][tid]);
+    }
+    park8<kMax>(B, slot, tile, acc);
+  }
+}
+
+// The heads and first eight incidence entries of a member's first bodies, one
+// per thread, kept for all body passes of a solve: they do not change, and
+// reading them is two trips to L2 that the gathers of q wait for.
+template <int kT>
+struct BodyCache {
+  double mi[kT];
+  int s[kT], e[kT];
+  uint32_t c[8][kT];
+};
+template <class K, int kT>
+__device__ inline void fill_body_cache(const K& a, const Team& t, BodyCache<kT>& k) {
   const int b = t.w0 + threadIdx.x;
   BodyHead h{0.0, 0, 0};
   if (b < t.w1) h = body_head(a, b);
@@ -324,19 +364,19 @@ __device__ inline void fill_body_cache(const K& a, const Team& t, BodyCache& k) 
 // Body pass of a member: w_b = minv_b (D^T x)_b for its bodies.  Past the kept
 // ones, heads load two rounds ahead and each body's first eight incidence
 // entries one round ahead, while the current round gathers.
-template <class T, bool kAR>
-__device__ inline void team_body_pass(const KArgs<T>& a, const Team& t, const BodyCache& k,
+template <class T, bool kAR, int kT>
+__device__ inline void team_body_pass(const KArgs<T>& a, const Team& t, const BodyCache<kT>& k,
                                       typename Vec4<T>::type* w, const typename Vec4<T>::type* q) {
   const int e = t.w1;
   int b = t.w0 + threadIdx.x;
   if (b >= e) return;
   BodyHead h{k.mi[threadIdx.x], k.s[threadIdx.x], k.e[threadIdx.x]}, hn{0.0, 0, 0};
-  if (b + kThreads < e) hn = body_head(a, b + kThreads);
+  if (b + kT < e) hn = body_head(a, b + kT);
   uint32_t c[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) c[j] = k.c[j][threadIdx.x];
-  for (; b < e; b += kThreads) {
-    const int bnn = b + 2 * kThreads;
+  for (; b < e; b += kT) {
+    const int bnn = b + 2 * kT;
     BodyHead hnn{0.0, 0, 0};
     if (bnn < e) hnn = body_head(a, bnn);
     uint32_t cn[8];
