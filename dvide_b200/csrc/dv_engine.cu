@@ -61,7 +61,8 @@ void fill_step_stats(const StepRecord& r, int s, dv_step_stats* out) {
 Engine::~Engine() {
   if (st_) cudaStreamSynchronize(st_);
   drop_graph();
-  for (void* p : allocs_) cudaFree(p);
+  free_spare();
+  for (const auto& p : allocs_) cudaFree(p.first);
   allocs_.clear();
   if (h_ew_) cudaFreeHost(h_ew_);
   if (h_sst_) cudaFreeHost(h_sst_);
@@ -70,6 +71,15 @@ Engine::~Engine() {
   if (h_red_) cudaFreeHost(h_red_);
   for (cudaEvent_t e : ev_) cudaEventDestroy(e);
   if (own_stream_ && st_) cudaStreamDestroy(st_);
+}
+
+void Engine::free_spare() {
+  for (const auto& b : spare_) {
+    cudaFree(b.second);
+    held_bytes_ -= b.first;
+  }
+  spare_.clear();
+  spare_bytes_ = 0;
 }
 
 static const char* const kPartnerLimitText =
@@ -150,11 +160,11 @@ int Engine::ensure_slots() {
   return DV_OK;
 }
 
-// One CTA per contact tile of a settled scene and some to spare, up to the
-// co-resident maximum: a settled body has 3.7 contacts, so its tiles are nearly
-// twice its 256-body ranges; CTAs without a tile leave at once.
+// One CTA per contact tile and some to spare (a settled body has 3.7 contacts,
+// half as many CTAs of twice the threads may run), up to the co-resident
+// maximum; CTAs without a tile leave at once.
 int Engine::default_grid(int max_ctas) const {
-  return std::max(1, std::min(max_ctas, d.nb / 64 + 1));
+  return std::max(1, std::min(max_ctas, d.nb / 32 + 1));
 }
 
 int Engine::upload_segments() {

@@ -8,7 +8,9 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <map>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "dv_internal.cuh"
@@ -109,6 +111,7 @@ class Engine {
   // step() call after the failing step.  Batches keep stepping other scenes.
   int set_stop_on_segment_error(bool on);
   int64_t launches() const { return launches_; }
+  size_t held_bytes() const { return held_bytes_; }  // device memory
 
   // Positions / velocities of bodies [b0, b0 + n) as 3 doubles per body,
   // between host arrays and the device's double4 layout: one contiguous copy
@@ -176,7 +179,12 @@ class Engine {
 
   cudaStream_t st_ = nullptr;
   bool own_stream_ = false;
-  std::vector<void*> allocs_;
+  std::unordered_map<void*, size_t> allocs_;  // device memory and its sizes
+  size_t held_bytes_ = 0;                     // ... of them and the spare blocks
+  std::multimap<size_t, void*> spare_;        // freed blocks by size
+  size_t spare_bytes_ = 0;
+  static constexpr size_t kSpareBytes = size_t(256) << 20;
+  void free_spare();
   std::vector<SegParams> hseg_;
   std::vector<dv_params> P_;
   std::vector<double> time_;
@@ -226,17 +234,39 @@ class Engine {
   double* h_red_ = nullptr;           // pinned, 16 slots
 };
 
+// Device memory of an engine.  A freed block stays with the engine for its next
+// allocation of at most that and at least half that size, up to kSpareBytes in
+// all: a layout change of a server takes and gives back some twenty blocks, and
+// cudaMalloc and cudaFree of each cost 0.1 to 0.5 ms and wait for the device.
+// All work on a block runs on the engine's stream, so the next user's follows
+// the last one's.  Spare blocks go back when an allocation fails and with the engine.
 template <class T>
 inline int Engine::dalloc(T** p, size_t n) {
   if (n == 0) n = 1;
+  const size_t bytes = n * sizeof(T);
   void* q = nullptr;
-  cudaError_t e = cudaMalloc(&q, n * sizeof(T));
+  auto it = spare_.lower_bound(bytes);
+  if (it != spare_.end() && it->first / 2 <= bytes) {
+    q = it->second;
+    allocs_[q] = it->first;
+    spare_bytes_ -= it->first;
+    spare_.erase(it);
+    *p = reinterpret_cast<T*>(q);
+    return DV_OK;
+  }
+  cudaError_t e = cudaMalloc(&q, bytes);
+  if (e == cudaErrorMemoryAllocation && !spare_.empty()) {
+    cudaGetLastError();
+    free_spare();
+    e = cudaMalloc(&q, bytes);
+  }
   if (e != cudaSuccess) {
     *p = nullptr;
     cudaGetLastError();
     return dv_record_cuda_error(e, "cudaMalloc", __FILE__, __LINE__);
   }
-  allocs_.push_back(q);
+  allocs_[q] = bytes;
+  held_bytes_ += bytes;
   *p = reinterpret_cast<T*>(q);
   return DV_OK;
 }
@@ -244,9 +274,18 @@ inline int Engine::dalloc(T** p, size_t n) {
 template <class T>
 inline void Engine::dfree(T*& p) {
   if (!p) return;
-  cudaFree(p);
-  auto it = std::find(allocs_.begin(), allocs_.end(), (void*)p);
-  if (it != allocs_.end()) allocs_.erase(it);
+  auto it = allocs_.find((void*)p);
+  if (it != allocs_.end()) {
+    const size_t bytes = it->second;
+    allocs_.erase(it);
+    if (spare_bytes_ + bytes <= kSpareBytes) {
+      spare_.emplace(bytes, (void*)p);
+      spare_bytes_ += bytes;
+    } else {
+      cudaFree(p);
+      held_bytes_ -= bytes;
+    }
+  }
   p = nullptr;
 }
 
