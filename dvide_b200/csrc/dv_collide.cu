@@ -23,8 +23,9 @@
 // Each body's partners with larger id are sorted, so a segment's contacts come
 // out in lexicographic (A, B) order, the order of the reference's sorted unique
 // 64-bit pair keys (CollisionDetector.cu:319-325).  The narrowphase
-// (sphere-sphere, sphere-box; box-box is never a contact) also emits the
-// tangent frame of System.cu:753-762, so no separate Jacobian is built.
+// (sphere-sphere, sphere-box; box-box is never a contact) emits the normal; the
+// tangent frame of System.cu:753-762 follows from it where it is used, so no
+// separate Jacobian is built.
 //
 // Sizes that change every step (contacts, tiles) are read on the device, so
 // the whole pipeline runs without a host round trip and can be captured in a
@@ -357,24 +358,16 @@ struct CollideArgs {
   uint32_t* ida;
   uint32_t* idb;
   double* F;
-  float* nf;
   double* gap;
   double* loc;
 };
 
 __device__ inline void write_contact(const CollideArgs& a, size_t c, int ia, int ib,
-                                     const NpOut& o, bool exact) {
+                                     const NpOut& o) {
   a.ida[c] = (uint32_t)ia;
   a.idb[c] = (uint32_t)ib;
-  d3 u, v;
-  frame_from_normal(o.n, &u, &v, exact);
   size_t S = a.ccap;
   a.F[0 * S + c] = o.n.x; a.F[1 * S + c] = o.n.y; a.F[2 * S + c] = o.n.z;
-  a.F[3 * S + c] = u.x;   a.F[4 * S + c] = u.y;   a.F[5 * S + c] = u.z;
-  a.F[6 * S + c] = v.x;   a.F[7 * S + c] = v.y;   a.F[8 * S + c] = v.z;
-  a.nf[0 * S + c] = (float)o.n.x;
-  a.nf[1 * S + c] = (float)o.n.y;
-  a.nf[2 * S + c] = (float)o.n.z;
   a.gap[c] = o.gap;
   a.loc[0 * S + c] = o.loc.x;
   a.loc[1 * S + c] = o.loc.y;
@@ -516,7 +509,7 @@ __global__ void __launch_bounds__(kThreads) k_sphere_write(CollideArgs a) {
       const int B = (int)a.kept[(size_t)j * kKeep + e];
       NpOut o;
       narrowphase(a.p4, a.g4, A, B, P.env, P.exact != 0, &o);
-      write_contact(a, base + e, A, B, o, P.exact != 0);
+      write_contact(a, base + e, A, B, o);
     }
   }
   unsigned more = __ballot_sync(0xffffffffu, n > kKeep && n <= kMaxPerBody && (lane & 7) == 0);
@@ -534,7 +527,7 @@ __global__ void __launch_bounds__(kThreads) k_sphere_write(CollideArgs a) {
       for (int k = 0; k < n2; ++k) rank += s_buf[warp][k] < B ? 1 : 0;
       NpOut o;
       narrowphase(a.p4, a.g4, A2, B, P.env, P.exact != 0, &o);
-      write_contact(a, base + rank, A2, B, o, P.exact != 0);
+      write_contact(a, base + rank, A2, B, o);
     }
     __syncwarp();
   }
@@ -637,7 +630,7 @@ __global__ void __launch_bounds__(kThreads) k_sphere_pairs_wide(CollideArgs a) {
       const int B = s_ids[e];
       NpOut o;
       narrowphase(a.p4, a.g4, A, B, env, exact, &o);
-      write_contact(a, base + e, A, B, o, exact);
+      write_contact(a, base + e, A, B, o);
     }
   }
 }
@@ -693,7 +686,7 @@ __global__ void __launch_bounds__(kThreads) k_box_pairs(CollideArgs a, int* __re
   pre += __popc(bal & ((1u << lane) - 1u));
   size_t pos = (size_t)(a.cbase[L] + a.sst[sg].delta) +
                (size_t)(chunk_off[crow + blockIdx.x] - chunk_off[crow]) + pre;
-  write_contact(a, pos, L, B, o, P.exact != 0);
+  write_contact(a, pos, L, B, o);
 }
 
 // Binary search of the tile starts: the last segment with tstart <= t and tiles.
@@ -799,6 +792,7 @@ __global__ void __launch_bounds__(1024) k_seg_layout(int nseg, int nb,
       S.c0 = (int)ec;
       S.t0 = (int)et;
       S.nt = (int)nt;
+      S.exact = seg[s].exact;
       S.delta = (int)(ec - (seg[s].active ? cbase[seg[s].b0] : 0));
       seg_tstart[s] = (int)et;
     }
@@ -1054,7 +1048,6 @@ CollideArgs make_args(SceneDev& sd) {
   a.ida = sd.ida;
   a.idb = sd.idb;
   a.F = sd.F;
-  a.nf = sd.nf;
   a.gap = sd.gap;
   a.loc = sd.loc;
   return a;

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kThreads) k_violation_items_flat(
     const double* __restrict__ bil_gam, const double* __restrict__ bil_b,
     const int2* __restrict__ bil_off, const double* __restrict__ F, const double* __restrict__ gap,
     const uint32_t* __restrict__ ida, const uint32_t* __restrict__ idb,
-    const double4* __restrict__ v4, double h, double mu, double* __restrict__ items) {
+    const double4* __restrict__ v4, bool exact, double h, double mu, double* __restrict__ items) {
   int k = blockIdx.x * kThreads + threadIdx.x;
   if (k >= nc) return;
   const double* vd = reinterpret_cast<const double*>(v4);
@@ -139,8 +139,13 @@ __global__ void __launch_bounds__(kThreads) k_violation_items_flat(
     const int c = c0 + (int)(q / 3);
     const double4 va = v4[ida[c]], vb = v4[idb[c]];
     const double d0 = va.x - vb.x, d1 = va.y - vb.y, d2 = va.z - vb.z;
-    const double* f = F + (size_t)(3 * row) * S + c;
-    const double dv = (f[0] * d0 + f[S] * d1) + f[2 * S] * d2;
+    d3 f = mk3(F[c], F[S + c], F[2 * S + c]);
+    if (row) {
+      d3 u, v;
+      frame_from_normal(f, &u, &v, exact);
+      f = row == 1 ? u : v;
+    }
+    const double dv = (f.x * d0 + f.y * d1) + f.z * d2;
     return (row == 0 ? gap[c] / h : 0.0) + dv;
   };
   const long long j = 3LL * k;
@@ -208,7 +213,7 @@ int Engine::ccp_violation(int s, double* out4) {
     k_violation_items_flat<<<(nc + kThreads - 1) / kThreads, kThreads, 0, st_>>>(
         nc, hseg_[s].nbil, X.c0, d.ccap, hseg_[s].wbase, d.wtotal, d.gamma,
         d.bil_gam + hseg_[s].bil0, d.bil_b + hseg_[s].bil0, d.bil_off + hseg_[s].bil0, d.F, d.gap,
-        d.ida, d.idb, d.v4, P_[s].h, P_[s].mu, items);
+        d.ida, d.idb, d.v4, X.exact != 0, P_[s].h, P_[s].mu, items);
   else
     k_violation_items<<<(nc + kThreads - 1) / kThreads, kThreads, 0, st_>>>(
         nc, X.c0, d.ccap, hseg_[s].wbase, d.wtotal, d.gamma, d.F, d.gap, d.ida, d.idb, d.v4,

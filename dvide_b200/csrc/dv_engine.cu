@@ -108,7 +108,7 @@ int Engine::alloc_contacts(size_t cap) {
   // segment ranges start on multiples of 256 and the solve kernel copies
   // 32-contact plane segments with bulk asynchronous copies
   cap = (cap + kContactAlign - 1) / kContactAlign * kContactAlign;
-  dfree(q.ida); dfree(q.idb); dfree(q.F); dfree(q.nf); dfree(q.gap); dfree(q.loc);
+  dfree(q.ida); dfree(q.idb); dfree(q.F); dfree(q.gap); dfree(q.loc);
   dfree(q.r); dfree(q.blk);
   for (int k = 0; k < 5; ++k) dfree(q.G[k]);
   dfree(q.q); dfree(q.inc); dfree(q.part); dfree(q.tseg);
@@ -117,8 +117,7 @@ int Engine::alloc_contacts(size_t cap) {
   q.tcap = (int)(cap / kTileItems) + q.nseg + 1 + (q.nbil + kTileItems - 1) / kTileItems;
   TRY(dalloc(&q.ida, cap));
   TRY(dalloc(&q.idb, cap));
-  TRY(dalloc(&q.F, 9 * cap));
-  TRY(dalloc(&q.nf, 3 * cap));
+  TRY(dalloc(&q.F, 3 * cap));
   TRY(dalloc(&q.gap, cap));
   TRY(dalloc(&q.loc, 3 * cap));
   TRY(dalloc(&q.r, 3 * cap));
@@ -1161,10 +1160,29 @@ __global__ void __launch_bounds__(kThreads) k_rows_to_planes(const double* __res
   for (int j = 0; j < k; ++j) dst[j * stride + first + i] = src[(size_t)i * k + j];
 }
 
+// A contact's frame from its normal (System.cu:753-762).
+__device__ inline void frame_at(const double* __restrict__ F, size_t S, int c, bool exact, d3 (&f)[3]) {
+  f[0] = mk3(F[c], F[S + c], F[2 * S + c]);
+  frame_from_normal(f[0], &f[1], &f[2], exact);
+}
+__global__ void __launch_bounds__(kThreads) k_frames(const double* __restrict__ F, size_t S, int c0, int nc,
+                                                    bool exact, double* __restrict__ out) {
+  const int i = blockIdx.x * kThreads + threadIdx.x;
+  if (i >= nc) return;
+  d3 f[3];
+  frame_at(F, S, c0 + i, exact, f);
+  for (int r = 0; r < 3; ++r) {
+    out[9 * (size_t)i + 3 * r] = f[r].x;
+    out[9 * (size_t)i + 3 * r + 1] = f[r].y;
+    out[9 * (size_t)i + 3 * r + 2] = f[r].z;
+  }
+}
+
 // System.cu:1259-1295: normal and friction force per contact, gamma 0 past the
 // warm start's length m.
 __global__ void __launch_bounds__(kThreads) k_contact_forces(const double* __restrict__ F, size_t S, int c0,
-                                                            int nc, const double* __restrict__ gamma,
+                                                            int nc, bool exact,
+                                                            const double* __restrict__ gamma,
                                                             size_t WS, size_t w0, int m, double h,
                                                             double* __restrict__ normal,
                                                             double* __restrict__ friction) {
@@ -1172,11 +1190,16 @@ __global__ void __launch_bounds__(kThreads) k_contact_forces(const double* __res
   if (i >= nc) return;
   const double g0 = i < m ? gamma[w0 + i] : 0.0, g1 = i < m ? gamma[WS + w0 + i] : 0.0,
                g2 = i < m ? gamma[2 * WS + w0 + i] : 0.0;
-  for (int k = 0; k < 3; ++k) {
-    const double* f = F + (size_t)k * S + c0 + i;
-    normal[3 * (size_t)i + k] = (g0 * f[0]) / h;
-    friction[3 * (size_t)i + k] = (g1 * f[3 * S] + g2 * f[6 * S]) / h;
-  }
+  d3 f[3];
+  frame_at(F, S, c0 + i, exact, f);
+  double* n = normal + 3 * (size_t)i;
+  double* t = friction + 3 * (size_t)i;
+  n[0] = (g0 * f[0].x) / h;
+  n[1] = (g0 * f[0].y) / h;
+  n[2] = (g0 * f[0].z) / h;
+  t[0] = (g1 * f[1].x + g2 * f[2].x) / h;
+  t[1] = (g1 * f[1].y + g2 * f[2].y) / h;
+  t[2] = (g1 * f[1].z + g2 * f[2].z) / h;
 }
 
 int blocks_of(int n) { return (n + kThreads - 1) / kThreads; }
@@ -1219,12 +1242,20 @@ int Engine::copy_schur_vector_out(int c0, int nc, double* r) {
   return download(r, stage3_, sizeof(double) * 3 * (size_t)nc);
 }
 
+int Engine::copy_frames_out(int s, double* F) {
+  const int nc = h_sst_[s].nc;
+  if (nc <= 0) return DV_OK;
+  TRY(ensure_stage(9 * (size_t)nc));
+  k_frames<<<blocks_of(nc), kThreads, 0, st_>>>(d.F, d.ccap, h_sst_[s].c0, nc, h_sst_[s].exact != 0, stage3_);
+  return download(F, stage3_, sizeof(double) * 9 * (size_t)nc);
+}
+
 int Engine::copy_contact_forces_out(int s, double* normal, double* friction) {
   const int nc = h_sst_[s].nc, c0 = h_sst_[s].c0;
   if (nc <= 0) return DV_OK;
   TRY(ensure_stage(6 * (size_t)nc));
   double* f = stage3_ + 3 * (size_t)nc;
-  k_contact_forces<<<blocks_of(nc), kThreads, 0, st_>>>(d.F, d.ccap, c0, nc, d.gamma, d.wtotal,
+  k_contact_forces<<<blocks_of(nc), kThreads, 0, st_>>>(d.F, d.ccap, c0, nc, h_sst_[s].exact != 0, d.gamma, d.wtotal,
                                                        (size_t)hseg_[s].wbase,
                                                        std::min(h_sst_[s].gsize, hseg_[s].wcap), P_[s].h,
                                                        stage3_, f);

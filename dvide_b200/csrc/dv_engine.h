@@ -125,10 +125,11 @@ class Engine {
   // k planes of n values (stride apart, from item `first`) as n rows of k.
   int copy_rows_out(const double* planes, size_t stride, size_t first, int n, int k, double* out);
   // Contact quantities in the reference's layouts, interleaved on the device:
-  // normal and gap (4 per contact), the Schur vector (3), and the forces per
-  // contact of segment s (3 each; either may be null).
+  // normal and gap (4 per contact), the Schur vector (3), the frames of segment
+  // s (9) and its forces per contact (3 each; either may be null).
   int copy_normals_out(int c0, int nc, double* nP);
   int copy_schur_vector_out(int c0, int nc, double* r);
+  int copy_frames_out(int s, double* F);
   int copy_contact_forces_out(int s, double* normal, double* friction);
 
   // System::getCCPViolation (System.cu:1590-1643) and the energies

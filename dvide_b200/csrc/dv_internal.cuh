@@ -18,8 +18,8 @@
 //   contacts:     per segment sorted by (A, B) like the reference's
 //                 thrust::unique of 64-bit pair keys (CollisionDetector.cu:
 //                 319-325); segment s owns [c0, c0 + nc), c0 a multiple of 256.
-//                 ids A/B (uint32, global body ids), normal n as 3 planes (plus
-//                 u, v for the frame accessors), gap, location (3 planes); every
+//                 ids A/B (uint32, global body ids), normal n as 3 planes, gap,
+//                 location (3 planes); every
 //                 per-contact 3-vector is 3 planes of stride `ccap` (structure
 //                 of arrays, coalesced loads).
 //   tiles:        512 contacts; segment s owns tiles [t0, t0 + nt); tile k of
@@ -94,6 +94,7 @@ struct SegState {
   int gsize;            // warm-start length (System::gamma_d / 3); kept when nc = 0
   unsigned err;         // error bits of this segment's last step
   int members;          // CTAs of its team in this launch (engines of several segments)
+  int exact;            // mode of the contacts' frames: SegParams::exact at their detection
   SolveResult ctl;
 };
 
@@ -126,7 +127,7 @@ constexpr int kWideGrid = 256;
 constexpr int kWidePartners = 8192;
 // Partners per sphere that the count pass keeps for the write pass, and the
 // bodies up to which an engine takes the short forms of collision detection.
-constexpr int kKeepPartners = 16;
+constexpr int kKeepPartners = 8;
 constexpr int kFewBodies = 6144;
 
 // Tiles that a team's member takes at most when there are more than the grid
@@ -181,8 +182,7 @@ struct SceneDev {
   size_t ccap = 0;            // contact slots
   int tcap = 0;               // tiles
   uint32_t *ida = nullptr, *idb = nullptr;
-  double* F = nullptr;        // 9 planes (n, u, v)
-  float* nf = nullptr;        // 3 planes: n rounded to float (mixed-precision solve)
+  double* F = nullptr;        // 3 planes: the normal (B -> A)
   double* gap = nullptr;
   double* loc = nullptr;      // 3 planes
   double* r = nullptr;        // 3 planes (float planes in the mixed solve)

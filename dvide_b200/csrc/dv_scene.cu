@@ -209,8 +209,7 @@ DV_API int dv_get_frames(dv_scene* s, double* F) {
   if (!s || !F) return DV_ERR_ARG;
   Engine& E = s->E;
   TRY(E.sync_state());
-  const int nc = E.seg_state(0).nc, c0 = E.seg_state(0).c0;
-  return E.copy_rows_out(E.d.F, E.d.ccap, c0, nc, 9, F);
+  return E.copy_frames_out(0, F);
 }
 
 DV_API int dv_get_schur_vector(dv_scene* s, double* r) {

@@ -52,7 +52,6 @@ struct KArgs {
   const uint32_t* __restrict__ ida;
   const uint32_t* __restrict__ idb;
   const double* __restrict__ F;
-  const float* __restrict__ nf;
   const double* __restrict__ gap;
   T* r;
   T* fr;              // PGJ, PGS: frame words (FrameWords), 3 planes, written by the setup pass
@@ -99,8 +98,7 @@ struct Frame {
   T n0, n1, n2, u0, u1, u2, v0, v1, v2;
 };
 
-// The FP64 frame, recomputed from the stored normal with the narrowphase's own
-// function and the scene's mode (same bits as the stored u, v planes).
+// The FP64 frame of a normal in the scene's mode.
 __device__ inline Frame<double> frame_d(double n0, double n1, double n2, bool exact) {
   d3 u, v;
   frame_from_normal(mk3(n0, n1, n2), &u, &v, exact);
@@ -171,29 +169,18 @@ __device__ inline Frame<T> make_frame(T n0, T n1, T n2, const FrameWords<T>& w) 
   return f;
 }
 
-// Normal planes in the solve's precision.
-template <class T> __device__ inline const T* normal_planes(const KArgs<T>& a);
-template <> __device__ inline const double* normal_planes<double>(const KArgs<double>& a) {
-  return a.F;
-}
-template <> __device__ inline const float* normal_planes<float>(const KArgs<float>& a) {
-  return a.nf;
-}
-
 // The frame of contact c from the normal and the words that a solve's setup
 // pass left in the fr planes.
 template <class T>
 __device__ inline Frame<T> load_frame(const KArgs<T>& a, int c) {
-  const T* n = normal_planes<T>(a);
   const FrameWords<T> w{a.fr[c], a.fr[a.S + c], a.fr[2 * a.S + c]};
-  return make_frame<T>(n[c], n[a.S + c], n[2 * a.S + c], w);
+  return make_frame<T>((T)__ldg(a.F + c), (T)__ldg(a.F + a.S + c), (T)__ldg(a.F + 2 * a.S + c), w);
 }
 
 // Setup: forms the words of contact c, keeps them and returns the frame.
 template <class T>
 __device__ inline Frame<T> start_frame(const KArgs<T>& a, int c, bool exact) {
-  const T* n = normal_planes<T>(a);
-  const T n0 = n[c], n1 = n[a.S + c], n2 = n[2 * a.S + c];
+  const T n0 = (T)__ldg(a.F + c), n1 = (T)__ldg(a.F + a.S + c), n2 = (T)__ldg(a.F + 2 * a.S + c);
   const FrameWords<T> w = frame_words(n0, n1, n2, exact);
   a.fr[c] = w.a;
   a.fr[a.S + c] = w.b;
@@ -669,7 +656,6 @@ KArgs<T> make_kargs(SceneDev& sd, const SolveConfig& cfg) {
   a.ida = sd.ida;
   a.idb = sd.idb;
   a.F = sd.F;
-  a.nf = sd.nf;
   a.gap = sd.gap;
   a.r = reinterpret_cast<T*>(sd.r);
   a.fr = a.blk = reinterpret_cast<T*>(sd.blk);

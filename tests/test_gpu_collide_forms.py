@@ -22,8 +22,8 @@ def _cluster(nb):
 
 
 @pytest.mark.parametrize("make", [
-    # kept partners end at 16, the warp's list at 128
-    *[lambda n=n: scenes.crowd(n, max_iterations=10) for n in (15, 16, 17, 31, 33, 127, 130)],
+    # kept partners end at 8, the warp's list at 128
+    *[lambda n=n: scenes.crowd(n, max_iterations=10) for n in (7, 8, 9, 31, 33, 127, 130)],
     # the crowded sphere last: second in all its contacts; 24 is one thread's longest run
     *[lambda n=n: _reversed(scenes.crowd(n, max_iterations=10)) for n in (23, 24, 25, 26, 200)],
     lambda: _reversed(scenes.raspberry(1500, max_iterations=5)),
@@ -62,3 +62,19 @@ def test_families_and_many_small_scenes(native):
         for x, y in zip(few.state(i), many.state(i)):
             assert np.array_equal(x, y)
         assert few.scene_stats()[i] == many.scene_stats()[i]
+
+
+def test_frames_keep_the_mode_of_their_detection(native, oracle_mod):
+    """Frames and forces are those of the step, also after the mode is changed."""
+    sc = scenes.random_cluster(6, n=60)
+    sc.params["fp64_narrowphase"] = 1
+    g = native.NativeScene.from_scene(sc)
+    o = oracle_mod.OracleScene(sc)
+    g.step(1)
+    o.step(1)
+    forces = g.contact_forces()
+    g.set_params(fp64_narrowphase=0)
+    assert np.array_equal(g.frames(), o.frames())
+    for x, y in zip(g.contact_forces(), forces):
+        assert np.array_equal(x, y)
+    g.close()
