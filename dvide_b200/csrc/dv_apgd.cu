@@ -836,8 +836,7 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
           __syncthreads();
         }
 
-        // ---- the contact pass's sub-tiles of this member; its first two are
-        // copied while the body pass runs
+        // ---- the contact pass's sub-tiles of this member
         const int cur = C.cur, nw = C.nw, restart = C.restart;
         auto issue = [&](int j) {  // this warp's sub-tile j into stage j & 1
           const int t = team_tile(tm, tm.ntc, tile_of(j));
@@ -857,19 +856,21 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
                        2 * B::kHalfBytes, bar);
           }
         };
-        // this warp's earlier writes of the iterates, and its reads of the
-        // stages, come before the copies (once for the pass: a fence of global
-        // memory waits for the warp's stores)
-        asm volatile("fence.proxy.async;" ::: "memory");
-        __syncwarp();
-        issue(0);
-        issue(1);
         team_body_pass<T, kAR>(a, tm, bodies, wv, qv);
-        if (!team_sync(a, tm, false, [&]() { ctl_ahead(C); })) {
+        // while the barrier waits: the copies of the first two sub-tiles, and the
+        // next controller's scalars.  This warp's earlier writes of the iterates,
+        // and its reads of the stages, come before the copies (once for the pass:
+        // a fence of global memory waits for the warp's stores).
+        if (!team_sync(a, tm, false, [&]() {
+              asm volatile("fence.proxy.async;" ::: "memory");
+              __syncwarp();
+              issue(0);
+              issue(1);
+              if (threadIdx.x == 32) ctl_ahead(C);
+            })) {
           drain_warp_stages(stg, &a.ew->wait_limit_ns);
           return;
         }
-
         timer.mark(a, kPhaseBody);
 
         // N gamma_new, objective (APGD.cu:237-238), residual (:90-102); then the

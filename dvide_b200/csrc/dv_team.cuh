@@ -62,41 +62,41 @@ __device__ inline void red_add(unsigned* p, unsigned v) {
 // polls after it.  False after a time limit or another CTA's.  The first
 // barrier of a team (`joining`) may wait for members that are still busy with
 // earlier scenes: there the limit starts again while any team makes progress.
-// Meanwhile one thread of another warp runs `other`.
+// `other` is run by all threads between the arrival and the polls.
 struct Nothing {
   __device__ void operator()() const {}
 };
 template <class K, class Fn = Nothing>
 __device__ inline bool team_sync(const K& a, Team& t, bool joining = false, Fn other = Fn{}) {
   __syncthreads();
-  if (threadIdx.x == 32) other();
   if (threadIdx.x == 0) {
     if (a.nseg > 1 && t.rank == 0) red_add(&a.ew->progress, 1u);
-    if (t.m > 1) {
-      t.target += (unsigned)t.m;
-      const unsigned target = t.target;
-      red_add_release(t.bar, 1u);
-      unsigned polls = 0, seen = 0;
-      uint64_t t0 = 0;
-      while ((int)(ld_acquire(t.bar) - target) < 0) {
-        if (joining) __nanosleep(200);
-        if ((++polls & 1023u) == 0u) {
-          if (ld_acquire(&a.ew->err) & (kErrBarrierTimeout | kErrCopyTimeout)) {
-            t.fail = 1;
-            break;
-          }
-          const uint64_t now = global_ns();
-          if (t0 == 0) t0 = now;
-          if (joining) {
-            const unsigned p = ld_acquire(&a.ew->progress);
-            if (p != seen) t0 = now;
-            seen = p;
-          }
-          if (now - t0 > a.ew->wait_limit_ns) {
-            atomicOr(&a.ew->err, kErrBarrierTimeout);
-            t.fail = 1;
-            break;
-          }
+    if (t.m > 1) red_add_release(t.bar, 1u);
+  }
+  other();
+  if (threadIdx.x == 0 && t.m > 1) {
+    t.target += (unsigned)t.m;
+    const unsigned target = t.target;
+    unsigned polls = 0, seen = 0;
+    uint64_t t0 = 0;
+    while ((int)(ld_acquire(t.bar) - target) < 0) {
+      if (joining) __nanosleep(200);
+      if ((++polls & 1023u) == 0u) {
+        if (ld_acquire(&a.ew->err) & (kErrBarrierTimeout | kErrCopyTimeout)) {
+          t.fail = 1;
+          break;
+        }
+        const uint64_t now = global_ns();
+        if (t0 == 0) t0 = now;
+        if (joining) {
+          const unsigned p = ld_acquire(&a.ew->progress);
+          if (p != seen) t0 = now;
+          seen = p;
+        }
+        if (now - t0 > a.ew->wait_limit_ns) {
+          atomicOr(&a.ew->err, kErrBarrierTimeout);
+          t.fail = 1;
+          break;
         }
       }
     }
