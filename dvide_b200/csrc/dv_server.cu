@@ -118,9 +118,10 @@ struct dv_server {
       rc = E->init(in, cfg.precision);
       if (rc == DV_OK && user_stream) rc = E->set_stream(user_stream);
       // FP32 iterates fit three CTAs per SM (80 registers); results do not
-      // depend on the launch shape
+      // depend on the launch shape.  Round-robin tiles: 256 mixed scenes took 166
+      // ms a step that way and 179 in contiguous ranges, 200 small ones 4.8 and 5.7.
       if (rc == DV_OK) {
-        if (cfg.precision == DV_PREC_MIXED) E->set_launch(E->max_ctas_for(3), 1, 1, 3);
+        if (cfg.precision == DV_PREC_MIXED) E->set_launch(E->max_ctas_for(3), 1, 0, 3);
         else E->set_launch(E->max_ctas(), 1, 0, 2);
       }
     }

@@ -231,7 +231,7 @@ DV_API int dv_ccp_violation_noalloc(int32_t nc, int32_t nb, const double* gamma,
  * Batched scenes.  No counterpart in the reference (DVIDE steps one System
  * per process).  A batch steps many independent scenes together: one
  * collision pipeline and ONE persistent solve kernel per step for all of
- * them, each scene with its own parameters, contact set, warm start and APGD
+ * them (teams of CTAs, a scene each), each scene with its own parameters, contact set, warm start and APGD
  * convergence (a converged scene stops iterating while the others go on).
  * Every reduction of a scene runs over that scene's own tiles in a fixed
  * order, so each scene's results are bit-identical to the same scene stepped
@@ -255,9 +255,10 @@ typedef struct dv_scene_stats {
 } dv_scene_stats;
 
 typedef struct dv_tune_candidate {
-  int32_t grid;              /* CTAs of the persistent solve kernel */
-  int32_t chunk;             /* consecutive 512-contact tiles a CTA takes at a time */
-  int32_t contiguous;        /* 1: each CTA owns one contiguous tile range (scenes per CTA) */
+  int32_t grid;              /* CTAs of the persistent solve kernel, of 256 threads (a batch of one
+                                scene of at most 20480 bodies runs half as many of 512) */
+  int32_t chunk;             /* consecutive 512-contact tiles of a scene a CTA takes at a time */
+  int32_t contiguous;        /* 1: each CTA owns one contiguous tile range of its scene */
   int32_t blocks_per_sm;     /* 2 (128 registers per thread) or 3 (80; DV_PREC_MIXED only) */
   float ms_per_step;         /* measured device time per step */
 } dv_tune_candidate;
