@@ -70,7 +70,7 @@ Engine::~Engine() {
   if (h_sst_ring_) cudaFreeHost(h_sst_ring_);
   if (h_red_) cudaFreeHost(h_red_);
   for (cudaEvent_t e : ev_) cudaEventDestroy(e);
-  if (own_stream_ && st_) cudaStreamDestroy(st_);
+  if (own_st_) cudaStreamDestroy(own_st_);
 }
 
 void Engine::free_spare() {
@@ -242,9 +242,9 @@ int Engine::init(const std::vector<SceneInput>& scenes, int precision) {
   if (precision != DV_PREC_FP64 && precision != DV_PREC_MIXED) return DV_ERR_UNSUPPORTED;
   // arguments first: nothing touches the device for an invalid scene
   for (const SceneInput& sc : scenes) TRY(validate_scene(sc));
-  if (cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking) != cudaSuccess)
+  if (cudaStreamCreateWithFlags(&own_st_, cudaStreamNonBlocking) != cudaSuccess)
     return dv_record_cuda_error(cudaGetLastError(), "cudaStreamCreate", __FILE__, __LINE__);
-  own_stream_ = true;
+  st_ = own_st_;
   d.precision = precision;
   TRY(dalloc(&d.ew, 1));
   TRY(dalloc(&d.wide_ids, kWideSpheres));
@@ -642,11 +642,7 @@ void Engine::set_launch(int grid, int chunk, int contiguous, int blocks_per_sm) 
 
 int Engine::set_stream(cudaStream_t s) {
   DV_CUDA_TRY(cudaStreamSynchronize(st_));
-  if (s) {
-    if (own_stream_) cudaStreamDestroy(st_);
-    own_stream_ = false;
-    st_ = s;
-  }
+  if (s) st_ = s;
   return DV_OK;
 }
 

@@ -87,6 +87,7 @@ class Engine {
   bool graph_failed() const { return graph_failed_; }
 
   int set_stream(cudaStream_t s);
+  int use_own_stream() { return set_stream(own_st_); }
   cudaStream_t stream() const { return st_; }
   int set_segment_params(int s, const dv_params& P);
   const dv_params& segment_params(int s) const { return P_[s]; }
@@ -179,7 +180,7 @@ class Engine {
   void ordered_sum_dev(const double* items, int n, double* part, int slot);
 
   cudaStream_t st_ = nullptr;
-  bool own_stream_ = false;
+  cudaStream_t own_st_ = nullptr;  // the engine's own; st_ is it or the caller's
   std::unordered_map<void*, size_t> allocs_;  // device memory and its sizes
   size_t held_bytes_ = 0;                     // ... of them and the spare blocks
   std::multimap<size_t, void*> spare_;        // freed blocks by size

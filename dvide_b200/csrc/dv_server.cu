@@ -75,6 +75,7 @@ struct dv_server {
   double bytes_in_use = 0;
   bool departed = false;  // scenes left since the engine layout was built
   bool idle = false;      // nothing is resident in the engine
+  int device = 0;         // the engine's
   dv_server_stats st{};
 
   double now() const {
@@ -82,8 +83,10 @@ struct dv_server {
   }
 
   // Nothing is resident: the device memory is freed, up to what an idle server keeps.
+  // The caller's stream may end before the next requests: an idle engine has left it.
   void set_idle() {
-    if (E && E->held_bytes() > kIdleBytes) E.reset();
+    if (idle || !E) return;
+    if (E->held_bytes() > kIdleBytes || E->use_own_stream() != DV_OK) E.reset();
     idle = E != nullptr;
   }
 
@@ -101,13 +104,16 @@ struct dv_server {
       }
     }
     // an engine kept while idle serves any new scenes but those that only a
-    // fresh one takes
-    bool special = E && E->d.anti_relax;
+    // fresh one takes, and those of a caller that has moved to another device
+    int dev = 0;
+    DV_CUDA_TRY(cudaGetDevice(&dev));
+    bool special = E && (E->d.anti_relax || dev != device);
     for (const auto& r : next) special |= r->P.anti_relaxation != 0;
     if (idle && special) E.reset();
     int rc = DV_OK;
     if (E) {
-      rc = E->reconfigure(slots);
+      if (idle && user_stream) rc = E->set_stream(user_stream);
+      if (rc == DV_OK) rc = E->reconfigure(slots);
       if (rc != DV_OK && idle) E.reset();
     }
     idle = false;
@@ -115,6 +121,7 @@ struct dv_server {
       std::vector<SceneInput> in(slots.size());
       for (size_t i = 0; i < slots.size(); ++i) in[i] = slots[i].in;
       E.reset(new Engine());
+      device = dev;
       rc = E->init(in, cfg.precision);
       if (rc == DV_OK && user_stream) rc = E->set_stream(user_stream);
       // FP32 iterates fit three CTAs per SM (80 registers); results do not
@@ -319,7 +326,7 @@ DV_API int dv_server_destroy(dv_server* s) {
 DV_API int dv_server_set_stream(dv_server* s, void* cuda_stream) {
   if (!s) return DV_ERR_ARG;
   s->user_stream = (cudaStream_t)cuda_stream;
-  if (s->E && cuda_stream) return s->E->set_stream((cudaStream_t)cuda_stream);
+  if (s->E && !s->idle && cuda_stream) return s->E->set_stream((cudaStream_t)cuda_stream);
   return DV_OK;
 }
 
