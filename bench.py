@@ -95,10 +95,10 @@ def solve_bytes_one_product(nc, nb, sweeps, backtracks):
 
 
 # DRAM bytes per algorithmic byte of the solve kernel, measured with ncu
-# (dram__bytes_read.sum + dram__bytes_write.sum = 4.371 + 1.994 GB) on a
+# (dram__bytes_read.sum + dram__bytes_write.sum = 5.118 + 1.965 GB) on a
 # 30-iteration launch on this workload (11.415 GB algorithmic); the full launch
 # is scaled by it.
-TRAFFIC_PER_ALGORITHMIC_BYTE = 6.365664 / 11.415179
+TRAFFIC_PER_ALGORITHMIC_BYTE = 7.083004 / 11.415179
 
 
 def collide_bytes(nc, nb, npossible):
@@ -522,10 +522,10 @@ SERVED_SPEC_RECORD = {
     "workload": "12000 requests, Poisson 200/s for 60 s, 200 steps each (h 1e-3), spheres "
                 "log-uniform [500, 50000], mixed precision with up to 500 FP64 refinement "
                 "iterations, 150 GB budget",
-    "value": 21.16e6, "unit": "contact-steps/s (wall clock, arrivals included)",
-    "device_contact_steps_per_s": 23.27e6, "speedup_vs_plain": 11.7,
-    "time_per_step_ms": {"p50": 1317, "p99": 2260},
-    "completion_latency_s": {"p50": 479, "p99": 683},
+    "value": 31.18e6, "unit": "contact-steps/s (wall clock, arrivals included)",
+    "device_contact_steps_per_s": 35.22e6, "speedup_vs_plain": 9.2,
+    "time_per_step_ms": {"p50": 793, "p99": 1226},
+    "completion_latency_s": {"p50": 317, "p99": 450},
     "peak_resident_gb": 101.7, "completed": 12000,
     "source": "recorded, not measured in this run: profiles/served_poisson_200ps_60s.md "
               "(python bench.py --steps 3 --warmup 3 --no-batched --no-mixed-error "
