@@ -446,7 +446,7 @@ __device__ inline int find_partners(const CollideArgs& a, int A, int sg, int* bu
 // Count pass, one warp per sphere; up to kKeep partners (in a settled pile 3.7
 // on average) are kept in ascending order for the write pass, which otherwise
 // would search again.  On 200,000 settled spheres the two passes took 369 and 451
-// us when each read boxes and spheres body by body, and take 306 and 95.
+// us when each read boxes and spheres body by body, and take 305 and 86.
 __global__ void __launch_bounds__(kThreads) k_sphere_count(CollideArgs a) {
   __shared__ int s_buf[kWarpsPerCta][kMaxPerBody];
   __shared__ int s_cnt[kWarpsPerCta];

@@ -247,7 +247,7 @@ enum : unsigned {
   kErrPartners = 64u,     // a sphere has more contact partners than the pair kernel keeps
 };
 
-// Longest a CTA waits at a grid barrier before it records a timeout and
+// Longest a CTA waits at a team barrier before it records a timeout and
 // leaves the kernel (a barrier normally completes in microseconds).
 constexpr uint64_t kBarrierTimeoutNs = 2000000000ull;
 

@@ -231,7 +231,8 @@ DV_API int dv_ccp_violation_noalloc(int32_t nc, int32_t nb, const double* gamma,
  * Batched scenes.  No counterpart in the reference (DVIDE steps one System
  * per process).  A batch steps many independent scenes together: one
  * collision pipeline and ONE persistent solve kernel per step for all of
- * them (teams of CTAs, a scene each), each scene with its own parameters, contact set, warm start and APGD
+ * them (teams of CTAs, a scene each), each scene with its own parameters,
+ * contact set, warm start and APGD
  * convergence (a converged scene stops iterating while the others go on).
  * Every reduction of a scene runs over that scene's own tiles in a fixed
  * order, so each scene's results are bit-identical to the same scene stepped
@@ -381,7 +382,7 @@ DV_API int dv_server_result_state(dv_server* s, int64_t id, double* p, double* v
 DV_API int dv_server_get_stats(dv_server* s, dv_server_stats* out);
 
 /* Failure detection without a fault: runs the solve kernels' bounded waits
- * (grid barrier, bulk-copy mbarrier) against conditions that never become
+ * (team barrier, bulk-copy mbarrier) against conditions that never become
  * true -- a CTA that never arrives, bytes no copy brings -- with a limit of
  * limit_ms, and reports whether each wait ended by its time limit
  * (*barrier_timed_out, *copy_timed_out = 1) and the error bits it left.  The
