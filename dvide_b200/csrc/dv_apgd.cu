@@ -1337,7 +1337,6 @@ void plan_teams(SceneDev& sd, int grid, bool refine, cudaStream_t st, int64_t* l
     ++*launches;
   } else {
     cudaMemsetAsync(sd.team_bar, 0, sizeof(unsigned), st);
-    if (!refine) cudaMemsetAsync(&sd.sst->err, 0, sizeof(unsigned), st);
   }
 }
 

@@ -106,7 +106,9 @@ __device__ inline bool team_sync(const K& a, Team& t, bool joining = false, Fn o
 }
 
 // Takes the next slot of the plan; false when there is none left.  One scene
-// needs no plan: its team is the first m CTAs.
+// needs no plan: its team is the first m CTAs, and the first of them clears the
+// scene's error bits, as the plan does for the others: in a launch that works,
+// so the mark that a failed collision detection leaves on its scene stays.
 template <class K>
 __device__ inline bool join_team(const K& a, Team& t, int* slot_seen) {
   __syncthreads();  // the last scene's reads of the team are done
@@ -115,6 +117,7 @@ __device__ inline bool join_team(const K& a, Team& t, int* slot_seen) {
     if (a.nseg == 1) {
       m = *slot_seen ? 0 : team_size(a.sst[0].nt, a.nb, 1, gridDim.x);
       rank = blockIdx.x;
+      if (rank == 0 && m > 0 && !a.refine) a.sst[0].err = 0u;
       if (rank < m && (a.seg[0].active != 0) && (!a.refine || a.sst[0].ctl.refined)) s = 0;
     } else {
       const unsigned slot = atomicAdd(&a.ew->ticket, 1u);
