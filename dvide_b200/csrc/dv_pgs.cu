@@ -283,11 +283,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
             if (tm.rank == 0) {
               const int to = min(nc, from + kPgsChunk);
               odd |= pgs_sweep(a, tm, P, Gc, Gn, cone, from, to, strict != 0);
-              if (to == nc && threadIdx.x == 0) a.sst[s].ctl.mode = odd ? 1 : 0;
+              // a strict sweep leaves the word alone: members that are slow to
+              // leave the barrier may still read it
+              if (to == nc && !strict && threadIdx.x == 0) a.sst[s].ctl.mode = odd ? 1 : 0;
             }
             if (!sync(kPhaseStep)) return;
           }
-          if (__ldcg(&a.sst[s].ctl.mode) == 0) break;
+          if (strict || __ldcg(&a.sst[s].ctl.mode) == 0) break;
         }
         team_body_pass<double, false>(a, tm, bodies, wv, qv);
         if (!sync(kPhaseBody)) return;
