@@ -30,7 +30,10 @@
 // product to the parallel body and contact passes.  The working velocities
 // live in v4, which the update at the end of the step overwrites, as the
 // reference's sweep overwrites System::v.
+#include <string.h>
+
 #include <algorithm>
+#include <vector>
 
 #include "dv_team.cuh"
 
@@ -68,8 +71,11 @@ __device__ inline void pgs_ctl(PgsSolve& C, const double* m, const SegParams& P)
 // Contacts [from, to) of the scene, from gamma in Gc to gamma in Gn, by one CTA
 // (all its threads).  `strict`: fixed bodies' contacts one after another too.
 // Returns, in every thread, whether a fixed body's velocity would have changed
-// (only without `strict`).
-__device__ bool pgs_sweep(const KArgs<double>& a, const Team& tm, const SegParams& P, const double* Gc,
+// (only without `strict`).  Every round updates at least the first contact that
+// is left; one that updates none, because the counts and the incidence disagree,
+// ends the sweep with an error instead of a wait without end.
+enum PgsSweep : int { kSweepDone = 0, kSweepOdd = 1, kSweepStalled = 2 };
+__device__ PgsSweep pgs_sweep(const KArgs<double>& a, const Team& tm, const SegParams& P, const double* Gc,
                           double* Gn, const Cone<double>& cone, int from, int to, bool strict) {
   const size_t S = a.S;
   const double h = P.h;
@@ -103,7 +109,10 @@ __device__ bool pgs_sweep(const KArgs<double>& a, const Team& tm, const SegParam
     const bool wait_a = strict || mia != 0.0, wait_b = strict || mib != 0.0;
     while (__syncthreads_or(todo)) {
       const bool go = todo && (!wait_a || done_of[ia] == at.x) && (!wait_b || done_of[ib] == at.y);
-      __syncthreads();  // every thread has read the counts
+      if (!__syncthreads_or(go)) {  // every thread has read the counts
+        if (threadIdx.x == 0) atomicOr(&a.ew->err, kErrBarrierTimeout);
+        return kSweepStalled;
+      }
       if (!go) continue;
       const double4 va = v[ia], vb = v[ib];
       double g0 = o0 - ob * (f.n0 * va.x + f.n1 * va.y + f.n2 * va.z - f.n0 * vb.x - f.n1 * vb.y -
@@ -141,7 +150,7 @@ __device__ bool pgs_sweep(const KArgs<double>& a, const Team& tm, const SegParam
       todo = false;
     }
   }
-  return __syncthreads_or(odd);
+  return __syncthreads_or(odd) ? kSweepOdd : kSweepDone;
 }
 
 __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
@@ -282,7 +291,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
           for (int from = 0; from < nc; from += kPgsChunk) {
             if (tm.rank == 0) {
               const int to = min(nc, from + kPgsChunk);
-              odd |= pgs_sweep(a, tm, P, Gc, Gn, cone, from, to, strict != 0);
+              const PgsSweep r = pgs_sweep(a, tm, P, Gc, Gn, cone, from, to, strict != 0);
+              if (r == kSweepStalled) return;
+              odd |= r == kSweepOdd;
               // a strict sweep leaves the word alone: members that are slow to
               // leave the barrier may still read it
               if (to == nc && !strict && threadIdx.x == 0) a.sst[s].ctl.mode = odd ? 1 : 0;
@@ -390,7 +401,96 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
   timer.store(a);
 }
 
+// A sweep over a chain of contacts (contact c between bodies c and c + 1), with
+// the contacts' places among their bodies' as they are, or one further on: then
+// no contact is ever next.
+constexpr int kStallBodies = 64;
+__global__ void __launch_bounds__(kThreads) k_selftest_sweep(KArgs<double> a, int* out) {
+  __shared__ Team tm;
+  if (threadIdx.x == 0) tm.c0 = 0;
+  __syncthreads();
+  const Cone<double> cone = make_cone<double>(0.5);
+  const PgsSweep r = pgs_sweep(a, tm, a.seg[0], a.G[0], a.G[1], cone, 0, kStallBodies - 1, false);
+  if (threadIdx.x == 0) *out = r == kSweepStalled;
+}
+
 }  // namespace
+
+}  // namespace dv
+
+extern "C" {
+
+DV_API int dv_selftest_stalled_sweep(int32_t further, int32_t* stalled, uint32_t* error_bits) {
+  using namespace dv;
+  constexpr int S = kStallBodies;
+  // planes of S doubles: v and q (4 each), the five iterates, F, frame words (3
+  // each), gap, minv, ids, counts
+  enum { kV = 0, kQ = 4, kG = 8, kF = 23, kFr = 26, kGap = 29, kMinv, kIds, kCount, kPlanes };
+  std::vector<double> h((size_t)kPlanes * S, 0.0);
+  uint32_t* ids = reinterpret_cast<uint32_t*>(h.data() + kIds * S);
+  int2* place = reinterpret_cast<int2*>(h.data() + (kG + 9) * S);
+  for (int i = 0; i < S; ++i) {
+    h[kMinv * S + i] = 1.0;
+    h[(kF + 2) * S + i] = h[kFr * S + i] = h[(kFr + 2) * S + i] = 1.0;
+    ids[i] = (uint32_t)i;
+    ids[S + i] = (uint32_t)std::min(i + 1, S - 1);
+    place[i] = make_int2((i > 0 ? 1 : 0) + (further ? 1 : 0), further ? 1 : 0);
+  }
+  SegParams P{};
+  P.h = 1.0;
+  P.mu = 0.5;
+  EngineWords words{};
+  struct Block {
+    double* w;
+    SegParams* seg;
+    EngineWords* ew;
+    int* out;
+  } b{nullptr, nullptr, nullptr, nullptr};
+  int r = -1;
+  auto run = [&]() -> int {
+    DV_CUDA_TRY(cudaMalloc(&b.w, h.size() * sizeof(double)));
+    DV_CUDA_TRY(cudaMalloc(&b.seg, sizeof(P)));
+    DV_CUDA_TRY(cudaMalloc(&b.ew, sizeof(words)));
+    DV_CUDA_TRY(cudaMalloc(&b.out, sizeof(int)));
+    DV_CUDA_TRY(cudaMemcpy(b.w, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
+    DV_CUDA_TRY(cudaMemcpy(b.seg, &P, sizeof(P), cudaMemcpyHostToDevice));
+    DV_CUDA_TRY(cudaMemcpy(b.ew, &words, sizeof(words), cudaMemcpyHostToDevice));
+    KArgs<double> a;
+    memset((void*)&a, 0, sizeof(a));
+    a.S = S;
+    a.v4 = reinterpret_cast<double4*>(b.w + kV * S);
+    a.qd = reinterpret_cast<double4*>(b.w + kQ * S);
+    for (int k = 0; k < 5; ++k) a.G[k] = b.w + (kG + 3 * k) * S;
+    a.F = b.w + kF * S;
+    a.fr = b.w + kFr * S;
+    a.gap = b.w + kGap * S;
+    a.minv = b.w + kMinv * S;
+    a.ida = reinterpret_cast<const uint32_t*>(b.w + kIds * S);
+    a.idb = a.ida + S;
+    a.body_count = reinterpret_cast<int*>(b.w + kCount * S);
+    a.seg = b.seg;
+    a.ew = b.ew;
+    k_selftest_sweep<<<1, kThreads>>>(a, b.out);
+    DV_CUDA_TRY(cudaGetLastError());
+    DV_CUDA_TRY(cudaDeviceSynchronize());
+    DV_CUDA_TRY(cudaMemcpy(&r, b.out, sizeof(int), cudaMemcpyDeviceToHost));
+    DV_CUDA_TRY(cudaMemcpy(&words, b.ew, sizeof(words), cudaMemcpyDeviceToHost));
+    return DV_OK;
+  };
+  const int rc = run();
+  cudaFree(b.w);
+  cudaFree(b.seg);
+  cudaFree(b.ew);
+  cudaFree(b.out);
+  if (rc != DV_OK) return rc;
+  if (stalled) *stalled = r;
+  if (error_bits) *error_bits = words.err;
+  return DV_OK;
+}
+
+}  // extern "C"
+
+namespace dv {
 
 void launch_pgs_solve(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t* launches,
                       bool solve_only) {

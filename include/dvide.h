@@ -389,6 +389,11 @@ DV_API int dv_server_get_stats(dv_server* s, dv_server_stats* out);
  * device stays usable afterwards. */
 DV_API int dv_selftest_bounded_waits(int32_t limit_ms, int32_t* barrier_timed_out,
                                      int32_t* copy_timed_out, uint32_t* error_bits);
+/* The same for the PGS sweep's rounds, which wait for one another by counts: a
+ * sweep over a chain of contacts, with `further` != 0 one whose counts never come
+ * up.  It must end with *stalled = 1 and the barrier-timeout bit; without, it
+ * runs through (*stalled = 0). */
+DV_API int dv_selftest_stalled_sweep(int32_t further, int32_t* stalled, uint32_t* error_bits);
 
 #ifdef __cplusplus
 }
