@@ -1121,10 +1121,15 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
     const unsigned err = C.err | (live ? __ldcg(&a.sst[s].err) : 0u);
     const bool refine_next = kMixed && P.refine > 0 && live && err == 0u && !(C.residual < P.tol);
 
+    // Where an error ends the call (plain scenes), one in the FP32 phase of a
+    // solve with refinement leaves the scene as it was: the update is the FP64
+    // phase's, which it does not get to.
+    const bool stay = kMixed && P.refine > 0 && err != 0u && a.ew->stop_on_seg_err;
+
     // ---- f_c = D^T gamma; v = Minv (k + f_c); f_contact = f_c / h; p += h v.
     // Scenes with neither contacts nor bilateral rows: v = Minv k, f_contact = 0
     // (System.cu:577-581); the rows' impulses enter f_c like the contacts'.
-    if (!a.solve_only && !refine_next) {
+    if (!a.solve_only && !refine_next && !stay) {
       for (int b = tm.w0 + threadIdx.x; b < tm.w1; b += kT) {
         const double h = P.h;
         double4 k = a.k4[b];

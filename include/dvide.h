@@ -79,7 +79,9 @@ typedef struct dv_params {
                                APGD iterations after the FP32 ones, started from the FP32
                                best iterate, for every solve whose FP32 phase ended above
                                the tolerance (iteration cap, or no new best residual for 50
-                               accepted iterations) */
+                               accepted iterations).  A solver error in the FP32 phase of
+                               a plain scene ends its step before the update: positions,
+                               velocities and contact forces stay */
 } dv_params;
 
 /* Per-step report (System.cu:586-599 and APGD.cu:351-357). */
