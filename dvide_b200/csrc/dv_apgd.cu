@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
       {
         int nslot = 0;
         for (int i = 0;; ++i) {
-          const int t = team_tile(tm, tm.nt, i);
+          const int t = team_tile(tm, i);
           if (t < 0) break;
           const int k0 = t * kTileItems, gsize = tm.gsize;
           const double h = P.h;
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
       {
         int nslot = 0;
         for (int i = 0;; ++i) {
-          const int t = team_tile(tm, tm.nt, i);
+          const int t = team_tile(tm, i);
           if (t < 0) break;
           const int k0 = t * kTileItems;
           double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -674,7 +674,7 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
           // (nothing would hide the copies), the lines of the next sub-tile go to L2.
           const bool staged = tm.ntc > tm.m;
           auto bring = [&](int j) {
-            const int t = team_tile(tm, tm.ntc, tile_of(j));
+            const int t = contact_tile(tm, tile_of(j));
             const int kw = t * kTileItems + sub_of(j) * kSub + gwarp * 32;
             if (t < 0 || kw >= nc) return;
             const size_t blk = (size_t)(c0 + kw) >> 5;
@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
           bool failed = false;
           int j = 0;  // sub-tile of this member
           for (int i = 0;; ++i) {
-            const int t = team_tile(tm, tm.nt, i);
+            const int t = team_tile(tm, i);
             if (t < 0) break;
             const int k0 = t * kTileItems;
             double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -839,7 +839,7 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
         // ---- the contact pass's sub-tiles of this member
         const int cur = C.cur, nw = C.nw, restart = C.restart;
         auto issue = [&](int j) {  // this warp's sub-tile j into stage j & 1
-          const int t = team_tile(tm, tm.ntc, tile_of(j));
+          const int t = contact_tile(tm, tile_of(j));
           const int kw = t * kTileItems + sub_of(j) * kSub + gwarp * 32;
           if (t >= 0 && kw < nc && lane == 0) {
             const int sidx = j & 1;
@@ -882,7 +882,7 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
           T* Xn = a.G[nw];
           T* X2 = a.G[C.nw2];
           for (int j = 0;; ++j) {
-            const int t = team_tile(tm, tm.ntc, tile_of(j));
+            const int t = contact_tile(tm, tile_of(j));
             if (t < 0) break;
             const int sidx = j & 1, sub = sub_of(j);
             if (j && !failed) {
@@ -999,7 +999,7 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
             nslot = 0;
             const T* wt = reinterpret_cast<const T*>(wv);
             for (int i = 0;; ++i) {
-              const int t = team_tile(tm, tm.nt, i);
+              const int t = team_tile(tm, i);
               if (t < 0) break;
               const int kb = bil_tile_k0(t, 0, nc);
               if (kb < 0) continue;
@@ -1032,7 +1032,7 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
         int nslot = 0;
         const int best = C.best;
         for (int i = 0;; ++i) {
-          const int t = team_tile(tm, tm.nt, i);
+          const int t = team_tile(tm, i);
           if (t < 0) break;
           double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
           if (best >= 0) {
@@ -1069,7 +1069,7 @@ __global__ void __launch_bounds__(kThreads* kGroups, kMinB) k_step_solve(KArgs<T
         const bool keep = a.refine && best < 0;
         const T* src = best >= 0 ? a.G[best] : nullptr;
         for (int i = 0;; ++i) {
-          const int t = team_tile(tm, tm.nt, i);
+          const int t = team_tile(tm, i);
           if (t < 0) break;
           const int kb = a.nbil ? bil_tile_k0(t, 0, nc) : -1;
           if (kb >= 0) {

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
       if (!sync(kPhaseSetup, true)) return;
       // ---- r = D (Minv k) + b; gamma_0 = (1, 0, 0) -> G[0]; B; q = F gamma_0
       for (int i = 0;; ++i) {
-        const int t = team_tile(tm, tm.nt, i);
+        const int t = team_tile(tm, i);
         if (t < 0) break;
         const double h = P.h;
         for (int m = 0; m < kItemsPerThread; ++m) {
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
         const T* Gc = a.G[C.cur];
         T* Gn = a.G[C.cur ^ 1];
         for (int i = 0;; ++i) {
-          const int t = team_tile(tm, tm.nt, i);
+          const int t = team_tile(tm, i);
           if (t < 0) break;
           double mx[3] = {0.0, 0.0, 0.0};
           for (int m = 0; m < kItemsPerThread; ++m) {
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
       // ---- gamma -> warm-start region; q = F gamma (FP64)
       const T* src = a.G[C.cur];
       for (int i = 0;; ++i) {
-        const int t = team_tile(tm, tm.nt, i);
+        const int t = team_tile(tm, i);
         if (t < 0) break;
         for (int m = 0; m < kItemsPerThread; ++m) {
           const int k = t * kTileItems + m * kThreads + threadIdx.x;

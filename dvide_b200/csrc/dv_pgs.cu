@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
       // ---- r = D (Minv k) + b; gamma_0 = (1, 0, 0) -> G[0]; B; q = F gamma_0
       const int shift = a.sst[s].delta;
       for (int i = 0;; ++i) {
-        const int t = team_tile(tm, tm.nt, i);
+        const int t = team_tile(tm, i);
         if (t < 0) break;
         const double h = P.h;
         for (int m = 0; m < kItemsPerThread; ++m) {
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
         if (!sync(kPhaseBody)) return;
         int nslot = 0;
         for (int i = 0;; ++i) {
-          const int t = team_tile(tm, tm.nt, i);
+          const int t = team_tile(tm, i);
           if (t < 0) break;
           double mx[3] = {0.0, 0.0, 0.0};
           for (int m = 0; m < kItemsPerThread; ++m) {
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
       // ---- gamma -> warm-start region (System::gamma_d); q = F gamma (FP64)
       const double* src = a.G[C.cur];
       for (int i = 0;; ++i) {
-        const int t = team_tile(tm, tm.nt, i);
+        const int t = team_tile(tm, i);
         if (t < 0) break;
         for (int m = 0; m < kItemsPerThread; ++m) {
           const int k = t * kTileItems + m * kThreads + threadIdx.x;

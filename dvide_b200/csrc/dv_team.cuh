@@ -17,6 +17,7 @@
 #pragma once
 
 #include "dv_solve.cuh"
+#include "dv_tiles.h"
 
 namespace dv {
 
@@ -31,24 +32,15 @@ struct Team {
   int t0, ntc, nt;  // first tile; contact tiles; with the bilateral rows' tiles
   int w0, w1;       // this member's bodies
   int gsize;
-  int chunk, contiguous;
+  TileShare share;
   int fail;
   unsigned target;  // arrivals that open the next barrier
   unsigned* bar;
 };
 
-// Tile i of this member's share of n tiles (-1 past the end): round robin in
-// chunks of `chunk` consecutive tiles, or one contiguous range per member.
-__device__ inline int team_tile(const Team& t, int n, int i) {
-  if (t.contiguous) {
-    const int lo = (int)((long long)n * t.rank / t.m);
-    const int hi = (int)((long long)n * (t.rank + 1) / t.m);
-    return lo + i < hi ? lo + i : -1;
-  }
-  const int k = t.chunk;
-  const int x = k == 1 ? t.rank + i * t.m : (t.rank + (i / k) * t.m) * k + i % k;
-  return x < n ? x : -1;
-}
+// The member's walks over the contact tiles, and over all tiles (dv_tiles.h).
+__device__ inline int contact_tile(const Team& t, int i) { return share_tile(t.share, t.ntc, i); }
+__device__ inline int team_tile(const Team& t, int i) { return scene_tile(t.share, t.ntc, t.nt, i); }
 
 __device__ inline void red_add_release(unsigned* p, unsigned v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
@@ -145,8 +137,7 @@ __device__ inline bool join_team(const K& a, Team& t, int* slot_seen) {
       t.w0 = P.b0 + min(n, rank * per);
       t.w1 = P.b0 + min(n, (rank + 1) * per);
       t.gsize = X.gsize;
-      t.chunk = a.chunk;
-      t.contiguous = a.contiguous;
+      t.share = TileShare{rank, m, a.chunk, a.contiguous};
       t.fail = 0;
       t.target = 0;
       t.bar = a.team_bar + (size_t)s * kTeamBarStride;
