@@ -49,6 +49,7 @@
 // Work is split in tiles of 512 contacts (2 per thread).  Every wait has a
 // time limit.
 #include <algorithm>
+#include <atomic>
 
 #include "dv_team.cuh"
 
@@ -1274,23 +1275,33 @@ constexpr size_t solve_smem_bytes() {
          (kGroups == 2 ? sizeof(PairBuf) : 0);
 }
 
+// Co-resident CTAs of a form of the kernel on the current device, asked for once
+// per device (a member of a team that never runs would be waited for).
 template <class T, int G, int MB, bool AR>
-void prepare_kernel() {
-  static bool done = false;
-  if (done) return;
-  cudaFuncSetAttribute(k_step_solve<T, G, MB, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)solve_smem_bytes<T, G>());
-  done = true;
+int resident_ctas() {
+  constexpr int kDevices = 64;
+  static std::atomic<int> known[kDevices];
+  int dev = 0, sms = 0, per_sm = 0;
+  cudaGetDevice(&dev);
+  const bool keep = dev >= 0 && dev < kDevices;
+  if (keep && known[dev].load(std::memory_order_relaxed)) return known[dev].load(std::memory_order_relaxed);
+  const size_t smem = solve_smem_bytes<T, G>();
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_step_solve<T, G, MB, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_solve<T, G, MB, AR>, kThreads * G, smem);
+  const int n = sms * std::max(per_sm, 1);
+  if (keep && e == cudaSuccess && per_sm > 0) known[dev].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 template <class T, int G, int MB, bool AR = false>
 void launch_typed(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t* launches,
                   bool solve_only, bool refine) {
-  prepare_kernel<T, G, MB, AR>();
   KArgs<T> a = make_kargs<T>(sd, cfg);
   a.solve_only = solve_only ? 1 : 0;
   a.refine = refine ? 1 : 0;
-  const int grid = G == 2 ? std::max(1, cfg.grid / 2) : cfg.grid;
+  const int grid = std::min(G == 2 ? std::max(1, cfg.grid / 2) : cfg.grid, resident_ctas<T, G, MB, AR>());
   plan_teams(sd, grid, refine, st, launches);
   void* params[] = {&a};
   cudaLaunchCooperativeKernel((const void*)k_step_solve<T, G, MB, AR>, grid, kThreads * G, params,
@@ -1313,26 +1324,14 @@ void launch_form(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t*
     launch_typed<T, 1, 2, AR>(sd, cfg, st, launches, solve_only, refine);
 }
 
-template <class T, int MB>
-int max_ctas_of() {
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  prepare_kernel<T, 1, MB, false>();
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_step_solve<T, 1, MB, false>, kThreads,
-                                                solve_smem_bytes<T, 1>());
-  if (per_sm < 1) per_sm = 1;
-  return sms * per_sm;
-}
-
 }  // namespace
 
 // Co-resident CTAs of the solve kernel for a precision and a register budget
 // (blocks_per_sm 2: 128 registers per thread; 3: 80, FP32 iterates only).
 int apgd_max_ctas(int precision, int blocks_per_sm) {
   if (precision == DV_PREC_MIXED)
-    return blocks_per_sm == 3 ? max_ctas_of<float, 3>() : max_ctas_of<float, 2>();
-  return max_ctas_of<double, 2>();
+    return blocks_per_sm == 3 ? resident_ctas<float, 1, 3, false>() : resident_ctas<float, 1, 2, false>();
+  return resident_ctas<double, 1, 2, false>();
 }
 
 void plan_teams(SceneDev& sd, int grid, bool refine, cudaStream_t st, int64_t* launches) {

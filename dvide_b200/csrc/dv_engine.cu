@@ -736,12 +736,15 @@ int Engine::capture_graph() {
     cudaGetLastError();
     return DV_ERR_UNSUPPORTED;
   }
+  const cudaError_t before = cudaPeekAtLastError();
   collide(d, st_, &dummy);
   launch_step_solve(d, cfg_, st_, &dummy);
+  // a launch that was refused is not in the graph, which would replay without it
+  const bool refused = before == cudaSuccess && cudaPeekAtLastError() != cudaSuccess;
   e = cudaStreamEndCapture(st_, &graph_);
-  if (e != cudaSuccess || !graph_) {
+  if (e != cudaSuccess || refused || !graph_) {
     cudaGetLastError();
-    graph_ = nullptr;
+    drop_graph();
     return DV_ERR_UNSUPPORTED;
   }
   e = cudaGraphInstantiate(&graph_exec_, graph_, 0);
