@@ -46,6 +46,7 @@ namespace {
 constexpr int kWarpsPerCta = kThreads / 32;
 constexpr int kMaxPerBody = 128;  // partners with larger id per sphere
 constexpr int kKeep = kKeepPartners;
+constexpr int kAgainCtas = 592;   // CTAs that search listed spheres again at most
 
 __device__ inline unsigned long long ordered_bits(double x) {
   unsigned long long u = (unsigned long long)__double_as_longlong(x);
@@ -71,6 +72,7 @@ __global__ void k_seg_reset(int nseg, GridInfo* __restrict__ grid, SegState* __r
   if (s == 0) {
     ew->npossible = 0;
     ew->n_wide = 0;
+    ew->n_again = 0;
   }
   if (s >= nseg) return;
   for (int d = 0; d < 3; ++d) {
@@ -345,6 +347,7 @@ struct CollideArgs {
   const uint32_t* sorted_bodies;  // small bodies sorted by cell
   const double4* spheres;         // (x, y, z, r) in the same order
   uint32_t* kept;                 // kKeep partners per small body, from the count pass
+  uint32_t* again;                // small bodies with more, at most kMaxPerBody (ew->n_again)
   const int* cstart;
   const int* cend;
   const GridInfo* grid;
@@ -469,6 +472,7 @@ __global__ void __launch_bounds__(kThreads) k_sphere_count(CollideArgs a) {
     a.cnt_cand[A] = ncand;
     a.cnt_cont[A] = n;
     // more partners than the write pass lists: k_sphere_pairs_wide writes them
+    if (n > kKeep && n <= kMaxPerBody) a.again[atomicAdd(&a.ew->n_again, 1)] = (uint32_t)j;
     if (n > kMaxPerBody) {
       const int k = atomicAdd(&a.ew->n_wide, 1);
       if (k < kWideSpheres && n <= kWidePartners) {
@@ -485,53 +489,53 @@ __global__ void __launch_bounds__(kThreads) k_sphere_count(CollideArgs a) {
   }
 }
 
-// Write pass, eight lanes per sphere: the contacts of the kept partners at the
-// sphere's slot.  A sphere with more than kKeep and at most kMaxPerBody
-// partners is searched again by its whole warp.
-__global__ void __launch_bounds__(kThreads) k_sphere_write(CollideArgs a) {
+// Write pass.  The first `kept_ctas` CTAs, eight lanes per sphere: the contacts
+// of the kept partners at the sphere's slot.  The others, a warp per sphere: the
+// spheres that the count pass listed, with more than kKeep and at most
+// kMaxPerBody partners, are searched again.  (Searched by the warp that wrote its
+// four spheres' kept partners, a crowd of 129 such spheres took four searches one
+// after another.)
+__global__ void __launch_bounds__(kThreads) k_sphere_write(CollideArgs a, int kept_ctas) {
   __shared__ int s_buf[kWarpsPerCta][kMaxPerBody];
   __shared__ int s_cnt[kWarpsPerCta];
   if (a.ew->err) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int j0 = (blockIdx.x * kWarpsPerCta + warp) * 4;
-  if (j0 >= a.n_small) return;
-  const int j = j0 + (lane >> 3);
-  int A = -1, sg = 0, n = 0;
-  if (j < a.n_small) {
-    A = a.small_ids[j];
-    sg = a.bseg[A];
-    if (a.seg[sg].active) n = a.cnt_cont[A];
-  }
-  if (n > 0 && n <= kKeep) {
+  if ((int)blockIdx.x < kept_ctas) {
+    const int j = (blockIdx.x * kThreads + threadIdx.x) >> 3;
+    if (j >= a.n_small) return;
+    const int A = a.small_ids[j], sg = a.bseg[A];
     const SegParams& P = a.seg[sg];
-    const size_t base = (size_t)(a.cbase[A] + a.sst[sg].delta);
-    for (int e = lane & 7; e < n; e += 8) {
+    const int n = P.active ? a.cnt_cont[A] : 0;
+    if (n > kKeep) return;
+    const int e = lane & 7;
+    if (e < n) {
+      const size_t base = (size_t)(a.cbase[A] + a.sst[sg].delta);
       const int B = (int)a.kept[(size_t)j * kKeep + e];
       NpOut o;
       narrowphase(a.p4, a.g4, A, B, P.env, P.exact != 0, &o);
       write_contact(a, base + e, A, B, o);
     }
+    return;
   }
-  unsigned more = __ballot_sync(0xffffffffu, n > kKeep && n <= kMaxPerBody && (lane & 7) == 0);
-  while (more) {
-    const int l = __ffs(more) - 1;
-    more &= more - 1;
-    const int A2 = __shfl_sync(0xffffffffu, A, l), sg2 = __shfl_sync(0xffffffffu, sg, l);
-    const SegParams& P = a.seg[sg2];
+  const int listed = a.ew->n_again, step = ((int)gridDim.x - kept_ctas) * kWarpsPerCta;
+  for (int w = ((int)blockIdx.x - kept_ctas) * kWarpsPerCta + warp; w < listed; w += step) {
+    const int A = a.small_ids[a.again[w]], sg = a.bseg[A];
+    const SegParams& P = a.seg[sg];
     int ncand;
-    const int n2 = min(find_partners(a, A2, sg2, s_buf[warp], &s_cnt[warp], &ncand), kMaxPerBody);
-    const size_t base = (size_t)(a.cbase[A2] + a.sst[sg2].delta);
-    for (int e = lane; e < n2; e += 32) {
+    const int n = min(find_partners(a, A, sg, s_buf[warp], &s_cnt[warp], &ncand), kMaxPerBody);
+    const size_t base = (size_t)(a.cbase[A] + a.sst[sg].delta);
+    for (int e = lane; e < n; e += 32) {
       const int B = s_buf[warp][e];
       int rank = 0;
-      for (int k = 0; k < n2; ++k) rank += s_buf[warp][k] < B ? 1 : 0;
+      for (int k = 0; k < n; ++k) rank += s_buf[warp][k] < B ? 1 : 0;
       NpOut o;
-      narrowphase(a.p4, a.g4, A2, B, P.env, P.exact != 0, &o);
-      write_contact(a, base + rank, A2, B, o);
+      narrowphase(a.p4, a.g4, A, B, P.env, P.exact != 0, &o);
+      write_contact(a, base + rank, A, B, o);
     }
     __syncwarp();
   }
 }
+static_assert(kKeep == 8, "eight lanes write a sphere's kept partners");
 
 // The write pass for the spheres the count pass listed in wide_ids (more than
 // kMaxPerBody partners with larger ids): each CTA takes listed spheres in turn;
@@ -917,6 +921,7 @@ __global__ void __launch_bounds__(1024) k_front_few(
   if (tid == 0) {
     ew->npossible = 0;
     ew->n_wide = 0;
+    ew->n_again = 0;
   }
   __syncthreads();
   for (int i0 = 0; i0 < nb; i0 += 1024) body_aabb(i0 + tid, p4, g4, bseg, seg, nb, amin, amax, grid);
@@ -952,40 +957,70 @@ __global__ void __launch_bounds__(1024) k_front_few(
   }
 }
 
-// The incidence: per body its contacts as B, then as A, ascending.
+// The incidence: per body its contacts as B, then as A, ascending.  Runs of B
+// contacts come in the order of the atomics and are sorted: short ones by a
+// thread, longer ones by a warp (each entry's rank), the longest by the CTA
+// (bitonic), the last two in shared memory.  A body has at most nb - 1 contacts.
+constexpr int kShortRun = 24, kWarpRun = 256, kLongRun = 32 * kWarpRun;
+static_assert(kFewBodies <= kLongRun, "a run fits the shared memory");
 __global__ void __launch_bounds__(1024) k_incidence_few(
     int nb, const uint32_t* __restrict__ idb, const int* __restrict__ tseg,
     const SegState* __restrict__ sst, const int* __restrict__ bseg, const int* __restrict__ cbase,
-    const int* __restrict__ acnt, int* cnt, uint32_t* slot, uint32_t* scratch, int* istart, uint32_t* inc,
+    const int* __restrict__ acnt, int* cnt, uint32_t* slot, uint32_t* longest, int* istart, uint32_t* inc,
     const EngineWords* __restrict__ ew) {
-  constexpr int kShort = 24;  // longest run that one thread sorts
-  __shared__ int s_long;
+  __shared__ __align__(16) uint32_t s_run[kLongRun];
+  __shared__ int s_longest;
   if (ew->err) return;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nt = ew->ntiles;
-  if (tid == 0) s_long = 0;
+  if (tid == 0) s_longest = 0;
   for (int b = tid; b < nb; b += 1024) cnt[b] = 0;
   __syncthreads();
+  // a warp takes a whole tile where tiles abound (many scenes of a few contacts
+  // each), a quarter where they do not
+  const int unit = nt >= 128 ? kTileItems : kTileItems / 4, units = kTileItems / unit;
+  // four contacts per lane at once: their loads, and their atomics, do not wait
+  // for one another
   auto each_contact = [&](auto fn) {
-    for (int i = tid; i < nt * kTileItems; i += 1024) {
-      const int t = i / kTileItems;
+    for (int u = warp; u < nt * units; u += 32) {
+      const int t = u / units;
       const SegState& S = sst[tseg[t]];
-      const int k = (t - S.t0) * kTileItems + i % kTileItems;
-      if (k < S.nc) fn(S.c0 + k);
+      const int k0 = (t - S.t0) * kTileItems + (u - t * units) * unit, k1 = min(k0 + unit, S.nc), c0 = S.c0;
+      for (int k = k0 + lane; k < k1; k += 128) {
+        uint32_t b[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) b[q] = k + 32 * q < k1 ? idb[c0 + k + 32 * q] : ~0u;
+        fn(c0 + k, b);
+      }
     }
   };
-  each_contact([&](int c) { slot[c] = (uint32_t)atomicAdd(&cnt[idb[c]], 1); });
+  each_contact([&](int c, const uint32_t (&b)[4]) {
+    int at[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) at[q] = b[q] != ~0u ? atomicAdd(&cnt[b[q]], 1) : 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (b[q] != ~0u) slot[c + 32 * q] = (uint32_t)at[q];
+  });
   __syncthreads();
   scan_one_cta(nb, [&](int b) { return __ldcg(cnt + b) + acnt[b]; }, istart);
   __syncthreads();
-  each_contact([&](int c) { inc[istart[idb[c]] + (int)slot[c]] = (uint32_t)c | 0x80000000u; });
+  each_contact([&](int c, const uint32_t (&b)[4]) {
+    int at[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) at[q] = b[q] != ~0u ? istart[b[q]] + (int)slot[c + 32 * q] : 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (b[q] != ~0u) inc[at[q]] = (uint32_t)(c + 32 * q) | 0x80000000u;
+  });
   __syncthreads();
-  for (int b = tid; b < nb; b += 1024) {
-    const int n = __ldcg(cnt + b), na = acnt[b];
-    uint32_t* run = inc + istart[b];
-    if (n > kShort) {
-      s_long = 1;
-    } else {
+  for (int base = warp * 32; base < nb; base += 1024) {
+    const int b = base + lane;
+    const int n = b < nb ? __ldcg(cnt + b) : 0, na = b < nb ? acnt[b] : 0;
+    const int first = na ? cbase[b] + sst[bseg[b]].delta : 0;
+    const int at = b < nb ? istart[b] : 0;
+    uint32_t* run = inc + at;
+    if (n <= kShortRun) {
       for (int i = 1; i < n; ++i) {
         const uint32_t x = run[i];
         int k = i - 1;
@@ -993,25 +1028,63 @@ __global__ void __launch_bounds__(1024) k_incidence_few(
         run[k + 1] = x;
       }
     }
-    if (na) {
-      const int first = cbase[b] + sst[bseg[b]].delta;
+    if (na <= kShortRun)
       for (int k = 0; k < na; ++k) run[n + k] = (uint32_t)(first + k);
+    // the lanes' longer runs, each by the whole warp
+    for (unsigned m = __ballot_sync(0xffffffffu, na > kShortRun); m; m &= m - 1) {
+      const int l = __ffs(m) - 1;
+      const int na2 = __shfl_sync(0xffffffffu, na, l), first2 = __shfl_sync(0xffffffffu, first, l);
+      uint32_t* r = inc + __shfl_sync(0xffffffffu, at + n, l);
+      for (int k = lane; k < na2; k += 32) r[k] = (uint32_t)(first2 + k);
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, n > kShortRun); m; m &= m - 1) {
+      const int l = __ffs(m) - 1;
+      const int n2 = __shfl_sync(0xffffffffu, n, l);
+      uint32_t* r = inc + __shfl_sync(0xffffffffu, at, l);
+      if (n2 > kWarpRun) {
+        if (lane == 0) longest[atomicAdd(&s_longest, 1)] = (uint32_t)(base + l);
+        continue;
+      }
+      uint32_t* sr = s_run + warp * kWarpRun;
+      const int m4 = (n2 + 3) & ~3;
+      for (int i = lane; i < m4; i += 32) sr[i] = i < n2 ? r[i] : ~0u;
+      __syncwarp();
+      for (int i = lane; i < n2; i += 32) {
+        const uint32_t x = sr[i];
+        int rank = 0;
+        for (int k = 0; k < m4; k += 4) {
+          const uint4 y = *reinterpret_cast<const uint4*>(sr + k);
+          rank += (y.x < x ? 1 : 0) + (y.y < x ? 1 : 0) + (y.z < x ? 1 : 0) + (y.w < x ? 1 : 0);
+        }
+        r[rank] = x;
+      }
+      __syncwarp();
     }
   }
   __syncthreads();
-  if (!s_long) return;
-  for (int b = 0; b < nb; ++b) {  // long runs: the whole CTA, by rank
-    const int n = __ldcg(cnt + b);
-    if (n <= kShort) continue;
-    uint32_t* run = inc + istart[b];
-    for (int i = tid; i < n; i += 1024) scratch[i] = run[i];
+  const int nlong = s_longest;
+  for (int j = 0; j < nlong; ++j) {
+    const int b = (int)longest[j];
+    const int n = min(__ldcg(cnt + b), kLongRun);
+    uint32_t* r = inc + istart[b];
+    int m = kWarpRun;
+    while (m < n) m <<= 1;
+    for (int i = tid; i < m; i += 1024) s_run[i] = i < n ? r[i] : 0xffffffffu;
     __syncthreads();
-    for (int i = tid; i < n; i += 1024) {
-      const uint32_t x = scratch[i];
-      int rank = 0;
-      for (int k = 0; k < n; ++k) rank += scratch[k] < x ? 1 : 0;
-      run[rank] = x;
+    for (int k = 2; k <= m; k <<= 1) {
+      for (int d = k >> 1; d > 0; d >>= 1) {
+        for (int p = tid; p < m / 2; p += 1024) {
+          const int i = 2 * p - (p & (d - 1)), l = i + d;  // the pair's places, d apart
+          const uint32_t x = s_run[i], y = s_run[l];
+          if ((x > y) == ((i & k) == 0)) {
+            s_run[i] = y;
+            s_run[l] = x;
+          }
+        }
+        __syncthreads();
+      }
     }
+    for (int i = tid; i < n; i += 1024) r[i] = s_run[i];
     __syncthreads();
   }
 }
@@ -1036,6 +1109,7 @@ CollideArgs make_args(SceneDev& sd) {
   a.sorted_bodies = sd.valA;
   a.spheres = sd.spheres;
   a.kept = sd.kept;
+  a.again = sd.keyB;  // free between the two sorts
   a.cstart = sd.cell_start;
   a.cend = sd.cell_end;
   a.grid = sd.grid;
@@ -1067,9 +1141,16 @@ void collide(SceneDev& sd, cudaStream_t st, int64_t* launches) {
   const int nb = sd.nb;
   if (nb == 0) return;
   const int park = sd.ncell_cap - 1;  // cell of spheres in inactive segments
-  // Short or long form, device time of detection: 1,000 spheres 80 or 183 us,
-  // 5,003 spheres 186 or 213, 64 scenes of 20,500 bodies 0.45 ms more than long.
-  const bool few = nb <= kFewBodies && sd.ncell_cap <= 16 * kFewBodies;
+  // Short or long form, by bodies; the incidence, whose work is the contacts', by
+  // the slots they have: an engine starts with four per body, and a crowd's grow.
+  // Device time of detection, short and long: 1,000 spheres 64 and 157 us, 6,000
+  // 164 and 224, 64 scenes of 20,500 bodies 0.45 ms more than long; with 992,000
+  // contacts of 1,501 spheres 12 ms (incidence short) and 1.0; 6,000 spheres of
+  // 44,000 contacts 246 us (long incidence alone) and 237, 4,000 of 48,000 214 and
+  // 228; 201 spheres of 17,800 contacts 327 us and 304.
+  const size_t slots = (size_t)std::min(kFewContacts, 96 * nb) + kContactAlign * (size_t)sd.nseg;
+  const bool few_contacts = nb <= kFewBodies && sd.ccap <= slots;
+  const bool few = nb <= (few_contacts ? kFewBodies : kFewBodies * 2 / 3) && sd.ncell_cap <= 16 * kFewBodies;
   if (few) {
     k_front_few<<<1, 1024, 0, st>>>(sd.nseg, nb, sd.small_ids, sd.n_small, sd.bseg, sd.seg, sd.p4,
                                     sd.geom4, sd.amin, sd.amax, sd.grid, sd.cell, sd.cell_start,
@@ -1124,8 +1205,9 @@ void collide(SceneDev& sd, cudaStream_t st, int64_t* launches) {
       exclusive_scan_i32(sd.large_chunk, sd.large_chunk_off, nchunks, sd.scan_tmp, st, launches);
   }
   if (sd.n_small > 0) {
-    const int per_cta = 4 * kWarpsPerCta;
-    k_sphere_write<<<(sd.n_small + per_cta - 1) / per_cta, kThreads, 0, st>>>(a);
+    const int kept_ctas = blocks_for(8LL * sd.n_small);
+    const int again_ctas = std::min((sd.n_small + kWarpsPerCta - 1) / kWarpsPerCta, kAgainCtas);
+    k_sphere_write<<<kept_ctas + again_ctas, kThreads, 0, st>>>(a, kept_ctas);
     k_sphere_pairs_wide<<<std::min(kWideGrid, sd.n_small), kThreads, 0, st>>>(a);
     *launches += 2;
   }
@@ -1133,7 +1215,7 @@ void collide(SceneDev& sd, cudaStream_t st, int64_t* launches) {
     k_box_pairs<true><<<box_grid, kThreads, 0, st>>>(a, nullptr, sd.large_chunk_off);
     ++*launches;
   }
-  if (few) {
+  if (few && few_contacts) {
     k_incidence_few<<<1, 1024, 0, st>>>(nb, sd.idb, sd.tseg, sd.sst, sd.bseg, sd.cbase, sd.cnt_cont,
                                         sd.cnt_cand, sd.keyA, sd.valA, sd.inc_start, sd.inc, sd.ew);
     ++*launches;

@@ -117,6 +117,7 @@ struct EngineWords {
   unsigned ticket;
   unsigned progress;
   int n_wide;           // spheres of this step with more partners than the warp pair kernel lists
+  int n_again;          // ... with more than are kept, and listed
 };
 
 // Spheres per step whose partners (larger ids) exceed the warp pair kernel's
@@ -129,6 +130,7 @@ constexpr int kWidePartners = 8192;
 // bodies up to which an engine takes the short forms of collision detection.
 constexpr int kKeepPartners = 8;
 constexpr int kFewBodies = 6144;
+constexpr int kFewContacts = 32768;  // contact slots of an engine whose incidence one CTA forms
 
 // Tiles that a team's member takes at most when there are more than the grid
 // has CTAs, and the distance of the teams' arrival counters (a line each).
