@@ -58,7 +58,13 @@ void fill_step_stats(const StepRecord& r, int s, dv_step_stats* out) {
     if (rc_ != DV_OK) return rc_; \
   } while (0)
 
+Engine::Engine(bool keep_blocks) : keep_blocks_(keep_blocks) {
+  cudaGetDevice(&device_);
+  if (keep_blocks_) Holders::add(this);
+}
+
 Engine::~Engine() {
+  if (keep_blocks_) Holders::remove(this);
   if (st_) cudaStreamSynchronize(st_);
   drop_graph();
   free_spare();
@@ -73,13 +79,14 @@ Engine::~Engine() {
   if (own_st_) cudaStreamDestroy(own_st_);
 }
 
-void Engine::free_spare() {
-  for (const auto& b : spare_) {
-    cudaFree(b.second);
-    held_bytes_ -= b.first;
-  }
+size_t Engine::free_spare() {
+  std::lock_guard<std::recursive_mutex> g(Holders::lock());
+  const size_t bytes = spare_bytes_;
+  for (const auto& b : spare_) cudaFree(b.second);
   spare_.clear();
+  held_bytes_ -= bytes;
   spare_bytes_ = 0;
+  return bytes;
 }
 
 static const char* const kPartnerLimitText =

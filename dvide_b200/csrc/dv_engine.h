@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "dv_internal.cuh"
+#include "dv_reclaim.h"
 
 namespace dv {
 
@@ -40,9 +41,11 @@ struct StepRecord {
   int time_index = 0;
 };
 
-class Engine {
+class Engine final : private Holder {
  public:
-  Engine() = default;
+  // keep_blocks: freed blocks stay for the next allocations (servers, whose
+  // layouts change all the time)
+  explicit Engine(bool keep_blocks = false);
   ~Engine();
   Engine(const Engine&) = delete;
   Engine& operator=(const Engine&) = delete;
@@ -112,7 +115,11 @@ class Engine {
   // step() call after the failing step.  Batches keep stepping other scenes.
   int set_stop_on_segment_error(bool on);
   int64_t launches() const { return launches_; }
-  size_t held_bytes() const { return held_bytes_; }  // device memory
+  size_t held_bytes() const {  // device memory, spare blocks among it
+    std::lock_guard<std::recursive_mutex> g(Holders::lock());
+    return held_bytes_;
+  }
+  size_t free_spare();
 
   // Positions / velocities of bodies [b0, b0 + n) as 3 doubles per body,
   // between host arrays and the device's double4 layout: one contiguous copy
@@ -183,10 +190,12 @@ class Engine {
   cudaStream_t own_st_ = nullptr;  // the engine's own; st_ is it or the caller's
   std::unordered_map<void*, size_t> allocs_;  // device memory and its sizes
   size_t held_bytes_ = 0;                     // ... of them and the spare blocks
-  std::multimap<size_t, void*> spare_;        // freed blocks by size
+  const bool keep_blocks_;
+  int device_ = 0;
+  std::multimap<size_t, void*> spare_;        // freed blocks by size (under Holders::lock)
   size_t spare_bytes_ = 0;
   static constexpr size_t kSpareBytes = size_t(256) << 20;
-  void free_spare();
+  size_t reclaim(int device) override { return device == device_ ? free_spare() : 0; }
   std::vector<SegParams> hseg_;
   std::vector<dv_params> P_;
   std::vector<double> time_;
@@ -236,37 +245,41 @@ class Engine {
   double* h_red_ = nullptr;           // pinned, 16 slots
 };
 
-// Device memory of an engine.  A freed block stays with the engine for its next
-// allocation of at most that and at least half that size, up to kSpareBytes in
-// all: a layout change of a server takes and gives back some twenty blocks, and
-// cudaMalloc and cudaFree of each cost 0.1 to 0.5 ms and wait for the device.
-// All work on a block runs on the engine's stream, so the next user's follows
-// the last one's.  Spare blocks go back when an allocation fails and with the engine.
+// Device memory of an engine.  With keep_blocks a freed block stays with the
+// engine for its next allocation of at most that and at least half that size, up
+// to kSpareBytes in all: a layout change of a server takes and gives back some
+// twenty blocks, and cudaMalloc and cudaFree of each cost 0.1 to 0.5 ms and wait
+// for the device.  All work on a block runs on the engine's stream, so the next
+// user's follows the last one's.  Spare blocks go back with the engine, and when
+// an allocation of any engine of the process fails.
 template <class T>
 inline int Engine::dalloc(T** p, size_t n) {
   if (n == 0) n = 1;
   const size_t bytes = n * sizeof(T);
   void* q = nullptr;
-  auto it = spare_.lower_bound(bytes);
-  if (it != spare_.end() && it->first / 2 <= bytes) {
-    q = it->second;
-    allocs_[q] = it->first;
-    spare_bytes_ -= it->first;
-    spare_.erase(it);
-    *p = reinterpret_cast<T*>(q);
-    return DV_OK;
+  if (keep_blocks_) {
+    std::lock_guard<std::recursive_mutex> g(Holders::lock());
+    auto it = spare_.lower_bound(bytes);
+    if (it != spare_.end() && it->first / 2 <= bytes) {
+      q = it->second;
+      allocs_[q] = it->first;
+      spare_bytes_ -= it->first;
+      spare_.erase(it);
+      *p = reinterpret_cast<T*>(q);
+      return DV_OK;
+    }
   }
   cudaError_t e = cudaMalloc(&q, bytes);
-  if (e == cudaErrorMemoryAllocation && !spare_.empty()) {
+  if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    free_spare();
-    e = cudaMalloc(&q, bytes);
+    if (Holders::reclaim_all(device_)) e = cudaMalloc(&q, bytes);
   }
   if (e != cudaSuccess) {
     *p = nullptr;
     cudaGetLastError();
     return dv_record_cuda_error(e, "cudaMalloc", __FILE__, __LINE__);
   }
+  std::lock_guard<std::recursive_mutex> g(Holders::lock());
   allocs_[q] = bytes;
   held_bytes_ += bytes;
   *p = reinterpret_cast<T*>(q);
@@ -280,7 +293,8 @@ inline void Engine::dfree(T*& p) {
   if (it != allocs_.end()) {
     const size_t bytes = it->second;
     allocs_.erase(it);
-    if (spare_bytes_ + bytes <= kSpareBytes) {
+    std::lock_guard<std::recursive_mutex> g(Holders::lock());
+    if (keep_blocks_ && spare_bytes_ + bytes <= kSpareBytes) {
       spare_.emplace(bytes, (void*)p);
       spare_bytes_ += bytes;
     } else {

@@ -55,10 +55,39 @@ double pct(std::vector<float> v, double q) {
   return v[i];
 }
 
-// Device memory that an idle server keeps for its next requests at most.  A
-// burst of 40 requests on a new engine spent 28 of 45 ms of its first round on
-// allocations.
+// Device memory that an idle server keeps for its next requests at most, as far
+// as its budget goes.  A burst of 40 requests on a new engine spent 28 of 45 ms of
+// its first round on allocations.
 constexpr size_t kIdleBytes = size_t(1) << 30;
+
+// The engine of an idle server.  It has left the caller's stream, which may end
+// before the next requests, and goes back when an allocation of another engine
+// fails.
+class ParkedEngine final : private Holder {
+ public:
+  ParkedEngine() { Holders::add(this); }
+  ~ParkedEngine() { Holders::remove(this); }
+  void put(std::unique_ptr<Engine> e, int device) {
+    std::lock_guard<std::recursive_mutex> g(Holders::lock());
+    e_ = std::move(e);
+    device_ = device;
+  }
+  // null: none, or given back
+  std::unique_ptr<Engine> take() {
+    std::lock_guard<std::recursive_mutex> g(Holders::lock());
+    return std::move(e_);
+  }
+
+ private:
+  size_t reclaim(int device) override {
+    if (!e_ || device != device_) return 0;
+    const size_t bytes = e_->held_bytes();
+    e_.reset();
+    return bytes;
+  }
+  std::unique_ptr<Engine> e_;
+  int device_ = 0;
+};
 
 }  // namespace
 
@@ -74,7 +103,7 @@ struct dv_server {
   std::map<int64_t, std::pair<std::vector<double>, std::vector<double>>> states;
   double bytes_in_use = 0;
   bool departed = false;  // scenes left since the engine layout was built
-  bool idle = false;      // nothing is resident in the engine
+  ParkedEngine parked;    // E while nothing is resident
   int device = 0;         // the engine's
   dv_server_stats st{};
 
@@ -83,11 +112,16 @@ struct dv_server {
   }
 
   // Nothing is resident: the device memory is freed, up to what an idle server keeps.
-  // The caller's stream may end before the next requests: an idle engine has left it.
   void set_idle() {
-    if (idle || !E) return;
-    if (E->held_bytes() > kIdleBytes || E->use_own_stream() != DV_OK) E.reset();
-    idle = E != nullptr;
+    if (!E) return;
+    const double most = std::min((double)kIdleBytes, cfg.hbm_budget_bytes);
+    if ((double)E->held_bytes() <= most && E->use_own_stream() == DV_OK) parked.put(std::move(E), device);
+    E.reset();
+  }
+
+  // What layouts and grown buffers have freed is held within the budget only.
+  void trim() {
+    if ((double)E->held_bytes() > cfg.hbm_budget_bytes) E->free_spare();
   }
 
   // Rebuilds the engine for `next`: kept[i] = segment index of next[i] in the
@@ -107,20 +141,22 @@ struct dv_server {
     // fresh one takes, and those of a caller that has moved to another device
     int dev = 0;
     DV_CUDA_TRY(cudaGetDevice(&dev));
-    bool special = E && (E->d.anti_relax || dev != device);
-    for (const auto& r : next) special |= r->P.anti_relaxation != 0;
-    if (idle && special) E.reset();
+    const bool reused = !E && (E = parked.take()) != nullptr;
+    if (reused) {
+      bool special = E->d.anti_relax || dev != device;
+      for (const auto& r : next) special |= r->P.anti_relaxation != 0;
+      if (special) E.reset();
+    }
     int rc = DV_OK;
     if (E) {
-      if (idle && user_stream) rc = E->set_stream(user_stream);
+      if (reused && user_stream) rc = E->set_stream(user_stream);
       if (rc == DV_OK) rc = E->reconfigure(slots);
-      if (rc != DV_OK && idle) E.reset();
+      if (rc != DV_OK && reused) E.reset();
     }
-    idle = false;
     if (!E) {
       std::vector<SceneInput> in(slots.size());
       for (size_t i = 0; i < slots.size(); ++i) in[i] = slots[i].in;
-      E.reset(new Engine());
+      E.reset(new Engine(true));
       device = dev;
       rc = E->init(in, cfg.precision);
       if (rc == DV_OK && user_stream) rc = E->set_stream(user_stream);
@@ -132,6 +168,7 @@ struct dv_server {
         else E->set_launch(E->max_ctas(), 1, 0, 2);
       }
     }
+    trim();
     if (rc == DV_OK && cfg.use_graph) E->set_graph(true);  // falls back to launches on failure
     st.reconfigures += 1;
     return rc;
@@ -172,7 +209,7 @@ struct dv_server {
       return DV_OK;
     }
     if (changed || !E) {
-      if (!E || idle)
+      if (!E)
         for (int& k : kept) k = -1;
       int rc = rebuild(next, kept);
       if (rc != DV_OK) {
@@ -188,6 +225,7 @@ struct dv_server {
     for (auto& r : active) k = std::min(k, r->nsteps - r->done);
     k = std::max(k, 1);
     int rc = E->step(k);
+    trim();
     if (rc == DV_ERR_ARG) {
       // a scene over the pair kernels' partner limits fails the step for every
       // scene: retire the requests whose scenes did it (with DV_ERR_ARG and
@@ -326,7 +364,7 @@ DV_API int dv_server_destroy(dv_server* s) {
 DV_API int dv_server_set_stream(dv_server* s, void* cuda_stream) {
   if (!s) return DV_ERR_ARG;
   s->user_stream = (cudaStream_t)cuda_stream;
-  if (s->E && !s->idle && cuda_stream) return s->E->set_stream((cudaStream_t)cuda_stream);
+  if (s->E && cuda_stream) return s->E->set_stream((cudaStream_t)cuda_stream);
   return DV_OK;
 }
 

@@ -319,6 +319,10 @@ DV_API int64_t dv_batch_launch_count(dv_batch* b);
  * dv_server_submit when a request arrives, dv_server_round repeatedly (one
  * round = admissions, steps_per_round steps, retirements), dv_server_poll for
  * finished requests.  Times are seconds on the server's steady clock.
+ * Freed device memory stays with the server for its next layouts, up to 256 MB,
+ * and an idle server keeps up to 1 GB in all, both within hbm_budget_bytes; it
+ * goes back with dv_server_destroy, and when an allocation of any scene, batch
+ * or server of the process fails.
  * ------------------------------------------------------------------------ */
 typedef struct dv_server dv_server;
 
