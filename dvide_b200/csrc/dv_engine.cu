@@ -139,18 +139,37 @@ int Engine::alloc_contacts(size_t cap) {
   TRY(dalloc(&q.part, (size_t)16 * q.tcap));
   TRY(dalloc(&q.tseg, (size_t)q.tcap));
   TRY(ensure_slots());
-  size_t rc = std::max((size_t)q.nb, cap);
-  if (rc > q.radix_cap) {
-    dfree(q.keyA); dfree(q.valA); dfree(q.keyB); dfree(q.valB); dfree(q.radix_hist);
-    q.radix_cap = rc;
-    TRY(dalloc(&q.keyA, rc));
-    TRY(dalloc(&q.valA, rc));
-    TRY(dalloc(&q.keyB, rc));
-    TRY(dalloc(&q.valB, rc));
-    q.radix_hist_cap = radix_hist_size(rc);
-    TRY(dalloc(&q.radix_hist, q.radix_hist_cap));
+  const size_t hist = radix_hist_size(cap);
+  if (hist > q.radix_hist_cap) {
+    dfree(q.radix_hist);
+    q.radix_hist_cap = 0;
+    TRY(dalloc(&q.radix_hist, hist));
+    q.radix_hist_cap = hist;
   }
+  place_collision_scratch();
   return DV_OK;
+}
+
+// What collision detection alone uses lies over what the solve alone uses: boxes,
+// spheres in cell order and kept partners (128 bytes per body) over q, cells (16
+// per body) and sort keys (16 per contact slot) over the last iterate.  Both run
+// on the engine's stream, one after the other, and each writes what it reads.
+// There are four slots per body at least, so all of it fits, and the device
+// memory of a scene stays within what a server counts for it.
+void Engine::place_collision_scratch() {
+  SceneDev& q = d;
+  const size_t nb = (size_t)q.nb;
+  q.amin = q.q;
+  q.amax = q.amin + nb;
+  q.spheres = q.amax + nb;
+  q.kept = reinterpret_cast<uint32_t*>(q.spheres + nb);
+  static_assert(3 * sizeof(double4) + kKeepPartners * sizeof(uint32_t) <= 4 * sizeof(double4), "fits four slots of q");
+  q.cell = reinterpret_cast<int4*>(q.G[4]);
+  q.keyA = reinterpret_cast<uint32_t*>(q.cell + nb);
+  q.valA = q.keyA + q.ccap;
+  q.keyB = q.valA + q.ccap;
+  q.valB = q.keyB + q.ccap;
+  static_assert(sizeof(int4) + 4 * 4 * sizeof(uint32_t) <= 4 * 6 * sizeof(double), "fits four slots of an iterate");
 }
 
 // The teams of a launch have a slot per member: at most one per tile, one per
@@ -515,18 +534,12 @@ int Engine::reconfigure(const std::vector<SlotSpec>& slots) {
   // ---- per-body scratch, segment tables, collision and contact capacity
   if (nb2 > nb_cap_) {
     int cap = std::max(nb2, nb_cap_ + nb_cap_ / 4);
-    dfree(d.k4); dfree(d.w4); dfree(d.fc4); dfree(d.amin); dfree(d.amax); dfree(d.cell);
-    dfree(d.spheres); dfree(d.kept);
+    dfree(d.k4); dfree(d.w4); dfree(d.fc4);
     dfree(d.cnt_cont); dfree(d.cnt_cand); dfree(d.cbase); dfree(d.binc_start); dfree(d.inc_start);
     dfree(d.bseg);
     TRY(dalloc(&d.k4, cap));
     TRY(dalloc(&d.w4, cap));
     TRY(dalloc(&d.fc4, cap));
-    TRY(dalloc(&d.amin, cap));
-    TRY(dalloc(&d.amax, cap));
-    TRY(dalloc(&d.cell, cap));
-    TRY(dalloc(&d.spheres, cap));
-    TRY(dalloc(&d.kept, (size_t)cap * kKeepPartners));
     TRY(dalloc(&d.cnt_cont, cap));
     TRY(dalloc(&d.cnt_cand, cap));
     TRY(dalloc(&d.cbase, (size_t)cap + 1));
@@ -598,6 +611,7 @@ int Engine::reconfigure(const std::vector<SlotSpec>& slots) {
   d.ncell_cap = ncell2;
   if (ccap2 > d.ccap || (int)(d.ccap / kTileItems) + nseg2 + 1 > d.tcap || !d.ida)
     TRY(alloc_contacts(std::max(ccap2, d.ccap)));
+  place_collision_scratch();
   TRY(ensure_slots());
   hseg_ = hs2;
   P_ = P2;

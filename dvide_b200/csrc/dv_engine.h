@@ -171,6 +171,7 @@ class Engine final : private Holder {
                     int col);
   int stage_to_gamma(int s, int n);
   int ensure_slots();
+  void place_collision_scratch();
   int default_grid(int max_ctas) const;
   template <class T>
   int ensure(T** p, int* cap, size_t need);

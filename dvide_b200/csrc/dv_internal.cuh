@@ -159,13 +159,12 @@ struct SceneDev {
   int* small_ids = nullptr;   // sphere bodies binned in the grid, grouped by segment
   int* large_ids = nullptr;   // boxes, tested against all bodies of their segment
   int max_seg_chunks = 0;     // largest ceil(segment bodies / 256)
-  // collision scratch
+  // collision scratch, over q and G[4] (Engine::place_collision_scratch)
   double4 *amin = nullptr, *amax = nullptr;   // shifted AABBs
   int4* cell = nullptr;                       // cell coords + global linear id
   double4* spheres = nullptr;                 // gridded spheres (x, y, z, r) in cell order
   uint32_t* kept = nullptr;                   // kKeepPartners partners per gridded sphere
-  uint32_t *keyA = nullptr, *valA = nullptr, *keyB = nullptr, *valB = nullptr;  // radix buffers
-  size_t radix_cap = 0;
+  uint32_t *keyA = nullptr, *valA = nullptr, *keyB = nullptr, *valB = nullptr;  // radix buffers, ccap
   uint32_t* radix_hist = nullptr;
   size_t radix_hist_cap = 0;
   int* cell_start = nullptr;

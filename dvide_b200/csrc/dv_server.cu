@@ -35,14 +35,19 @@ struct Request {
   int seg = -1;  // segment index in the current engine layout
 };
 
-// Admission estimate of a resident scene's device memory: carried body
-// arrays and per-body scratch, contact slots (4 per body) with their solver
-// vectors, and the warm-start region (6 per body).
+// Admission estimate of a resident scene's device memory: what an engine holds
+// per body, per contact slot (4 per body; collision detection's own arrays lie
+// over the solve's) and per warm slot (6 per body).
 double estimate_bytes(int nb) {
-  const double per_body = 6 * 32 + 3 * 32 + 2 * 32 + 16 + 4 * 8;
-  const double per_contact = 8 + 72 + 12 + 8 + 24 + 24 + 10 * 24 + 32 + 8 + 16;
-  const double per_warm = 24;
-  return (double)nb * (per_body + 4.0 * per_contact + 6.0 * per_warm) + 64.0 * 1024.0;
+  // state, force and geometry, k, w and the contact force; inverse mass, family,
+  // segment, warm range, counts and offsets, list, cells; the state's staging
+  const double per_body = 4 * 32 + 3 * 32 + 8 + 4 + 4 + 8 + 5 * 4 + 4 + 32 + 48;
+  // ids, normal, gap, location, r, constants, five iterates, q, incidence
+  const double per_contact = 8 + 24 + 8 + 24 + 24 + 80 + 5 * 48 + 32 + 8;
+  const double per_warm = 24 + 4;
+  // partials, tiles, slots, histograms
+  const double rest = 8;
+  return (double)nb * (per_body + 4.0 * per_contact + 6.0 * per_warm + rest) + 64.0 * 1024.0;
 }
 
 double pct(std::vector<float> v, double q) {

@@ -77,3 +77,23 @@ def test_idle_server_holds_no_more_than_its_budget(native, used):
         g.close()
         srv.close()
     assert used(start) <= 4 * MB
+
+
+def test_resident_scene_stays_within_its_estimate(native, used):
+    """1.5 million bodies far apart: 96 MB for the blocks' granularity (some 45
+    blocks of 2 MB at most); the estimate is 3.5 GB."""
+    n = 1_500_000
+    sc = scenes.free_balls(n)
+    small = native.NativeServer(precision=native.DV_PREC_FP64)
+    small.submit(scenes.free_balls(3), 2)
+    while small.round():
+        pass
+    small.close()
+    start = used()
+    srv = native.NativeServer(precision=native.DV_PREC_FP64, hbm_budget_bytes=2.4e3 * n)
+    srv.submit(sc, 9)  # more than a round
+    assert srv.round()
+    estimate = srv.stats()["bytes_in_use"]
+    held = used(start)
+    srv.close()
+    assert held <= estimate + 96 * MB, (held / n, estimate / n)
