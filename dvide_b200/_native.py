@@ -32,7 +32,7 @@ EXPORTS = [
     "dv_contact_forces_per_collision", "dv_get_step_stats", "dv_status_string", "dv_last_error",
     "dv_scene_launch_count", "dv_get_step_history", "dv_clear_step_history",
     "dv_get_phase_times", "dv_ccp_violation_noalloc", "dv_selftest_bounded_waits",
-    "dv_selftest_stalled_sweep",
+    "dv_selftest_bounded_join", "dv_selftest_stalled_sweep",
     "dv_batch_create", "dv_batch_destroy", "dv_batch_set_stream", "dv_batch_step",
     "dv_batch_num_scenes", "dv_batch_get_state", "dv_batch_set_state", "dv_batch_scene_stats",
     "dv_batch_step_history", "dv_batch_get_gamma", "dv_batch_ccp_violation",
@@ -494,6 +494,16 @@ def selftest_bounded_waits(limit_ms=50):
     check(lib().dv_selftest_bounded_waits(int(limit_ms), C.byref(b), C.byref(c), C.byref(e)),
           "dv_selftest_bounded_waits")
     return b.value, c.value, e.value
+
+
+def selftest_bounded_join(limit_ms=50, passes=0):
+    """Lets the wait of a team that forms run out, after `passes` signs of
+    progress of another team (dv_selftest_bounded_join); returns (timed_out,
+    ms after the last progress, error_bits)."""
+    r, ms, e = C.c_int32(), C.c_double(), C.c_uint32()
+    check(lib().dv_selftest_bounded_join(int(limit_ms), int(passes), C.byref(r), C.byref(ms), C.byref(e)),
+          "dv_selftest_bounded_join")
+    return r.value, ms.value, e.value
 
 
 def selftest_stalled_sweep(further):

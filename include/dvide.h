@@ -395,6 +395,13 @@ DV_API int dv_server_get_stats(dv_server* s, dv_server_stats* out);
  * device stays usable afterwards. */
 DV_API int dv_selftest_bounded_waits(int32_t limit_ms, int32_t* barrier_timed_out,
                                      int32_t* copy_timed_out, uint32_t* error_bits);
+/* The same for the barrier at which a team of a batch or a server forms: its
+ * limit starts again while other teams make progress.  Another team passes
+ * `passes` barriers, a quarter of limit_ms apart, and stops; the wait must end
+ * (*timed_out = 1) about limit_ms after the last of them. */
+DV_API int dv_selftest_bounded_join(int32_t limit_ms, int32_t passes, int32_t* timed_out,
+                                    double* ms_after_progress, uint32_t* error_bits);
+
 /* The same for the PGS sweep's rounds, which wait for one another by counts: a
  * sweep over a chain of contacts, with `further` != 0 one whose counts never come
  * up.  It must end with *stalled = 1 and the barrier-timeout bit; without, it
