@@ -1236,7 +1236,7 @@ __global__ void __launch_bounds__(1024) k_team_plan(int nseg, const SegParams* _
     if (!takes(s)) continue;
     order[atomicAdd(&s_bin[bin_of(sst[s].nt)], 1)] = s;
     sst[s].members = team_size(sst[s].nt, seg[s].b1 - seg[s].b0, per, grid);
-    for (int i = 0; i < kTeamBarStride; i += kTeamBarStride) team_bar[(size_t)s * kTeamBarStride + i] = 0u;
+    team_bar[(size_t)s * kTeamBarStride] = 0u;
   }
   __syncthreads();
   for (int base = 0; base < n; base += 1024) {

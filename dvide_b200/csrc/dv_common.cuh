@@ -154,22 +154,6 @@ __device__ inline double warp_max(double v) {
   return v;
 }
 
-__device__ inline double block_max256(double v, double* scratch) {
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  v = warp_max(v);
-  __syncthreads();
-  if (lane == 0) scratch[warp] = v;
-  __syncthreads();
-  double r = 0.0;
-  if (warp == 0) {
-    double w = (lane < 8) ? scratch[lane] : 0.0;
-#pragma unroll
-    for (int off = 4; off >= 1; off >>= 1) w = fmax(w, __shfl_down_sync(0xffffffffu, w, off));
-    r = w;
-  }
-  return r;
-}
-
 // ---------------------------------------------------------------------------
 // Memory-model helpers for the persistent kernels.
 // ---------------------------------------------------------------------------
@@ -177,17 +161,6 @@ __device__ inline unsigned ld_acquire(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-__device__ inline void st_release(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ inline unsigned atom_add_acq_rel(unsigned* p, unsigned v) {
-  unsigned old;
-  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;"
-               : "=r"(old)
-               : "l"(p), "r"(v)
-               : "memory");
-  return old;
 }
 __device__ inline uint64_t global_ns() {
   uint64_t t;

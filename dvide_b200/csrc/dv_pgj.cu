@@ -61,7 +61,7 @@ __device__ inline void pgj_ctl(PgjSolve& C, const double* m, const SegParams& P)
 template <class T>
 __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
   using V = typename Vec4<T>::type;
-  __shared__ double scratch[kNQ * 8 + 8];
+  __shared__ double scratch[kMaxima * kWarps];
   __shared__ DeferBuf s_def;
   __shared__ Team tm;
   __shared__ BodyCache<kThreads> bodies;
@@ -203,8 +203,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgj_solve(KArgs<T> a) {
         }
         fold_parked_max<3>(a, s_def, nslot);
         if (!sync(kPhaseProduct)) return;
-        double mm[3];
-        fold_tiles_sm<0, 3>(a, tm.t0, tm.nt, nullptr, mm, 0, scratch);
+        double mm[kMaxima];
+        fold_tile_maxima(a, tm.t0, tm.nt, mm, scratch);
         if (threadIdx.x == 0) pgj_ctl(C, mm, P);
         __syncthreads();
       }

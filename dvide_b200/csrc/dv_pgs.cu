@@ -154,7 +154,7 @@ __device__ PgsSweep pgs_sweep(const KArgs<double>& a, const Team& tm, const SegP
 }
 
 __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
-  __shared__ double scratch[kNQ * 8 + 8];
+  __shared__ double scratch[kMaxima * kWarps];
   __shared__ DeferBuf s_def;
   __shared__ Team tm;
   __shared__ BodyCache<kThreads> bodies;
@@ -334,8 +334,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
         }
         fold_parked_max<3>(a, s_def, nslot);
         if (!sync(kPhaseProduct)) return;
-        double mm[3];
-        fold_tiles_sm<0, 3>(a, tm.t0, tm.nt, nullptr, mm, 0, scratch);
+        double mm[kMaxima];
+        fold_tile_maxima(a, tm.t0, tm.nt, mm, scratch);
         if (threadIdx.x == 0) {
           C.cur ^= 1;
           pgs_ctl(C, mm, P);

@@ -14,8 +14,6 @@ namespace dv {
 
 namespace {
 
-constexpr int kNQ = 7;      // partial-sum slots per tile
-constexpr int kQMax = kNQ;  // slot of the per-tile maximum
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxWarps = 16;  // warps of the largest CTA that has stages
 constexpr int kSub = kThreads;  // contacts per sub-tile
@@ -252,99 +250,56 @@ __device__ inline double dot3i(A a0, A a1, A a2, B b0, B b1, B b2) {
   return ((double)a0 * (double)b0 + (double)a1 * (double)b1) + (double)a2 * (double)b2;
 }
 
-// Folds NS sums (warp_fold, then the 8-warp tree) and NM maxima of each thread
-// with one exchange through shared memory (NS + NM <= 8); thread 0 gets the
-// results.
-template <int NS, int NM>
-__device__ inline void block_fold_sums_maxes(double* v, double* m, double* scratch) {
+// Folds a scene's tile maxima, planes 0 to NM - 1 of its nt tiles from t0 on, to
+// thread 0.  Four tiles' loads per plane are in flight at once.
+template <int NM, class K>
+__device__ inline void fold_tile_maxima(const K& a, int t0, int nt, double (&out)[NM], double* scratch) {
+  constexpr int U = 4;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double* p = a.part + t0;
+  double mx[NM];
 #pragma unroll
-  for (int qi = 0; qi < NS; ++qi) v[qi] = warp_fold(v[qi]);
+  for (int q = 0; q < NM; ++q) mx[q] = 0.0;
+  for (int t = threadIdx.x; t < nt; t += U * kThreads) {
+    double x[NM][U];
 #pragma unroll
-  for (int qi = 0; qi < NM; ++qi) m[qi] = warp_max(m[qi]);
+    for (int u = 0; u < U; ++u) {
+      const int at = t + u * kThreads;
+#pragma unroll
+      for (int q = 0; q < NM; ++q) x[q][u] = at < nt ? __ldcg(p + (size_t)q * a.tcap + at) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int q = 0; q < NM; ++q) mx[q] = fmax(mx[q], x[q][u]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NM; ++q) mx[q] = warp_max(mx[q]);
   __syncthreads();
   if (lane == 0) {
 #pragma unroll
-    for (int qi = 0; qi < NS; ++qi) scratch[qi * 8 + warp] = v[qi];
-#pragma unroll
-    for (int qi = 0; qi < NM; ++qi) scratch[(NS + qi) * 8 + warp] = m[qi];
+    for (int q = 0; q < NM; ++q) scratch[q * kWarps + warp] = mx[q];
   }
   __syncthreads();
   if (warp == 0) {
 #pragma unroll
-    for (int qi = 0; qi < NS; ++qi) {
-      double w = (lane < 8) ? scratch[qi * 8 + lane] : 0.0;
+    for (int q = 0; q < NM; ++q) {
+      double w = lane < kWarps ? scratch[q * kWarps + lane] : 0.0;
 #pragma unroll
-      for (int off = 4; off >= 1; off >>= 1) w = w + __shfl_down_sync(0xffffffffu, w, off);
-      v[qi] = w;
-    }
-#pragma unroll
-    for (int qi = 0; qi < NM; ++qi) {
-      double w = (lane < 8) ? scratch[(NS + qi) * 8 + lane] : 0.0;
-#pragma unroll
-      for (int off = 4; off >= 1; off >>= 1) w = fmax(w, __shfl_down_sync(0xffffffffu, w, off));
-      m[qi] = w;
+      for (int off = kWarps / 2; off >= 1; off >>= 1) w = fmax(w, __shfl_down_sync(0xffffffffu, w, off));
+      out[q] = w;
     }
   }
   __syncthreads();
 }
 
-// Segment controller side: folds the segment's per-tile partials, NS sums
-// (planes 0..NS-1) in the fixed order -- slot j sums the segment's tiles j,
-// j+256, ... in turn, then the 256-slot tree -- and NM maxima (planes
-// mplane0, mplane0+1, ...).  All loads of a chunk of U tiles are in flight
-// before its sums, which keep the slot order: one L2 round trip per chunk.
-template <int NS, int NM, class K>
-__device__ inline void fold_tiles_sm(const K& a, int t0, int nt, double* sum_out, double* max_out,
-                                     int mplane0, double* scratch) {
-  constexpr int U = (NS + NM) <= 2 ? 8 : 4;
-  constexpr int AS = NS > 0 ? NS : 1, AM = NM > 0 ? NM : 1;
-  const double* p = a.part + t0;
-  const size_t tc = (size_t)a.tcap;
-  double sum[AS], mx[AM];
-#pragma unroll
-  for (int qi = 0; qi < AS; ++qi) sum[qi] = 0.0;
-#pragma unroll
-  for (int qi = 0; qi < AM; ++qi) mx[qi] = 0.0;
-  int t = threadIdx.x;
-  for (; t + (U - 1) * kThreads < nt; t += U * kThreads) {
-    double xs[AS][U], xm[AM][U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-#pragma unroll
-      for (int qi = 0; qi < NS; ++qi) xs[qi][u] = __ldcg(p + qi * tc + t + u * kThreads);
-#pragma unroll
-      for (int qi = 0; qi < NM; ++qi)
-        xm[qi][u] = __ldcg(p + (size_t)(mplane0 + qi) * tc + t + u * kThreads);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-#pragma unroll
-      for (int qi = 0; qi < NS; ++qi) sum[qi] = sum[qi] + xs[qi][u];
-#pragma unroll
-      for (int qi = 0; qi < NM; ++qi) mx[qi] = fmax(mx[qi], xm[qi][u]);
-    }
-  }
-  for (; t < nt; t += kThreads) {
-#pragma unroll
-    for (int qi = 0; qi < NS; ++qi) sum[qi] = sum[qi] + __ldcg(p + qi * tc + t);
-#pragma unroll
-    for (int qi = 0; qi < NM; ++qi) mx[qi] = fmax(mx[qi], __ldcg(p + (size_t)(mplane0 + qi) * tc + t));
-  }
-  block_fold_sums_maxes<NS, NM>(sum, mx, scratch);
-#pragma unroll
-  for (int qi = 0; qi < NS; ++qi) sum_out[qi] = sum[qi];
-#pragma unroll
-  for (int qi = 0; qi < NM; ++qi) max_out[qi] = mx[qi];
-}
-
 // Deferred tile folds: the warps park their maxima of a tile and go on to the
 // next; fold_parked_max() completes the parked tiles.
-constexpr int kMaxDefer = 8;
+constexpr int kMaxDefer = 8, kMaxima = 3;
 struct DeferBuf {
-  double w[kMaxDefer][kNQ + 1][kWarps];  // [slot][quantity][warp]
+  double w[kMaxDefer][kMaxima][kWarps];  // [slot][quantity][warp]
   int tile[kMaxDefer];
-  int fail;                              // a warp's copy wait timed out
 };
 
 // ---- maxima reductions of PGJ and PGS (only maxima: no summation order) ----
@@ -496,9 +451,6 @@ __device__ inline void seg_error(const K& a, int s, unsigned bit) {
   if (a.ew->stop_on_seg_err) atomicOr(&a.ew->err, bit);
 }
 
-// w_b = minv_b * (D^T x)_b of one body; fixed bodies keep w = 0.
-// kAR: also v = Minv (k + D^T x) for the anti-relaxation (APGD.cu:338-340;
-// 0 for fixed bodies, whose v enters only as squares).
 // The words a body's gather starts from, its inverse mass and the bounds of its
 // incidence run, loaded together so that they cost one memory round trip.
 struct BodyHead {
@@ -515,16 +467,19 @@ __device__ inline BodyHead body_head(const K& a, int b) {
   return h;
 }
 
-// kPre: c0 holds the body's first eight incidence entries, loaded a round
-// ahead by the body pass (zero past its run).
-template <class T, bool kAR = false, bool kPre = false>
+// w_b = minv_b * (D^T x)_b of one body; fixed bodies keep w = 0.
+// kAR: also v = Minv (k + D^T x) for the anti-relaxation (APGD.cu:338-340;
+// 0 for fixed bodies, whose v enters only as squares).
+// c0 holds the body's first eight incidence entries, loaded a round ahead by the
+// body pass (zero past its run).
+template <class T, bool kAR>
 __device__ inline void body_w(const KArgs<T>& a, typename Vec4<T>::type* w,
                               const typename Vec4<T>::type* q, int b, const BodyHead& h,
-                              const uint32_t* c0 = nullptr) {
+                              const uint32_t* c0) {
   using V = typename Vec4<T>::type;
   const double mi = h.mi;
   if (mi != 0.0) {
-    V s = kPre ? gather_q_pre<T, V>(a, q, h.s, h.e, c0) : gather_q<T, V>(a, q, h.s, h.e);
+    V s = gather_q_pre<T, V>(a, q, h.s, h.e, c0);
     if (a.nbil) add_bilateral<T, V>(a.bil_inc_start, a.bil_inc, a.bq, b, s);
     T m = (T)mi;
     V o;

@@ -246,7 +246,7 @@ __device__ inline void fold_parked8(ParkBuf& B, double* part, int tcap, int n) {
   __syncthreads();
 }
 
-// Folds a scene's tile partials (the order of fold_tiles_sm: slot j sums tiles
+// Folds a scene's tile partials (in a fixed order: slot j sums tiles
 // j, j + 256, ..., then the 256-slot tree), NS sums and, with kMax, a maximum
 // in plane 7, into out[].  Every member of a team calls it after the pass's
 // barrier and runs the scene's controller on its own copy of the scalars: the
@@ -376,7 +376,7 @@ __device__ inline void team_body_pass(const KArgs<T>& a, const Team& t, const Bo
     uint32_t cn[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) cn[j] = (hn.s + j < hn.e) ? __ldg(a.inc + hn.s + j) : 0u;
-    body_w<T, kAR, true>(a, w, q, b, h, c);
+    body_w<T, kAR>(a, w, q, b, h, c);
     h = hn;
     hn = hnn;
 #pragma unroll
