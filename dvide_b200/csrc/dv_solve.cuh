@@ -260,19 +260,23 @@ __device__ inline void fold_tile_maxima(const K& a, int t0, int nt, double (&out
   double mx[NM];
 #pragma unroll
   for (int q = 0; q < NM; ++q) mx[q] = 0.0;
-  for (int t = threadIdx.x; t < nt; t += U * kThreads) {
+  int t = threadIdx.x;
+  for (; t + (U - 1) * kThreads < nt; t += U * kThreads) {
     double x[NM][U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int at = t + u * kThreads;
 #pragma unroll
-      for (int q = 0; q < NM; ++q) x[q][u] = at < nt ? __ldcg(p + (size_t)q * a.tcap + at) : 0.0;
+      for (int q = 0; q < NM; ++q) x[q][u] = __ldcg(p + (size_t)q * a.tcap + t + u * kThreads);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
 #pragma unroll
       for (int q = 0; q < NM; ++q) mx[q] = fmax(mx[q], x[q][u]);
     }
+  }
+  for (; t < nt; t += kThreads) {
+#pragma unroll
+    for (int q = 0; q < NM; ++q) mx[q] = fmax(mx[q], __ldcg(p + (size_t)q * a.tcap + t));
   }
 #pragma unroll
   for (int q = 0; q < NM; ++q) mx[q] = warp_max(mx[q]);
