@@ -72,11 +72,14 @@ __device__ inline void pgs_ctl(PgsSolve& C, const double* m, const SegParams& P)
 // (all its threads).  `strict`: fixed bodies' contacts one after another too.
 // Returns, in every thread, whether a fixed body's velocity would have changed
 // (only without `strict`).  Every round updates at least the first contact that
-// is left; one that updates none, because the counts and the incidence disagree,
-// ends the sweep with an error instead of a wait without end.
+// is left, so none of a window waits for more rounds than the window has contacts;
+// one that does, because the counts and the incidence disagree, gives up, and the
+// sweep ends with an error.
 enum PgsSweep : int { kSweepDone = 0, kSweepOdd = 1, kSweepStalled = 2 };
 __device__ PgsSweep pgs_sweep(const KArgs<double>& a, const Team& tm, const SegParams& P, const double* Gc,
                           double* Gn, const Cone<double>& cone, int from, int to, bool strict) {
+  __shared__ int s_stalled;
+  if (threadIdx.x == 0) s_stalled = 0;
   const size_t S = a.S;
   const double h = P.h;
   const double* Bc = a.G[4];
@@ -107,13 +110,17 @@ __device__ PgsSweep pgs_sweep(const KArgs<double>& a, const Team& tm, const SegP
       at = place[c];
     }
     const bool wait_a = strict || mia != 0.0, wait_b = strict || mib != 0.0;
+    int waited = 0;
     while (__syncthreads_or(todo)) {
       const bool go = todo && (!wait_a || done_of[ia] == at.x) && (!wait_b || done_of[ib] == at.y);
-      if (!__syncthreads_or(go)) {  // every thread has read the counts
-        if (threadIdx.x == 0) atomicOr(&a.ew->err, kErrBarrierTimeout);
-        return kSweepStalled;
+      __syncthreads();  // every thread has read the counts
+      if (!go) {
+        if (++waited > kThreads && todo) {
+          todo = false;
+          s_stalled = 1;
+        }
+        continue;
       }
-      if (!go) continue;
       const double4 va = v[ia], vb = v[ib];
       double g0 = o0 - ob * (f.n0 * va.x + f.n1 * va.y + f.n2 * va.z - f.n0 * vb.x - f.n1 * vb.y -
                              f.n2 * vb.z + bn);
@@ -150,7 +157,9 @@ __device__ PgsSweep pgs_sweep(const KArgs<double>& a, const Team& tm, const SegP
       todo = false;
     }
   }
-  return __syncthreads_or(odd) ? kSweepOdd : kSweepDone;
+  odd = __syncthreads_or(odd);
+  if (s_stalled && threadIdx.x == 0) atomicOr(&a.ew->err, kErrBarrierTimeout);
+  return s_stalled ? kSweepStalled : odd ? kSweepOdd : kSweepDone;
 }
 
 __global__ void __launch_bounds__(kThreads, 2) k_pgs_solve(KArgs<double> a) {
