@@ -46,7 +46,7 @@ namespace {
 constexpr int kWarpsPerCta = kThreads / 32;
 constexpr int kMaxPerBody = 128;  // partners with larger id per sphere
 constexpr int kKeep = kKeepPartners;
-constexpr int kAgainCtas = 592;   // CTAs that search listed spheres again at most
+constexpr int kAgainCtas = 148;   // CTAs that only search listed spheres again at most
 
 __device__ inline unsigned long long ordered_bits(double x) {
   unsigned long long u = (unsigned long long)__double_as_longlong(x);
@@ -489,36 +489,32 @@ __global__ void __launch_bounds__(kThreads) k_sphere_count(CollideArgs a) {
   }
 }
 
-// Write pass.  The first `kept_ctas` CTAs, eight lanes per sphere: the contacts
-// of the kept partners at the sphere's slot.  The others, a warp per sphere: the
-// spheres that the count pass listed, with more than kKeep and at most
-// kMaxPerBody partners, are searched again.  (Searched by the warp that wrote its
-// four spheres' kept partners, a crowd of 129 such spheres took four searches one
-// after another.)
-__global__ void __launch_bounds__(kThreads) k_sphere_write(CollideArgs a, int kept_ctas) {
+// Write pass.  Eight lanes per sphere: the contacts of the kept partners at the
+// sphere's slot.  Then, a warp per sphere: the spheres that the count pass listed,
+// with more than kKeep and at most kMaxPerBody partners, are searched again.
+// (Searched by the warp that wrote its four spheres' kept partners, a crowd of 129
+// such spheres took four searches one after another.)
+__global__ void __launch_bounds__(kThreads) k_sphere_write(CollideArgs a) {
   __shared__ int s_buf[kWarpsPerCta][kMaxPerBody];
   __shared__ int s_cnt[kWarpsPerCta];
   if (a.ew->err) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if ((int)blockIdx.x < kept_ctas) {
-    const int j = (blockIdx.x * kThreads + threadIdx.x) >> 3;
-    if (j >= a.n_small) return;
+  const int j = (blockIdx.x * kThreads + threadIdx.x) >> 3, e0 = lane & 7;
+  if (j < a.n_small) {
     const int A = a.small_ids[j], sg = a.bseg[A];
     const SegParams& P = a.seg[sg];
     const int n = P.active ? a.cnt_cont[A] : 0;
-    if (n > kKeep) return;
-    const int e = lane & 7;
-    if (e < n) {
+    if (n <= kKeep && e0 < n) {
       const size_t base = (size_t)(a.cbase[A] + a.sst[sg].delta);
-      const int B = (int)a.kept[(size_t)j * kKeep + e];
+      const int B = (int)a.kept[(size_t)j * kKeep + e0];
       NpOut o;
       narrowphase(a.p4, a.g4, A, B, P.env, P.exact != 0, &o);
-      write_contact(a, base + e, A, B, o);
+      write_contact(a, base + e0, A, B, o);
     }
-    return;
   }
-  const int listed = a.ew->n_again, step = ((int)gridDim.x - kept_ctas) * kWarpsPerCta;
-  for (int w = ((int)blockIdx.x - kept_ctas) * kWarpsPerCta + warp; w < listed; w += step) {
+  __syncwarp();
+  const int listed = a.ew->n_again;
+  for (int w = blockIdx.x * kWarpsPerCta + warp; w < listed; w += gridDim.x * kWarpsPerCta) {
     const int A = a.small_ids[a.again[w]], sg = a.bseg[A];
     const SegParams& P = a.seg[sg];
     int ncand;
@@ -1205,9 +1201,9 @@ void collide(SceneDev& sd, cudaStream_t st, int64_t* launches) {
       exclusive_scan_i32(sd.large_chunk, sd.large_chunk_off, nchunks, sd.scan_tmp, st, launches);
   }
   if (sd.n_small > 0) {
-    const int kept_ctas = blocks_for(8LL * sd.n_small);
-    const int again_ctas = std::min((sd.n_small + kWarpsPerCta - 1) / kWarpsPerCta, kAgainCtas);
-    k_sphere_write<<<kept_ctas + again_ctas, kThreads, 0, st>>>(a, kept_ctas);
+    // a warp per sphere where that is a CTA per SM at most
+    const int one_each = std::min((sd.n_small + kWarpsPerCta - 1) / kWarpsPerCta, kAgainCtas);
+    k_sphere_write<<<std::max(blocks_for(8LL * sd.n_small), one_each), kThreads, 0, st>>>(a);
     k_sphere_pairs_wide<<<std::min(kWideGrid, sd.n_small), kThreads, 0, st>>>(a);
     *launches += 2;
   }
