@@ -60,11 +60,11 @@ void fill_step_stats(const StepRecord& r, int s, dv_step_stats* out) {
 
 Engine::Engine(bool keep_blocks) : keep_blocks_(keep_blocks) {
   cudaGetDevice(&device_);
-  if (keep_blocks_) Holders::add(this);
+  Holders::add(this);
 }
 
 Engine::~Engine() {
-  if (keep_blocks_) Holders::remove(this);
+  Holders::remove(this);
   if (st_) cudaStreamSynchronize(st_);
   drop_graph();
   free_spare();
@@ -121,7 +121,9 @@ int Engine::alloc_contacts(size_t cap) {
   dfree(q.q); dfree(q.inc); dfree(q.part); dfree(q.tseg);
   dfree(q.ar_r0); dfree(q.ar_v);
   q.ccap = cap;
-  q.tcap = (int)(cap / kTileItems) + q.nseg + 1 + (q.nbil + kTileItems - 1) / kTileItems;
+  // room for a tile of bilateral rows before there are any: the first row of a
+  // scene need not make its contact buffers again
+  q.tcap = (int)(cap / kTileItems) + q.nseg + 1 + std::max(1, (q.nbil + kTileItems - 1) / kTileItems);
   TRY(dalloc(&q.ida, cap));
   TRY(dalloc(&q.idb, cap));
   TRY(dalloc(&q.F, 3 * cap));
@@ -303,6 +305,14 @@ int Engine::ensure(T** p, int* cap, size_t need) {
 }
 
 int Engine::reconfigure(const std::vector<SlotSpec>& slots) {
+  in_layout_ = true;
+  const int rc = lay_out(slots);
+  in_layout_ = false;
+  if (!keep_blocks_) free_spare();
+  return rc;
+}
+
+int Engine::lay_out(const std::vector<SlotSpec>& slots) {
   const int nseg2 = (int)slots.size();
   if (nseg2 == 0) return DV_ERR_ARG;
   for (const SlotSpec& sl : slots) {
@@ -1048,15 +1058,21 @@ int Engine::upload_bilateral() {
     inc.insert(inc.end(), per[b].begin(), per[b].end());
   }
   start[nb] = (int)inc.size();
-  dfree(d.bil_off); dfree(d.bil_info); dfree(d.bil_inc_start); dfree(d.bil_inc);
-  dfree(d.bil_work); dfree(d.bil_gam); dfree(d.bil_b);
-  TRY(dalloc(&d.bil_off, n));
-  TRY(dalloc(&d.bil_info, n));
-  TRY(dalloc(&d.bil_inc_start, (size_t)nb + 1));
-  TRY(dalloc(&d.bil_inc, inc.size()));
-  TRY(dalloc(&d.bil_work, 12 * (size_t)n));
-  TRY(dalloc(&d.bil_gam, n));
-  TRY(dalloc(&d.bil_b, n));
+  // rows come one by one: the arrays grow by doubling (planes of bil_work: nbil apart)
+  if ((size_t)n > bil_cap_) {
+    const size_t cap = std::max<size_t>(16, 2 * (size_t)n);
+    dfree(d.bil_off); dfree(d.bil_info); dfree(d.bil_inc); dfree(d.bil_work); dfree(d.bil_gam);
+    dfree(d.bil_b);
+    bil_cap_ = 0;
+    TRY(dalloc(&d.bil_off, cap));
+    TRY(dalloc(&d.bil_info, cap));
+    TRY(dalloc(&d.bil_inc, 2 * cap));
+    TRY(dalloc(&d.bil_work, 12 * cap));
+    TRY(dalloc(&d.bil_gam, cap));
+    TRY(dalloc(&d.bil_b, cap));
+    bil_cap_ = cap;
+  }
+  if (!d.bil_inc_start) TRY(dalloc(&d.bil_inc_start, (size_t)nb + 1));
   if (!d.seg_time) TRY(dalloc(&d.seg_time, (size_t)d.nseg));
   DV_CUDA_TRY(cudaMemcpyAsync(d.bil_off, off.data(), sizeof(int2) * n, cudaMemcpyHostToDevice, st_));
   DV_CUDA_TRY(cudaMemcpyAsync(d.bil_info, info.data(), sizeof(double4) * n, cudaMemcpyHostToDevice, st_));

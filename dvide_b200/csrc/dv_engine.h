@@ -171,6 +171,7 @@ class Engine final : private Holder {
                     int col);
   int stage_to_gamma(int s, int n);
   int ensure_slots();
+  int lay_out(const std::vector<SlotSpec>& slots);
   void place_collision_scratch();
   int default_grid(int max_ctas) const;
   template <class T>
@@ -192,6 +193,7 @@ class Engine final : private Holder {
   std::unordered_map<void*, size_t> allocs_;  // device memory and its sizes
   size_t held_bytes_ = 0;                     // ... of them and the spare blocks
   const bool keep_blocks_;
+  bool in_layout_ = false;                    // freed blocks serve the layout being made
   int device_ = 0;
   std::multimap<size_t, void*> spare_;        // freed blocks by size (under Holders::lock)
   size_t spare_bytes_ = 0;
@@ -204,6 +206,7 @@ class Engine final : private Holder {
   // bilateral rows (host copy; segment 0 of a one-segment engine)
   std::vector<int> bil_a_, bil_b_;
   std::vector<double> bil_vel_, bil_t0_, bil_p0_;
+  size_t bil_cap_ = 0;  // rows that the device arrays hold
   int max_ctas_ = 1;
   SolveConfig cfg_{1, 1, 0, 2};
   bool cfg_user_ = false;
@@ -246,11 +249,11 @@ class Engine final : private Holder {
   double* h_red_ = nullptr;           // pinned, 16 slots
 };
 
-// Device memory of an engine.  With keep_blocks a freed block stays with the
-// engine for its next allocation of at most that and at least half that size, up
-// to kSpareBytes in all: a layout change of a server takes and gives back some
-// twenty blocks, and cudaMalloc and cudaFree of each cost 0.1 to 0.5 ms and wait
-// for the device.  All work on a block runs on the engine's stream, so the next
+// Device memory of an engine.  While a layout is made, and with keep_blocks at all
+// times, a freed block stays with the engine for its next allocation of at most
+// that and at least half that size, up to kSpareBytes in all: a layout takes and
+// gives back some twenty blocks, and cudaMalloc and cudaFree of each cost 0.1 to
+// 0.5 ms and wait for the device.  All work on a block runs on the engine's stream, so the next
 // user's follows the last one's.  Spare blocks go back with the engine, and when
 // an allocation of any engine of the process fails.
 template <class T>
@@ -258,7 +261,7 @@ inline int Engine::dalloc(T** p, size_t n) {
   if (n == 0) n = 1;
   const size_t bytes = n * sizeof(T);
   void* q = nullptr;
-  if (keep_blocks_) {
+  if (keep_blocks_ || in_layout_) {
     std::lock_guard<std::recursive_mutex> g(Holders::lock());
     auto it = spare_.lower_bound(bytes);
     if (it != spare_.end() && it->first / 2 <= bytes) {
@@ -295,7 +298,7 @@ inline void Engine::dfree(T*& p) {
     const size_t bytes = it->second;
     allocs_.erase(it);
     std::lock_guard<std::recursive_mutex> g(Holders::lock());
-    if (keep_blocks_ && spare_bytes_ + bytes <= kSpareBytes) {
+    if ((keep_blocks_ || in_layout_) && spare_bytes_ + bytes <= kSpareBytes) {
       spare_.emplace(bytes, (void*)p);
       spare_bytes_ += bytes;
     } else {
