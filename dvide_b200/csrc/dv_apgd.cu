@@ -1314,7 +1314,11 @@ void launch_typed(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t
 // then at most about one per SM.  Solve per step in 512- and 256-thread CTAs:
 // 1,000 spheres 1.63 and 1.73 ms, 20,011 mixed 8.16 and 8.95; 200,000 spheres
 // 44 and 34 ms (their stages leave the body pass a sixth of the L1); 64 scenes
-// 2.9 and 2.7 ms (their 160 tiles need a second wave).
+// 2.9 and 2.7 ms (their 160 tiles need a second wave).  Setup and one iteration
+// near the line, FP64: 20,000 spheres 113 and 119 us, 30,000 131 and 139, 40,000
+// 164 and 160.  A pile below the line that is dense enough for more tiles than SMs
+// gains nothing or pays a little: 238 tiles 225 and 225 us, 517 tiles 25.7 and 23.1
+// us per iteration.
 template <class T, bool AR = false>
 void launch_form(SceneDev& sd, const SolveConfig& cfg, cudaStream_t st, int64_t* launches,
                  bool solve_only, bool refine = false) {

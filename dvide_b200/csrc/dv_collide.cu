@@ -31,8 +31,9 @@
 // the whole pipeline runs without a host round trip and can be captured in a
 // CUDA graph.  Engines of at most kFewBodies bodies take short forms of it, one
 // CTA each, for everything before, between and after the pair kernels: there a
-// step of some fifty launches is bound by the launches themselves (2 us each).  EngineWords::err is sticky: once set, every later kernel of the
-// step returns at once.
+// step of some fifty launches is bound by the launches themselves (2 us each).
+// EngineWords::err is sticky: once set, every later kernel of the step returns at
+// once.
 #include <stdio.h>
 
 #include <algorithm>

@@ -899,8 +899,8 @@ int Engine::step(int n) {
     for (int i = 0; i < m; ++i) {
       const EngineWords& w = h_ew_ring_[i];
       const SegState* ss = h_sst_ring_ + (size_t)i * d.nseg;
-      // a step counts when its solve reached the update (steps_done advanced)
-      // or, for engine-level errors, not at all
+      // a step with an engine-level error does not count: no kernel after the
+      // one that found it has touched the state
       unsigned hard = w.err & (kErrCapacity | kErrPartners | kErrBarrierTimeout | kErrCopyTimeout);
       if (hard) {
         failed = i;

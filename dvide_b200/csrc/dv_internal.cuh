@@ -132,9 +132,10 @@ constexpr int kKeepPartners = 8;
 constexpr int kFewBodies = 6144;
 constexpr int kFewContacts = 32768;  // contact slots of an engine whose incidence one CTA forms
 
-// Tiles that a team's member takes at most when there are more than the grid
-// has CTAs, and the distance of the teams' arrival counters (a line each).
-constexpr int kPairBodies = 20480;  // bodies of a scene that 512-thread CTAs solve
+// Bodies of a scene that 512-thread CTAs solve; tiles that a team's member takes
+// at most when there are more than the grid has CTAs; the distance of the teams'
+// arrival counters (a line each).
+constexpr int kPairBodies = 20480;
 constexpr int kTeamTiles = 4;
 constexpr int kTeamBarStride = 32;
 
