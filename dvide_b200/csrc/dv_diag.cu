@@ -183,10 +183,20 @@ int Engine::ensure_red(size_t n) {
     if (cudaMallocHost(&h_red_, 16 * sizeof(double)) != cudaSuccess)
       return dv_record_cuda_error(cudaErrorMemoryAllocation, "cudaMallocHost", __FILE__, __LINE__);
   }
-  if (n <= d_red_cap_) return DV_OK;
-  dfree(d_red_);
-  d_red_cap_ = n;
-  return dalloc(&d_red_, n);
+  // over another iterate than the rows' stage
+  if (n <= 6 * d.ccap) {
+    d_red_ = d.G[1];
+    return DV_OK;
+  }
+  if (n > wide_red_cap_) {
+    dfree(wide_red_);
+    wide_red_cap_ = 0;
+    const int rc = dalloc(&wide_red_, n);
+    if (rc != DV_OK) return rc;
+    wide_red_cap_ = n;
+  }
+  d_red_ = wide_red_;
+  return DV_OK;
 }
 
 // Ordered sum of `n` device items; the result lands in h_red_[slot] after a sync.

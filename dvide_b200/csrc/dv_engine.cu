@@ -1301,12 +1301,22 @@ int Engine::copy_contact_forces_out(int s, double* normal, double* friction) {
   return DV_OK;
 }
 
+// Rows on their way between host and device lie over an iterate of the solve,
+// which nothing reads between two steps: reading a scene takes no memory of its
+// own, also the first time (0.3 to 0.5 ms per block that a call would allocate).
+// Rows of more than six per contact slot, the frames, have a block.
 int Engine::ensure_stage(size_t n) {
-  if (n <= stage3_cap_) return DV_OK;
-  dfree(stage3_);
-  stage3_cap_ = 0;
-  TRY(dalloc(&stage3_, n));
-  stage3_cap_ = n;
+  if (n <= 6 * d.ccap) {
+    stage3_ = d.G[0];
+    return DV_OK;
+  }
+  if (n > wide_stage_cap_) {
+    dfree(wide_stage_);
+    wide_stage_cap_ = 0;
+    TRY(dalloc(&wide_stage_, n));
+    wide_stage_cap_ = n;
+  }
+  stage3_ = wide_stage_;
   return DV_OK;
 }
 

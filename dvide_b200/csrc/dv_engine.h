@@ -241,11 +241,13 @@ class Engine final : private Holder {
   std::vector<double> snap_time_;
   std::vector<int> snap_time_index_;
   // staging of host transfers: bodies or contacts as rows
-  double* stage3_ = nullptr;
-  size_t stage3_cap_ = 0;
+  double* stage3_ = nullptr;          // since the last ensure_stage
+  double* wide_stage_ = nullptr;
+  size_t wide_stage_cap_ = 0;
   // diagnostics scratch
-  double* d_red_ = nullptr;
-  size_t d_red_cap_ = 0;
+  double* d_red_ = nullptr;           // since the last ensure_red
+  double* wide_red_ = nullptr;
+  size_t wide_red_cap_ = 0;
   double* h_red_ = nullptr;           // pinned, 16 slots
 };
 

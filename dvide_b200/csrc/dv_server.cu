@@ -40,13 +40,13 @@ struct Request {
 // over the solve's) and per warm slot (6 per body).
 double estimate_bytes(int nb) {
   // state, force and geometry, k, w and the contact force; inverse mass, family,
-  // segment, warm range, counts and offsets, list, cells; the state's staging
-  const double per_body = 4 * 32 + 3 * 32 + 8 + 4 + 4 + 8 + 5 * 4 + 4 + 32 + 48;
+  // segment, warm range, counts and offsets, list, cells
+  const double per_body = 4 * 32 + 3 * 32 + 8 + 4 + 4 + 8 + 5 * 4 + 4 + 32;
   // ids, normal, gap, location, r, constants, five iterates, q, incidence
   const double per_contact = 8 + 24 + 8 + 24 + 24 + 80 + 5 * 48 + 32 + 8;
   const double per_warm = 24 + 4;
-  // partials, tiles, slots, histograms
-  const double rest = 8;
+  // partials, tiles, slots, histograms (8), and room to spare
+  const double rest = 56;
   return (double)nb * (per_body + 4.0 * per_contact + 6.0 * per_warm + rest) + 64.0 * 1024.0;
 }
 
