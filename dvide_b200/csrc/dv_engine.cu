@@ -470,18 +470,16 @@ int Engine::lay_out(const std::vector<SlotSpec>& slots) {
   TRY(dalloc(&nws, nbz));
   TRY(dalloc(&nwc, nbz));
   {
-    const size_t ns = std::max<size_t>(sp4.size(), 1);
-    double4 *tp = nullptr, *tv = nullptr, *tf = nullptr, *tg = nullptr;
-    double* tm = nullptr;
-    int *tfam = nullptr, *tmap = nullptr;
-    TRY(dalloc(&tp, ns));
-    TRY(dalloc(&tv, ns));
-    TRY(dalloc(&tf, ns));
-    TRY(dalloc(&tg, ns));
-    TRY(dalloc(&tm, ns));
-    TRY(dalloc(&tfam, ns));
-    TRY(dalloc(&tmap, nbz));
-    const size_t k = sp4.size();
+    const size_t ns = std::max<size_t>(sp4.size(), 1), k = sp4.size();
+    // A layout of new scenes only takes its bodies as they come; one that carries
+    // scenes gathers both from one staged block.
+    const bool fresh = k == nbz;
+    double4* staged = nullptr;
+    if (!fresh) TRY(dalloc(&staged, 4 * ns + (ns * 12 + nbz * 4 + sizeof(double4) - 1) / sizeof(double4)));
+    double4 *tp = fresh ? np4 : staged, *tv = fresh ? nv4 : tp + ns, *tf = fresh ? nf4 : tv + ns,
+            *tg = fresh ? ng4 : tf + ns;
+    double* tm = fresh ? nminv : reinterpret_cast<double*>(tg + ns);
+    int* tfam = fresh ? nfam : reinterpret_cast<int*>(tm + ns);
     if (k) {
       DV_CUDA_TRY(cudaMemcpyAsync(tp, sp4.data(), sizeof(double4) * k, cudaMemcpyHostToDevice, st));
       DV_CUDA_TRY(cudaMemcpyAsync(tv, sv4.data(), sizeof(double4) * k, cudaMemcpyHostToDevice, st));
@@ -490,12 +488,18 @@ int Engine::lay_out(const std::vector<SlotSpec>& slots) {
       DV_CUDA_TRY(cudaMemcpyAsync(tm, sminv.data(), sizeof(double) * k, cudaMemcpyHostToDevice, st));
       DV_CUDA_TRY(cudaMemcpyAsync(tfam, sfam.data(), sizeof(int) * k, cudaMemcpyHostToDevice, st));
     }
-    DV_CUDA_TRY(cudaMemcpyAsync(tmap, map2.data(), sizeof(int) * nbz, cudaMemcpyHostToDevice, st));
-    k_gather_bodies<<<(nb2 + kThreads - 1) / kThreads, kThreads, 0, st>>>(
-        nb2, tmap, d.p4, d.v4, d.f4, d.geom4, d.minv, d.family, d.ws, d.wc, tp, tv, tf, tg, tm,
-        tfam, np4, nv4, nf4, ng4, nminv, nfam, nws, nwc);
-    ++launches_;
-    DV_CUDA_TRY(cudaGetLastError());
+    if (fresh) {
+      DV_CUDA_TRY(cudaMemsetAsync(nws, 0, sizeof(int) * nbz, st));
+      DV_CUDA_TRY(cudaMemsetAsync(nwc, 0, sizeof(int) * nbz, st));
+    } else {
+      int* tmap = tfam + ns;
+      DV_CUDA_TRY(cudaMemcpyAsync(tmap, map2.data(), sizeof(int) * nbz, cudaMemcpyHostToDevice, st));
+      k_gather_bodies<<<(nb2 + kThreads - 1) / kThreads, kThreads, 0, st>>>(
+          nb2, tmap, d.p4, d.v4, d.f4, d.geom4, d.minv, d.family, d.ws, d.wc, tp, tv, tf, tg, tm,
+          tfam, np4, nv4, nf4, ng4, nminv, nfam, nws, nwc);
+      ++launches_;
+      DV_CUDA_TRY(cudaGetLastError());
+    }
     // warm-start arena
     double* ng = nullptr;
     uint32_t* nid = nullptr;
@@ -530,7 +534,7 @@ int Engine::lay_out(const std::vector<SlotSpec>& slots) {
       dfree(tn);
     }
     DV_CUDA_TRY(cudaStreamSynchronize(st));
-    dfree(tp); dfree(tv); dfree(tf); dfree(tg); dfree(tm); dfree(tfam); dfree(tmap);
+    dfree(staged);
     dfree(d.p4); dfree(d.v4); dfree(d.f4); dfree(d.geom4); dfree(d.minv); dfree(d.family);
     dfree(d.gamma); dfree(d.wid); dfree(d.ws); dfree(d.wc);
     d.p4 = np4; d.v4 = nv4; d.f4 = nf4; d.geom4 = ng4; d.minv = nminv; d.family = nfam;
