@@ -14,9 +14,12 @@ MB = 1 << 20
 @pytest.fixture()
 def used():
     """Device bytes in use since the fixture's start, the modules loaded."""
+    import gc
+
     import torch
     torch.cuda.init()
     torch.zeros(1, device="cuda")
+    gc.collect()  # scenes that earlier tests left behind
 
     def free():
         torch.cuda.synchronize()
